@@ -356,6 +356,7 @@ def attention_tcgen05_jobs(head_dim: int, dtype: torch.dtype, softcap: bool = Fa
 
 TCGEN05_HEAD_DIMS = (64, 128)
 WIDE_TILE = 128                  # queries per tile of the tcgen05 prompt attention
+WIDE_PAIR = 2 * WIDE_TILE        # the same where a CTA takes two tiles
 _attention_tcgen05_libs = {}
 
 
@@ -395,8 +396,8 @@ def _sink(sink, hq: Optional[int] = None) -> tuple:
 
 
 def attn_prefill_wide(q, out, k_cache, v_cache, req_slot, block_table, wide_req, wide_q0, q_start, q_len, ctx_len, hq, hkv,
-                      page_size, scale, window, sink=None, keep_first: int = 0, softcap: Optional[float] = None) -> None:
-    """Attention of portions on tcgen05: q, out [tokens, hq, D]; tiles of 128 queries as (request, first query).
+                      page_size, scale, window, sink=None, keep_first: int = 0, softcap: Optional[float] = None, span: int = WIDE_TILE) -> None:
+    """Attention of portions on tcgen05: q, out [tokens, hq, D]; tiles of `span` (128 or 256) queries as (request, first query).
     `softcap`: a score s becomes softcap * tanh(s / softcap) before the softmax.  `sink`: see `_sink`.  `keep_first`: the sequence's first keys that stay in sight behind a window."""
     dim = k_cache.shape[-1]
     _need(q, torch.bfloat16, "q", 3); _need(out, torch.bfloat16, "out", 3); _need(k_cache, torch.bfloat16, "k_cache", 4)
@@ -409,7 +410,7 @@ def attn_prefill_wide(q, out, k_cache, v_cache, req_slot, block_table, wide_req,
     lib = _attention_tcgen05(dim, softcap is not None)
     _check(lib.cisr_attn_prefill_tcgen05(_p(q), _p(out), q.shape[0], _p(k_cache), _p(v_cache), k_cache.shape[0], _p(req_slot),
                                          _p(block_table), block_table.shape[1], _p(wide_req), _p(wide_q0), wide_req.numel(),
-                                         _p(q_start), _p(q_len), _p(ctx_len), hq, hkv, page_size, ctypes.c_float(scale),
+                                         span, _p(q_start), _p(q_len), _p(ctx_len), hq, hkv, page_size, ctypes.c_float(scale),
                                          _softcap(softcap), int(window or 0), int(keep_first or 0), *_sink(sink, hq), _stream()), "attn_prefill_wide")
 
 

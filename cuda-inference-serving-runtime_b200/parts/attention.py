@@ -121,8 +121,9 @@ class GQAAttention(Mixer):
         out = torch.empty((tokens, hq, dim), dtype=self.dtype, device=device)
         plan = ctx.plan_for(self)
         if plan.info["n_tiles"] and kernels.attn_prefill_wide_ok(q, cache.k, cache.page_size):
-            kernels.attn_prefill_wide(q, out, cache.k, cache.v, ctx.req_slot, cache.block_table, plan["wide_req"], plan["wide_q0"],
-                                      ctx.q_start, ctx.q_len, ctx.ctx_len, hq, hkv, cache.page_size, self.scale, self.window)
+            tiles, span = wide_tiles(plan, hq)
+            kernels.attn_prefill_wide(q, out, cache.k, cache.v, ctx.req_slot, cache.block_table, *tiles, ctx.q_start, ctx.q_len,
+                                      ctx.ctx_len, hq, hkv, cache.page_size, self.scale, self.window, span=span)
         elif plan.info["n_tiles"]:
             kernels.attn_prefill(q, out, cache.k, cache.v, ctx.req_slot, cache.block_table, plan["tile_req"], plan["tile_q0"],
                                  ctx.q_start, ctx.q_len, ctx.ctx_len, hq, hkv, cache.page_size, self.scale, self.window)
@@ -159,18 +160,30 @@ def decode_ranges(longest_context: int) -> int:
     return n
 
 
+WIDE_CTAS = 148            # CTAs of the tcgen05 prompt attention that run at once: one per SM
+
+
+def wide_tiles(plan, heads: int) -> tuple:
+    """The tile list for the tcgen05 prompt attention, and its queries per tile.  A CTA does most work per copy with 256
+    queries; where CTAs of 128 all run at once, twice as many of half the length end sooner (2048 queries, 9 heads of 64: 26
+    us against 36; 300 queries, 32 heads of 128: 14.5 against 15.6; 512 CTAs of 128 queries: 72 against 57)."""
+    if plan.info["n_wide"] * heads <= WIDE_CTAS:
+        return (plan["wide_req"], plan["wide_q0"]), kernels.WIDE_TILE
+    return (plan["pair_req"], plan["pair_q0"]), kernels.WIDE_PAIR
+
+
 ATTENTION_PLAN_KEY = ("paged_attention", kernels.PREFILL_TILE, kernels.WIDE_TILE, DECODE_RANGE)
 
 
 def attention_step_plan(host):
     """Which CTAs the attention kernels launch for a step: portions of more than one token are cut into query
-    tiles (request, first query), once per tile size of the two prompt kernels, a portion's last tile first (it
+    tiles (request, first query), once per tile size of the prompt kernels, a portion's last tile first (it
     has the longest key loop); single tokens are listed for the split kernel, whose number of key ranges comes
     from the longest context among them (or from the bound a captured graph was made for).  Every mixer that runs
     the paged attention kernels shares this plan (`ATTENTION_PLAN_KEY`)."""
     from ..engine.batch import StepPlan
 
-    tile_req, tile_q0, wide_req, wide_q0, dec_req = [], [], [], [], []
+    tile_req, tile_q0, wide_req, wide_q0, pair_req, pair_q0, dec_req = [], [], [], [], [], [], []
     longest = 0
     for r, n in enumerate(host.q_len):
         if n == 1:
@@ -183,12 +196,15 @@ def attention_step_plan(host):
             for q0 in reversed(range(0, n, kernels.WIDE_TILE)):
                 wide_req.append(r)
                 wide_q0.append(q0)
+            for q0 in reversed(range(0, n, kernels.WIDE_PAIR)):
+                pair_req.append(r)
+                pair_q0.append(q0)
     if dec_req and host.ctx_bound:
         longest = max(longest, host.ctx_bound)
     as_i32 = lambda values: np.asarray(values, dtype=np.int32)
     return StepPlan(
         arrays={"tile_req": as_i32(tile_req), "tile_q0": as_i32(tile_q0), "wide_req": as_i32(wide_req),
-                "wide_q0": as_i32(wide_q0), "dec_req": as_i32(dec_req)},
+                "wide_q0": as_i32(wide_q0), "pair_req": as_i32(pair_req), "pair_q0": as_i32(pair_q0), "dec_req": as_i32(dec_req)},
         info={"n_tiles": len(tile_req), "n_wide": len(wide_req), "n_decode": len(dec_req),
               "n_splits": decode_ranges(longest)})
 
@@ -203,9 +219,9 @@ def paged_attention(plan, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, cac
     tokens, _, dim = q.shape
     out = torch.empty_like(q)
     if plan.info["n_tiles"] and kernels.attn_prefill_wide_ok(q, k, cache.page_size):
-        kernels.attn_prefill_wide(q, out, k, v, ctx.req_slot, cache.block_table, plan["wide_req"], plan["wide_q0"],
-                                  ctx.q_start, ctx.q_len, ctx.ctx_len, hq, hkv, cache.page_size, scale, window, sink=sink,
-                                  keep_first=keep_first, softcap=softcap)
+        tiles, span = wide_tiles(plan, hq)
+        kernels.attn_prefill_wide(q, out, k, v, ctx.req_slot, cache.block_table, *tiles, ctx.q_start, ctx.q_len, ctx.ctx_len, hq, hkv,
+                                  cache.page_size, scale, window, sink=sink, keep_first=keep_first, softcap=softcap, span=span)
     elif plan.info["n_tiles"]:
         kernels.attn_prefill(q, out, k, v, ctx.req_slot, cache.block_table, plan["tile_req"], plan["tile_q0"],
                              ctx.q_start, ctx.q_len, ctx.ctx_len, hq, hkv, cache.page_size, scale, window, sink=sink,
