@@ -1,0 +1,297 @@
+// The chunk products of the recurrences with a matrix state per head (gated_linear.cu, lightning.cu).  For a chunk of n <= 64
+// tokens with S0 the state before it, L_t the sum of the logarithms of the decays up to token t, and gains g:
+//     gain    sum_i exp(L_n - L_i) g_i k_i v_i^T                             a tile of 64 x 64 of [N, dv] per CTA
+//     scores  q_t . k_i                                                      a CTA per chunk and group
+//     read    exp(L_t) S0^T q_t + sum_{i <= t} exp(L_t - L_i) g_i (q_t . k_i) v_i     64 tokens x 64 value columns per CTA
+// Every product is 64 x 64 x 64 at a time, float on the tensor cores (split_mma.cuh), 256 threads and 55 KB of shared
+// memory: three CTAs share an SM, and one loads and splits its operands while the others multiply.
+// What bounds it: loading and splitting the operands (and silu, where it is taken here) beside a quarter of the tensor rate.
+// Measured at 2048 tokens, against tiles on the CUDA cores: lightning, 16 heads of 128 x 128, gains with scores 64 us and
+// reads 50 (before 57 without scores and 141 with them); a matrix memory of 8 heads of 128 x 256, 2100 tokens, 45 and 47
+// (59 and 65).
+#pragma once
+#include "split_mma.cuh"
+
+namespace {
+constexpr int CHUNK = 64;
+constexpr int CHUNK_THREADS = 256;
+constexpr size_t CHUNK_SMEM = 2 * sizeof(SplitTile);
+
+struct ChunkArgs {
+    const float* q; const float* k; const float* v;      // at their first column; rows of `*_stride` floats
+    int q_stride, k_stride, v_stride;
+    const float* la; const float* g;                     // [tokens][heads]: logarithms of the decays, gains; null:
+    const float* decay;                                  // [heads] one decay per head, gains of one
+    float* state; long long state_stride;
+    const int* req_slot; const int* q_start; const int* q_len;
+    const int* chunk_req; const int* chunk_t0; const int* req_chunk0;
+    float* scores;                                       // [chunks][groups][CHUNK][CHUNK]
+    float* blocks;                                       // [chunks][heads][N * dv (+ N)]
+    float* chunk_decay;                                  // [chunks][heads] (may be null)
+    float* y; float* yn;                                 // [tokens][heads][dv], [tokens][heads]
+    float q_scale;
+    int heads, groups, N, dv, least;
+};
+
+__device__ __forceinline__ float chunk_silu(float z) { return z / (1.f + expf(-z)); }
+
+// Rows [0, nr) x columns [0, nc) of src (row stride `stride`), zeros elsewhere: asked for, and later put into a tile, so that
+// several tiles' loads are on their way together.  put: silu of each where asked, then each row times weight(row).
+constexpr int PER_THREAD = CHUNK * CHUNK / 4 / CHUNK_THREADS;        // runs of four floats of a tile per thread
+struct RawTile { float4 v[PER_THREAD]; };
+template <bool VEC>
+__device__ __forceinline__ void fetch_tile(RawTile& raw, const float* __restrict__ src, size_t stride, int nr, int nc) {
+#pragma unroll
+    for (int u = 0; u < PER_THREAD; ++u) {
+        const int i = threadIdx.x + u * CHUNK_THREADS, r = i >> 4, c = (i & 15) * 4;
+        const float* p = src + (size_t)r * stride + c;
+        if (VEC) {
+            raw.v[u] = (r < nr && c < nc) ? *reinterpret_cast<const float4*>(p) : make_float4(0.f, 0.f, 0.f, 0.f);
+        } else {
+            raw.v[u].x = (r < nr && c < nc) ? p[0] : 0.f; raw.v[u].y = (r < nr && c + 1 < nc) ? p[1] : 0.f;
+            raw.v[u].z = (r < nr && c + 2 < nc) ? p[2] : 0.f; raw.v[u].w = (r < nr && c + 3 < nc) ? p[3] : 0.f;
+        }
+    }
+}
+template <bool SILU, typename W>
+__device__ __forceinline__ void put_tile(SplitTile& dst, const RawTile& raw, W weight) {
+#pragma unroll
+    for (int u = 0; u < PER_THREAD; ++u) {
+        const int i = threadIdx.x + u * CHUNK_THREADS, r = i >> 4, c = (i & 15) * 4;
+        float4 v = raw.v[u];
+        if (SILU) { v.x = chunk_silu(v.x); v.y = chunk_silu(v.y); v.z = chunk_silu(v.z); v.w = chunk_silu(v.w); }
+        const float w = weight(r);
+        split_store4(dst, r, c, make_float4(v.x * w, v.y * w, v.z * w, v.w * w));
+    }
+}
+struct One { __device__ __forceinline__ float operator()(int) const { return 1.f; } };
+
+// L [CHUNK]: sums of the logarithms up to each token of the chunk, in double: their differences are what counts, and behind a
+// run of strong decays a float sum would have lost the digits of the weak ones.  Tokens beyond the portion add nothing.
+// `gain` receives g (zero beyond the portion).
+__device__ __forceinline__ void stage_decays(const ChunkArgs& a, int h, int token0, int n, double* L, float* gain) {
+    if (threadIdx.x < 32) {
+        const int t = 2 * threadIdx.x;
+        if (a.decay) {
+            const double lg = log((double)a.decay[h]);
+            L[t] = lg * min(t + 1, n);
+            L[t + 1] = lg * min(t + 2, n);
+        } else {
+            const double x = t < n ? (double)a.la[(size_t)(token0 + t) * a.heads + h] : 0.0;
+            const double y = t + 1 < n ? (double)a.la[(size_t)(token0 + t + 1) * a.heads + h] : 0.0;
+            double sum = x + y;
+#pragma unroll
+            for (int off = 1; off < 32; off <<= 1) {
+                const double before = __shfl_up_sync(0xffffffffu, sum, off);
+                if ((int)threadIdx.x >= off) sum += before;
+            }
+            L[t + 1] = sum;
+            L[t] = sum - y;
+        }
+    } else if (threadIdx.x >= 64 && threadIdx.x < 64 + CHUNK) {
+        const int t = threadIdx.x - 64;
+        gain[t] = t < n ? (a.decay ? 1.f : a.g[(size_t)(token0 + t) * a.heads + h]) : 0.f;
+    }
+}
+
+// a warp's 16 x 32 part of a 64 x 64 result, element pairs (row, col, col + 1) handed to `put`
+template <typename P>
+__device__ __forceinline__ void for_result(const float (&acc)[4][4], int m0, int n0, P put) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int half = 0; half < 2; ++half)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) put(m0 + 8 * half + (lane >> 2), n0 + 8 * j + 2 * (lane & 3), acc[j][2 * half], acc[j][2 * half + 1]);
+}
+template <bool VEC>
+__device__ __forceinline__ void put_pair(float* dst, int left, float x, float y) {       // `left` columns are there (VEC: an even number)
+    if (VEC) {
+        if (left > 0) *reinterpret_cast<float2*>(dst) = make_float2(x, y);
+    } else {
+        if (left > 0) dst[0] = x;
+        if (left > 1) dst[1] = y;
+    }
+}
+
+// q_t . k_i of one chunk and group (n tokens from row token0 on), every pair of tokens
+template <bool VEC, bool SILU>
+__device__ __forceinline__ void chunk_scores(const ChunkArgs& a, int chunk, int grp, int n, size_t token0, SplitTile& Q, SplitTile& K, int m0, int n0w) {
+    float acc[4][4] = {};
+    for (int n0 = 0; n0 < a.N; n0 += CHUNK) {
+        const int nc = min(CHUNK, a.N - n0);
+        RawTile q, k;
+        fetch_tile<VEC>(q, a.q + token0 * a.q_stride + grp * a.N + n0, a.q_stride, n, nc);
+        fetch_tile<VEC>(k, a.k + token0 * a.k_stride + grp * a.N + n0, a.k_stride, n, nc);
+        if (n0) __syncthreads();
+        put_tile<SILU>(Q, q, One());
+        put_tile<SILU>(K, k, One());
+        __syncthreads();
+        if (n0w <= m0 + 15) split_product<false, false>(acc, Q, K, m0, n0w, (nc + 15) >> 4);      // pairs with i > t are never read
+    }
+    float* out = a.scores + ((size_t)chunk * a.groups + grp) * CHUNK * CHUNK;
+    for_result(acc, m0, n0w, [&](int t, int i, float x, float y) { *reinterpret_cast<float2*>(out + t * CHUNK + i) = make_float2(x, y); });
+}
+
+// grid (chunk, head, tiles of [N, dv] + 1): the last z makes the scores of the chunk's groups, in the CTAs of the first heads
+template <bool VEC, bool NORM, bool SILU>
+__global__ void __launch_bounds__(CHUNK_THREADS, 3)
+chunk_gains_kernel(const ChunkArgs a) {
+    extern __shared__ __align__(16) unsigned char chunk_smem[];
+    __shared__ double L[CHUNK];
+    __shared__ float w[CHUNK];
+    SplitTile& K = reinterpret_cast<SplitTile*>(chunk_smem)[0];
+    SplitTile& V = reinterpret_cast<SplitTile*>(chunk_smem)[1];
+    pdl_trigger();
+    const int chunk = blockIdx.x, h = blockIdx.y, warp = threadIdx.x >> 5, m0 = 16 * (warp >> 1), n0w = 32 * (warp & 1);
+    const bool scores = blockIdx.z == gridDim.z - 1;
+    const int row_tiles = (a.N + CHUNK - 1) / CHUNK;
+    const int n0 = ((int)blockIdx.z % row_tiles) * CHUNK, c0 = ((int)blockIdx.z / row_tiles) * CHUNK;
+    const int grp = h / (a.heads / a.groups);
+    const int r = a.chunk_req[chunk], t0 = a.chunk_t0[chunk], n = min(CHUNK, a.q_len[r] - t0);
+    const int token0 = a.q_start[r] + t0;
+    const int nr = min(CHUNK, a.N - n0), nc = min(CHUNK, a.dv - c0);
+    pdl_wait();
+    if (scores) {
+        if (h < a.groups) chunk_scores<VEC, SILU>(a, chunk, h, n, (size_t)token0, K, V, m0, n0w);
+        return;
+    }
+    RawTile k, v;
+    fetch_tile<VEC>(k, a.k + (size_t)token0 * a.k_stride + grp * a.N + n0, a.k_stride, n, nr);
+    fetch_tile<VEC>(v, a.v + (size_t)token0 * a.v_stride + h * a.dv + c0, a.v_stride, n, nc);
+    stage_decays(a, h, token0, n, L, w);
+    put_tile<SILU>(K, k, One());
+    __syncthreads();
+    if (threadIdx.x < CHUNK) w[threadIdx.x] *= expf((float)(L[CHUNK - 1] - L[threadIdx.x]));
+    if (a.chunk_decay && blockIdx.z == 0 && threadIdx.x == 0) a.chunk_decay[(size_t)chunk * a.heads + h] = expf((float)L[CHUNK - 1]);
+    __syncthreads();
+    put_tile<SILU>(V, v, [&](int t) { return w[t]; });
+    __syncthreads();
+    float acc[4][4] = {};
+    split_product<true, true>(acc, K, V, m0, n0w, (n + 15) >> 4);
+    const size_t per_head = (size_t)a.N * a.dv + (NORM ? a.N : 0);
+    float* out = a.blocks + ((size_t)chunk * a.heads + h) * per_head;
+    for_result(acc, m0, n0w, [&](int row, int c, float x, float y) {
+        if (row < nr) put_pair<VEC>(out + (size_t)(n0 + row) * a.dv + c0 + c, nc - c, x, y);
+    });
+    if (NORM && c0 == 0 && (int)threadIdx.x < nr) {
+        float sum = 0.f;
+        for (int i = 0; i < n; ++i)
+            sum = fmaf(w[i], to_float(K.part[0][i][threadIdx.x]) + (to_float(K.part[1][i][threadIdx.x]) + to_float(K.part[2][i][threadIdx.x])), sum);
+        out[(size_t)a.N * a.dv + n0 + threadIdx.x] = sum;
+    }
+}
+
+// grid (chunk, head, 64 value columns): the running product of [q exp(L) | scores with their decays] and [S0 ; v]
+template <bool VEC, bool NORM, bool SILU>
+__global__ void __launch_bounds__(CHUNK_THREADS, 3)
+chunk_reads_kernel(const ChunkArgs a) {
+    extern __shared__ __align__(16) unsigned char chunk_smem[];
+    __shared__ double L[CHUNK];
+    __shared__ float gain[CHUNK], carried[CHUNK], nvec[CHUNK];
+    SplitTile& A = reinterpret_cast<SplitTile*>(chunk_smem)[0];
+    SplitTile& B = reinterpret_cast<SplitTile*>(chunk_smem)[1];
+    pdl_trigger();
+    const int chunk = blockIdx.x, h = blockIdx.y, c0 = blockIdx.z * CHUNK, tid = threadIdx.x, warp = tid >> 5, m0 = 16 * (warp >> 1), n0w = 32 * (warp & 1);
+    const int grp = h / (a.heads / a.groups);
+    const int r = a.chunk_req[chunk], t0 = a.chunk_t0[chunk], n = min(CHUNK, a.q_len[r] - t0);
+    const int token0 = a.q_start[r] + t0, nc = min(CHUNK, a.dv - c0);
+    const size_t per_head = (size_t)a.N * a.dv + (NORM ? a.N : 0);
+    const float* block = a.blocks + ((size_t)chunk * a.heads + h) * per_head;
+    const bool norm_here = NORM && c0 == 0;
+    const int nt = tid >> 2, nq = (tid & 3) * 16;             // normaliser: four threads per token, a quarter of a row each
+    float norm = 0.f;
+    pdl_wait();
+    stage_decays(a, h, token0, n, L, gain);
+    float acc[4][4] = {};
+    for (int n0 = 0; n0 < a.N; n0 += CHUNK) {
+        const int nr = min(CHUNK, a.N - n0);
+        RawTile q, s0;
+        fetch_tile<VEC>(q, a.q + (size_t)token0 * a.q_stride + grp * a.N + n0, a.q_stride, n, nr);
+        fetch_tile<VEC>(s0, block + (size_t)n0 * a.dv + c0, a.dv, nr, nc);
+        if (n0) __syncthreads();
+        put_tile<SILU>(A, q, One());
+        put_tile<false>(B, s0, One());
+        if (norm_here && tid < CHUNK) nvec[tid] = tid < nr ? block[(size_t)a.N * a.dv + n0 + tid] : 0.f;
+        __syncthreads();
+        split_product<false, true>(acc, A, B, m0, n0w, (nr + 15) >> 4);
+        if (norm_here)
+            for (int i = 0; i < 16; i += 8) {
+                float q[8];
+                split_read8(A, nt, nq + i, q);
+#pragma unroll
+                for (int e = 0; e < 8; ++e) norm = fmaf(q[e], nvec[nq + i + e], norm);
+            }
+    }
+    const float* G = a.scores + ((size_t)chunk * a.groups + grp) * CHUNK * CHUNK;
+    RawTile v, sc;
+    fetch_tile<VEC>(v, a.v + (size_t)token0 * a.v_stride + h * a.dv + c0, a.v_stride, n, nc);
+    fetch_tile<true>(sc, G, CHUNK, CHUNK, CHUNK);
+    if (tid < CHUNK) carried[tid] = expf((float)L[tid]);
+    __syncthreads();
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+        const float f = carried[m0 + 8 * half + ((tid & 31) >> 2)];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) { acc[j][2 * half] *= f; acc[j][2 * half + 1] *= f; }
+    }
+    norm *= carried[nt];
+    put_tile<SILU>(B, v, One());
+#pragma unroll
+    for (int u = 0; u < PER_THREAD; ++u) {
+        const int i4 = tid + u * CHUNK_THREADS, t = i4 >> 4, i = (i4 & 15) * 4;
+        float p[4] = {0.f, 0.f, 0.f, 0.f};
+        if (i <= t) {
+            const float sv[4] = {sc.v[u].x, sc.v[u].y, sc.v[u].z, sc.v[u].w};
+            const double Lt = L[t];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) p[e] = i + e <= t ? sv[e] * gain[i + e] * expf((float)(Lt - L[i + e])) : 0.f;
+        }
+        split_store4(A, t, i, make_float4(p[0], p[1], p[2], p[3]));
+    }
+    __syncthreads();
+    split_product<false, true>(acc, A, B, m0, n0w, m0 / 16 + 1);         // P holds nothing right of the diagonal
+    if (norm_here) {
+        for (int i = 0; i < 16; i += 8) {
+            float p[8];
+            split_read8(A, nt, nq + i, p);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) norm += p[e];
+        }
+        norm += __shfl_xor_sync(0xffffffffu, norm, 1);
+        norm += __shfl_xor_sync(0xffffffffu, norm, 2);
+        if (nq == 0 && nt < n) a.yn[(size_t)(token0 + nt) * a.heads + h] = norm * a.q_scale;
+    }
+    for_result(acc, m0, n0w, [&](int t, int c, float x, float y) {
+        if (t < n) put_pair<VEC>(a.y + ((size_t)(token0 + t) * a.heads + h) * a.dv + c0 + c, nc - c, x * a.q_scale, y * a.q_scale);
+    });
+}
+
+// Whether rows of four floats may be read (and pairs written) as one: widths, strides and addresses that allow it.
+inline bool chunk_vectors_ok(const ChunkArgs& a) {
+    return a.N % 4 == 0 && a.dv % 4 == 0 && a.q_stride % 4 == 0 && a.k_stride % 4 == 0 && a.v_stride % 4 == 0 &&
+           !(((uintptr_t)a.q | (uintptr_t)a.k | (uintptr_t)a.v | (uintptr_t)a.blocks | (uintptr_t)a.y) & 15);
+}
+template <bool VEC, bool NORM, bool SILU>
+int launch_chunk_gains(const ChunkArgs& a, int n_chunks, cudaStream_t s, bool pdl) {
+    static bool configured = false;
+    if (!configured) {
+        cudaError_t e = cudaFuncSetAttribute(chunk_gains_kernel<VEC, NORM, SILU>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CHUNK_SMEM);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(chunk_gains_kernel<VEC, NORM, SILU>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+        if (e != cudaSuccess) return (int)e;
+        configured = true;
+    }
+    const int tiles = ((a.N + CHUNK - 1) / CHUNK) * ((a.dv + CHUNK - 1) / CHUNK);
+    return launch_kernel(chunk_gains_kernel<VEC, NORM, SILU>, dim3(n_chunks, a.heads, tiles + 1), dim3(CHUNK_THREADS), CHUNK_SMEM, s, pdl, a);
+}
+template <bool VEC, bool NORM, bool SILU>
+int launch_chunk_reads(const ChunkArgs& a, int n_chunks, cudaStream_t s, bool pdl) {
+    static bool configured = false;
+    if (!configured) {
+        cudaError_t e = cudaFuncSetAttribute(chunk_reads_kernel<VEC, NORM, SILU>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CHUNK_SMEM);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(chunk_reads_kernel<VEC, NORM, SILU>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+        if (e != cudaSuccess) return (int)e;
+        configured = true;
+    }
+    return launch_kernel(chunk_reads_kernel<VEC, NORM, SILU>, dim3(n_chunks, a.heads, (a.dv + CHUNK - 1) / CHUNK), dim3(CHUNK_THREADS), CHUNK_SMEM, s, pdl, a);
+}
+}  // namespace

@@ -23,34 +23,18 @@
 //                   same launch the scores q_t . k_i per (chunk, group), which every head of a group reads
 //           scan    walks a request's chunks element by element: a block receives the state BEFORE its chunk
 //           reads   the read-outs of every chunk at once: one running product over [q exp(L) | scores with their decays] and [S0 ; v]
-//           Each is a 64 x 64 tile per CTA of 128 threads with 8 x 4 results per thread, float on the CUDA cores.
-// The sums L are kept in double: their differences are what counts, and behind a run of strong decays a float sum would
-// have lost the digits of the weak ones.
-#include "common.cuh"
+//           Each is a 64 x 64 tile per CTA, float through the tensor cores (chunk_linear.cuh).
+#include "chunk_linear.cuh"
 
 static bool g_pdl = false;
 CISR_EXPORT void cisr_gated_set_pdl(int on) { g_pdl = on != 0; }
 
-constexpr int CHUNK = 64;
 constexpr int MAX_ROWS = 512;        // largest N: 16 row groups of at most 32 rows
 CISR_EXPORT int cisr_gated_chunk_tokens() { return CHUNK; }
 CISR_EXPORT int cisr_gated_max_key_dim() { return MAX_ROWS; }
 
 namespace {
-struct Args {
-    const float* q; const float* k; const float* v;      // at their first column; rows of `*_stride` floats
-    int q_stride, k_stride, v_stride;
-    const float* la; const float* g;                     // [tokens][heads]
-    float* state; long long state_stride;
-    const int* req_slot; const int* q_start; const int* q_len;
-    const int* chunk_req; const int* chunk_t0; const int* req_chunk0;
-    float* scores;                                       // [chunks][groups][CHUNK][CHUNK]
-    float* blocks;                                       // [chunks][heads][N * dv (+ N)]
-    float* chunk_decay;                                  // [chunks][heads]
-    float* y; float* yn;                                 // [tokens][heads][dv], [tokens][heads]
-    float q_scale;
-    int heads, groups, N, dv, least;
-};
+typedef ChunkArgs Args;
 
 // ------------------------------------------------------------------ token by token
 constexpr int TB = 8;                // tokens staged together
@@ -175,159 +159,7 @@ gated_walk_kernel(const Args a) {
     }
 }
 
-// ------------------------------------------------------------------ chunk by chunk
-constexpr int LDT = CHUNK + 4;       // row stride of a 64 x 64 tile in shared memory: 16-byte rows, eight neighbouring rows in different banks
-constexpr int THREADS = 128;
-
-// rows [0, nr) x columns [0, nc) of src (row stride `stride`) into dst [64][LDT], zeros elsewhere
-template <bool VEC>
-__device__ __forceinline__ void stage(float* dst, const float* __restrict__ src, size_t stride, int nr, int nc) {
-    if (VEC) {
-        float4 raw[8];
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            const int i = threadIdx.x + u * THREADS, r = i >> 4, c = (i & 15) * 4;
-            raw[u] = (r < nr && c < nc) ? *reinterpret_cast<const float4*>(src + (size_t)r * stride + c) : make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            const int i = threadIdx.x + u * THREADS, r = i >> 4, c = (i & 15) * 4;
-            *reinterpret_cast<float4*>(dst + r * LDT + c) = raw[u];
-        }
-    } else {
-#pragma unroll 8
-        for (int i = threadIdx.x; i < CHUNK * CHUNK; i += THREADS) {
-            const int r = i >> 6, c = i & 63;
-            dst[r * LDT + c] = (r < nr && c < nc) ? src[(size_t)r * stride + c] : 0.f;
-        }
-    }
-}
-
-// Sums of la up to each token of the chunk (double), by the first warp: lane l owns tokens 2 l and 2 l + 1.  Tokens beyond
-// the portion add nothing.  `gain` receives g (zero beyond the portion).
-__device__ __forceinline__ void stage_decays(const Args& a, int h, int token0, int n, double* L, float* gain) {
-    if (threadIdx.x < 32) {
-        const int t = 2 * threadIdx.x;
-        const double x = t < n ? (double)a.la[(size_t)(token0 + t) * a.heads + h] : 0.0;
-        const double y = t + 1 < n ? (double)a.la[(size_t)(token0 + t + 1) * a.heads + h] : 0.0;
-        double sum = x + y;
-#pragma unroll
-        for (int off = 1; off < 32; off <<= 1) {
-            const double before = __shfl_up_sync(0xffffffffu, sum, off);
-            if ((int)threadIdx.x >= off) sum += before;
-        }
-        L[t + 1] = sum;
-        L[t] = sum - y;
-    } else if (threadIdx.x >= 64) {
-        const int t = threadIdx.x - 64;
-        gain[t] = t < n ? a.g[(size_t)(token0 + t) * a.heads + h] : 0.f;
-    }
-}
-
-// q_t . k_i of one chunk and group (n tokens from row token0 on), every pair of tokens
-template <bool VEC>
-__device__ __forceinline__ void chunk_scores(const Args& a, int chunk, int grp, int n, size_t token0, float* Q, float* K) {
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    float acc[8][4] = {};
-    for (int n0 = 0; n0 < a.N; n0 += CHUNK) {
-        const int nc = min(CHUNK, a.N - n0);
-        if (n0) __syncthreads();
-        stage<VEC>(Q, a.q + token0 * a.q_stride + grp * a.N + n0, a.q_stride, n, nc);
-        stage<VEC>(K, a.k + token0 * a.k_stride + grp * a.N + n0, a.k_stride, n, nc);
-        __syncthreads();
-        const int k4s = (nc + 3) >> 2;
-        for (int k4 = 0; k4 < k4s; ++k4) {
-            float4 k[4];
-#pragma unroll
-            for (int y = 0; y < 4; ++y) k[y] = *reinterpret_cast<const float4*>(K + (tx + 16 * y) * LDT + 4 * k4);
-#pragma unroll
-            for (int x = 0; x < 8; ++x) {
-                const float4 q = *reinterpret_cast<const float4*>(Q + (ty + 8 * x) * LDT + 4 * k4);
-#pragma unroll
-                for (int y = 0; y < 4; ++y) {
-                    acc[x][y] = fmaf(q.x, k[y].x, acc[x][y]); acc[x][y] = fmaf(q.y, k[y].y, acc[x][y]);
-                    acc[x][y] = fmaf(q.z, k[y].z, acc[x][y]); acc[x][y] = fmaf(q.w, k[y].w, acc[x][y]);
-                }
-            }
-        }
-    }
-    float* out = a.scores + ((size_t)chunk * a.groups + grp) * CHUNK * CHUNK;
-#pragma unroll
-    for (int x = 0; x < 8; ++x)
-#pragma unroll
-        for (int y = 0; y < 4; ++y) out[(ty + 8 * x) * CHUNK + tx + 16 * y] = acc[x][y];
-}
-
-// grid (chunk, head, tiles of [N, dv] + 1): the last z makes the scores of the chunk's groups, in the CTAs of the first heads
-template <bool VEC, bool NORM>
-__global__ void __launch_bounds__(THREADS, 5)
-gated_gains_kernel(const Args a) {
-    extern __shared__ __align__(16) float smem[];
-    __shared__ double L[CHUNK];
-    __shared__ float w[CHUNK];
-    float* K = smem;
-    float* V = K + CHUNK * LDT;
-    pdl_trigger();
-    const int chunk = blockIdx.x, h = blockIdx.y, tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    const bool scores = blockIdx.z == gridDim.z - 1;
-    const int row_tiles = (a.N + CHUNK - 1) / CHUNK;
-    const int n0 = ((int)blockIdx.z % row_tiles) * CHUNK, c0 = ((int)blockIdx.z / row_tiles) * CHUNK;
-    const int grp = h / (a.heads / a.groups);
-    const int r = a.chunk_req[chunk], t0 = a.chunk_t0[chunk], n = min(CHUNK, a.q_len[r] - t0);
-    const int token0 = a.q_start[r] + t0;
-    const int nr = min(CHUNK, a.N - n0), nc = min(CHUNK, a.dv - c0);
-    pdl_wait();
-    if (scores) {
-        if (h < a.groups) chunk_scores<VEC>(a, chunk, h, n, (size_t)token0, K, V);
-        return;
-    }
-    stage_decays(a, h, token0, n, L, w);
-    stage<VEC>(K, a.k + (size_t)token0 * a.k_stride + grp * a.N + n0, a.k_stride, n, nr);
-    stage<VEC>(V, a.v + (size_t)token0 * a.v_stride + h * a.dv + c0, a.v_stride, n, nc);
-    __syncthreads();
-    if (threadIdx.x < CHUNK) w[threadIdx.x] *= expf((float)(L[CHUNK - 1] - L[threadIdx.x]));
-    if (blockIdx.z == 0 && threadIdx.x == 0) a.chunk_decay[(size_t)chunk * a.heads + h] = expf((float)L[CHUNK - 1]);
-    __syncthreads();
-    float acc[2][4][4] = {};
-    for (int i = 0; i < n; ++i) {
-        const float wi = w[i];
-        float4 v = *reinterpret_cast<const float4*>(V + i * LDT + 4 * tx);
-        v.x *= wi; v.y *= wi; v.z *= wi; v.w *= wi;
-#pragma unroll
-        for (int half = 0; half < 2; ++half) {
-            const float4 k = *reinterpret_cast<const float4*>(K + i * LDT + 32 * half + 4 * ty);
-            const float kv[4] = {k.x, k.y, k.z, k.w};
-#pragma unroll
-            for (int x = 0; x < 4; ++x) {
-                acc[half][x][0] = fmaf(kv[x], v.x, acc[half][x][0]); acc[half][x][1] = fmaf(kv[x], v.y, acc[half][x][1]);
-                acc[half][x][2] = fmaf(kv[x], v.z, acc[half][x][2]); acc[half][x][3] = fmaf(kv[x], v.w, acc[half][x][3]);
-            }
-        }
-    }
-    const size_t per_head = (size_t)a.N * a.dv + (NORM ? a.N : 0);
-    float* out = a.blocks + ((size_t)chunk * a.heads + h) * per_head;
-#pragma unroll
-    for (int half = 0; half < 2; ++half)
-#pragma unroll
-        for (int x = 0; x < 4; ++x) {
-            const int row = 32 * half + 4 * ty + x;
-            if (row >= nr) continue;
-            float* dst = out + (size_t)(n0 + row) * a.dv + c0 + 4 * tx;
-            if (VEC) {
-                if (4 * tx < nc) *reinterpret_cast<float4*>(dst) = make_float4(acc[half][x][0], acc[half][x][1], acc[half][x][2], acc[half][x][3]);
-            } else {
-#pragma unroll
-                for (int e = 0; e < 4; ++e)
-                    if (4 * tx + e < nc) dst[e] = acc[half][x][e];
-            }
-        }
-    if (NORM && c0 == 0 && (int)threadIdx.x < nr) {
-        float sum = 0.f;
-        for (int i = 0; i < n; ++i) sum = fmaf(w[i], K[i * LDT + threadIdx.x], sum);
-        out[(size_t)a.N * a.dv + n0 + threadIdx.x] = sum;
-    }
-}
-
+// ------------------------------------------------------------------ chunk by chunk: chunk_linear.cuh, and the scan between its two launches
 // grid (requests, heads, elements / (256 VEC)): a thread owns VEC neighbouring elements of the head's [N * dv (+ N)] state
 template <int VEC, bool NORM>
 __global__ void __launch_bounds__(256)
@@ -387,101 +219,6 @@ gated_scan_kernel(const Args a) {
     for (int j = 0; j < VEC; ++j) kept[j] = S[j];
 }
 
-// acc[x][y] += sum_k A[ty + 8 x][k] B[k][4 tx + y] over the first 4 * k4s rows of B
-__device__ __forceinline__ void tile_product(const float* A, const float* B, int tx, int ty, int k4s, float (&acc)[8][4]) {
-    for (int k4 = 0; k4 < k4s; ++k4) {
-        float4 b[4];
-#pragma unroll
-        for (int kk = 0; kk < 4; ++kk) b[kk] = *reinterpret_cast<const float4*>(B + (4 * k4 + kk) * LDT + 4 * tx);
-#pragma unroll
-        for (int x = 0; x < 8; ++x) {
-            const float4 av = *reinterpret_cast<const float4*>(A + (ty + 8 * x) * LDT + 4 * k4);
-            const float f[4] = {av.x, av.y, av.z, av.w};
-#pragma unroll
-            for (int kk = 0; kk < 4; ++kk) {
-                acc[x][0] = fmaf(f[kk], b[kk].x, acc[x][0]); acc[x][1] = fmaf(f[kk], b[kk].y, acc[x][1]);
-                acc[x][2] = fmaf(f[kk], b[kk].z, acc[x][2]); acc[x][3] = fmaf(f[kk], b[kk].w, acc[x][3]);
-            }
-        }
-    }
-}
-
-template <bool VEC, bool NORM>
-__global__ void __launch_bounds__(THREADS, 5)
-gated_reads_kernel(const Args a) {
-    extern __shared__ __align__(16) float smem[];
-    __shared__ double L[CHUNK];
-    __shared__ float gain[CHUNK], carried[CHUNK], nvec[CHUNK];
-    float* A = smem;
-    float* B = A + CHUNK * LDT;
-    pdl_trigger();
-    const int chunk = blockIdx.x, h = blockIdx.y, c0 = blockIdx.z * CHUNK, tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-    const int grp = h / (a.heads / a.groups);
-    const int r = a.chunk_req[chunk], t0 = a.chunk_t0[chunk], n = min(CHUNK, a.q_len[r] - t0);
-    const int token0 = a.q_start[r] + t0, nc = min(CHUNK, a.dv - c0);
-    const size_t per_head = (size_t)a.N * a.dv + (NORM ? a.N : 0);
-    const float* block = a.blocks + ((size_t)chunk * a.heads + h) * per_head;
-    const bool norm_here = NORM && c0 == 0;
-    const int nt = tid >> 1, nhalf = (tid & 1) * 32;          // normaliser: two threads per token, half a row each
-    float norm = 0.f;
-    pdl_wait();
-    stage_decays(a, h, token0, n, L, gain);
-    float acc[8][4] = {};
-    for (int n0 = 0; n0 < a.N; n0 += CHUNK) {
-        const int nr = min(CHUNK, a.N - n0);
-        if (n0) __syncthreads();
-        stage<VEC>(A, a.q + (size_t)token0 * a.q_stride + grp * a.N + n0, a.q_stride, n, nr);
-        stage<VEC>(B, block + (size_t)n0 * a.dv + c0, a.dv, nr, nc);
-        if (norm_here && tid < CHUNK) nvec[tid] = tid < nr ? block[(size_t)a.N * a.dv + n0 + tid] : 0.f;
-        __syncthreads();
-        tile_product(A, B, tx, ty, (nr + 3) >> 2, acc);
-        if (norm_here)
-            for (int i = 0; i < 32; ++i) norm = fmaf(A[nt * LDT + nhalf + i], nvec[nhalf + i], norm);
-    }
-    if (tid < CHUNK) carried[tid] = expf((float)L[tid]);
-    __syncthreads();
-#pragma unroll
-    for (int x = 0; x < 8; ++x) {
-        const float f = carried[ty + 8 * x];
-#pragma unroll
-        for (int y = 0; y < 4; ++y) acc[x][y] *= f;
-    }
-    norm *= carried[nt];
-    stage<VEC>(B, a.v + (size_t)token0 * a.v_stride + h * a.dv + c0, a.v_stride, n, nc);
-    const float* G = a.scores + ((size_t)chunk * a.groups + grp) * CHUNK * CHUNK;
-#pragma unroll
-    for (int u = 0; u < 8; ++u) {
-        const int i4 = tid + u * THREADS, t = i4 >> 4, i = (i4 & 15) * 4;
-        const float4 raw = *reinterpret_cast<const float4*>(G + t * CHUNK + i);
-        const float sc[4] = {raw.x, raw.y, raw.z, raw.w};
-        float p[4];
-        const double Lt = L[t];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) p[e] = i + e <= t ? sc[e] * gain[i + e] * expf((float)(Lt - L[i + e])) : 0.f;
-        *reinterpret_cast<float4*>(A + t * LDT + i) = make_float4(p[0], p[1], p[2], p[3]);
-    }
-    __syncthreads();
-    tile_product(A, B, tx, ty, CHUNK / 4, acc);
-    if (norm_here) {
-        for (int i = 0; i < 32; ++i) norm += A[nt * LDT + nhalf + i];
-        norm += __shfl_xor_sync(0xffffffffu, norm, 1);
-        if (nhalf == 0 && nt < n) a.yn[(size_t)(token0 + nt) * a.heads + h] = norm * a.q_scale;
-    }
-#pragma unroll
-    for (int x = 0; x < 8; ++x) {
-        const int t = ty + 8 * x;
-        if (t >= n) continue;
-        float* dst = a.y + ((size_t)(token0 + t) * a.heads + h) * a.dv + c0 + 4 * tx;
-        if (VEC) {
-            if (4 * tx < nc) *reinterpret_cast<float4*>(dst) = make_float4(acc[x][0] * a.q_scale, acc[x][1] * a.q_scale, acc[x][2] * a.q_scale, acc[x][3] * a.q_scale);
-        } else {
-#pragma unroll
-            for (int e = 0; e < 4; ++e)
-                if (4 * tx + e < nc) dst[e] = acc[x][e] * a.q_scale;
-        }
-    }
-}
-
 template <int ROWS, int VEC, bool NORM>
 int launch_walk(const Args& a, int n_req, cudaStream_t s) {
     constexpr int NP = 16 * ROWS, COLS = 16 * VEC;
@@ -504,16 +241,7 @@ int walk(const Args& a, int n_req, cudaStream_t s) {
 
 template <bool VEC, bool NORM>
 int chunks(const Args& a, int n_req, int n_chunks, cudaStream_t s) {
-    const size_t smem = sizeof(float) * 2 * CHUNK * LDT;       // 34 KB: within the default limit
-    const int row_tiles = (a.N + CHUNK - 1) / CHUNK, col_tiles = (a.dv + CHUNK - 1) / CHUNK;
-    static bool configured = false;
-    if (!configured) {       // five CTAs per SM want more shared memory than the default split gives
-        cudaError_t e = cudaFuncSetAttribute(gated_gains_kernel<VEC, NORM>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(gated_reads_kernel<VEC, NORM>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-        if (e != cudaSuccess) return (int)e;
-        configured = true;
-    }
-    int st = launch_kernel(gated_gains_kernel<VEC, NORM>, dim3(n_chunks, a.heads, row_tiles * col_tiles + 1), dim3(THREADS), smem, s, g_pdl, a);
+    int st = launch_chunk_gains<VEC, NORM, false>(a, n_chunks, s, g_pdl);
     if (st) return st;
     const int elements = a.N * a.dv + (NORM ? a.N : 0);
     // two elements per thread where every block and every state row begins on 8 bytes and no pair straddles matrix and normaliser
@@ -521,7 +249,7 @@ int chunks(const Args& a, int n_req, int n_chunks, cudaStream_t s) {
     if (pairs) st = launch_kernel(gated_scan_kernel<2, NORM>, dim3(n_req, a.heads, (elements / 2 + 255) / 256), dim3(256), 0, s, g_pdl, a);
     else st = launch_kernel(gated_scan_kernel<1, NORM>, dim3(n_req, a.heads, (elements + 255) / 256), dim3(256), 0, s, g_pdl, a);
     if (st) return st;
-    return launch_kernel(gated_reads_kernel<VEC, NORM>, dim3(n_chunks, a.heads, col_tiles), dim3(THREADS), smem, s, g_pdl, a);
+    return launch_chunk_reads<VEC, NORM, false>(a, n_chunks, s, g_pdl);
 }
 }  // namespace
 
@@ -535,7 +263,7 @@ CISR_EXPORT int cisr_gated_recurrence(const float* q, int q_stride, const float*
                                       float* scores, float* blocks, float* chunk_decay, void* stream) {
     if (n_req <= 0) return 0;
     if (heads <= 0 || groups <= 0 || heads % groups || N <= 0 || N > MAX_ROWS || dv <= 0) return -2;
-    Args a;
+    Args a = {};
     a.q = q; a.k = k; a.v = v; a.q_stride = q_stride; a.k_stride = k_stride; a.v_stride = v_stride; a.la = la; a.g = g; a.state = state;
     a.state_stride = state_stride; a.req_slot = req_slot; a.q_start = q_start; a.q_len = q_len; a.chunk_req = chunk_req; a.chunk_t0 = chunk_t0;
     a.req_chunk0 = req_chunk0; a.scores = scores; a.blocks = blocks; a.chunk_decay = chunk_decay; a.y = y; a.yn = yn; a.q_scale = q_scale;
@@ -546,8 +274,7 @@ CISR_EXPORT int cisr_gated_recurrence(const float* q, int q_stride, const float*
     int st = 0;
     if (chunked) {
         if (!chunk_req || !chunk_t0 || !req_chunk0 || !scores || !blocks || !chunk_decay) return -2;
-        const bool vec = N % 4 == 0 && dv % 4 == 0 && q_stride % 4 == 0 && k_stride % 4 == 0 && v_stride % 4 == 0 &&
-                         !(((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)blocks | (uintptr_t)y) & 15);
+        const bool vec = chunk_vectors_ok(a);
         if (vec) st = yn ? chunks<true, true>(a, n_req, n_chunks, s) : chunks<true, false>(a, n_req, n_chunks, s);
         else st = yn ? chunks<false, true>(a, n_req, n_chunks, s) : chunks<false, false>(a, n_req, n_chunks, s);
         if (st) return st;

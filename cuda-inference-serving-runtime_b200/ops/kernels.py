@@ -1021,7 +1021,7 @@ def lightning_recurrence(proj: torch.Tensor, q_col: int, k_col: int, v_col: int,
     value_dim].  `least` > 0 with `chunks` = (chunk_req, chunk_t0, req_chunk0, n_chunks): the requests that bring at least
     that many tokens run chunk by chunk (per chunk of LIGHTNING_CHUNK tokens its request and its first token inside the
     portion, per request the index of its first chunk: int32 on the device), the `n_short` others token by token; 0: all
-    token by token.  `columns_per_cta` (16, 32, 64; 0: by the size of the launch): value columns a CTA of the chunked form takes."""
+    token by token.  `columns_per_cta` is accepted and changes nothing: a CTA of the chunked form takes 64 value columns."""
     _need(proj, torch.float32, "proj", 2); _need(decay, torch.float32, "decay", 1); _need(state, torch.float32, "state", 2)
     _need(o, torch.float32, "o", 2)
     for name, t in (("req_slot", req_slot), ("q_start", q_start), ("q_len", q_len)):
@@ -1030,7 +1030,7 @@ def lightning_recurrence(proj: torch.Tensor, q_col: int, k_col: int, v_col: int,
     if (decay.numel() != heads or state.shape[1] != heads * key_dim * value_dim or o.shape != (tokens, heads * value_dim)
             or max(q_col, k_col) + heads * key_dim > cols or v_col + heads * value_dim > cols or key_dim > LIGHTNING_MAX_KEY_DIM):
         raise KernelError("lightning_recurrence: shapes disagree")
-    chunk_req = chunk_t0 = req_chunk0 = scratch = None
+    chunk_req = chunk_t0 = req_chunk0 = scratch = scores = None
     n_chunks = 0
     if least > 0 and chunks is not None and chunks[3] > 0:
         chunk_req, chunk_t0, req_chunk0, n_chunks = chunks
@@ -1038,12 +1038,13 @@ def lightning_recurrence(proj: torch.Tensor, q_col: int, k_col: int, v_col: int,
             _need(t, torch.int32, name, 1)
         if chunk_req.numel() < n_chunks or chunk_t0.numel() < n_chunks or req_chunk0.numel() < n_req:
             raise KernelError("lightning_recurrence: the chunk lists are too short")
+        scores = torch.empty((n_chunks, heads, LIGHTNING_CHUNK, LIGHTNING_CHUNK), dtype=torch.float32, device=proj.device)
         scratch = torch.empty((n_chunks, heads, key_dim, value_dim), dtype=torch.float32, device=proj.device)
     launches = (3 if n_chunks else 0) + (1 if not n_chunks or n_short else 0)
     _check(_lightning().cisr_lightning_recurrence(_p(proj), cols, q_col, k_col, v_col, _p(decay), _p(state), ctypes.c_longlong(state.shape[1]),
                                                   _p(req_slot), _p(q_start), _p(q_len), _p(o), heads, key_dim, value_dim, n_req,
                                                   int(least if n_chunks else 0), int(n_chunks), int(n_short), _p(chunk_req), _p(chunk_t0),
-                                                  _p(req_chunk0), _p(scratch), int(columns_per_cta), _stream()), "lightning_recurrence",
+                                                  _p(req_chunk0), _p(scratch), _p(scores), _stream()), "lightning_recurrence",
            own=launches)
     return o
 

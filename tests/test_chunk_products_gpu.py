@@ -1,0 +1,84 @@
+"""The chunked recurrences whose products run as split bfloat16 parts on the tensor cores, at sizes around their 64 x 64
+tiles, against the recurrence token by token in float64."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+# 64 terms per product with four roundings, a few products and exponentials per result: some 2^-24 each, 4e-7 in all
+BOUND = 4e-7
+
+
+def i32(a):
+    return torch.tensor(a, dtype=torch.int32, device="cuda")
+
+
+def step_lists(lens):
+    req, t0, first = [], [], []
+    for r, n in enumerate(lens):
+        first.append(len(req))
+        for t in range(0, n, 64):
+            req.append(r); t0.append(t)
+    starts = [sum(lens[:i]) for i in range(len(lens))]
+    return starts, (i32(req), i32(t0), i32(first), len(req))
+
+
+def error(got, want):
+    assert torch.isfinite(got).all()
+    return float((got.double() - want).norm() / want.norm())
+
+
+SIZES = [(64, 64, [64]), (128, 128, [65, 127]), (50, 37, [64, 130]), (72, 50, [191]), (4, 4, [64, 200]), (130, 66, [128, 129])]
+
+
+@pytest.mark.parametrize("dk,dv,lens", SIZES)
+def test_lightning_chunks(dk, dv, lens):
+    from cisr_b200.ops import kernels
+    heads, g = 3, torch.Generator(device="cuda").manual_seed(dk + dv)
+    starts, chunks = step_lists(lens)
+    proj = torch.randn(sum(lens), heads * (2 * dk + dv), generator=g, device="cuda")
+    decay = torch.tensor([0.96, 0.998, 1.0], device="cuda")
+    state = torch.randn(len(lens), heads * dk * dv, generator=g, device="cuda")
+    silu = lambda x: x * torch.sigmoid(x)
+    q, k, v = (silu(x) for x in proj.double().split([heads * dk, heads * dk, heads * dv], 1))
+    want, ends = [], []
+    for r, n in enumerate(lens):
+        S = state[r].double().view(heads, dv, dk).transpose(1, 2).clone()
+        for t in range(starts[r], starts[r] + n):
+            S = decay.double()[:, None, None] * S + k[t].view(heads, dk, 1) * v[t].view(heads, 1, dv)
+            want.append(torch.einsum("hkv,hk->hv", S, q[t].view(heads, dk)).reshape(-1))
+        ends.append(S.transpose(1, 2).reshape(-1))
+    o = torch.full((sum(lens), heads * dv), float("nan"), device="cuda")
+    kernels.lightning_recurrence(proj, 0, heads * dk, 2 * heads * dk, decay, state, i32(range(len(lens))), i32(starts), i32(lens), len(lens), o, heads, dk, dv,
+                                 least=64, chunks=chunks)
+    assert error(o, torch.stack(want)) < BOUND and error(state, torch.stack(ends)) < BOUND
+
+
+@pytest.mark.parametrize("norm", [False, True])
+@pytest.mark.parametrize("N,dv,lens", SIZES)
+def test_gated_chunks(N, dv, lens, norm):
+    from cisr_b200.ops import kernels
+    heads, groups, g = 4, 2, torch.Generator(device="cuda").manual_seed(N + dv)
+    starts, chunks = step_lists(lens)
+    T = sum(lens)
+    rand = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    q, k, v = rand(T, groups * N), rand(T, groups * N), rand(T, heads * dv)
+    la, gain = -3.0 * torch.rand(T, heads, generator=g, device="cuda") ** 6, torch.rand(T, heads, generator=g, device="cuda")
+    state = rand(len(lens), heads * N * (dv + int(norm)))
+    y, yn = torch.full((T, heads, dv), float("nan"), device="cuda"), torch.full((T, heads), float("nan"), device="cuda") if norm else None
+    Q, K = (x.double().view(T, groups, N).repeat_interleave(2, 1) for x in (q, k))
+    V = v.double().view(T, heads, dv)
+    want, want_n, ends = [], [], []
+    for r, n in enumerate(lens):
+        S = state[r, :heads * N * dv].double().view(heads, N, dv).clone()
+        m = state[r, heads * N * dv:].double().view(heads, N).clone() if norm else torch.zeros(heads, N, device="cuda", dtype=torch.float64)
+        for t in range(starts[r], starts[r] + n):
+            e, gk = la[t].double().exp(), gain[t].double()[:, None] * K[t]
+            S, m = e[:, None, None] * S + gk[:, :, None] * V[t][:, None], e[:, None] * m + gk
+            want.append(0.5 * torch.einsum("hkv,hk->hv", S, Q[t]))
+            want_n.append(0.5 * (m * Q[t]).sum(-1))
+        ends.append(torch.cat([S.reshape(-1)] + ([m.reshape(-1)] if norm else [])))
+    kernels.gated_recurrence(q, 0, k, 0, v, 0, la, gain, state, i32(range(len(lens))), i32(starts), i32(lens), len(lens), y, groups, N, q_scale=0.5, yn=yn,
+                             least=64, chunks=chunks)
+    assert error(y, torch.stack(want)) < BOUND and error(state, torch.stack(ends)) < BOUND
+    if norm:
+        assert error(yn, torch.stack(want_n)) < BOUND
