@@ -20,7 +20,7 @@
 // A request's row of the state tensor holds [heads][key_dim][value_dim] and then [taps - 1][conv channels], all float.
 // A portion of a prompt and a single decoded token take the same path, so a position's result does not depend on
 // how the sequence was cut.  Everything that enters the recurrence is float.
-#include "common.cuh"
+#include "split_mma.cuh"
 
 static bool g_pdl = false;
 CISR_EXPORT void cisr_delta_set_pdl(int on) { g_pdl = on != 0; }
@@ -72,6 +72,84 @@ delta_prepare_kernel(const float* __restrict__ proj, int row_stride, const float
     for (int hd = threadIdx.x; hd < heads; hd += blockDim.x) {
         beta[(size_t)t * heads + hd] = 1.f / (1.f + expf(-row[b_col + hd]));
         decay[(size_t)t * heads + hd] = expf(-expf(a_log[hd]) * softplus(row[a_col + hd] + dt_bias[hd]));
+    }
+}
+
+// The same for many tokens and four taps, PREPARE_TOKENS neighbouring tokens per CTA and four neighbouring channels per thread:
+// an input row is loaded once for the four tokens that use it and the weights once for all, where a CTA per token loads
+// four rows and the weights for one (2048 tokens of 3072 channels: 49 us by token, 29 so).  q and k pass through shared
+// memory for their norms, v goes straight out.
+constexpr int PREPARE_TOKENS = 4;
+__global__ void __launch_bounds__(256, 3)
+delta_prepare_tile_kernel(const float* __restrict__ proj, int row_stride, const float* __restrict__ conv_w, const float* __restrict__ state,
+                          long long state_stride, long long keep_offset, const float* __restrict__ a_log, const float* __restrict__ dt_bias,
+                          const int* __restrict__ token_req, const int* __restrict__ req_slot, const int* __restrict__ q_start,
+                          float* __restrict__ qkv, float* __restrict__ beta, float* __restrict__ decay, int heads, int kvh, int dk, int dv,
+                          float norm_eps, int tokens) {
+    extern __shared__ __align__(16) float act[];          // [PREPARE_TOKENS][q and k channels]
+    __shared__ int local[PREPARE_TOKENS], slot[PREPARE_TOKENS];
+    pdl_trigger();
+    const int t0 = blockIdx.x * PREPARE_TOKENS, count = min(PREPARE_TOKENS, tokens - t0);
+    if ((int)threadIdx.x < count) {
+        const int req = token_req[t0 + threadIdx.x];
+        local[threadIdx.x] = t0 + threadIdx.x - q_start[req];       // index of the token inside its portion
+        slot[threadIdx.x] = req_slot[req];
+    }
+    pdl_wait();
+    __syncthreads();
+    const int nqk = 2 * kvh * dk, channels = nqk + heads * dv;
+    for (int c = 4 * threadIdx.x; c < channels; c += 4 * blockDim.x) {
+        float4 w[4], x[PREPARE_TOKENS + 3];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) w[e] = *reinterpret_cast<const float4*>(conv_w + (size_t)(c + e) * 4);
+#pragma unroll
+        for (int i = 0; i < PREPARE_TOKENS + 3; ++i) {
+            const int row = t0 - 3 + i;
+            x[i] = row >= 0 && i < count + 3 ? *reinterpret_cast<const float4*>(proj + (size_t)row * row_stride + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+#pragma unroll
+        for (int i = 0; i < PREPARE_TOKENS; ++i) {
+            if (i >= count) break;
+            float4 in[4] = {x[i], x[i + 1], x[i + 2], x[i + 3]};
+            if (local[i] < 3) {                           // inputs before the portion: the request's kept ones [3][channels], oldest first
+                const float* keep = state + (size_t)slot[i] * state_stride + keep_offset + c;
+#pragma unroll
+                for (int j = 0; j < 3; ++j)
+                    if (local[i] < 3 - j) {
+                        const float* old = keep + (size_t)(j + local[i]) * channels;
+                        in[j] = make_float4(old[0], old[1], old[2], old[3]);
+                    }
+            }
+            float4 r;
+            const auto channel = [&](const float4& wc, float a, float b, float d, float e) {
+                return silu(fmaf(wc.w, e, fmaf(wc.z, d, fmaf(wc.y, b, fmaf(wc.x, a, 0.f)))));
+            };
+            r.x = channel(w[0], in[0].x, in[1].x, in[2].x, in[3].x);
+            r.y = channel(w[1], in[0].y, in[1].y, in[2].y, in[3].y);
+            r.z = channel(w[2], in[0].z, in[1].z, in[2].z, in[3].z);
+            r.w = channel(w[3], in[0].w, in[1].w, in[2].w, in[3].w);
+            if (c < nqk) *reinterpret_cast<float4*>(act + i * nqk + c) = r;
+            else *reinterpret_cast<float4*>(qkv + (size_t)(t0 + i) * channels + c) = r;
+        }
+    }
+    __syncthreads();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, n_warps = blockDim.x >> 5;
+    for (int pair = warp; pair < count * 2 * kvh; pair += n_warps) {      // q heads, then k heads, of each token
+        const int i = pair / (2 * kvh), head = pair - i * 2 * kvh;
+        const float* x = act + i * nqk + head * dk;
+        float sq = 0.f;
+        for (int d = lane; d < dk; d += 32) sq += x[d] * x[d];
+        sq = warp_sum(sq);
+        const float inv = (1.f / sqrtf(sq + norm_eps)) * (head < kvh ? 1.f / sqrtf((float)dk) : 1.f);
+        float* dst = qkv + (size_t)(t0 + i) * channels + head * dk;
+        for (int d = lane; d < dk; d += 32) dst[d] = x[d] * inv;
+    }
+    const int b_col = channels + heads * dv, a_col = b_col + heads;
+    for (int e = threadIdx.x; e < count * heads; e += blockDim.x) {
+        const int i = e / heads, hd = e - i * heads;
+        const float* row = proj + (size_t)(t0 + i) * row_stride;
+        beta[(size_t)(t0 + i) * heads + hd] = 1.f / (1.f + expf(-row[b_col + hd]));
+        decay[(size_t)(t0 + i) * heads + hd] = expf(-expf(a_log[hd]) * softplus(row[a_col + hd] + dt_bias[hd]));
     }
 }
 
@@ -487,6 +565,437 @@ delta_chunk_walk_kernel(const float* __restrict__ qkv, const float* __restrict__
     }
 }
 
+// ------------------------------------------------------------------ heads of up to 64 x 64: one small product per chunk in order
+// With T, P, c as above, Ub = T diag(beta) V and W = T diag(beta c) K need no state either, and
+//     U = Ub - W S0,   O = (diag(c) Q - P W) S0 + P Ub,   S_C = c_C S0 - (Kd^T W) S0 + Kd^T Ub,   Kd = diag(c_C / c) K.
+// So everything but one product of 64 x 64 with the state per chunk is made for every chunk of the step at once:
+//   delta_chunk_forms   a CTA per (chunk, head): N = Kd^T W (as split parts), G = Kd^T Ub, R = diag(c) Q - P W and c_C into the
+//                       scratch, P Ub into the output.  Eight products of 64 x 64 x 64, float through the tensor cores (split_mma.cuh),
+//                       and T by blocks: four blocks of 16 in one step, then 32 and 64 by products
+//   delta_chunk_states  a CTA per (request, head, 16 value columns): S <- c_C S - N S + G chunk by chunk, the product on the
+//                       tensor cores with S in the registers of its result; G's place receives the state before its chunk
+//   delta_chunk_reads   a CTA per (chunk, head): out += R S0
+// The walk over a chunk's own products in order took 256 us for 2048 tokens of 32 heads, and the tables before it 120, most
+// of it the inversion row by row; these three take 110, 41 and 26 us. Error of outputs and
+// states against 64 bits 1.0e-7 to 1.6e-7, where the walk has 1.7e-7 to 8.8e-7.
+constexpr int FORM_THREADS = 256;
+constexpr int FORM_G = 3 * CHUNK * CHUNK / 2, FORM_R = FORM_G + CHUNK * CHUNK, FORM_C = FORM_R + CHUNK * CHUNK;
+constexpr int FORM_FLOATS = FORM_C + 4;                    // of scratch per (chunk, head): N [3][64][64] bfloat16, G (later S0), R, c_C
+constexpr int AF_LD = CHUNK + 4;                           // row stride of A and T as floats
+constexpr size_t FORMS_SMEM = 4 * sizeof(SplitTile);
+
+// four neighbouring floats of every sixteenth row: asked for together, put as split parts with a factor per row
+struct FormTile { float4 v[4]; };
+template <bool VEC>
+__device__ __forceinline__ void fetch_form(FormTile& raw, const float* __restrict__ src, size_t stride, int nr, int nc) {
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        const int i = threadIdx.x + u * FORM_THREADS, r = i >> 4, c = (i & 15) * 4;
+        const float* p = src + (size_t)r * stride + c;
+        if (VEC) raw.v[u] = (r < nr && c < nc) ? *reinterpret_cast<const float4*>(p) : make_float4(0.f, 0.f, 0.f, 0.f);
+        else {
+            raw.v[u].x = (r < nr && c < nc) ? p[0] : 0.f; raw.v[u].y = (r < nr && c + 1 < nc) ? p[1] : 0.f;
+            raw.v[u].z = (r < nr && c + 2 < nc) ? p[2] : 0.f; raw.v[u].w = (r < nr && c + 3 < nc) ? p[3] : 0.f;
+        }
+    }
+}
+template <typename W>
+__device__ __forceinline__ void put_form(SplitTile& dst, const FormTile& raw, W weight) {
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        const int i = threadIdx.x + u * FORM_THREADS, r = i >> 4, c = (i & 15) * 4;
+        const float w = weight(r);
+        split_store4(dst, r, c, make_float4(raw.v[u].x * w, raw.v[u].y * w, raw.v[u].z * w, raw.v[u].w * w));
+    }
+}
+__device__ __forceinline__ void split_store2(SplitTile& t, int row, int col, float x, float y) {       // col even
+    uint32_t p[3];
+    split_pair(x, y, p);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) *reinterpret_cast<uint32_t*>(&t.part[i][row][col]) = p[i];
+}
+// a warp's 16 x 32 part of a result, pairs (row, col, col + 1)
+template <typename F>
+__device__ __forceinline__ void for_pairs(const float (&acc)[4][4], int m0, int n0, F put) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int half = 0; half < 2; ++half)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) put(m0 + 8 * half + (lane >> 2), n0 + 8 * j + 2 * (lane & 3), acc[j][2 * half], acc[j][2 * half + 1]);
+}
+
+// T = (I + A)^-1 for the strictly lower triangle A [64][AF_LD] (its upper triangle is scratch): the diagonal blocks of 16 by
+// substitution, a column per lane; then twice the block below the diagonal, -T22 (A21 T11), from blocks of half the size.
+__device__ __forceinline__ void invert_unit_lower(float* __restrict__ A, float* __restrict__ T) {
+    const int tid = threadIdx.x;
+    for (int i = tid; i < CHUNK * CHUNK; i += FORM_THREADS) {
+        const int r = i >> 6, c = i & 63;
+        if ((c >> 4) > (r >> 4)) T[r * AF_LD + c] = 0.f;
+    }
+    if (tid < 64) {
+        const int b = (tid >> 4) * 16, c = tid & 15;
+        float x[16];
+#pragma unroll
+        for (int t = 0; t < 16; ++t) {
+            float v = t == c ? 1.f : 0.f;
+#pragma unroll
+            for (int i = 0; i < t; ++i) v = fmaf(-A[(b + t) * AF_LD + b + i], x[i], v);
+            x[t] = v;                                       // zero above the diagonal: every term before it is
+            T[(b + t) * AF_LD + b + c] = v;
+        }
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int half = 16; half < CHUNK; half *= 2) {
+        // pairs of blocks at 2 half p; runs of four columns: r inside the block below, c inside the block beside
+        const int runs = half / 4, per_pair = half * runs, total = per_pair * (CHUNK / (2 * half));
+        for (int i = tid; i < total; i += FORM_THREADS) {
+            const int p = i / per_pair, e = i - p * per_pair, r = e / runs, c = 4 * (e - r * runs), base = 2 * half * p;
+            float4 y = make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int k = 0; k < half; ++k) {
+                const float a = A[(base + half + r) * AF_LD + base + k];
+                const float4 t = *reinterpret_cast<const float4*>(T + (base + k) * AF_LD + base + c);
+                y.x = fmaf(a, t.x, y.x); y.y = fmaf(a, t.y, y.y); y.z = fmaf(a, t.z, y.z); y.w = fmaf(a, t.w, y.w);
+            }
+            *reinterpret_cast<float4*>(A + (base + r) * AF_LD + base + half + c) = y;      // the block above the diagonal is free
+        }
+        __syncthreads();
+        for (int i = tid; i < total; i += FORM_THREADS) {
+            const int p = i / per_pair, e = i - p * per_pair, r = e / runs, c = 4 * (e - r * runs), base = 2 * half * p;
+            float4 y = make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int k = 0; k < half; ++k) {
+                const float a = -T[(base + half + r) * AF_LD + base + half + k];
+                const float4 t = *reinterpret_cast<const float4*>(A + (base + k) * AF_LD + base + half + c);
+                y.x = fmaf(a, t.x, y.x); y.y = fmaf(a, t.y, y.y); y.z = fmaf(a, t.z, y.z); y.w = fmaf(a, t.w, y.w);
+            }
+            *reinterpret_cast<float4*>(T + (base + half + r) * AF_LD + base + c) = y;
+        }
+        __syncthreads();
+    }
+}
+
+template <bool VEC>
+__global__ void __launch_bounds__(FORM_THREADS, 2)
+delta_chunk_forms_kernel(const float* __restrict__ qkv, const float* __restrict__ beta, const float* __restrict__ decay,
+                         const int* __restrict__ chunk_req, const int* __restrict__ chunk_t0, const int* __restrict__ q_start,
+                         const int* __restrict__ q_len, float* __restrict__ scratch, float* __restrict__ out, int heads, int kvh, int dk, int dv) {
+    extern __shared__ __align__(16) unsigned char form_smem[];
+    __shared__ double L[CHUNK];
+    __shared__ float bt[CHUNK], ct[CHUNK];
+    SplitTile* tile = reinterpret_cast<SplitTile*>(form_smem);
+    float* Af = reinterpret_cast<float*>(tile + 2);        // [64][AF_LD] in the third tile's place, T in the fourth's
+    float* Tf = reinterpret_cast<float*>(tile + 3);
+    static_assert(CHUNK * AF_LD * sizeof(float) <= sizeof(SplitTile), "");
+    pdl_trigger();
+    const int chunk = blockIdx.x, head = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, m0 = 16 * (warp >> 1), n0 = 32 * (warp & 1);
+    const int req = chunk_req[chunk], t0 = chunk_t0[chunk], count = min(CHUNK, q_len[req] - t0), first = q_start[req] + t0;
+    const int g = head / (heads / kvh), channels = 2 * kvh * dk + heads * dv;
+    const float* q = qkv + (size_t)first * channels + g * dk;
+    const float* k = q + kvh * dk;
+    const float* v = qkv + (size_t)first * channels + 2 * kvh * dk + head * dv;
+    pdl_wait();
+    FormTile kq, raw;
+    fetch_form<VEC>(raw, q, channels, count, dk);
+    fetch_form<VEC>(kq, k, channels, count, dk);
+    if (tid < 32) {                                        // sums of the logarithms of the decays, in double; none beyond the portion
+        const int t = 2 * tid;
+        const double x = t < count ? (double)fmaxf(logf(decay[(size_t)(first + t) * heads + head]), -80.f) : 0.0;
+        const double y = t + 1 < count ? (double)fmaxf(logf(decay[(size_t)(first + t + 1) * heads + head]), -80.f) : 0.0;
+        double sum = x + y;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const double before = __shfl_up_sync(0xffffffffu, sum, off);
+            if (tid >= off) sum += before;
+        }
+        L[t + 1] = sum;
+        L[t] = sum - y;
+        ct[t] = expf((float)(sum - y));
+        ct[t + 1] = expf((float)sum);
+    } else if (tid >= 64 && tid < 128) {
+        bt[tid - 64] = tid - 64 < count ? beta[(size_t)(first + tid - 64) * heads + head] : 0.f;
+    }
+    put_form(tile[1], raw, [](int) { return 1.f; });
+    put_form(tile[0], kq, [](int) { return 1.f; });
+    __syncthreads();
+    const int k_steps = (dk + 15) >> 4;
+    {
+        float kk[4][4] = {}, qk[4][4] = {};
+        if (n0 <= m0 + 15) {
+            split_product<false, false>(kk, tile[0], tile[0], m0, n0, k_steps);
+            split_product<false, false>(qk, tile[1], tile[0], m0, n0, k_steps);
+        }
+        fetch_form<VEC>(raw, v, channels, count, dv);      // wanted after the inversion
+        __syncthreads();                                   // Q has been read: P takes its place
+        for_pairs(kk, m0, n0, [&](int t, int i, float x, float y) {
+            const float r0 = i < t ? expf((float)(L[t] - L[i])) : 0.f, r1 = i + 1 < t ? expf((float)(L[t] - L[i + 1])) : 0.f;
+            *reinterpret_cast<float2*>(Af + t * AF_LD + i) = make_float2(bt[t] * r0 * x, bt[t] * r1 * y);
+        });
+        for_pairs(qk, m0, n0, [&](int t, int i, float x, float y) {
+            split_store2(tile[1], t, i, i <= t ? expf((float)(L[t] - L[i])) * x : 0.f, i + 1 <= t ? expf((float)(L[t] - L[i + 1])) * y : 0.f);
+        });
+    }
+    __syncthreads();
+    invert_unit_lower(Af, Tf);
+    {
+        float4 t4[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int i = tid + u * FORM_THREADS;
+            t4[u] = *reinterpret_cast<const float4*>(Tf + (i >> 4) * AF_LD + (i & 15) * 4);
+        }
+        __syncthreads();                                   // T has been read: its parts take its place
+#pragma unroll
+        for (int u = 0; u < 4; ++u) { const int i = tid + u * FORM_THREADS; split_store4(tile[3], i >> 4, (i & 15) * 4, t4[u]); }
+    }
+    put_form(tile[2], raw, [&](int t) { return bt[t]; });
+    put_form(tile[0], kq, [&](int t) { return bt[t] * ct[t]; });
+    __syncthreads();
+    {
+        float ub[4][4] = {}, w[4][4] = {};
+        split_product<false, true>(ub, tile[3], tile[2], m0, n0, m0 / 16 + 1);      // T holds nothing right of the diagonal
+        split_product<false, true>(w, tile[3], tile[0], m0, n0, m0 / 16 + 1);
+        __syncthreads();
+        for_pairs(ub, m0, n0, [&](int t, int c, float x, float y) { split_store2(tile[2], t, c, x, y); });
+        for_pairs(w, m0, n0, [&](int t, int c, float x, float y) { split_store2(tile[3], t, c, x, y); });
+    }
+    put_form(tile[0], kq, [&](int t) { return expf((float)(L[CHUNK - 1] - L[t])); });
+    __syncthreads();
+    float* forms = scratch + ((size_t)chunk * heads + head) * FORM_FLOATS;
+    float* G = forms + FORM_G;
+    float* R = forms + FORM_R;
+    if (tid == 0) forms[FORM_C] = ct[CHUNK - 1];
+    const int t_steps = (count + 15) >> 4;
+    {
+        float acc[4][4] = {};
+        split_product<true, true>(acc, tile[0], tile[3], m0, n0, t_steps);
+        for_pairs(acc, m0, n0, [&](int r, int c, float x, float y) {
+            uint32_t p[3];
+            split_pair(x, y, p);
+#pragma unroll
+            for (int i = 0; i < 3; ++i) reinterpret_cast<uint32_t*>(forms)[(i * CHUNK * CHUNK + r * CHUNK + c) >> 1] = p[i];
+        });
+    }
+    {
+        float acc[4][4] = {};
+        split_product<true, true>(acc, tile[0], tile[2], m0, n0, t_steps);
+        for_pairs(acc, m0, n0, [&](int r, int c, float x, float y) { *reinterpret_cast<float2*>(G + r * CHUNK + c) = make_float2(x, y); });
+    }
+    {
+        float acc[4][4] = {};
+        split_product<false, true>(acc, tile[1], tile[3], m0, n0, m0 / 16 + 1);
+        for_pairs(acc, m0, n0, [&](int t, int d, float x, float y) {
+            const float q0 = t < count && d < dk ? q[(size_t)t * channels + d] : 0.f, q1 = t < count && d + 1 < dk ? q[(size_t)t * channels + d + 1] : 0.f;
+            *reinterpret_cast<float2*>(R + t * CHUNK + d) = make_float2(fmaf(ct[t], q0, -x), fmaf(ct[t], q1, -y));
+        });
+    }
+    {
+        float acc[4][4] = {};
+        split_product<false, true>(acc, tile[1], tile[2], m0, n0, m0 / 16 + 1);
+        for_pairs(acc, m0, n0, [&](int t, int c, float x, float y) {
+            if (t >= count) return;
+            float* dst = out + ((size_t)(first + t) * heads + head) * dv + c;
+            if (VEC) { if (c < dv) *reinterpret_cast<float2*>(dst) = make_float2(x, y); }
+            else { if (c < dv) dst[0] = x; if (c + 1 < dv) dst[1] = y; }
+        });
+    }
+}
+
+constexpr int STATE_COLS = 16, STATE_STAGES = 3, STATE_THREADS = 128;
+constexpr int STATE_LD = 24;                               // row stride of S's parts: 48 bytes, eight rows in different banks
+struct StateParts { __nv_bfloat16 part[3][CHUNK][STATE_LD]; };
+struct StateStage { SplitTile n; float g[CHUNK][STATE_COLS]; };
+constexpr size_t STATES_SMEM = STATE_STAGES * sizeof(StateStage) + 2 * sizeof(StateParts);
+
+__global__ void __launch_bounds__(STATE_THREADS)
+delta_chunk_states_kernel(float* __restrict__ scratch, const int* __restrict__ req_chunk0, float* __restrict__ state, long long state_stride,
+                          const int* __restrict__ req_slot, const int* __restrict__ q_len, int heads, int dk, int dv, int least) {
+    extern __shared__ __align__(16) unsigned char form_smem[];
+    StateStage* stage = reinterpret_cast<StateStage*>(form_smem);
+    StateParts* parts = reinterpret_cast<StateParts*>(stage + STATE_STAGES);      // [2]
+    pdl_trigger();
+    const int req = blockIdx.x, head = blockIdx.y, col0 = blockIdx.z * STATE_COLS, tid = threadIdx.x, lane = tid & 31, m0 = 16 * (tid >> 5);
+    const int row = m0 + (lane >> 2), col = 2 * (lane & 3);      // this thread has rows row, row + 8 and columns col, col + 1, col + 8, col + 9
+    const int n = q_len[req], n_chunks = (n + CHUNK - 1) / CHUNK;
+    float* S = state + (size_t)req_slot[req] * state_stride + (size_t)head * dk * dv;
+    pdl_wait();
+    if (n < least) return;
+    float* forms = scratch + ((size_t)req_chunk0[req] * heads + head) * FORM_FLOATS;
+    const size_t step = (size_t)heads * FORM_FLOATS;
+    auto fetch = [&](int chunk) {                          // N and G of a chunk into their stage; an empty group beyond the last
+        if (chunk < n_chunks) {
+            StateStage& to = stage[chunk % STATE_STAGES];
+            const float* from = forms + chunk * step;
+#pragma unroll
+            for (int u = 0; u < 3 * CHUNK * 8 / STATE_THREADS; ++u) {
+                const int i = tid + u * STATE_THREADS, r = (i >> 3) & 63, k = (i & 7) * 8;
+                copy16(reinterpret_cast<float*>(&to.n.part[i >> 9][r][k]), from + (i >> 9) * (CHUNK * CHUNK / 2) + ((r * CHUNK + k) >> 1));
+            }
+#pragma unroll
+            for (int u = 0; u < CHUNK * 4 / STATE_THREADS; ++u) {
+                const int i = tid + u * STATE_THREADS, r = i >> 2, c = 4 * (i & 3);
+                copy16(&to.g[r][c], from + FORM_G + r * CHUNK + col0 + c);
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+#pragma unroll
+    for (int s = 0; s < STATE_STAGES - 1; ++s) fetch(s);
+    float now[2][4];                                       // as a result of the tensor core has it: [columns 8 j ..][row, row + 8]
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int r = row + 8 * (e >> 1), c = col0 + 8 * j + col + (e & 1);
+            now[j][e] = r < dk && c < dv ? S[(size_t)r * dv + c] : 0.f;
+        }
+    const int l7 = lane & 7, lo = (lane >> 3) & 1, hi = lane >> 4;
+    float keep = n_chunks > 0 ? forms[FORM_C] : 0.f;
+    for (int chunk = 0; chunk < n_chunks; ++chunk) {
+        StateParts& Sp = parts[chunk & 1];
+        const StateStage& at = stage[chunk % STATE_STAGES];
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                uint32_t p[3];
+                split_pair(now[j][2 * half], now[j][2 * half + 1], p);
+#pragma unroll
+                for (int i = 0; i < 3; ++i) *reinterpret_cast<uint32_t*>(&Sp.part[i][row + 8 * half][8 * j + col]) = p[i];
+            }
+        asm volatile("cp.async.wait_group %0;" ::"n"(STATE_STAGES - 2) : "memory");
+        __syncthreads();                                   // S is whole, N and G have landed, and the stage before this one is free
+        fetch(chunk + STATE_STAGES - 1);
+        const float f = keep;
+        if (chunk + 1 < n_chunks) keep = forms[(chunk + 1) * step + FORM_C];
+        float sum[2][4];
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                const int r = row + 8 * half, c = 8 * j + col;
+                const float2 g = *reinterpret_cast<const float2*>(&at.g[r][c]);
+                *reinterpret_cast<float2*>(forms + chunk * step + FORM_G + r * CHUNK + col0 + c) = make_float2(now[j][2 * half], now[j][2 * half + 1]);
+                sum[j][2 * half] = g.x; sum[j][2 * half + 1] = g.y;
+            }
+#pragma unroll
+        for (int k = 0; k < CHUNK; k += 16) {
+            uint32_t a[3][4], b[3][4];
+#pragma unroll
+            for (int p = 0; p < 3; ++p) {
+                load_matrices<false>(a[p], &at.n.part[p][m0 + l7 + 8 * lo][k + 8 * hi]);
+                load_matrices<true>(b[p], &Sp.part[p][k + l7 + 8 * lo][8 * hi]);
+            }
+            constexpr int PA[6] = {2, 0, 1, 1, 0, 0}, PB[6] = {0, 2, 1, 0, 1, 0};       // as split_product sums
+            float t[2][4] = {};
+#pragma unroll
+            for (int q = 0; q < 6; ++q)
+#pragma unroll
+                for (int j = 0; j < 2; ++j) mma_bf16(t[j], a[PA[q]], b[PB[q]][2 * j], b[PB[q]][2 * j + 1]);
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) sum[j][e] -= t[j][e];
+        }
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) now[j][e] = fmaf(f, now[j][e], sum[j][e]);
+    }
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int r = row + 8 * (e >> 1), c = col0 + 8 * j + col + (e & 1);
+            if (r < dk && c < dv) S[(size_t)r * dv + c] = now[j][e];
+        }
+}
+
+template <bool VEC>
+__global__ void __launch_bounds__(FORM_THREADS, 3)
+delta_chunk_reads_kernel(const float* __restrict__ scratch, const int* __restrict__ chunk_req, const int* __restrict__ chunk_t0,
+                         const int* __restrict__ q_start, const int* __restrict__ q_len, float* __restrict__ out, int heads, int dk, int dv) {
+    extern __shared__ __align__(16) unsigned char form_smem[];
+    SplitTile* tile = reinterpret_cast<SplitTile*>(form_smem);
+    pdl_trigger();
+    const int chunk = blockIdx.x, head = blockIdx.y, warp = threadIdx.x >> 5, m0 = 16 * (warp >> 1), n0 = 32 * (warp & 1);
+    const int req = chunk_req[chunk], t0 = chunk_t0[chunk], count = min(CHUNK, q_len[req] - t0), first = q_start[req] + t0;
+    const float* S0 = scratch + ((size_t)chunk * heads + head) * FORM_FLOATS + FORM_G;
+    pdl_wait();
+    FormTile s, r;
+    fetch_form<true>(s, S0, CHUNK, CHUNK, CHUNK);
+    fetch_form<true>(r, S0 + CHUNK * CHUNK, CHUNK, CHUNK, CHUNK);
+    put_form(tile[0], r, [](int) { return 1.f; });
+    put_form(tile[1], s, [](int) { return 1.f; });
+    __syncthreads();
+    float acc[4][4] = {};
+    split_product<false, true>(acc, tile[0], tile[1], m0, n0, (dk + 15) >> 4);
+    for_pairs(acc, m0, n0, [&](int t, int c, float x, float y) {
+        if (t >= count) return;
+        float* dst = out + ((size_t)(first + t) * heads + head) * dv + c;
+        if (VEC) {
+            if (c < dv) { const float2 o = *reinterpret_cast<float2*>(dst); *reinterpret_cast<float2*>(dst) = make_float2(o.x + x, o.y + y); }
+        } else {
+            if (c < dv) dst[0] += x;
+            if (c + 1 < dv) dst[1] += y;
+        }
+    });
+}
+
+template <bool VEC>
+int launch_forms(const float* qkv, const float* beta, const float* decay, const int* chunk_req, const int* chunk_t0, int n_chunks,
+                 const int* req_chunk0, float* scratch, float* state, long long state_stride, const int* req_slot, const int* q_start,
+                 const int* q_len, float* out, int heads, int kvh, int dk, int dv, int n_req, int least, cudaStream_t s) {
+    static bool configured = false;
+    if (!configured) {
+        cudaError_t e = cudaFuncSetAttribute(delta_chunk_forms_kernel<VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FORMS_SMEM);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(delta_chunk_states_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)STATES_SMEM);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(delta_chunk_reads_kernel<VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(2 * sizeof(SplitTile)));
+        if (e != cudaSuccess) return (int)e;
+        configured = true;
+    }
+    int st = launch_kernel(delta_chunk_forms_kernel<VEC>, dim3(n_chunks, heads), dim3(FORM_THREADS), FORMS_SMEM, s, g_pdl, qkv, beta, decay, chunk_req,
+                           chunk_t0, q_start, q_len, scratch, out, heads, kvh, dk, dv);
+    if (st) return st;
+    st = launch_kernel(delta_chunk_states_kernel, dim3(n_req, heads, (dv + STATE_COLS - 1) / STATE_COLS), dim3(STATE_THREADS), STATES_SMEM, s, g_pdl, scratch,
+                       req_chunk0, state, state_stride, req_slot, q_len, heads, dk, dv, least);
+    if (st) return st;
+    return launch_kernel(delta_chunk_reads_kernel<VEC>, dim3(n_chunks, heads), dim3(FORM_THREADS), 2 * sizeof(SplitTile), s, g_pdl, (const float*)scratch,
+                         chunk_req, chunk_t0, q_start, q_len, out, heads, dk, dv);
+}
+
+// The same where a head's values come in runs of four: LANES lanes share a (token, head), each with its runs, so a warp has
+// several of them under way (2048 tokens of 32 heads of 64: 24 us with a warp and two numbers a lane each, 11 so).
+template <typename OT, int LANES>
+__global__ void __launch_bounds__(256)
+delta_output_runs_kernel(const float* __restrict__ o, const float* __restrict__ proj, int row_stride, int gate_col,
+                         const float* __restrict__ norm_w, float eps, OT* __restrict__ out, int out_stride, int heads, int dv, int tokens) {
+    pdl_trigger();
+    pdl_wait();
+    const size_t pair = ((size_t)blockIdx.x * 256 + threadIdx.x) / LANES, t = pair / heads;
+    const int head = (int)(pair - t * heads), lane = threadIdx.x % LANES;
+    const bool live = t < (size_t)tokens && 4 * lane < dv;
+    float4 x = make_float4(0.f, 0.f, 0.f, 0.f), gate = x, w = x;
+    if (live) {
+        x = *reinterpret_cast<const float4*>(o + pair * dv + 4 * lane);
+        gate = *reinterpret_cast<const float4*>(proj + t * row_stride + gate_col + head * dv + 4 * lane);
+        w = *reinterpret_cast<const float4*>(norm_w + 4 * lane);
+    }
+    float sq = x.x * x.x + x.y * x.y + x.z * x.z + x.w * x.w;
+#pragma unroll
+    for (int off = LANES / 2; off; off >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, off);
+    if (!live) return;
+    const float inv = 1.f / sqrtf(sq / (float)dv + eps);
+    OT* dst = out + t * out_stride + head * dv + 4 * lane;
+    const float r[4] = {x.x * inv * w.x * silu(gate.x), x.y * inv * w.y * silu(gate.y), x.z * inv * w.z * silu(gate.z), x.w * inv * w.w * silu(gate.w)};
+    if (sizeof(OT) == 2) {
+        uint2 p;
+        p.x = bf16_pair(r[0], r[1]); p.y = bf16_pair(r[2], r[3]);
+        *reinterpret_cast<uint2*>(dst) = p;
+    } else {
+        *reinterpret_cast<float4*>(dst) = make_float4(r[0], r[1], r[2], r[3]);
+    }
+}
+
 template <typename OT>
 __global__ void __launch_bounds__(128)
 delta_output_kernel(const float* __restrict__ o, const float* __restrict__ proj, int row_stride, int gate_col,
@@ -507,6 +1016,21 @@ delta_output_kernel(const float* __restrict__ o, const float* __restrict__ proj,
     OT* dst = out + t * out_stride + head * dv;
     for (int d = lane; d < dv; d += 32) dst[d] = from_float<OT>(src[d] * inv * norm_w[d] * silu(gate[d]));
 }
+
+template <typename OT>
+int launch_output(const float* o, const float* proj, int row_stride, int gate_col, const float* norm_w, float eps, OT* out, int out_stride, int heads,
+                  int dv, int tokens, cudaStream_t s) {
+    const size_t pairs = (size_t)tokens * heads;
+    if (dv <= 128 && dv % 4 == 0 && row_stride % 4 == 0 && gate_col % 4 == 0 && out_stride % 4 == 0 &&
+        !(((uintptr_t)o | (uintptr_t)proj | (uintptr_t)norm_w | (uintptr_t)out) & 15)) {
+#define DELTA_OUTPUT_RUNS(LANES) launch_kernel(delta_output_runs_kernel<OT, LANES>, dim3((unsigned)((pairs * LANES + 255) / 256)), dim3(256), 0, s, g_pdl, o, proj, \
+                                               row_stride, gate_col, norm_w, eps, out, out_stride, heads, dv, tokens)
+        return dv <= 32 ? DELTA_OUTPUT_RUNS(8) : dv <= 64 ? DELTA_OUTPUT_RUNS(16) : DELTA_OUTPUT_RUNS(32);
+#undef DELTA_OUTPUT_RUNS
+    }
+    return launch_kernel(delta_output_kernel<OT>, dim3((unsigned)((pairs + 3) / 4)), dim3(128), 0, s, g_pdl, o, proj, row_stride, gate_col, norm_w, eps, out,
+                         out_stride, heads, dv, tokens);
+}
 }  // namespace
 
 CISR_EXPORT int cisr_delta_prepare(const float* proj, int row_stride, const float* conv_w, int taps, const float* state,
@@ -525,6 +1049,12 @@ CISR_EXPORT int cisr_delta_prepare(const float* proj, int row_stride, const floa
         if (e != cudaSuccess) return (int)e;
         configured = smem;
     }
+    const int nqk = 2 * kvh * dk;
+    if (tokens > 64 && taps == 4 && channels % 4 == 0 && nqk % 4 == 0 && row_stride % 4 == 0 && sizeof(float) * PREPARE_TOKENS * nqk <= 48 * 1024 &&
+        !(((uintptr_t)proj | (uintptr_t)conv_w | (uintptr_t)qkv) & 15))
+        return launch_kernel(delta_prepare_tile_kernel, dim3((tokens + PREPARE_TOKENS - 1) / PREPARE_TOKENS), dim3(256), sizeof(float) * PREPARE_TOKENS * nqk,
+                             (cudaStream_t)stream, g_pdl, proj, row_stride, conv_w, state, state_stride, keep_offset, a_log, dt_bias, token_req,
+                             req_slot, q_start, qkv, beta, decay, heads, kvh, dk, dv, norm_eps, tokens);
     const int threads = (tokens <= 64 && channels >= 1024) ? 1024 : 256;      // few tokens (a decode step): a token's channels on more threads
     return launch_kernel(delta_prepare_kernel, dim3(tokens), dim3(threads), smem, (cudaStream_t)stream, g_pdl, proj, row_stride, conv_w, taps,
                          state, state_stride, keep_offset, a_log, dt_bias, token_req, req_slot, q_start, qkv, beta, decay, heads, kvh,
@@ -602,7 +1132,7 @@ CISR_EXPORT int cisr_delta_recurrence(const float* qkv, const float* beta, const
 }
 
 CISR_EXPORT int cisr_delta_chunk_tokens() { return CHUNK; }
-CISR_EXPORT long long cisr_delta_chunk_table_floats() { return 2 * CHUNK * CHUNK + CHUNK; }
+CISR_EXPORT long long cisr_delta_chunk_table_floats() { return FORM_FLOATS; }        // enough for either form's scratch
 
 // The recurrence for the requests of the step that bring at least `least` tokens, chunk by chunk.  chunk_req / chunk_t0:
 // per chunk its request and first token inside the portion; req_chunk0: per request the index of its first chunk (requests
@@ -614,6 +1144,12 @@ CISR_EXPORT int cisr_delta_chunks(const float* qkv, const float* beta, const flo
     if (n_chunks <= 0 || n_req <= 0) return 0;
     if (dk <= 0 || dk > 256 || dv <= 0 || heads % kvh || least < 1) return -2;
     cudaStream_t s = (cudaStream_t)stream;
+    // Heads of up to 64 x 64 fit the tiles of the forms; wider ones walk their chunks' own products in order.
+    if (dk <= CHUNK && dv <= CHUNK && ((uintptr_t)tables & 15) == 0) {
+        const bool vec = dk % 4 == 0 && dv % 4 == 0 && (2 * kvh * dk + heads * dv) % 4 == 0 && !(((uintptr_t)qkv | (uintptr_t)out) & 15);
+        return (vec ? launch_forms<true> : launch_forms<false>)(qkv, beta, decay, chunk_req, chunk_t0, n_chunks, req_chunk0, tables, state, state_stride,
+                                                               req_slot, q_start, q_len, out, heads, kvh, dk, dv, n_req, least, s);
+    }
     const size_t smem_tables = sizeof(float) * ((size_t)2 * CHUNK * (dk + 1) + 4 * CHUNK * (CHUNK + 1) + 2 * CHUNK);
     const size_t smem_walk = sizeof(float) * ((size_t)2 * CHUNK * chunk_row_stride(dk) + 2 * CHUNK * (CHUNK + 4) + (size_t)dk * 16 +
                                               2 * CHUNK * 16 + 3 * CHUNK);        // sized for 16 columns, also where a CTA takes 8
@@ -651,12 +1187,8 @@ CISR_EXPORT int cisr_delta_chunks(const float* qkv, const float* beta, const flo
 CISR_EXPORT int cisr_delta_output(const float* o, const float* proj, int row_stride, int gate_col, const float* norm_w, float eps,
                                   void* out, int out_dtype, int out_stride, int heads, int dv, int tokens, void* stream) {
     if (tokens <= 0) return 0;
-    const size_t pairs = (size_t)tokens * heads;
-    const dim3 grid((unsigned)((pairs + 3) / 4));
     cudaStream_t s = (cudaStream_t)stream;
     if (out_dtype == CISR_BF16)
-        return launch_kernel(delta_output_kernel<__nv_bfloat16>, grid, dim3(128), 0, s, g_pdl, o, proj, row_stride, gate_col, norm_w, eps,
-                             (__nv_bfloat16*)out, out_stride, heads, dv, tokens);
-    return launch_kernel(delta_output_kernel<float>, grid, dim3(128), 0, s, g_pdl, o, proj, row_stride, gate_col, norm_w, eps,
-                         (float*)out, out_stride, heads, dv, tokens);
+        return launch_output(o, proj, row_stride, gate_col, norm_w, eps, (__nv_bfloat16*)out, out_stride, heads, dv, tokens, s);
+    return launch_output(o, proj, row_stride, gate_col, norm_w, eps, (float*)out, out_stride, heads, dv, tokens, s);
 }

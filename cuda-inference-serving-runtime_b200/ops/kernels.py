@@ -879,7 +879,7 @@ def bias_add(out: torch.Tensor, bias: torch.Tensor) -> torch.Tensor:
 _delta_state = {}
 DELTA_MAX_KEY_DIM = 256
 DELTA_CHUNK = 64                                       # tokens per chunk of the chunked recurrence
-DELTA_CHUNK_TABLE = 2 * DELTA_CHUNK * DELTA_CHUNK + DELTA_CHUNK   # floats of scratch per (chunk, head)
+DELTA_CHUNK_TABLE = 7 * DELTA_CHUNK * DELTA_CHUNK // 2 + 4       # floats of scratch per (chunk, head)
 
 
 def _delta():
@@ -918,8 +918,9 @@ def delta_keep(proj, state, req_slot, q_start, q_len, n_req, taps, channels, mat
 
 def delta_chunks(qkv, beta, decay, chunk_req, chunk_t0, n_chunks, req_chunk0, state, req_slot, q_start, q_len, o, n_req, heads, kv_heads,
                  key_dim, value_dim, least) -> None:
-    """The recurrence for the requests that bring at least `least` tokens, a chunk of DELTA_CHUNK tokens at a time: two
-    launches (the chunks' tables, all at once; then the walk from chunk to chunk).  chunk_req, chunk_t0: per chunk its
+    """The recurrence for the requests that bring at least `least` tokens, a chunk of DELTA_CHUNK tokens at a time: three
+    launches for heads of up to 64 x 64 (the chunks' forms, all at once; the states from chunk to chunk; the read-outs, all
+    at once), two for wider ones (the chunks' tables; the walk from chunk to chunk).  chunk_req, chunk_t0: per chunk its
     request and its first token inside the portion; req_chunk0: per request the index of its first chunk."""
     for name, t in (("chunk_req", chunk_req), ("chunk_t0", chunk_t0), ("req_chunk0", req_chunk0)):
         _need(t, torch.int32, name, 1)
@@ -928,7 +929,8 @@ def delta_chunks(qkv, beta, decay, chunk_req, chunk_t0, n_chunks, req_chunk0, st
     tables = torch.empty((n_chunks, heads, DELTA_CHUNK_TABLE), dtype=torch.float32, device=qkv.device)
     _check(_delta().cisr_delta_chunks(_p(qkv), _p(beta), _p(decay), _p(chunk_req), _p(chunk_t0), n_chunks, _p(req_chunk0), _p(tables),
                                       _p(state), ctypes.c_longlong(state.shape[1]), _p(req_slot), _p(q_start), _p(q_len), _p(o), heads,
-                                      kv_heads, key_dim, value_dim, n_req, int(least), _stream()), "delta_chunks", own=2)
+                                      kv_heads, key_dim, value_dim, n_req, int(least), _stream()), "delta_chunks",
+           own=3 if max(key_dim, value_dim) <= DELTA_CHUNK else 2)
 
 
 def delta_recurrence(qkv, beta, decay, state, req_slot, q_start, q_len, o, n_req, heads, kv_heads, key_dim, value_dim, lanes=0, below=0) -> None:

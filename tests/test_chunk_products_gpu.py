@@ -82,3 +82,30 @@ def test_gated_chunks(N, dv, lens, norm):
     assert error(y, torch.stack(want)) < BOUND and error(state, torch.stack(ends)) < BOUND
     if norm:
         assert error(yn, torch.stack(want_n)) < BOUND
+
+
+@pytest.mark.parametrize("dk,dv,heads,kvh,lens", [(64, 64, 4, 1, [64, 65, 200]), (48, 40, 2, 1, [127, 128]), (33, 7, 3, 3, [129]), (16, 16, 2, 2, [64]), (64, 1, 1, 1, [191])])
+def test_delta_forms(dk, dv, heads, kvh, lens):
+    from cisr_b200.ops import kernels
+    g = torch.Generator(device="cuda").manual_seed(dk + dv)
+    starts, (req, t0, first, n_chunks) = step_lists(lens)
+    T = sum(lens)
+    unit = lambda: torch.nn.functional.normalize(torch.randn(T, kvh, dk, generator=g, device="cuda"), dim=-1)
+    q, k, v = unit() * dk ** -0.5, unit(), torch.randn(T, heads, dv, generator=g, device="cuda")
+    qkv = torch.cat([x.reshape(T, -1) for x in (q, k, v)], dim=1).contiguous()
+    beta = torch.rand(T, heads, generator=g, device="cuda")
+    decay = torch.exp(-3.0 * torch.rand(T, heads, generator=g, device="cuda") ** 6)
+    state = torch.randn(len(lens), heads * dk * dv, generator=g, device="cuda")
+    Q, K = (x.double().repeat_interleave(heads // kvh, 1) for x in (q, k))
+    want, ends = [], []
+    for r, n in enumerate(lens):
+        S = state[r].double().view(heads, dk, dv).clone()
+        for t in range(starts[r], starts[r] + n):
+            S = decay[t].double()[:, None, None] * S
+            u = beta[t].double()[:, None] * (v[t].double() - torch.einsum("hkv,hk->hv", S, K[t]))
+            S = S + K[t][:, :, None] * u[:, None]
+            want.append(torch.einsum("hkv,hk->hv", S, Q[t]))
+        ends.append(S.reshape(-1))
+    o = torch.full((T, heads, dv), float("nan"), device="cuda")
+    kernels.delta_chunks(qkv, beta, decay, req, t0, n_chunks, first, state, i32(range(len(lens))), i32(starts), i32(lens), o, len(lens), heads, kvh, dk, dv, 64)
+    assert error(o, torch.stack(want)) < BOUND and error(state, torch.stack(ends)) < BOUND
