@@ -1609,12 +1609,13 @@ def moe_sort(chosen: torch.Tensor, experts: int, row_of: torch.Tensor, src_token
            "moe_sort")
 
 
-def moe_gather(h: torch.Tensor, src_token: torch.Tensor, sorted_h: torch.Tensor) -> torch.Tensor:
-    """sorted_h[row] = h[src_token[row]], zeros where src_token[row] < 0 (bfloat16 rows of 16-byte multiples)."""
+def moe_gather(h: torch.Tensor, src_token: torch.Tensor, sorted_h: torch.Tensor, fill: bool = True) -> torch.Tensor:
+    """sorted_h[row] = h[src_token[row]] (bfloat16 rows of 16-byte multiples); where src_token[row] < 0 zeros, or with
+    `fill` False whatever the row holds."""
     _need(h, torch.bfloat16, "h", 2); _need(sorted_h, torch.bfloat16, "sorted_h", 2); _need(src_token, torch.int32, "src_token", 1)
     if sorted_h.shape != (src_token.numel(), h.shape[1]):
         raise KernelError("moe_gather: shapes disagree")
-    _check(_moe().cisr_moe_gather(_p(h), _p(src_token), _p(sorted_h), sorted_h.shape[0], h.shape[1], _stream()), "moe_gather")
+    _check(_moe().cisr_moe_gather(_p(h), _p(src_token), _p(sorted_h), sorted_h.shape[0], h.shape[1], int(fill), _stream()), "moe_gather")
     return sorted_h
 
 
@@ -1656,7 +1657,8 @@ def moe_grouped(h: torch.Tensor, w_up: torch.Tensor, w_down: torch.Tensor, chose
     src_token = torch.empty(rows, dtype=torch.int32, device=device)
     tile_group = torch.empty(rows // MOE_TILE, dtype=torch.int32, device=device)
     moe_sort(chosen, experts, row_of, src_token, tile_group)
-    sorted_h = moe_gather(h, src_token, torch.empty((rows, hidden), dtype=torch.bfloat16, device=device))
+    # a padding row's products are read by no one, and a row's depend on it alone: the padding is not filled
+    sorted_h = moe_gather(h, src_token, torch.empty((rows, hidden), dtype=torch.bfloat16, device=device), fill=False)
     if gate_limit is None:
         act = gemm_tcgen05_grouped(sorted_h, w_up, torch.empty((rows, ff), dtype=torch.bfloat16, device=device), tile_group, tokens * top,
                                    activation=activation)
@@ -2154,7 +2156,7 @@ _DESCRIBE = {
     "moe_select": lambda logits, *a, **kw: (int(logits.shape[0]), int(logits.shape[1])),
     "moe_rows": lambda h, w_up, w_down, chosen, *a, **kw: (int(h.shape[0]), int(w_up.shape[0]), int(w_up.shape[1]), int(w_up.shape[2]), int(chosen.shape[1])),
     "moe_sort": lambda chosen, experts, *a: (int(chosen.shape[0]), int(chosen.shape[1]), int(experts)),
-    "moe_gather": lambda h, src_token, sorted_h: (int(sorted_h.shape[0]), int(sorted_h.shape[1])),
+    "moe_gather": lambda h, src_token, sorted_h, fill=True: (int(sorted_h.shape[0]), int(sorted_h.shape[1])),
     "moe_combine": lambda sorted_out, row_of, weight, out, out_scale=None, h=None: (int(out.shape[0]), int(weight.shape[1]), int(out.shape[1])),
     "gemm_tcgen05_grouped": lambda a, w, out, tile_group, rows_in_use=None, activation="relu_squared":
         (int(rows_in_use or a.shape[0]), int(w.shape[0]), int(w.shape[1]), int(w.shape[2]), out.dtype == torch.bfloat16),
