@@ -2,7 +2,8 @@
 // operands, float accumulation in tensor memory.  Used for steps with more tokens than the weight-streaming
 // kernels take (prompt portions, large decode batches).
 //
-//   * persistent CTAs, each walking output tiles of 128 x BN (BN = 256, 128 or 64, chosen from the number of
+//   * products of one round of tiles have a kernel of their own (gemm_tcgen05_split_kernel, further down); the others
+//     go to persistent CTAs, each walking output tiles of 128 x BN (BN = 256, 192, 128 or 64, chosen from the number of
 //     tiles: see the launchers), with two accumulators of BN columns in tensor memory so that the epilogue of
 //     one tile runs under the products of the next
 //   * warp 0: one thread issues TMA loads (cp.async.bulk.tensor.2d, 128-byte swizzle) of the A tile
@@ -75,21 +76,38 @@ struct Smem {
     static constexpr size_t TOTAL = TILES + 1024 /* alignment slack */ + 256 /* barriers */;
 };
 
-// The epilogue of one output tile for one thread: `row` is the thread's output row, `lane_base` the tensor-memory
-// address of its lane in the tile's accumulator, n0 the tile's first column (feature).
+// A tile's result is taken 32 columns at a time: in units of 32 columns (PLAIN, RELU2), of 32 gate and the 32 up columns of
+// the same features (SWIGLU, GATED), or of 32 rotation pairs of a head (ROPE: columns c and c + dim / 2).
 template <int BN, int EPI>
+__device__ __forceinline__ constexpr int epilogue_units() { return EPI == EPI_PLAIN || EPI == EPI_RELU2 ? BN / 32 : BN / 64; }
+template <int BN, int EPI>
+__device__ __forceinline__ void unit_columns(const Epilogue& ep, int unit, int& lo, int& hi) {
+    lo = 32 * unit; hi = 0;
+    if (paired_rows(EPI)) hi = BN / 2 + lo;
+    if (EPI == EPI_ROPE) {
+        const int per_head = ep.dim / 64;
+        lo = (unit / per_head) * ep.dim + (unit % per_head) * 32;
+        hi = lo + ep.dim / 2;
+    }
+}
+// The epilogue of units [u0, u1) of an output tile for one thread: `row` is the thread's output row, n0 the tile's first column
+// (feature); load(column, v) gives 32 columns of the row's sums (called by whole warps).
 // `pos`, `page` (ROPE): the row's position and the cache page it is written to, looked up by the caller while the tile
 // was still being accumulated (-1: a padding row, or a row beyond the step).
-__device__ __forceinline__ void epilogue_tile(const Epilogue& ep, uint32_t lane_base, int row, int m, int n, int n0, int pos, int page) {
-    if (EPI == EPI_PLAIN) {
+template <int BN, int EPI, typename Load>
+__device__ __forceinline__ void epilogue_tile(const Epilogue& ep, Load load, int u0, int u1, int row, int m, int n, int n0, int pos, int page) {
 #pragma unroll 1
-        for (int c = 0; c < BN; c += 32) {
-            uint32_t v[32];
-            tmem_load32(lane_base + (uint32_t)c, v);
+    for (int unit = u0; unit < u1; ++unit) {
+        int lo_col, hi_col;
+        unit_columns<BN, EPI>(ep, unit, lo_col, hi_col);
+        uint32_t v[32];
+        load(lo_col, v);
+        if (EPI == EPI_PLAIN) {
             if (ep.out_mult != 0.f) {
 #pragma unroll
                 for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) * ep.out_mult);
             }
+            const int c = lo_col;
             if (row < m) {
                 float* dst = ep.out_f32 + (size_t)row * n + n0 + c;
                 if (n0 + c + 32 <= n && (n & 3) == 0) {
@@ -113,62 +131,48 @@ __device__ __forceinline__ void epilogue_tile(const Epilogue& ep, uint32_t lane_
                         if (n0 + c + j < n) dst[j] = ep.accumulate ? dst[j] + __uint_as_float(v[j]) : __uint_as_float(v[j]);
                 }
             }
-        }
-    } else if (EPI == EPI_RELU2) {
-        // out = act(product) as bfloat16 [m, n]: the activation of an expert's first product (max(z, 0)^2, or the exact gelu)
-        const bool gelu = ep.act == 1;
-#pragma unroll 1
-        for (int c = 0; c < BN; c += 32) {
-            uint32_t v[32];
-            tmem_load32(lane_base + (uint32_t)c, v);
+        } else if (EPI == EPI_RELU2) {
+            // out = act(product) as bfloat16 [m, n]: the activation of an expert's first product (max(z, 0)^2, or the exact gelu)
+            const bool gelu = ep.act == 1;
             float act[32];
 #pragma unroll
             for (int j = 0; j < 32; ++j) {
                 const float z = __uint_as_float(v[j]), r = fmaxf(z, 0.f);
                 act[j] = gelu ? 0.5f * z * (1.f + erff(z * 0.70710678118654752f)) : r * r;
             }
-            if (row < m && n0 + c < n) store_bf16x32(ep.out_bf16 + (size_t)row * n + n0 + c, act, n - (n0 + c));
-        }
-    } else if (EPI == EPI_GATED) {
-        // the clamped gated activation of an expert's stacked gate and up rows, as bfloat16 [m, inter]
-        const float limit = ep.limit, alpha = ep.alpha;
-#pragma unroll 1
-        for (int c = 0; c < BN / 2; c += 32) {
-            uint32_t g[32], u[32];
-            tmem_load32(lane_base + (uint32_t)c, g);
-            tmem_load32(lane_base + (uint32_t)(BN / 2 + c), u);
+            if (row < m && n0 + lo_col < n) store_bf16x32(ep.out_bf16 + (size_t)row * n + n0 + lo_col, act, n - (n0 + lo_col));
+        } else if (paired_rows(EPI)) {
+            // The divisions go without the ordinary one's second path (2^-22 and less, beside the 2^-9 that act is rounded to):
+            // with it the 64 quotients of a thread ran one after the other, 10 us of a launch of few rows.  Denominators above
+            // 2^126 give 0, where the quotient is at most 2^-119.
+            uint32_t u[32];
+            load(hi_col, u);
             float act[32];
+            if (EPI == EPI_GATED) {
+                // the clamped gated activation of stacked gate and up rows, as bfloat16 [m, inter]
+                const float limit = ep.limit, alpha = ep.alpha;
 #pragma unroll
-            for (int j = 0; j < 32; ++j) {
-                const float gv = fminf(__uint_as_float(g[j]), limit), uv = fminf(fmaxf(__uint_as_float(u[j]), -limit), limit);
-                act[j] = gv / (1.f + expf(-alpha * gv)) * (uv + 1.f);
-            }
-            if (row < m && n0 + c < ep.inter)
-                store_bf16x32(ep.out_bf16 + (size_t)row * ep.inter + n0 + c, act, ep.inter - (n0 + c));
-        }
-    } else if (EPI == EPI_SWIGLU) {
-        // silu(z) = z / (1 + exp(-z)) and gelu(z) = z / (1 + exp(-2 sqrt(2 / pi) (z + 0.044715 z^3))) differ in the exponent only
-        const float lin = ep.act == 1 ? 2.f * 0.7978845608028654f : 1.f, cub = ep.act == 1 ? 0.044715f : 0.f;
-#pragma unroll 1
-        for (int c = 0; c < BN / 2; c += 32) {
-            uint32_t g[32], u[32];
-            tmem_load32(lane_base + (uint32_t)c, g);
-            tmem_load32(lane_base + (uint32_t)(BN / 2 + c), u);
-            float act[32];
+                for (int j = 0; j < 32; ++j) {
+                    const float gv = fminf(__uint_as_float(v[j]), limit), uv = fminf(fmaxf(__uint_as_float(u[j]), -limit), limit);
+                    act[j] = __fdividef(gv, 1.f + expf(-alpha * gv)) * (uv + 1.f);
+                }
+            } else {
+                // silu(z) = z / (1 + exp(-z)) and gelu(z) = z / (1 + exp(-2 sqrt(2 / pi) (z + 0.044715 z^3))) differ in the exponent only
+                const float lin = ep.act == 1 ? 2.f * 0.7978845608028654f : 1.f, cub = ep.act == 1 ? 0.044715f : 0.f;
 #pragma unroll
-            for (int j = 0; j < 32; ++j) {
-                const float gv = __uint_as_float(g[j]);
-                act[j] = gv / (1.f + expf(-lin * (gv + cub * gv * gv * gv))) * __uint_as_float(u[j]);
+                for (int j = 0; j < 32; ++j) {
+                    const float gv = __uint_as_float(v[j]);
+                    act[j] = __fdividef(gv, 1.f + expf(-lin * (gv + cub * gv * gv * gv))) * __uint_as_float(u[j]);
+                }
             }
-            if (row < m && n0 + c < ep.inter)
-                store_bf16x32(ep.out_bf16 + (size_t)row * ep.inter + n0 + c, act, ep.inter - (n0 + c));
-        }
-    } else {
-        // whole heads of the stacked q, k, v projection: BN / dim heads per tile, rotation pairs (i, i + dim / 2)
-        const int dim = ep.dim, half = dim / 2;
-#pragma unroll 1
-        for (int h0 = 0; h0 < BN; h0 += dim) {
-            const int hh = (n0 + h0) / dim;                        // head index in the stacked projection
+            if (row < m && n0 + lo_col < ep.inter)
+                store_bf16x32(ep.out_bf16 + (size_t)row * ep.inter + n0 + lo_col, act, ep.inter - (n0 + lo_col));
+        } else {
+            // whole heads of the stacked q, k, v projection: BN / dim heads per tile, rotation pairs (i, i + dim / 2)
+            const int dim = ep.dim, half = dim / 2;
+            const int hh = (n0 + lo_col) / dim, c = lo_col % dim;  // head index in the stacked projection, first pair of the unit
+            uint32_t hi[32];
+            load(hi_col, hi);
             if (hh >= ep.hq + 2 * ep.hkv) break;
             const bool is_q = hh < ep.hq, is_k = !is_q && hh < ep.hq + ep.hkv;
             bf16* dst = nullptr;
@@ -180,34 +184,28 @@ __device__ __forceinline__ void epilogue_tile(const Epilogue& ep, uint32_t lane_
                           (((size_t)page * ep.hkv + kvh) * ep.page_size + pos % ep.page_size) * dim;
                 }
             }
-#pragma unroll 1
-            for (int c = 0; c < half; c += 32) {
-                uint32_t lo[32], hi[32];
-                tmem_load32(lane_base + (uint32_t)(h0 + c), lo);
-                tmem_load32(lane_base + (uint32_t)(h0 + half + c), hi);
-                float first[32], second[32];
-                if ((is_q || is_k) && row < m) {
-                    const float4* cs = reinterpret_cast<const float4*>(ep.cos_t + (size_t)row * half + c);   // half is a multiple of 32
-                    const float4* sn = reinterpret_cast<const float4*>(ep.sin_t + (size_t)row * half + c);
+            float first[32], second[32];
+            if ((is_q || is_k) && row < m) {
+                const float4* cs = reinterpret_cast<const float4*>(ep.cos_t + (size_t)row * half + c);   // half is a multiple of 32
+                const float4* sn = reinterpret_cast<const float4*>(ep.sin_t + (size_t)row * half + c);
 #pragma unroll
-                    for (int j = 0; j < 32; j += 4) {
-                        const float4 cv = cs[j >> 2], sv = sn[j >> 2];
-                        const float cc[4] = {cv.x, cv.y, cv.z, cv.w}, ss[4] = {sv.x, sv.y, sv.z, sv.w};
+                for (int j = 0; j < 32; j += 4) {
+                    const float4 cv = cs[j >> 2], sv = sn[j >> 2];
+                    const float cc[4] = {cv.x, cv.y, cv.z, cv.w}, ss[4] = {sv.x, sv.y, sv.z, sv.w};
 #pragma unroll
-                        for (int u = 0; u < 4; ++u) {
-                            const float a = __uint_as_float(lo[j + u]), b = __uint_as_float(hi[j + u]);
-                            first[j + u] = a * cc[u] - b * ss[u];
-                            second[j + u] = b * cc[u] + a * ss[u];
-                        }
+                    for (int e = 0; e < 4; ++e) {
+                        const float x = __uint_as_float(v[j + e]), y = __uint_as_float(hi[j + e]);
+                        first[j + e] = x * cc[e] - y * ss[e];
+                        second[j + e] = y * cc[e] + x * ss[e];
                     }
-                } else {
+                }
+            } else {
 #pragma unroll
-                    for (int j = 0; j < 32; ++j) { first[j] = __uint_as_float(lo[j]); second[j] = __uint_as_float(hi[j]); }
-                }
-                if (dst) {
-                    store_bf16x32(dst + c, first, 32);
-                    store_bf16x32(dst + half + c, second, 32);
-                }
+                for (int j = 0; j < 32; ++j) { first[j] = __uint_as_float(v[j]); second[j] = __uint_as_float(hi[j]); }
+            }
+            if (dst) {
+                store_bf16x32(dst + c, first, 32);
+                store_bf16x32(dst + half + c, second, 32);
             }
         }
     }
@@ -352,7 +350,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             if (!ok) break;
             tcgen05_fence_after();
             const uint32_t lane_base = tmem_base + (uint32_t)(acc * BN) + ((uint32_t)(quarter * 32) << 16);
-            epilogue_tile<BN, EPI>(ep, lane_base, row, m, n, n0, pos, page);
+            epilogue_tile<BN, EPI>(ep, [&](int c, uint32_t (&v)[32]) { tmem_load32(lane_base + (uint32_t)c, v); }, 0, epilogue_units<BN, EPI>(), row, m, n, n0, pos, page);
             tcgen05_fence_before();
             __syncwarp();
             if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(acc_empty + acc)) : "memory");
@@ -363,6 +361,221 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     tcgen05_fence_before();
     __syncthreads();
     if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(tmem_columns(BN)) : "memory");
+}
+
+// ---------------------------------------------------------------- few tiles: one per CTA, K over a cluster
+// For products of one round of CTAs.  A CTA has MT tiles of 128 rows by BN columns (MT accumulators side by side in tensor memory,
+// which share every weight tile), and the CTAs of a cluster (1, 2 or 4, along z) an equal share of K each.  The cluster's partial
+// sums meet in shared memory: each CTA lays down the units that each other one finishes, in the ring, which its own products have
+// left; one barrier.cluster says that every inbox is free; bulk copies bring the runs over; and each CTA adds its units' shares in
+// the order of K.  A last barrier.cluster keeps every CTA until its own runs are read.
+//
+// What bounds it: one SM takes 110 to 150 B/ns from L2, whatever the tile, so a tile's K takes its time however few tiles there
+// are.  Narrow tiles (64 columns) and K cut over a cluster put more SMs on the same bytes; the meeting costs 2 us.  us with the
+// weights in L2, before (the persistent kernel) and in this one, 64 / 200 / 512 rows: 4096 x 14336 66 / 69 / 75, 28 / 35 / 55;
+// 4096 x 4096 22 / 23 / 25, 12 / 14 / 19; 2048 x 8192 38 / 40 / 42, 14 / 16 / 22; 576 x 576 6.6 / 7.2 / 7.4, 4.8 / 6.0 / 6.1.
+// The shares of a unit are added 32 columns at a time: with the loop over the shares inside the loop over the columns the
+// compiler read them one after the other, 15 us a launch.
+template <int BN, int MT, int STAGES>
+struct SplitSmem {
+    static constexpr size_t A_BYTES = (size_t)MT * BM * BK * sizeof(bf16);
+    static constexpr size_t B_BYTES = (size_t)BN * BK * sizeof(bf16);
+    static constexpr size_t STAGE = A_BYTES + B_BYTES, TILES = STAGES * STAGE;
+    static constexpr size_t TOTAL = TILES + 1024 /* alignment slack */ + 256 /* barriers */;
+    // what a CTA sends away and what it receives, (shares - 1) / shares of the tile each, lie side by side in the ring
+    static constexpr bool CAN_SPLIT = MT == 1 && BN <= 128;
+    static_assert(!CAN_SPLIT || 2 * (size_t)BN * BM * sizeof(float) * 3 / 4 <= TILES, "the runs of four shares");
+};
+
+__device__ __forceinline__ void cluster_meet() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+template <int BN, int MT, int STAGES, int EPI>
+__global__ void __launch_bounds__(192, 1)
+gemm_tcgen05_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
+                          const Epilogue ep, int m, int n, int k, int* __restrict__ error) {
+    CISR_TRACE_SCOPE(TRACE_GEMM_TCGEN05);
+    extern __shared__ unsigned char smem_raw[];
+    typedef SplitSmem<BN, MT, STAGES> S;
+    unsigned char* tiles = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    uint64_t* full_bar = reinterpret_cast<uint64_t*>(tiles + S::TILES);
+    uint64_t* empty_bar = full_bar + STAGES;
+    uint64_t* acc_full = empty_bar + STAGES;
+    uint64_t* inbox_full = acc_full + 1;                                       // the other CTAs' shares have arrived
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(inbox_full + 1);
+    constexpr int TILE_N = paired_rows(EPI) ? BN / 2 : BN;
+    constexpr int COLUMNS = MT * BN;                                           // of tensor memory: 64 to 512, a power of two
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+    const int shares = (int)gridDim.z, rank = (int)blockIdx.z;                 // the cluster is the z dimension
+    const int n0 = (int)blockIdx.x * TILE_N, m0 = (int)blockIdx.y * MT * BM;
+    const int all_blocks = (k + BK - 1) / BK, kb0 = all_blocks * rank / shares, k_blocks = all_blocks * (rank + 1) / shares - kb0;
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < STAGES; ++s) { mbar_init(full_bar + s, 1); mbar_init(empty_bar + s, 1); }
+        mbar_init(acc_full, 1);
+        mbar_init(inbox_full, 1);
+        mbar_init_fence();
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(COLUMNS) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tcgen05_fence_before();
+    __syncthreads();
+    tcgen05_fence_after();
+    const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+    bool ok = true;
+    pdl_trigger();
+
+    if (warp == 0) {
+        if (lane == 0) {
+            auto load_b = [&](int s, int kb) {
+                unsigned char* b_tile = tiles + s * S::STAGE + S::A_BYTES;
+                if (paired_rows(EPI)) {       // two boxes of BN/2 rows: gate rows n0.., up rows inter + n0..
+                    tma_load_2d(b_tile, &map_w, (kb0 + kb) * BK, n0, full_bar + s);
+                    tma_load_2d(b_tile + S::B_BYTES / 2, &map_w, (kb0 + kb) * BK, ep.inter + n0, full_bar + s);
+                } else {
+                    tma_load_2d(b_tile, &map_w, (kb0 + kb) * BK, n0, full_bar + s);
+                }
+            };
+            auto load_a = [&](int s, int kb) {
+#pragma unroll
+                for (int t = 0; t < MT; ++t) tma_load_2d(tiles + s * S::STAGE + t * (S::A_BYTES / MT), &map_a, (kb0 + kb) * BK, m0 + t * BM, full_bar + s);
+            };
+            // the weights do not come from the kernel before: the first stages' tiles of them are requested before the wait on it
+            const int early = k_blocks < STAGES ? k_blocks : STAGES;
+            for (int kb = 0; kb < early; ++kb) {
+                mbar_expect_tx(full_bar + kb, (uint32_t)S::STAGE);
+                load_b(kb, kb);
+            }
+            pdl_wait();
+            CISR_TRACE_WAITED();
+            for (int kb = 0; kb < early; ++kb) load_a(kb, kb);
+            for (int kb = early; kb < k_blocks; ++kb) {
+                const int s = kb % STAGES;
+                ok = mbar_wait(empty_bar + s, ((kb / STAGES) & 1) ^ 1);
+                if (!ok) break;
+                mbar_expect_tx(full_bar + s, (uint32_t)S::STAGE);
+                load_a(s, kb);
+                load_b(s, kb);
+            }
+        }
+    } else if (warp == 1) {
+        constexpr uint32_t idesc = umma_idesc(BN);
+        const uint64_t desc_a = umma_desc(tiles), desc_b = umma_desc(tiles + S::A_BYTES);      // addresses below 256 KB: sums stay in the field
+        for (int kb = 0; kb < k_blocks; ++kb) {
+            const int s = kb % STAGES;
+            ok = __all_sync(0xffffffffu, mbar_wait(full_bar + s, (kb / STAGES) & 1));
+            if (!ok) break;
+            tcgen05_fence_after();
+            const uint64_t at = (uint64_t)s * (S::STAGE >> 4);
+#pragma unroll
+            for (int t = 0; t < MT; ++t)
+#pragma unroll
+                for (int kk = 0; kk < BK / UMMA_K; ++kk)
+                    umma_bf16_elect(tmem_base + (uint32_t)(t * BN), desc_a + at + t * (S::A_BYTES / MT >> 4) + 2 * kk, desc_b + at + 2 * kk, idesc, (kb | kk) != 0);
+            umma_commit_elect(empty_bar + s);
+        }
+        if (ok) umma_commit_elect(acc_full);
+    }
+    const int quarter = warp & 3;                                              // epilogue warps: the 32 lanes this warp may read
+    int pos[MT], page[MT];
+    if (warp >= 2) {
+        pdl_wait();      // outputs may alias what the kernel before still reads; step metadata is older than that kernel
+#pragma unroll
+        for (int t = 0; t < MT; ++t) {
+            const int row = m0 + t * BM + quarter * 32 + lane;
+            pos[t] = 0; page[t] = -1;
+            if (EPI == EPI_ROPE && row < m) {
+                pos[t] = ep.positions[row];
+                page[t] = ep.block_table[(size_t)ep.req_slot[ep.token_req[row]] * ep.table_width + pos[t] / ep.page_size];
+            }
+        }
+        ok = mbar_wait(acc_full, 0);
+        tcgen05_fence_after();
+    }
+    const uint32_t lanes = (uint32_t)(quarter * 32) << 16;
+    constexpr int UNITS = epilogue_units<BN, EPI>();
+    if (S::CAN_SPLIT && shares > 1) {
+        // every thread meets the barriers, also where a wait ran out (its sums are then not written)
+        __syncwarp();
+        const int per_cta = UNITS / shares, sides = EPI == EPI_PLAIN || EPI == EPI_RELU2 ? 1 : 2;
+        const int run = per_cta * sides * 32 * BM;                             // floats that one CTA sends another: [unit][side][32 columns][128 rows]
+        float* outbox = reinterpret_cast<float*>(tiles);                       // [shares - 1] runs, by receiver
+        float* inbox = outbox + (size_t)(shares - 1) * run;                    // [shares - 1] runs, by sender
+        const int row_in = quarter * 32 + lane;
+        if (warp >= 2) {
+            for (int to = 0; to < shares; ++to) {
+                if (to == rank) continue;
+                float* box = outbox + (size_t)(to < rank ? to : to - 1) * run + row_in;
+                for (int u = 0; u < per_cta; ++u) {
+                    int lo, hi;
+                    unit_columns<BN, EPI>(ep, to * per_cta + u, lo, hi);
+                    for (int side = 0; side < sides; ++side) {
+                        uint32_t v[32];
+                        tmem_load32(tmem_base + lanes + (uint32_t)(side ? hi : lo), v);
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) box[j * BM] = __uint_as_float(v[j]);
+                        box += 32 * BM;
+                    }
+                }
+            }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // the runs before the copies that read them
+            if (warp == 2 && lane == 0) mbar_expect_tx(inbox_full, (uint32_t)((shares - 1) * run * sizeof(float)));
+            __syncwarp();
+        }
+        cluster_meet();                                                        // every CTA's products are done and its runs are written: the inboxes are free
+        if (warp == 2 && lane == 0) {
+            for (int to = 0; to < shares; ++to) {
+                if (to == rank) continue;
+                uint32_t there, bar;
+                asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(there) : "r"(smem_u32(inbox + (size_t)(rank < to ? rank : rank - 1) * run)), "r"(to));
+                asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(bar) : "r"(smem_u32(inbox_full)), "r"(to));
+                asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                             ::"r"(there), "r"(smem_u32(outbox + (size_t)(to < rank ? to : to - 1) * run)), "r"((uint32_t)(run * sizeof(float))), "r"(bar) : "memory");
+            }
+        }
+        __syncwarp();
+        if (warp >= 2) {
+            ok = mbar_wait(inbox_full, 0) && ok;
+            if (__all_sync(0xffffffffu, ok)) {
+                const float* next = inbox + row_in;                            // loads come in the order unit, side
+                epilogue_tile<BN, EPI>(ep, [&](int c, uint32_t (&v)[32]) {
+                    const float* from = next;
+                    next += 32 * BM;
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) v[j] = 0u;
+#pragma unroll 1
+                    for (int r = 0; r < shares; ++r) {                         // the shares in the order of K
+                        uint32_t share[32];
+                        if (r == rank) {
+                            tmem_load32(tmem_base + lanes + (uint32_t)c, share);
+                        } else {
+#pragma unroll
+                            for (int j = 0; j < 32; ++j) share[j] = __float_as_uint(from[j * BM]);
+                            from += run;
+                        }
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) + __uint_as_float(share[j]));
+                    }
+                }, rank * per_cta, (rank + 1) * per_cta, m0 + row_in, m, n, n0, pos[0], page[0]);
+            }
+        }
+        __syncwarp();
+        cluster_meet();                                                        // every run has arrived: no CTA leaves while its own are read
+    } else if (warp >= 2 && ok) {
+#pragma unroll
+        for (int t = 0; t < MT; ++t) {
+            const uint32_t lane_base = tmem_base + lanes + (uint32_t)(t * BN);
+            epilogue_tile<BN, EPI>(ep, [&](int c, uint32_t (&v)[32]) { tmem_load32(lane_base + (uint32_t)c, v); }, 0, UNITS,
+                                   m0 + t * BM + quarter * 32 + lane, m, n, n0, pos[t], page[t]);
+        }
+    }
+    if (!ok && lane == 0) atomicExch(error, 1);
+    tcgen05_fence_before();
+    __syncthreads();
+    if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(COLUMNS) : "memory");
 }
 
 // ---------------------------------------------------------------- host side
@@ -401,20 +614,58 @@ int launch(const void* a, const void* w, const Epilogue& ep, int m, int n, int k
 // occupy most of the device (one CTA per SM at that size).
 bool wide_tiles(int m, int tiles_n256) { return (long long)((m + BM - 1) / BM) * tiles_n256 >= 120; }
 
-// Fewer 128 x 128 tiles than SMs: every CTA runs one tile, alone on its SM, and the time is the ring's round trips to
-// L2 (a stage is asked for again only after its product), not the tensor pipe.  A deeper ring with the whole SM's
-// shared memory hides them, and while 128 x 64 tiles still fit the device at one per SM, twice as many CTAs share
-// the weights.  Returns 64 or 128 for the tile width of the deep ring, 0 for the ordinary choice (also with
-// CISR_GEMM_DEEP=0).  `cols`: output columns a 128-wide tile covers (64 features for the gated product).
-int few_tiles(int m, int n, int cols) {
+template <int BN, int MT, int STAGES, int EPI>
+int launch_split(const void* a, const void* w, const Epilogue& ep, int m, int n, int k, int shares, cudaStream_t s) {
+    CUtensorMap map_a, map_w;
+    int status = cached_map(&map_a, a, m, k, BM);
+    if (status) return status;
+    if ((status = cached_map(&map_w, w, n, k, paired_rows(EPI) ? BN / 2 : BN))) return status;
+    typedef SplitSmem<BN, MT, STAGES> S;
+    static bool configured = false;
+    if (!configured) {
+        cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_split_kernel<BN, MT, STAGES, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::TOTAL);
+        if (e != cudaSuccess) return (int)e;
+        configured = true;
+    }
+    const int cols = paired_rows(EPI) ? n / 2 : n, tile_n = paired_rows(EPI) ? BN / 2 : BN;
+    return launch_kernel_cluster(gemm_tcgen05_split_kernel<BN, MT, STAGES, EPI>, dim3((cols + tile_n - 1) / tile_n, (m + MT * BM - 1) / (MT * BM), shares),
+                                 dim3(192), S::TOTAL, s, g_pdl, shares, map_a, map_w, ep, m, n, k, g_error);
+}
+
+// How the kernel for few tiles takes a product of m rows and cols64 tiles of 64 columns, max64 and max128 the shares of K that tiles
+// of 64 and 128 columns can be cut in (0: no such tiles); mt 0: not at all, the persistent kernel is better (or CISR_GEMM_DEEP=0).
+// - K to 2048 and tiles of 64 columns fit the SMs at one each: those, cut in two from 24 blocks of K on where there is room.  us,
+//   64 and 128 columns wide: 576 x 576, 200 rows 6.0 and 7.6; 2048 x 2048, 64 rows 7.6 and 8.7; 512 rows 9.9 and 10.4.
+// - tiles of 128 columns fit: K cut in as many shares as fit, of at least eight blocks each.  A longer K wants the wider tiles,
+//   which read the activations half as often: 2048 x 8192, 64 rows, 64 CTAs either way: 14 us, 17 with 64 columns.
+// - more tiles, to 256 rows: one tile for all the rows, of 128 columns where that fits, or of 256.  28672 x 4096, gated, 200 rows
+//   56 us; 63 in the persistent kernel; 16384 x 2048 18 and 19.5.
+// - more rows or columns: the persistent kernel, whose epilogues run beside the next tile's products (2048 x 2048, 2048 rows: 19
+//   us; 24 here).
+struct SplitChoice { int bn, mt, shares; };
+SplitChoice split_choice(int m, int cols64, int k, int max64, int max128) {
     static int sms = 0, on = -1;
     if (!sms) { int device = 0; cudaGetDevice(&device); cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device); }
     if (on < 0) { const char* e = getenv("CISR_GEMM_DEEP"); on = !(e && e[0] == '0'); }
-    if (!on) return 0;
-    const long long tiles_m = (m + BM - 1) / BM;
-    if (tiles_m * ((n + cols / 2 - 1) / (cols / 2)) <= sms) return 64;
-    if (tiles_m * ((n + cols - 1) / cols) <= sms) return 128;
-    return 0;
+    const int blocks = (k + BK - 1) / BK, cols128 = (cols64 + 1) / 2;
+    const long long tiles_m = (m + BM - 1) / BM, tiles64 = tiles_m * cols64, tiles128 = tiles_m * cols128;
+    if (!on) return {0, 0, 0};
+    if (max64 && blocks <= 32 && tiles64 <= sms) return {64, 1, max64 >= 2 && blocks >= 24 && 2 * tiles64 <= sms ? 2 : 1};
+    if (tiles128 <= sms) {
+        int shares = 1;
+        while (2 * shares <= max128 && 2 * shares * tiles128 <= sms && blocks >= 16 * shares) shares *= 2;
+        return {128, 1, shares};
+    }
+    if (tiles_m > 2) return {0, 0, 0};
+    if (tiles_m == 2 && cols128 <= sms) return {128, 2, 1};
+    if ((cols128 + 1) / 2 <= sms) return {256, (int)tiles_m, 1};
+    return {0, 0, 0};
+}
+template <int EPI>
+int launch_split_choice(SplitChoice c, const void* a, const void* w, const Epilogue& ep, int m, int n, int k, cudaStream_t s) {
+    if (c.bn == 64) return launch_split<64, 1, 8, EPI>(a, w, ep, m, n, k, c.shares, s);
+    if (c.mt == 1) return c.bn == 256 ? launch_split<256, 1, 4, EPI>(a, w, ep, m, n, k, c.shares, s) : launch_split<128, 1, 6, EPI>(a, w, ep, m, n, k, c.shares, s);
+    return c.bn == 256 ? launch_split<256, 2, 3, EPI>(a, w, ep, m, n, k, c.shares, s) : launch_split<128, 2, 4, EPI>(a, w, ep, m, n, k, c.shares, s);
 }
 
 bool operands_ok(const void* a, const void* w, int k) {
@@ -447,11 +698,14 @@ CISR_EXPORT int cisr_gemm_tcgen05(const void* a, const void* w, float* out, int 
     Epilogue ep = {};
     ep.out_f32 = out; ep.accumulate = accumulate != 0; ep.out_mult = out_mult == 1.f ? 0.f : out_mult;
     cudaStream_t s = (cudaStream_t)stream;
-    if (n <= 64) return launch<64, 8, EPI_PLAIN>(a, w, ep, m, n, k, (n + 63) / 64, s);
+    if (n <= 64) {
+        // a router's few outputs: a column of row tiles, K cut in two where it is long (uncut, 16 CTAs wait for all of K one after another)
+        const int shares = k >= 2048 && (m + BM - 1) / BM <= 74 ? 2 : 1;
+        if (shares == 2) return launch_split<64, 1, 8, EPI_PLAIN>(a, w, ep, m, n, k, 2, s);
+        return launch<64, 8, EPI_PLAIN>(a, w, ep, m, n, k, 1, s);
+    }
+    if (const SplitChoice c = split_choice(m, (n + 63) / 64, k, 2, 4); c.mt) return launch_split_choice<EPI_PLAIN>(c, a, w, ep, m, n, k, s);
     if (wide_tiles(m, (n + 255) / 256)) return launch<256, 4, EPI_PLAIN>(a, w, ep, m, n, k, (n + 255) / 256, s);
-    const int deep = few_tiles(m, n, 128);
-    if (deep == 64) return launch<64, 8, EPI_PLAIN>(a, w, ep, m, n, k, (n + 63) / 64, s);
-    if (deep == 128) return launch<128, 6, EPI_PLAIN>(a, w, ep, m, n, k, (n + 127) / 128, s);
     return launch<128, 3, EPI_PLAIN>(a, w, ep, m, n, k, (n + 127) / 128, s);
 }
 
@@ -464,12 +718,15 @@ CISR_EXPORT int cisr_gemm_tcgen05_swiglu(const void* a, const void* w, void* out
     if (!operands_ok(a, w, k)) return -2;
     Epilogue ep = {};
     ep.out_bf16 = (bf16*)out; ep.inter = inter; ep.act = gate_act;
+    const SplitChoice few = split_choice(m, (inter + 31) / 32, k, 1, 2);
     if (gate_act == 2) {
         ep.limit = gate_limit; ep.alpha = 1.702f;
+        if (few.mt) return launch_split_choice<EPI_GATED>(few, a, w, ep, m, 2 * inter, k, (cudaStream_t)stream);
         if (wide_tiles(m, (inter + 127) / 128))
             return launch<256, 4, EPI_GATED>(a, w, ep, m, 2 * inter, k, (inter + 127) / 128, (cudaStream_t)stream);
         return launch<128, 3, EPI_GATED>(a, w, ep, m, 2 * inter, k, (inter + 63) / 64, (cudaStream_t)stream);
     }
+    if (few.mt) return launch_split_choice<EPI_SWIGLU>(few, a, w, ep, m, 2 * inter, k, (cudaStream_t)stream);
     if (wide_tiles(m, (inter + 127) / 128)) {
         // 128 x 256 tiles, or 128 x 192 where their last round would be much emptier: 192 tiles of 256 columns on 148 SMs
         // are two rounds for 1.3 rounds of work, 256 tiles of 192 columns are two rounds of three quarters the length
@@ -481,9 +738,6 @@ CISR_EXPORT int cisr_gemm_tcgen05_swiglu(const void* a, const void* w, void* out
             return launch<192, 4, EPI_SWIGLU>(a, w, ep, m, 2 * inter, k, (inter + 95) / 96, (cudaStream_t)stream);
         return launch<256, 4, EPI_SWIGLU>(a, w, ep, m, 2 * inter, k, (inter + 127) / 128, (cudaStream_t)stream);
     }
-    const int deep = few_tiles(m, inter, 64);
-    if (deep == 64) return launch<64, 8, EPI_SWIGLU>(a, w, ep, m, 2 * inter, k, (inter + 31) / 32, (cudaStream_t)stream);
-    if (deep == 128) return launch<128, 6, EPI_SWIGLU>(a, w, ep, m, 2 * inter, k, (inter + 63) / 64, (cudaStream_t)stream);
     return launch<128, 3, EPI_SWIGLU>(a, w, ep, m, 2 * inter, k, (inter + 63) / 64, (cudaStream_t)stream);
 }
 
@@ -502,10 +756,8 @@ CISR_EXPORT int cisr_gemm_tcgen05_rope(const void* a, const void* w, int m, int 
     ep.positions = positions; ep.token_req = token_req; ep.req_slot = req_slot; ep.block_table = block_table;
     ep.table_width = table_width; ep.page_size = page_size; ep.hq = hq; ep.hkv = hkv; ep.dim = dim;
     const int n = (hq + 2 * hkv) * dim;
+    if (const SplitChoice c = split_choice(m, (n + 63) / 64, k, dim == 64 ? 1 : 0, 2); c.mt) return launch_split_choice<EPI_ROPE>(c, a, w, ep, m, n, k, (cudaStream_t)stream);
     if (wide_tiles(m, (n + 255) / 256)) return launch<256, 4, EPI_ROPE>(a, w, ep, m, n, k, (n + 255) / 256, (cudaStream_t)stream);
-    const int deep = few_tiles(m, n, 128);
-    if (deep == 64 && dim == 64) return launch<64, 8, EPI_ROPE>(a, w, ep, m, n, k, (n + 63) / 64, (cudaStream_t)stream);   // a whole head per tile
-    if (deep) return launch<128, 6, EPI_ROPE>(a, w, ep, m, n, k, (n + 127) / 128, (cudaStream_t)stream);
     return launch<128, 3, EPI_ROPE>(a, w, ep, m, n, k, (n + 127) / 128, (cudaStream_t)stream);
 }
 
