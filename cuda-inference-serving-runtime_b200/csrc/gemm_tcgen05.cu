@@ -638,8 +638,9 @@ int launch_split(const void* a, const void* w, const Epilogue& ep, int m, int n,
 //   64 and 128 columns wide: 576 x 576, 200 rows 6.0 and 7.6; 2048 x 2048, 64 rows 7.6 and 8.7; 512 rows 9.9 and 10.4.
 // - tiles of 128 columns fit: K cut in as many shares as fit, of at least eight blocks each.  A longer K wants the wider tiles,
 //   which read the activations half as often: 2048 x 8192, 64 rows, 64 CTAs either way: 14 us, 17 with 64 columns.
-// - more tiles, to 256 rows: one tile for all the rows, of 128 columns where that fits, or of 256.  28672 x 4096, gated, 200 rows
-//   56 us; 63 in the persistent kernel; 16384 x 2048 18 and 19.5.
+// - tiles of 256 columns fit, or do for two row tiles that share them: those.  us, in the persistent kernel (whose 128 x 128 tiles
+//   read half as much again) and here: 4096 x 14336, 800 rows 170 and 88; 6144 x 4096, 512 rows 46 and 34; gated 28672 x 4096, 200
+//   rows 63 and 56; gated 3584 x 4096, 1024 rows 45 and 28.
 // - more rows or columns: the persistent kernel, whose epilogues run beside the next tile's products (2048 x 2048, 2048 rows: 19
 //   us; 24 here).
 struct SplitChoice { int bn, mt, shares; };
@@ -656,16 +657,15 @@ SplitChoice split_choice(int m, int cols64, int k, int max64, int max128) {
         while (2 * shares <= max128 && 2 * shares * tiles128 <= sms && blocks >= 16 * shares) shares *= 2;
         return {128, 1, shares};
     }
-    if (tiles_m > 2) return {0, 0, 0};
-    if (tiles_m == 2 && cols128 <= sms) return {128, 2, 1};
-    if ((cols128 + 1) / 2 <= sms) return {256, (int)tiles_m, 1};
+    if (tiles_m * ((cols128 + 1) / 2) <= sms) return {256, 1, 1};
+    if (tiles_m == 2 && (cols128 + 1) / 2 <= sms) return {256, 2, 1};
     return {0, 0, 0};
 }
 template <int EPI>
 int launch_split_choice(SplitChoice c, const void* a, const void* w, const Epilogue& ep, int m, int n, int k, cudaStream_t s) {
     if (c.bn == 64) return launch_split<64, 1, 8, EPI>(a, w, ep, m, n, k, c.shares, s);
-    if (c.mt == 1) return c.bn == 256 ? launch_split<256, 1, 4, EPI>(a, w, ep, m, n, k, c.shares, s) : launch_split<128, 1, 6, EPI>(a, w, ep, m, n, k, c.shares, s);
-    return c.bn == 256 ? launch_split<256, 2, 3, EPI>(a, w, ep, m, n, k, c.shares, s) : launch_split<128, 2, 4, EPI>(a, w, ep, m, n, k, c.shares, s);
+    if (c.bn == 128) return launch_split<128, 1, 6, EPI>(a, w, ep, m, n, k, c.shares, s);
+    return c.mt == 1 ? launch_split<256, 1, 4, EPI>(a, w, ep, m, n, k, 1, s) : launch_split<256, 2, 3, EPI>(a, w, ep, m, n, k, 1, s);
 }
 
 bool operands_ok(const void* a, const void* w, int k) {

@@ -18,7 +18,7 @@ def near(got, want, kk):
 
 @pytest.mark.parametrize("m,n,kk", [(1, 66, 1472), (200, 576, 1536), (300, 4736, 1536), (257, 64, 2048), (129, 33, 2056),  # 64 columns, K in 1 and 2
                                     (64, 4096, 4096), (128, 4737, 2056), (130, 9472, 2120), (700, 300, 4104),               # 128: 4, 2 and 1
-                                    (129, 9600, 520), (256, 18944, 72), (100, 19000, 520), (256, 18945, 520), (90, 37900, 72)])
+                                    (129, 9600, 520), (900, 4500, 200), (256, 18944, 72), (100, 19000, 520), (256, 18945, 520), (90, 37900, 72)])
 @pytest.mark.parametrize("accumulate", [False, True])
 def test_plain(m, n, kk, accumulate):
     from cisr_b200.ops import kernels
@@ -29,7 +29,7 @@ def test_plain(m, n, kk, accumulate):
     near(out, 0.5 * want + accumulate, kk)
 
 
-@pytest.mark.parametrize("m,inter,kk", [(200, 1500, 576), (64, 2368, 1536), (128, 2000, 4096), (200, 4800, 520), (100, 9500, 520), (256, 9500, 136)])
+@pytest.mark.parametrize("m,inter,kk", [(200, 1500, 576), (64, 2368, 1536), (128, 2000, 4096), (200, 4800, 520), (900, 2300, 200), (100, 9500, 520), (256, 9500, 136)])
 @pytest.mark.parametrize("gate", ["silu", "gelu_tanh", "gated_clamp"])
 def test_gated(m, inter, kk, gate):
     from cisr_b200.ops import kernels
@@ -48,7 +48,7 @@ def test_gated(m, inter, kk, gate):
     assert ((out.double() - want).abs() <= 1e-3 + 2 ** -7 * want.abs()).all()       # bfloat16's 2^-9 with room for the sums' error
 
 
-@pytest.mark.parametrize("m,hq,hkv,dim,kk", [(200, 9, 3, 64, 576), (64, 32, 8, 128, 4096), (130, 8, 8, 64, 4104), (200, 16, 4, 128, 2048), (200, 66, 5, 128, 520)])
+@pytest.mark.parametrize("m,hq,hkv,dim,kk", [(200, 9, 3, 64, 576), (64, 32, 8, 128, 4096), (130, 8, 8, 64, 4104), (200, 16, 4, 128, 2048), (200, 66, 5, 128, 520), (700, 32, 8, 128, 200)])
 def test_rotated(m, hq, hkv, dim, kk):
     from cisr_b200.ops import kernels
     a, w, _ = operands(m, (hq + 2 * hkv) * dim, kk)
