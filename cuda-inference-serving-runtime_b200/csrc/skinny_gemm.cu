@@ -33,6 +33,7 @@
 // Parity: these products are what runtime/blas.py:41-56 of the reference hands to cuBLAS with M = batch;
 // the fused neighbours are kernels/execution.cu:12-24 (residual + norm), :7-10 (SwiGLU), :28-40 (rotation
 // and cache write).  K must be a multiple of 8 (16-byte rows).
+#include "skinny_call.cuh"
 #include "common.cuh"
 
 namespace {
@@ -535,13 +536,17 @@ CISR_EXPORT void cisr_skinny_set_pdl(int on) { g_pdl = on != 0; }
 
 // One entry point; unused pointer groups are null.  Returns -2 for shapes it does not take (the caller then
 // uses the library product and the separate kernels).
-CISR_EXPORT int cisr_skinny_gemm(const void* w, int n, int k, const void* act, const float* x, const float* delta,
-                                 const void* norm_w, int norm_w_dtype, float eps, float* x_out, const int* rows, int m,
-                                 int epilogue, float* out_f32, void* out_bf16, int inter, const float* cos_t,
-                                 const float* sin_t, int rot_half, int interleaved, void* q_out, void* k_cache,
-                                 void* v_cache, const int* positions, const int* token_req, const int* req_slot,
-                                 const int* block_table, int table_width, int page_size, int hq, int hkv, int dim,
-                                 int accumulate, float out_mult, int gate_act, float gate_limit, void* stream) {
+CISR_EXPORT int cisr_skinny_gemm(const SkinnyCall* call) {
+    const void *w = call->w, *act = call->act, *norm_w = call->norm_w;
+    const float *x = (const float*)call->x, *delta = (const float*)call->delta, *cos_t = (const float*)call->cos_t, *sin_t = (const float*)call->sin_t;
+    const int *rows = (const int*)call->rows, *positions = (const int*)call->positions, *token_req = (const int*)call->token_req;
+    const int *req_slot = (const int*)call->req_slot, *block_table = (const int*)call->block_table;
+    float *x_out = (float*)call->x_out, *out_f32 = (float*)call->out_f32;
+    void *out_bf16 = call->out_bf16, *q_out = call->q_out, *k_cache = call->k_cache, *v_cache = call->v_cache, *stream = call->stream;
+    const float eps = (float)call->eps, out_mult = (float)call->out_mult, gate_limit = (float)call->gate_limit;
+    const int n = call->n, k = call->k, norm_w_dtype = call->norm_w_dtype, m = call->m, epilogue = call->epilogue, inter = call->inter;
+    const int rot_half = call->rot_half, interleaved = call->interleaved, table_width = call->table_width, page_size = call->page_size;
+    const int hq = call->hq, hkv = call->hkv, dim = call->dim, accumulate = call->accumulate, gate_act = call->gate_act;
     if (m <= 0) return 0;
     if (m > 64 || k % 8 || k <= 0 || n <= 0) return -2;
     if (epilogue == EPI_ROPE && (dim % 16 || dim > 256 || dim < 16 || n != (hq + 2 * hkv) * dim || 2 * rot_half > dim)) return -2;

@@ -29,6 +29,7 @@ BASE_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "--shared", "-Xcompiler", "-fPIC
               "--expt-relaxed-constexpr"]
 
 _loaded: Dict[str, ctypes.CDLL] = {}
+_plain: Dict[str, ctypes.CDLL] = {}      # those without definitions, by source name
 _lock = threading.Lock()
 
 
@@ -175,6 +176,8 @@ def _drop_superseded(target: Path) -> None:
 
 
 def load_library(source_name: str, defines: Optional[Mapping[str, object]] = None, extra: Sequence[str] = ()) -> ctypes.CDLL:
+    if not defines and not extra and source_name in _plain:        # the usual call, one per launch
+        return _plain[source_name]
     key = repr((source_name, sorted((defines or {}).items()), list(extra)))
     with _lock:
         lib = _loaded.get(key)
@@ -185,6 +188,8 @@ def load_library(source_name: str, defines: Optional[Mapping[str, object]] = Non
             except OSError as err:
                 raise BuildError(f"could not load {path}: {err}") from err
             _loaded[key] = lib
+            if not defines and not extra:
+                _plain[source_name] = lib
         return lib
 
 

@@ -9,6 +9,7 @@ from __future__ import annotations
 
 import ctypes
 import os
+import struct
 from typing import Optional
 
 import torch
@@ -1868,6 +1869,14 @@ def skinny_ok(tokens: int, w: torch.Tensor) -> bool:
     return padded * (w.shape[1] + 8) * 2 + 64 * padded * 4 * 2 <= 200 * 1024     # the tokens and the partial sums fit in shared memory
 
 
+# struct SkinnyCall of csrc/skinny_call.cuh: 19 addresses, three doubles, 15 ints
+_SKINNY_CALL = struct.Struct("@19P3d15i")
+
+
+def _at(t: Optional[torch.Tensor]) -> int:
+    return 0 if t is None else t.data_ptr()
+
+
 def skinny_gemm(w: torch.Tensor, tokens: int, *, act: Optional[torch.Tensor] = None, x: Optional[torch.Tensor] = None,
                 delta: Optional[torch.Tensor] = None, norm_w: Optional[torch.Tensor] = None, eps: float = 0.0,
                 x_out: Optional[torch.Tensor] = None, rows: Optional[torch.Tensor] = None, epilogue: int = EPI_PLAIN,
@@ -1922,25 +1931,27 @@ def skinny_gemm(w: torch.Tensor, tokens: int, *, act: Optional[torch.Tensor] = N
             _need(r[name], torch.int32, name)
         if r["rot_half"]:
             _need(r["cos"], torch.float32, "cos", 2); _need(r["sin"], torch.float32, "sin", 2)
-    args = (_p(w), n, k, _p(act), _p(x), _p(delta), _p(norm_w), dtype_code(norm_w.dtype) if norm_w is not None else 0,
-            ctypes.c_float(eps), _p(x_out), _p(rows), tokens, epilogue, _p(out_f32), _p(out_b16),
-            n // 2 if epilogue == EPI_SWIGLU else 0, _p(r.get("cos")), _p(r.get("sin")), int(r.get("rot_half", 0)),
-            int(bool(r.get("interleaved", False))), _p(r.get("q_out")), _p(r.get("k_cache")), _p(r.get("v_cache")),
-            _p(r.get("positions")), _p(r.get("token_req")), _p(r.get("req_slot")), _p(r.get("block_table")),
-            r["block_table"].shape[1] if rope else 0, int(r.get("page_size", 0)), int(r.get("hq", 0)), int(r.get("hkv", 0)),
-            int(r.get("dim", 0)), int(bool(accumulate)), ctypes.c_float(out_mult), *_gate(gate, gate_limit), _stream())
+    gate_act, _ = _gate(gate, gate_limit)
+    get = r.get
+    args = _SKINNY_CALL.pack(
+        w.data_ptr(), _at(act), _at(x), _at(delta), _at(norm_w), _at(x_out), _at(rows), _at(out_f32), _at(out_b16), _at(get("cos")),
+        _at(get("sin")), _at(get("q_out")), _at(get("k_cache")), _at(get("v_cache")), _at(get("positions")), _at(get("token_req")),
+        _at(get("req_slot")), _at(get("block_table")), _stream().value or 0, eps, out_mult, gate_limit or 0.0, n, k,
+        dtype_code(norm_w.dtype) if norm_w is not None else 0, tokens, epilogue, n // 2 if epilogue == EPI_SWIGLU else 0,
+        int(get("rot_half", 0)), int(bool(get("interleaved", False))), r["block_table"].shape[1] if rope else 0, int(get("page_size", 0)),
+        int(get("hq", 0)), int(get("hkv", 0)), int(get("dim", 0)), int(bool(accumulate)), gate_act)
     if (accumulate or out_mult != 1.0) and epilogue != EPI_PLAIN:
         raise KernelError("skinny_gemm: only the plain epilogue adds into its output or multiplies it")
     if kind not in ("auto", "latency", "stream"):
         raise KernelError(f"unknown kind {kind!r}")
     if kind == "stream" or (kind == "auto" and tokens <= STREAM_MAX_TOKENS and w.numel() * 2 >= STREAM_MIN_BYTES):
-        status = _stream_lib().cisr_stream_gemm(*args)
+        status = _stream_lib().cisr_stream_gemm(args)
         if status != -2:                  # -2: not a shape for the streaming kernel
             _check(status, "stream_gemm")
             return
         if kind == "stream":
             raise KernelError("stream_gemm does not take this shape")
-    _check(_skinny().cisr_skinny_gemm(*args), "skinny_gemm")
+    _check(_skinny().cisr_skinny_gemm(args), "skinny_gemm")
 
 
 STREAM_MAX_TOKENS = 16
