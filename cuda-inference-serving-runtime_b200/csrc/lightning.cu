@@ -226,10 +226,67 @@ __global__ void lightning_output_kernel(const float* __restrict__ o, const float
         out[(size_t)t * out_stride + j] = from_float<CT>(row[j] * unit * norm_w[j] * (1.f / (1.f + expf(-g[j]))));
 }
 
+// The same, four columns an access and the row and its gates in registers, all requested before the sum: bound by memory (2048
+// tokens of 2048: 42 MB, 6.4 us), where single columns asked for one float a thread and the gates only after the sum:
+// 18.4 us, now 10.5.
+// The sigmoid's division without the ordinary one's second path where the result is rounded to bfloat16 (2^-22 beside 2^-9).
+template <typename CT> __device__ __forceinline__ float sigmoid_of(float g) { return 1.f / (1.f + expf(-g)); }
+template <> __device__ __forceinline__ float sigmoid_of<__nv_bfloat16>(float g) { return __fdividef(1.f, 1.f + expf(-g)); }
+__device__ __forceinline__ void store4(float* to, const float (&v)[4]) { *reinterpret_cast<float4*>(to) = make_float4(v[0], v[1], v[2], v[3]); }
+__device__ __forceinline__ void store4(__nv_bfloat16* to, const float (&v)[4]) {
+    __nv_bfloat162 pair[2] = {__floats2bfloat162_rn(v[0], v[1]), __floats2bfloat162_rn(v[2], v[3])};
+    *reinterpret_cast<uint2*>(to) = *reinterpret_cast<uint2*>(pair);
+}
+constexpr int OUT_THREADS = 256, OUT_RUNS = 4;            // rows of up to 4 * 4 * 256 columns
+template <typename CT>
+__global__ void __launch_bounds__(OUT_THREADS)
+lightning_output_runs_kernel(const float* __restrict__ o, const float* __restrict__ gate, int gate_stride, int gate_col,
+                             const float* __restrict__ norm_w, float eps, CT* __restrict__ out, int out_stride, int width) {
+    __shared__ float scratch[32];
+    pdl_trigger();
+    pdl_wait();
+    const size_t t = blockIdx.x;
+    const float* row = o + t * width;
+    const float* gr = gate + t * gate_stride + gate_col;
+    float v[OUT_RUNS][4], g[OUT_RUNS][4], sq = 0.f;
+#pragma unroll
+    for (int r = 0; r < OUT_RUNS; ++r) {
+        const int j = 4 * (r * OUT_THREADS + (int)threadIdx.x);
+        const float4 a = j < width ? *reinterpret_cast<const float4*>(row + j) : make_float4(0.f, 0.f, 0.f, 0.f);
+        const float4 b = j < width ? *reinterpret_cast<const float4*>(gr + j) : make_float4(0.f, 0.f, 0.f, 0.f);
+        v[r][0] = a.x; v[r][1] = a.y; v[r][2] = a.z; v[r][3] = a.w;
+        g[r][0] = b.x; g[r][1] = b.y; g[r][2] = b.z; g[r][3] = b.w;
+    }
+#pragma unroll
+    for (int r = 0; r < OUT_RUNS; ++r)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) sq += v[r][e] * v[r][e];
+    const float unit = rsqrtf(block_sum(sq, scratch) / (float)width + eps);
+#pragma unroll
+    for (int r = 0; r < OUT_RUNS; ++r) {
+        const int j = 4 * (r * OUT_THREADS + (int)threadIdx.x);
+        if (j >= width) break;
+        const float4 w = *reinterpret_cast<const float4*>(norm_w + j);
+        const float ww[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) v[r][e] = v[r][e] * unit * ww[e] * sigmoid_of<CT>(g[r][e]);
+        store4(out + t * out_stride + j, v[r]);
+    }
+}
+
 CISR_EXPORT int cisr_lightning_output(const float* o, const float* gate, int gate_stride, int gate_col, const float* norm_w, float eps,
                                       void* out, int dtype, int out_stride, int width, int tokens, void* stream) {
     if (tokens <= 0) return 0;
     cudaStream_t s = (cudaStream_t)stream;
+    // rows of 512 to 4096 columns in whole aligned runs of four (below, most of the threads would have none)
+    const bool runs = width >= 512 && width <= 4 * OUT_THREADS * OUT_RUNS && !((width | gate_stride | gate_col | out_stride) & 3) &&
+                      !(((uintptr_t)o | (uintptr_t)gate | (uintptr_t)norm_w | (uintptr_t)out) & 15);
+    if (runs && dtype == CISR_BF16)
+        return launch_kernel(lightning_output_runs_kernel<__nv_bfloat16>, dim3(tokens), dim3(OUT_THREADS), 0, s, g_pdl, o, gate, gate_stride,
+                             gate_col, norm_w, eps, (__nv_bfloat16*)out, out_stride, width);
+    if (runs)
+        return launch_kernel(lightning_output_runs_kernel<float>, dim3(tokens), dim3(OUT_THREADS), 0, s, g_pdl, o, gate, gate_stride, gate_col,
+                             norm_w, eps, (float*)out, out_stride, width);
     const int threads = width >= 1024 ? 256 : 128;
     if (dtype == CISR_BF16)
         return launch_kernel(lightning_output_kernel<__nv_bfloat16>, dim3(tokens), dim3(threads), 0, s, g_pdl, o, gate, gate_stride, gate_col,
