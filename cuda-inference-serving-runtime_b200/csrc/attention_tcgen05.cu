@@ -66,6 +66,13 @@ constexpr int KV_BYTES = NSUB * KV_SUB;       // a K tile, or a V tile
 // tile only after the output products, one softmax later.  A tile is 16 KB at head size 64 and 32 KB at 128.
 constexpr int K_STAGES = D == 64 ? 4 : 3;
 constexpr int V_STAGES = D == 64 ? 4 : 2;
+// Two streams with the same queries leave room for one more value tile (stream 1's queries), which head size 128 takes.  Head
+// size 64 does not: its streams take the tiles in turn and a warp of its own waits for each stream's, so a ring of five would
+// hand every slot from one warp to the other, and a warp that skips a phase of a slot's barrier can pass it a phase early.
+// In an even ring every slot is one stream's.
+constexpr bool OWN_P = D == 64;
+__host__ __device__ constexpr int value_slots(bool shared) { return V_STAGES + (shared && !OWN_P); }
+static_assert(!OWN_P || (K_STAGES % 2 == 0 && value_slots(true) % 2 == 0), "a slot belongs to one stream");
 constexpr size_t SMEM_FIXED = 1024 + 2 * Q_BYTES + (K_STAGES + V_STAGES) * KV_BYTES + 256;
 constexpr float LOG2E = 1.4426950408889634f;
 constexpr float RESCALE_STEP = 8.f;           // the max may lag by this much (base-2 exponent) before O is rescaled
@@ -76,7 +83,6 @@ constexpr int THREADS = 32 * FIRST_SOFTMAX_WARP + SOFTMAX_THREADS;
 // the accumulators leave room for the probabilities in a place of their own (OWN_P), so a stream's next scores are
 // multiplied as soon as its threads have the scores at hand in registers; at 128 they go over the first half of the scores.
 constexpr uint32_t TMEM_O = 256, TMEM_P = 384;
-constexpr bool OWN_P = D == 64;
 // A softmax thread takes its row of scores from tensor memory once and keeps it in registers (head size 64), or twice, 32
 // columns at a time in a loop (128: first the max, then the exponentials).  A row in registers unrolls to four times the
 // code, whose fetch shows wherever a CTA walks few tiles: 7 portions of 70 queries, 32 heads of 128: 27.4 us against 25.8,
@@ -115,7 +121,7 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     unsigned char* Qs = base;                                   // [NSUB][128 queries][128 B]
     unsigned char* Kring = Qs + Q_BYTES;                        // [K_STAGES] key tiles, each [NSUB][BN keys][128 B]
     unsigned char* Vring = Kring + K_STAGES * KV_BYTES;         // [V_STAGES] value tiles, the same layout
-    unsigned char* Qs1 = Vring + V_STAGES * KV_BYTES;           // stream 1's queries, or one more value tile (of the same size) where it has none of its own
+    unsigned char* Qs1 = Vring + V_STAGES * KV_BYTES;           // stream 1's queries, or (head size 128) one more value tile where it has none of its own
     uint64_t* bars = reinterpret_cast<uint64_t*>(Qs1 + Q_BYTES);
     uint64_t* q_full = bars;                                    // [2] a stream's query tile has landed
     uint64_t* k_full = q_full + 2;                              // [K_STAGES] a key tile has landed
@@ -155,8 +161,8 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     const int count0 = shared ? (n_tiles + 1) / 2 : n_kept + (qpos0 + BM - k_begin + BN - 1) / BN;      // tiles of stream 0
     const int count1 = shared ? n_tiles / 2 : n_tiles;
     // a value tile's place in its ring, and the parity of its turn there
-    auto v_slot = [&](int j) { return shared ? j % (V_STAGES + 1) : j % V_STAGES; };
-    auto v_turn = [&](int j) { return (uint32_t)(shared ? j / (V_STAGES + 1) : j / V_STAGES) & 1; };
+    auto v_slot = [&](int j) { return shared ? j % value_slots(true) : j % value_slots(false); };
+    auto v_turn = [&](int j) { return (uint32_t)(shared ? j / value_slots(true) : j / value_slots(false)) & 1; };
     auto tile_k0 = [&](int j) { return j < n_kept ? j * BN : k_begin + (j - n_kept) * BN; };
     if (tid == 0) {
         // a tile is free when both streams' products are done; the tiles that stream 0 no longer sees are never waited for
@@ -218,7 +224,7 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         bool ok = true;
         for (int j = 0; j < n_tiles; ++j) {
             const int s = values ? v_slot(j) : j % K_STAGES;
-            if (j >= (values ? V_STAGES + shared : K_STAGES)) ok = warp_wait(empty + s, (values ? v_turn(j) : (j / K_STAGES) & 1) ^ 1);
+            if (j >= (values ? value_slots(shared) : K_STAGES)) ok = warp_wait(empty + s, (values ? v_turn(j) : (j / K_STAGES) & 1) ^ 1);
             if (!ok) break;
             if (lane == 0) mbar_expect_tx(full + s, (uint32_t)KV_BYTES);
             __syncwarp();
@@ -562,6 +568,10 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __g
 
 CISR_EXPORT int cisr_attn_tcgen05_head_dim() { return D; }
 CISR_EXPORT int cisr_attn_tcgen05_tile() { return BM; }
+// The slots of the key ring, or of the value ring for a tile whose streams share their queries or not, and how many warps issue
+// products (one per stream, or one for both): what a check of the rings' turns needs to know.
+CISR_EXPORT int cisr_attn_tcgen05_slots(int values, int shared) { return values ? value_slots(shared != 0) : K_STAGES; }
+CISR_EXPORT int cisr_attn_tcgen05_product_warps() { return OWN_P ? 2 : 1; }
 CISR_EXPORT void cisr_attn_tcgen05_set_pdl(int on) { g_pdl = on != 0; }
 
 // `error_flag`: one zeroed int in device memory that the kernel sets (to 5) when one of its waits ran out.
