@@ -80,6 +80,9 @@ delta_prepare_kernel(const float* __restrict__ proj, int row_stride, const float
 // four rows and the weights for one (2048 tokens of 3072 channels: 49 us by token, 29 so).  q and k pass through shared
 // memory for their norms, v goes straight out.
 constexpr int PREPARE_TOKENS = 4;
+// Shared memory of a launch, the tokens' indices with it: the kernel takes what a CTA has without asking for more, 48 KB.
+constexpr size_t prepare_tile_smem(int qk_channels) { return sizeof(float) * PREPARE_TOKENS * (size_t)qk_channels; }
+constexpr size_t PREPARE_TILE_STATIC = 2 * PREPARE_TOKENS * sizeof(int);
 __global__ void __launch_bounds__(256, 3)
 delta_prepare_tile_kernel(const float* __restrict__ proj, int row_stride, const float* __restrict__ conv_w, const float* __restrict__ state,
                           long long state_stride, long long keep_offset, const float* __restrict__ a_log, const float* __restrict__ dt_bias,
@@ -1050,9 +1053,9 @@ CISR_EXPORT int cisr_delta_prepare(const float* proj, int row_stride, const floa
         configured = smem;
     }
     const int nqk = 2 * kvh * dk;
-    if (tokens > 64 && taps == 4 && channels % 4 == 0 && nqk % 4 == 0 && row_stride % 4 == 0 && sizeof(float) * PREPARE_TOKENS * nqk <= 48 * 1024 &&
+    if (tokens > 64 && taps == 4 && channels % 4 == 0 && nqk % 4 == 0 && row_stride % 4 == 0 && prepare_tile_smem(nqk) + PREPARE_TILE_STATIC <= 48 * 1024 &&
         !(((uintptr_t)proj | (uintptr_t)conv_w | (uintptr_t)qkv) & 15))
-        return launch_kernel(delta_prepare_tile_kernel, dim3((tokens + PREPARE_TOKENS - 1) / PREPARE_TOKENS), dim3(256), sizeof(float) * PREPARE_TOKENS * nqk,
+        return launch_kernel(delta_prepare_tile_kernel, dim3((tokens + PREPARE_TOKENS - 1) / PREPARE_TOKENS), dim3(256), prepare_tile_smem(nqk),
                              (cudaStream_t)stream, g_pdl, proj, row_stride, conv_w, state, state_stride, keep_offset, a_log, dt_bias, token_req,
                              req_slot, q_start, qkv, beta, decay, heads, kvh, dk, dv, norm_eps, tokens);
     const int threads = (tokens <= 64 && channels >= 1024) ? 1024 : 256;      // few tokens (a decode step): a token's channels on more threads
