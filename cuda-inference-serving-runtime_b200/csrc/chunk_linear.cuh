@@ -53,7 +53,7 @@ __device__ __forceinline__ void fetch_tile(RawTile& raw, const float* __restrict
         }
     }
 }
-template <bool SILU, typename W>
+template <bool SILU, bool PLAIN, typename W>
 __device__ __forceinline__ void put_tile(SplitTile& dst, const RawTile& raw, W weight) {
 #pragma unroll
     for (int u = 0; u < PER_THREAD; ++u) {
@@ -61,7 +61,7 @@ __device__ __forceinline__ void put_tile(SplitTile& dst, const RawTile& raw, W w
         float4 v = raw.v[u];
         if (SILU) { v.x = chunk_silu(v.x); v.y = chunk_silu(v.y); v.z = chunk_silu(v.z); v.w = chunk_silu(v.w); }
         const float w = weight(r);
-        split_store4(dst, r, c, make_float4(v.x * w, v.y * w, v.z * w, v.w * w));
+        tile_store4<PLAIN>(dst, r, c, make_float4(v.x * w, v.y * w, v.z * w, v.w * w));
     }
 }
 struct One { __device__ __forceinline__ float operator()(int) const { return 1.f; } };
@@ -114,8 +114,8 @@ __device__ __forceinline__ void put_pair(float* dst, int left, float x, float y)
 }
 
 // q_t . k_i of one chunk and group (n tokens from row token0 on), every pair of tokens
-template <bool VEC, bool SILU>
-__device__ __forceinline__ void chunk_scores(const ChunkArgs& a, int chunk, int grp, int n, size_t token0, SplitTile& Q, SplitTile& K, int m0, int n0w) {
+template <bool VEC, bool SILU, bool PLAIN>
+__device__ __forceinline__ int chunk_scores(const ChunkArgs& a, int chunk, int grp, int n, size_t token0, SplitTile& Q, SplitTile& K, int m0, int n0w) {
     float acc[4][4] = {};
     for (int n0 = 0; n0 < a.N; n0 += CHUNK) {
         const int nc = min(CHUNK, a.N - n0);
@@ -123,25 +123,25 @@ __device__ __forceinline__ void chunk_scores(const ChunkArgs& a, int chunk, int 
         fetch_tile<VEC>(q, a.q + token0 * a.q_stride + grp * a.N + n0, a.q_stride, n, nc);
         fetch_tile<VEC>(k, a.k + token0 * a.k_stride + grp * a.N + n0, a.k_stride, n, nc);
         if (n0) __syncthreads();
-        put_tile<SILU>(Q, q, One());
-        put_tile<SILU>(K, k, One());
+        put_tile<SILU, PLAIN>(Q, q, One());
+        put_tile<SILU, PLAIN>(K, k, One());
         __syncthreads();
-        if (n0w <= m0 + 15) split_product<false, false>(acc, Q, K, m0, n0w, (nc + 15) >> 4);      // pairs with i > t are never read
+        if (n0w <= m0 + 15) tile_product<PLAIN, false, false>(acc, Q, K, m0, n0w, (nc + 15) >> 4);      // pairs with i > t are never read
     }
     float* out = a.scores + ((size_t)chunk * a.groups + grp) * CHUNK * CHUNK;
     for_result(acc, m0, n0w, [&](int t, int i, float x, float y) { *reinterpret_cast<float2*>(out + t * CHUNK + i) = make_float2(x, y); });
+    return not_finite(acc);
 }
 
 // grid (chunk, head, tiles of [N, dv] + 1): the last z makes the scores of the chunk's groups, in the CTAs of the first heads
-template <bool VEC, bool NORM, bool SILU>
-__global__ void __launch_bounds__(CHUNK_THREADS, 3)
-chunk_gains_kernel(const ChunkArgs a) {
+struct GainShared { double L[CHUNK]; float w[CHUNK]; };
+template <bool VEC, bool NORM, bool SILU, bool PLAIN>
+__device__ __forceinline__ int gains_pass(const ChunkArgs& a, GainShared& sh) {
     extern __shared__ __align__(16) unsigned char chunk_smem[];
-    __shared__ double L[CHUNK];
-    __shared__ float w[CHUNK];
+    double* L = sh.L;
+    float* w = sh.w;
     SplitTile& K = reinterpret_cast<SplitTile*>(chunk_smem)[0];
     SplitTile& V = reinterpret_cast<SplitTile*>(chunk_smem)[1];
-    pdl_trigger();
     const int chunk = blockIdx.x, h = blockIdx.y, warp = threadIdx.x >> 5, m0 = 16 * (warp >> 1), n0w = 32 * (warp & 1);
     const bool scores = blockIdx.z == gridDim.z - 1;
     const int row_tiles = (a.N + CHUNK - 1) / CHUNK;
@@ -150,24 +150,23 @@ chunk_gains_kernel(const ChunkArgs a) {
     const int r = a.chunk_req[chunk], t0 = a.chunk_t0[chunk], n = min(CHUNK, a.q_len[r] - t0);
     const int token0 = a.q_start[r] + t0;
     const int nr = min(CHUNK, a.N - n0), nc = min(CHUNK, a.dv - c0);
-    pdl_wait();
+    if (!PLAIN) pdl_wait();
     if (scores) {
-        if (h < a.groups) chunk_scores<VEC, SILU>(a, chunk, h, n, (size_t)token0, K, V, m0, n0w);
-        return;
+        return h < a.groups ? chunk_scores<VEC, SILU, PLAIN>(a, chunk, h, n, (size_t)token0, K, V, m0, n0w) : 0;
     }
     RawTile k, v;
     fetch_tile<VEC>(k, a.k + (size_t)token0 * a.k_stride + grp * a.N + n0, a.k_stride, n, nr);
     fetch_tile<VEC>(v, a.v + (size_t)token0 * a.v_stride + h * a.dv + c0, a.v_stride, n, nc);
     stage_decays(a, h, token0, n, L, w);
-    put_tile<SILU>(K, k, One());
+    put_tile<SILU, PLAIN>(K, k, One());
     __syncthreads();
     if (threadIdx.x < CHUNK) w[threadIdx.x] *= expf((float)(L[CHUNK - 1] - L[threadIdx.x]));
     if (a.chunk_decay && blockIdx.z == 0 && threadIdx.x == 0) a.chunk_decay[(size_t)chunk * a.heads + h] = expf((float)L[CHUNK - 1]);
     __syncthreads();
-    put_tile<SILU>(V, v, [&](int t) { return w[t]; });
+    put_tile<SILU, PLAIN>(V, v, [&](int t) { return w[t]; });
     __syncthreads();
     float acc[4][4] = {};
-    split_product<true, true>(acc, K, V, m0, n0w, (n + 15) >> 4);
+    tile_product<PLAIN, true, true>(acc, K, V, m0, n0w, (n + 15) >> 4);
     const size_t per_head = (size_t)a.N * a.dv + (NORM ? a.N : 0);
     float* out = a.blocks + ((size_t)chunk * a.heads + h) * per_head;
     for_result(acc, m0, n0w, [&](int row, int c, float x, float y) {
@@ -175,22 +174,30 @@ chunk_gains_kernel(const ChunkArgs a) {
     });
     if (NORM && c0 == 0 && (int)threadIdx.x < nr) {
         float sum = 0.f;
-        for (int i = 0; i < n; ++i)
-            sum = fmaf(w[i], to_float(K.part[0][i][threadIdx.x]) + (to_float(K.part[1][i][threadIdx.x]) + to_float(K.part[2][i][threadIdx.x])), sum);
+        for (int i = 0; i < n; ++i) sum = fmaf(w[i], tile_value<PLAIN>(K, i, threadIdx.x), sum);
         out[(size_t)a.N * a.dv + n0 + threadIdx.x] = sum;
     }
+    return not_finite(acc);
+}
+template <bool VEC, bool NORM, bool SILU>
+__device__ __noinline__ void gains_plain(const ChunkArgs& a, GainShared& sh) { gains_pass<VEC, NORM, SILU, true>(a, sh); }
+template <bool VEC, bool NORM, bool SILU>
+__global__ void __launch_bounds__(CHUNK_THREADS, 3)
+chunk_gains_kernel(const __grid_constant__ ChunkArgs a) {
+    __shared__ GainShared sh;
+    pdl_trigger();
+    if (__syncthreads_or(gains_pass<VEC, NORM, SILU, false>(a, sh))) gains_plain<VEC, NORM, SILU>(a, sh);
 }
 
 // grid (chunk, head, 64 value columns): the running product of [q exp(L) | scores with their decays] and [S0 ; v]
-template <bool VEC, bool NORM, bool SILU>
-__global__ void __launch_bounds__(CHUNK_THREADS, 3)
-chunk_reads_kernel(const ChunkArgs a) {
+struct ReadShared { double L[CHUNK]; float gain[CHUNK], carried[CHUNK], nvec[CHUNK]; };
+template <bool VEC, bool NORM, bool SILU, bool PLAIN>
+__device__ __forceinline__ int reads_pass(const ChunkArgs& a, ReadShared& sh) {
     extern __shared__ __align__(16) unsigned char chunk_smem[];
-    __shared__ double L[CHUNK];
-    __shared__ float gain[CHUNK], carried[CHUNK], nvec[CHUNK];
+    double* L = sh.L;
+    float *gain = sh.gain, *carried = sh.carried, *nvec = sh.nvec;
     SplitTile& A = reinterpret_cast<SplitTile*>(chunk_smem)[0];
     SplitTile& B = reinterpret_cast<SplitTile*>(chunk_smem)[1];
-    pdl_trigger();
     const int chunk = blockIdx.x, h = blockIdx.y, c0 = blockIdx.z * CHUNK, tid = threadIdx.x, warp = tid >> 5, m0 = 16 * (warp >> 1), n0w = 32 * (warp & 1);
     const int grp = h / (a.heads / a.groups);
     const int r = a.chunk_req[chunk], t0 = a.chunk_t0[chunk], n = min(CHUNK, a.q_len[r] - t0);
@@ -199,8 +206,8 @@ chunk_reads_kernel(const ChunkArgs a) {
     const float* block = a.blocks + ((size_t)chunk * a.heads + h) * per_head;
     const bool norm_here = NORM && c0 == 0;
     const int nt = tid >> 2, nq = (tid & 3) * 16;             // normaliser: four threads per token, a quarter of a row each
+    if (!PLAIN) pdl_wait();
     float norm = 0.f;
-    pdl_wait();
     stage_decays(a, h, token0, n, L, gain);
     float acc[4][4] = {};
     for (int n0 = 0; n0 < a.N; n0 += CHUNK) {
@@ -209,15 +216,15 @@ chunk_reads_kernel(const ChunkArgs a) {
         fetch_tile<VEC>(q, a.q + (size_t)token0 * a.q_stride + grp * a.N + n0, a.q_stride, n, nr);
         fetch_tile<VEC>(s0, block + (size_t)n0 * a.dv + c0, a.dv, nr, nc);
         if (n0) __syncthreads();
-        put_tile<SILU>(A, q, One());
-        put_tile<false>(B, s0, One());
+        put_tile<SILU, PLAIN>(A, q, One());
+        put_tile<false, PLAIN>(B, s0, One());
         if (norm_here && tid < CHUNK) nvec[tid] = tid < nr ? block[(size_t)a.N * a.dv + n0 + tid] : 0.f;
         __syncthreads();
-        split_product<false, true>(acc, A, B, m0, n0w, (nr + 15) >> 4);
+        tile_product<PLAIN, false, true>(acc, A, B, m0, n0w, (nr + 15) >> 4);
         if (norm_here)
             for (int i = 0; i < 16; i += 8) {
                 float q[8];
-                split_read8(A, nt, nq + i, q);
+                tile_read8<PLAIN>(A, nt, nq + i, q);
 #pragma unroll
                 for (int e = 0; e < 8; ++e) norm = fmaf(q[e], nvec[nq + i + e], norm);
             }
@@ -235,7 +242,7 @@ chunk_reads_kernel(const ChunkArgs a) {
         for (int j = 0; j < 4; ++j) { acc[j][2 * half] *= f; acc[j][2 * half + 1] *= f; }
     }
     norm *= carried[nt];
-    put_tile<SILU>(B, v, One());
+    put_tile<SILU, PLAIN>(B, v, One());
 #pragma unroll
     for (int u = 0; u < PER_THREAD; ++u) {
         const int i4 = tid + u * CHUNK_THREADS, t = i4 >> 4, i = (i4 & 15) * 4;
@@ -246,14 +253,14 @@ chunk_reads_kernel(const ChunkArgs a) {
 #pragma unroll
             for (int e = 0; e < 4; ++e) p[e] = i + e <= t ? sv[e] * gain[i + e] * expf((float)(Lt - L[i + e])) : 0.f;
         }
-        split_store4(A, t, i, make_float4(p[0], p[1], p[2], p[3]));
+        tile_store4<PLAIN>(A, t, i, make_float4(p[0], p[1], p[2], p[3]));
     }
     __syncthreads();
-    split_product<false, true>(acc, A, B, m0, n0w, m0 / 16 + 1);         // P holds nothing right of the diagonal
+    tile_product<PLAIN, false, true, true>(acc, A, B, m0, n0w, m0 / 16 + 1);         // P holds nothing right of the diagonal
     if (norm_here) {
         for (int i = 0; i < 16; i += 8) {
             float p[8];
-            split_read8(A, nt, nq + i, p);
+            tile_read8<PLAIN>(A, nt, nq + i, p);
 #pragma unroll
             for (int e = 0; e < 8; ++e) norm += p[e];
         }
@@ -264,6 +271,16 @@ chunk_reads_kernel(const ChunkArgs a) {
     for_result(acc, m0, n0w, [&](int t, int c, float x, float y) {
         if (t < n) put_pair<VEC>(a.y + ((size_t)(token0 + t) * a.heads + h) * a.dv + c0 + c, nc - c, x * a.q_scale, y * a.q_scale);
     });
+    return not_finite(acc);
+}
+template <bool VEC, bool NORM, bool SILU>
+__device__ __noinline__ void reads_plain(const ChunkArgs& a, ReadShared& sh) { reads_pass<VEC, NORM, SILU, true>(a, sh); }
+template <bool VEC, bool NORM, bool SILU>
+__global__ void __launch_bounds__(CHUNK_THREADS, 3)
+chunk_reads_kernel(const __grid_constant__ ChunkArgs a) {
+    __shared__ ReadShared sh;
+    pdl_trigger();
+    if (__syncthreads_or(reads_pass<VEC, NORM, SILU, false>(a, sh))) reads_plain<VEC, NORM, SILU>(a, sh);
 }
 
 // Whether rows of four floats may be read (and pairs written) as one: widths, strides and addresses that allow it.

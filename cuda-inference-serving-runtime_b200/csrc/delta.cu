@@ -602,20 +602,14 @@ __device__ __forceinline__ void fetch_form(FormTile& raw, const float* __restric
         }
     }
 }
-template <typename W>
+template <bool PLAIN, typename W>
 __device__ __forceinline__ void put_form(SplitTile& dst, const FormTile& raw, W weight) {
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
         const int i = threadIdx.x + u * FORM_THREADS, r = i >> 4, c = (i & 15) * 4;
         const float w = weight(r);
-        split_store4(dst, r, c, make_float4(raw.v[u].x * w, raw.v[u].y * w, raw.v[u].z * w, raw.v[u].w * w));
+        tile_store4<PLAIN>(dst, r, c, make_float4(raw.v[u].x * w, raw.v[u].y * w, raw.v[u].z * w, raw.v[u].w * w));
     }
-}
-__device__ __forceinline__ void split_store2(SplitTile& t, int row, int col, float x, float y) {       // col even
-    uint32_t p[3];
-    split_pair(x, y, p);
-#pragma unroll
-    for (int i = 0; i < 3; ++i) *reinterpret_cast<uint32_t*>(&t.part[i][row][col]) = p[i];
 }
 // a warp's 16 x 32 part of a result, pairs (row, col, col + 1)
 template <typename F>
@@ -666,7 +660,7 @@ __device__ __forceinline__ void invert_unit_lower(float* __restrict__ A, float* 
         for (int i = tid; i < total; i += FORM_THREADS) {
             const int p = i / per_pair, e = i - p * per_pair, r = e / runs, c = 4 * (e - r * runs), base = 2 * half * p;
             float4 y = make_float4(0.f, 0.f, 0.f, 0.f);
-            for (int k = 0; k < half; ++k) {
+            for (int k = 0; k <= r; ++k) {                 // T22 holds nothing right of its diagonal, and a NaN below must not meet it
                 const float a = -T[(base + half + r) * AF_LD + base + half + k];
                 const float4 t = *reinterpret_cast<const float4*>(A + (base + k) * AF_LD + base + half + c);
                 y.x = fmaf(a, t.x, y.x); y.y = fmaf(a, t.y, y.y); y.z = fmaf(a, t.z, y.z); y.w = fmaf(a, t.w, y.w);
@@ -677,26 +671,32 @@ __device__ __forceinline__ void invert_unit_lower(float* __restrict__ A, float* 
     }
 }
 
-template <bool VEC>
-__global__ void __launch_bounds__(FORM_THREADS, 2)
-delta_chunk_forms_kernel(const float* __restrict__ qkv, const float* __restrict__ beta, const float* __restrict__ decay,
-                         const int* __restrict__ chunk_req, const int* __restrict__ chunk_t0, const int* __restrict__ q_start,
-                         const int* __restrict__ q_len, float* __restrict__ scratch, float* __restrict__ out, int heads, int kvh, int dk, int dv) {
+struct FormArgs {
+    const float* qkv; const float* beta; const float* decay; const int* chunk_req; const int* chunk_t0; const int* q_start; const int* q_len;
+    float* scratch; float* out; int heads, kvh, dk, dv;
+};
+struct FormShared { double L[CHUNK]; float bt[CHUNK], ct[CHUNK]; };
+template <bool VEC, bool PLAIN>
+__device__ __forceinline__ int forms_pass(const FormArgs& a, FormShared& sh) {
+    const float *qkv = a.qkv, *beta = a.beta, *decay = a.decay;
+    const int *chunk_req = a.chunk_req, *chunk_t0 = a.chunk_t0, *q_start = a.q_start, *q_len = a.q_len;
+    float *scratch = a.scratch, *out = a.out;
+    const int heads = a.heads, kvh = a.kvh, dk = a.dk, dv = a.dv;
     extern __shared__ __align__(16) unsigned char form_smem[];
-    __shared__ double L[CHUNK];
-    __shared__ float bt[CHUNK], ct[CHUNK];
+    double* L = sh.L;
+    float *bt = sh.bt, *ct = sh.ct;
     SplitTile* tile = reinterpret_cast<SplitTile*>(form_smem);
     float* Af = reinterpret_cast<float*>(tile + 2);        // [64][AF_LD] in the third tile's place, T in the fourth's
     float* Tf = reinterpret_cast<float*>(tile + 3);
     static_assert(CHUNK * AF_LD * sizeof(float) <= sizeof(SplitTile), "");
-    pdl_trigger();
     const int chunk = blockIdx.x, head = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, m0 = 16 * (warp >> 1), n0 = 32 * (warp & 1);
     const int req = chunk_req[chunk], t0 = chunk_t0[chunk], count = min(CHUNK, q_len[req] - t0), first = q_start[req] + t0;
     const int g = head / (heads / kvh), channels = 2 * kvh * dk + heads * dv;
     const float* q = qkv + (size_t)first * channels + g * dk;
     const float* k = q + kvh * dk;
     const float* v = qkv + (size_t)first * channels + 2 * kvh * dk + head * dv;
-    pdl_wait();
+    if (!PLAIN) pdl_wait();
+    int bad = 0;
     FormTile kq, raw;
     fetch_form<VEC>(raw, q, channels, count, dk);
     fetch_form<VEC>(kq, k, channels, count, dk);
@@ -717,15 +717,15 @@ delta_chunk_forms_kernel(const float* __restrict__ qkv, const float* __restrict_
     } else if (tid >= 64 && tid < 128) {
         bt[tid - 64] = tid - 64 < count ? beta[(size_t)(first + tid - 64) * heads + head] : 0.f;
     }
-    put_form(tile[1], raw, [](int) { return 1.f; });
-    put_form(tile[0], kq, [](int) { return 1.f; });
+    put_form<PLAIN>(tile[1], raw, [](int) { return 1.f; });
+    put_form<PLAIN>(tile[0], kq, [](int) { return 1.f; });
     __syncthreads();
     const int k_steps = (dk + 15) >> 4;
     {
         float kk[4][4] = {}, qk[4][4] = {};
         if (n0 <= m0 + 15) {
-            split_product<false, false>(kk, tile[0], tile[0], m0, n0, k_steps);
-            split_product<false, false>(qk, tile[1], tile[0], m0, n0, k_steps);
+            tile_product<PLAIN, false, false>(kk, tile[0], tile[0], m0, n0, k_steps);
+            tile_product<PLAIN, false, false>(qk, tile[1], tile[0], m0, n0, k_steps);
         }
         fetch_form<VEC>(raw, v, channels, count, dv);      // wanted after the inversion
         __syncthreads();                                   // Q has been read: P takes its place
@@ -734,7 +734,7 @@ delta_chunk_forms_kernel(const float* __restrict__ qkv, const float* __restrict_
             *reinterpret_cast<float2*>(Af + t * AF_LD + i) = make_float2(bt[t] * r0 * x, bt[t] * r1 * y);
         });
         for_pairs(qk, m0, n0, [&](int t, int i, float x, float y) {
-            split_store2(tile[1], t, i, i <= t ? expf((float)(L[t] - L[i])) * x : 0.f, i + 1 <= t ? expf((float)(L[t] - L[i + 1])) * y : 0.f);
+            tile_store2<PLAIN>(tile[1], t, i, i <= t ? expf((float)(L[t] - L[i])) * x : 0.f, i + 1 <= t ? expf((float)(L[t] - L[i + 1])) * y : 0.f);
         });
     }
     __syncthreads();
@@ -748,20 +748,20 @@ delta_chunk_forms_kernel(const float* __restrict__ qkv, const float* __restrict_
         }
         __syncthreads();                                   // T has been read: its parts take its place
 #pragma unroll
-        for (int u = 0; u < 4; ++u) { const int i = tid + u * FORM_THREADS; split_store4(tile[3], i >> 4, (i & 15) * 4, t4[u]); }
+        for (int u = 0; u < 4; ++u) { const int i = tid + u * FORM_THREADS; tile_store4<PLAIN>(tile[3], i >> 4, (i & 15) * 4, t4[u]); }
     }
-    put_form(tile[2], raw, [&](int t) { return bt[t]; });
-    put_form(tile[0], kq, [&](int t) { return bt[t] * ct[t]; });
+    put_form<PLAIN>(tile[2], raw, [&](int t) { return bt[t]; });
+    put_form<PLAIN>(tile[0], kq, [&](int t) { return bt[t] * ct[t]; });
     __syncthreads();
     {
         float ub[4][4] = {}, w[4][4] = {};
-        split_product<false, true>(ub, tile[3], tile[2], m0, n0, m0 / 16 + 1);      // T holds nothing right of the diagonal
-        split_product<false, true>(w, tile[3], tile[0], m0, n0, m0 / 16 + 1);
+        tile_product<PLAIN, false, true, true>(ub, tile[3], tile[2], m0, n0, m0 / 16 + 1);      // T holds nothing right of the diagonal
+        tile_product<PLAIN, false, true, true>(w, tile[3], tile[0], m0, n0, m0 / 16 + 1);
         __syncthreads();
-        for_pairs(ub, m0, n0, [&](int t, int c, float x, float y) { split_store2(tile[2], t, c, x, y); });
-        for_pairs(w, m0, n0, [&](int t, int c, float x, float y) { split_store2(tile[3], t, c, x, y); });
+        for_pairs(ub, m0, n0, [&](int t, int c, float x, float y) { tile_store2<PLAIN>(tile[2], t, c, x, y); });
+        for_pairs(w, m0, n0, [&](int t, int c, float x, float y) { tile_store2<PLAIN>(tile[3], t, c, x, y); });
     }
-    put_form(tile[0], kq, [&](int t) { return expf((float)(L[CHUNK - 1] - L[t])); });
+    put_form<PLAIN>(tile[0], kq, [&](int t) { return expf((float)(L[CHUNK - 1] - L[t])); });
     __syncthreads();
     float* forms = scratch + ((size_t)chunk * heads + head) * FORM_FLOATS;
     float* G = forms + FORM_G;
@@ -770,7 +770,7 @@ delta_chunk_forms_kernel(const float* __restrict__ qkv, const float* __restrict_
     const int t_steps = (count + 15) >> 4;
     {
         float acc[4][4] = {};
-        split_product<true, true>(acc, tile[0], tile[3], m0, n0, t_steps);
+        tile_product<PLAIN, true, true>(acc, tile[0], tile[3], m0, n0, t_steps);
         for_pairs(acc, m0, n0, [&](int r, int c, float x, float y) {
             uint32_t p[3];
             split_pair(x, y, p);
@@ -780,12 +780,13 @@ delta_chunk_forms_kernel(const float* __restrict__ qkv, const float* __restrict_
     }
     {
         float acc[4][4] = {};
-        split_product<true, true>(acc, tile[0], tile[2], m0, n0, t_steps);
+        tile_product<PLAIN, true, true>(acc, tile[0], tile[2], m0, n0, t_steps);
         for_pairs(acc, m0, n0, [&](int r, int c, float x, float y) { *reinterpret_cast<float2*>(G + r * CHUNK + c) = make_float2(x, y); });
     }
     {
         float acc[4][4] = {};
-        split_product<false, true>(acc, tile[1], tile[3], m0, n0, m0 / 16 + 1);
+        tile_product<PLAIN, false, true, true>(acc, tile[1], tile[3], m0, n0, m0 / 16 + 1);
+        bad |= not_finite(acc);
         for_pairs(acc, m0, n0, [&](int t, int d, float x, float y) {
             const float q0 = t < count && d < dk ? q[(size_t)t * channels + d] : 0.f, q1 = t < count && d + 1 < dk ? q[(size_t)t * channels + d + 1] : 0.f;
             *reinterpret_cast<float2*>(R + t * CHUNK + d) = make_float2(fmaf(ct[t], q0, -x), fmaf(ct[t], q1, -y));
@@ -793,7 +794,8 @@ delta_chunk_forms_kernel(const float* __restrict__ qkv, const float* __restrict_
     }
     {
         float acc[4][4] = {};
-        split_product<false, true>(acc, tile[1], tile[2], m0, n0, m0 / 16 + 1);
+        tile_product<PLAIN, false, true, true>(acc, tile[1], tile[2], m0, n0, m0 / 16 + 1);
+        bad |= not_finite(acc);
         for_pairs(acc, m0, n0, [&](int t, int c, float x, float y) {
             if (t >= count) return;
             float* dst = out + ((size_t)(first + t) * heads + head) * dv + c;
@@ -801,6 +803,16 @@ delta_chunk_forms_kernel(const float* __restrict__ qkv, const float* __restrict_
             else { if (c < dv) dst[0] = x; if (c + 1 < dv) dst[1] = y; }
         });
     }
+    return bad;
+}
+template <bool VEC>
+__device__ __noinline__ void forms_plain(const FormArgs& a, FormShared& sh) { forms_pass<VEC, true>(a, sh); }
+template <bool VEC>
+__global__ void __launch_bounds__(FORM_THREADS, 2)
+delta_chunk_forms_kernel(const __grid_constant__ FormArgs a) {
+    __shared__ FormShared sh;
+    pdl_trigger();
+    if (__syncthreads_or(forms_pass<VEC, false>(a, sh))) forms_plain<VEC>(a, sh);
 }
 
 constexpr int STATE_COLS = 16, STATE_STAGES = 3, STATE_THREADS = 128;
@@ -913,28 +925,30 @@ delta_chunk_states_kernel(float* __restrict__ scratch, const int* __restrict__ r
         }
 }
 
-template <bool VEC>
-__global__ void __launch_bounds__(FORM_THREADS, 3)
-delta_chunk_reads_kernel(const float* __restrict__ scratch, const int* __restrict__ chunk_req, const int* __restrict__ chunk_t0,
-                         const int* __restrict__ q_start, const int* __restrict__ q_len, float* __restrict__ out, int heads, int dk, int dv) {
+struct ReadArgs {
+    const float* scratch; const int* chunk_req; const int* chunk_t0; const int* q_start; const int* q_len; float* out; int heads, dk, dv;
+};
+// a pass whose sums are not all finite adds nothing to the output: the plain one follows
+template <bool VEC, bool PLAIN>
+__device__ __forceinline__ int form_reads_pass(const ReadArgs& a) {
     extern __shared__ __align__(16) unsigned char form_smem[];
     SplitTile* tile = reinterpret_cast<SplitTile*>(form_smem);
-    pdl_trigger();
-    const int chunk = blockIdx.x, head = blockIdx.y, warp = threadIdx.x >> 5, m0 = 16 * (warp >> 1), n0 = 32 * (warp & 1);
-    const int req = chunk_req[chunk], t0 = chunk_t0[chunk], count = min(CHUNK, q_len[req] - t0), first = q_start[req] + t0;
-    const float* S0 = scratch + ((size_t)chunk * heads + head) * FORM_FLOATS + FORM_G;
-    pdl_wait();
+    const int chunk = blockIdx.x, head = blockIdx.y, warp = threadIdx.x >> 5, m0 = 16 * (warp >> 1), n0 = 32 * (warp & 1), dv = a.dv;
+    const int req = a.chunk_req[chunk], t0 = a.chunk_t0[chunk], count = min(CHUNK, a.q_len[req] - t0), first = a.q_start[req] + t0;
+    const float* S0 = a.scratch + ((size_t)chunk * a.heads + head) * FORM_FLOATS + FORM_G;
+    if (!PLAIN) pdl_wait();
     FormTile s, r;
     fetch_form<true>(s, S0, CHUNK, CHUNK, CHUNK);
     fetch_form<true>(r, S0 + CHUNK * CHUNK, CHUNK, CHUNK, CHUNK);
-    put_form(tile[0], r, [](int) { return 1.f; });
-    put_form(tile[1], s, [](int) { return 1.f; });
+    put_form<PLAIN>(tile[0], r, [](int) { return 1.f; });
+    put_form<PLAIN>(tile[1], s, [](int) { return 1.f; });
     __syncthreads();
     float acc[4][4] = {};
-    split_product<false, true>(acc, tile[0], tile[1], m0, n0, (dk + 15) >> 4);
+    tile_product<PLAIN, false, true>(acc, tile[0], tile[1], m0, n0, (a.dk + 15) >> 4);
+    if (!PLAIN && __syncthreads_or(not_finite(acc))) return 1;
     for_pairs(acc, m0, n0, [&](int t, int c, float x, float y) {
         if (t >= count) return;
-        float* dst = out + ((size_t)(first + t) * heads + head) * dv + c;
+        float* dst = a.out + ((size_t)(first + t) * a.heads + head) * dv + c;
         if (VEC) {
             if (c < dv) { const float2 o = *reinterpret_cast<float2*>(dst); *reinterpret_cast<float2*>(dst) = make_float2(o.x + x, o.y + y); }
         } else {
@@ -942,6 +956,15 @@ delta_chunk_reads_kernel(const float* __restrict__ scratch, const int* __restric
             if (c + 1 < dv) dst[1] += y;
         }
     });
+    return 0;
+}
+template <bool VEC>
+__device__ __noinline__ void form_reads_plain(const ReadArgs& a) { form_reads_pass<VEC, true>(a); }
+template <bool VEC>
+__global__ void __launch_bounds__(FORM_THREADS, 3)
+delta_chunk_reads_kernel(const __grid_constant__ ReadArgs a) {
+    pdl_trigger();
+    if (form_reads_pass<VEC, false>(a)) form_reads_plain<VEC>(a);
 }
 
 template <bool VEC>
@@ -956,14 +979,14 @@ int launch_forms(const float* qkv, const float* beta, const float* decay, const 
         if (e != cudaSuccess) return (int)e;
         configured = true;
     }
-    int st = launch_kernel(delta_chunk_forms_kernel<VEC>, dim3(n_chunks, heads), dim3(FORM_THREADS), FORMS_SMEM, s, g_pdl, qkv, beta, decay, chunk_req,
-                           chunk_t0, q_start, q_len, scratch, out, heads, kvh, dk, dv);
+    int st = launch_kernel(delta_chunk_forms_kernel<VEC>, dim3(n_chunks, heads), dim3(FORM_THREADS), FORMS_SMEM, s, g_pdl,
+                           FormArgs{qkv, beta, decay, chunk_req, chunk_t0, q_start, q_len, scratch, out, heads, kvh, dk, dv});
     if (st) return st;
     st = launch_kernel(delta_chunk_states_kernel, dim3(n_req, heads, (dv + STATE_COLS - 1) / STATE_COLS), dim3(STATE_THREADS), STATES_SMEM, s, g_pdl, scratch,
                        req_chunk0, state, state_stride, req_slot, q_len, heads, dk, dv, least);
     if (st) return st;
-    return launch_kernel(delta_chunk_reads_kernel<VEC>, dim3(n_chunks, heads), dim3(FORM_THREADS), 2 * sizeof(SplitTile), s, g_pdl, (const float*)scratch,
-                         chunk_req, chunk_t0, q_start, q_len, out, heads, dk, dv);
+    return launch_kernel(delta_chunk_reads_kernel<VEC>, dim3(n_chunks, heads), dim3(FORM_THREADS), 2 * sizeof(SplitTile), s, g_pdl,
+                         ReadArgs{scratch, chunk_req, chunk_t0, q_start, q_len, out, heads, dk, dv});
 }
 
 // The same where a head's values come in runs of four: LANES lanes share a (token, head), each with its runs, so a warp has

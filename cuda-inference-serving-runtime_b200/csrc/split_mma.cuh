@@ -2,8 +2,15 @@
 //
 // A float is three bfloat16: x = b0 + b1 + b2 with b0 = x rounded, b1 = (x - b0) rounded, b2 the rest.  Both subtractions
 // are exact and 3 x 8 bits hold a float's 24, so nothing of x is lost (but below about 2^-110, where the parts run out of
-// exponents, and at values that round to a bfloat16 infinity, whose rest is NaN).  Of the nine products of parts the six
-// largest are taken; what is left out is 2^-24 of the product and less, a float's own rounding.
+// exponents).  Of the nine products of parts the six largest are taken; what is left out is 2^-24 of the product and less, a
+// float's own rounding.  The split of a float into bfloat16 parts for products is Henry, Tang and Heinecke's ("Leveraging the
+// bfloat16 artificial intelligence datatype for higher-precision computations", 2019).
+//
+// Infinities, NaN and floats that round to a bfloat16 infinity have NaN among their parts, and zeros times those reach results
+// that hold nothing of the number.  Every result that such a number touches is NaN, so a kernel looks at its sums at the end
+// (not_finite) and, where any thread of the CTA has found one, makes its pass once more with PLAIN tiles and products: these
+// hold a float's bits and use float multiply-adds.  That pass is a function of its own, never inlined: the registers of the
+// usual one stay as they are.
 //
 // The float recurrences use it for their chunk products, which on the CUDA cores ran at a fifth of the multiply-add rate:
 // a thread's 8 x 4 tile there loads twelve 16-byte words per 128 multiply-adds and waits for them.  Measured on a B200: this
@@ -29,15 +36,41 @@ __device__ __forceinline__ void split_pair(float x, float y, uint32_t (&p)[3]) {
     x -= __uint_as_float(p[1] << 16); y -= __uint_as_float(p[1] & 0xffff0000u);
     p[2] = bf16_pair(x, y);
 }
-__device__ __forceinline__ void split_store4(SplitTile& t, int row, int col, float4 v) {       // col a multiple of 4
+// PLAIN: the upper and the lower halves of the floats' bits in the first two parts, zeros in the third
+template <bool PLAIN>
+__device__ __forceinline__ void tile_pair(float x, float y, uint32_t (&p)[3]) {
+    if (!PLAIN) return split_pair(x, y, p);
+    const uint32_t a = __float_as_uint(x), b = __float_as_uint(y);
+    p[0] = (a >> 16) | (b & 0xffff0000u); p[1] = (a & 0xffffu) | (b << 16); p[2] = 0u;
+}
+template <bool PLAIN>
+__device__ __forceinline__ void tile_store2(SplitTile& t, int row, int col, float x, float y) {       // col even
+    uint32_t p[3];
+    tile_pair<PLAIN>(x, y, p);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) *reinterpret_cast<uint32_t*>(&t.part[i][row][col]) = p[i];
+}
+template <bool PLAIN>
+__device__ __forceinline__ void tile_store4(SplitTile& t, int row, int col, float4 v) {       // col a multiple of 4
     uint32_t a[3], b[3];
-    split_pair(v.x, v.y, a);
-    split_pair(v.z, v.w, b);
+    tile_pair<PLAIN>(v.x, v.y, a);
+    tile_pair<PLAIN>(v.z, v.w, b);
 #pragma unroll
     for (int i = 0; i < 3; ++i) *reinterpret_cast<uint2*>(&t.part[i][row][col]) = make_uint2(a[i], b[i]);
 }
+template <bool PLAIN>
+__device__ __forceinline__ float tile_value(const SplitTile& t, int row, int col) {
+    if (PLAIN) return __uint_as_float(((uint32_t)__bfloat16_as_ushort(t.part[0][row][col]) << 16) | __bfloat16_as_ushort(t.part[1][row][col]));
+    return to_float(t.part[0][row][col]) + (to_float(t.part[1][row][col]) + to_float(t.part[2][row][col]));
+}
 // eight neighbouring floats of a tile's row put together again (col a multiple of 8)
-__device__ __forceinline__ void split_read8(const SplitTile& t, int row, int col, float (&v)[8]) {
+template <bool PLAIN>
+__device__ __forceinline__ void tile_read8(const SplitTile& t, int row, int col, float (&v)[8]) {
+    if (PLAIN) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] = tile_value<true>(t, row, col + j);
+        return;
+    }
 #pragma unroll
     for (int j = 0; j < 8; ++j) v[j] = 0.f;
 #pragma unroll
@@ -92,5 +125,40 @@ __device__ __forceinline__ void split_product(float (&acc)[4][4], const SplitTil
 #pragma unroll
             for (int e = 0; e < 4; ++e) acc[j][e] += t[j][e];
     }
+}
+
+// The same elements from tiles that hold floats, by multiply-adds in the order of k.  LOWER: A holds nothing right of its
+// diagonal, and what B has there is left out.
+template <bool A_KM, bool B_KN, bool LOWER>
+__device__ __forceinline__ void plain_product(float (&acc)[4][4], const SplitTile& A, const SplitTile& B, int m0, int n0, int steps) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+        const int m = m0 + 8 * half + (lane >> 2), last = LOWER ? min(16 * steps - 1, m) : 16 * steps - 1;
+#pragma unroll 1
+        for (int k = 0; k <= last; ++k) {
+            const float a = A_KM ? tile_value<true>(A, k, m) : tile_value<true>(A, m, k);
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const int n = n0 + 8 * j + 2 * (lane & 3) + e;
+                    acc[j][2 * half + e] = fmaf(a, B_KN ? tile_value<true>(B, k, n) : tile_value<true>(B, n, k), acc[j][2 * half + e]);
+                }
+        }
+    }
+}
+template <bool PLAIN, bool A_KM, bool B_KN, bool LOWER = false>
+__device__ __forceinline__ void tile_product(float (&acc)[4][4], const SplitTile& A, const SplitTile& B, int m0, int n0, int steps) {
+    if (PLAIN) plain_product<A_KM, B_KN, LOWER>(acc, A, B, m0, n0, steps);
+    else split_product<A_KM, B_KN>(acc, A, B, m0, n0, steps);
+}
+__device__ __forceinline__ int not_finite(const float (&acc)[4][4]) {
+    float z = 0.f;                        // 0 x finite is 0, else NaN, and a NaN stays
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) z = fmaf(acc[j][e], 0.f, z);
+    return z != 0.f;
 }
 }  // namespace
