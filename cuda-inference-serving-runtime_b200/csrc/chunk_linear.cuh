@@ -73,7 +73,8 @@ __device__ __forceinline__ void stage_decays(const ChunkArgs& a, int h, int toke
     if (threadIdx.x < 32) {
         const int t = 2 * threadIdx.x;
         if (a.decay) {
-            const double lg = log((double)a.decay[h]);
+            // a decay of zero: a logarithm whose differences are 0 for a token itself and give a factor of 0 before it
+            const double lg = a.decay[h] == 0.f ? -1e5 : log((double)a.decay[h]);
             L[t] = lg * min(t + 1, n);
             L[t + 1] = lg * min(t + 2, n);
         } else {

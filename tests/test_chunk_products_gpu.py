@@ -185,3 +185,9 @@ def test_delta_non_finite_values_reach_later_tokens_only(at):
     kernels.delta_chunks(qkv, beta, decay, req, t0, n_chunks, first, state, i32([0]), i32(starts), i32([T]), o, 1, heads, heads, dk, dv, 64)
     same_where_finite(o, torch.stack(want))
     same_where_finite(state, S.reshape(1, -1))
+
+
+def test_lightning_decay_of_zero():
+    """Each token alone: o = (q . k) v, also where a decay is too small for a float."""
+    for got, want in zip(*lightning_case([64, 130], 40, 24, 3, torch.tensor([0.0, 1e-46, 0.9], device="cuda"), lambda proj, state: None)):
+        same_where_finite(got, want)
