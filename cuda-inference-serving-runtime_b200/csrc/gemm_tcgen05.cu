@@ -46,6 +46,19 @@ struct Epilogue {                       // what the epilogue variants need beyon
     // rows [g * n, (g + 1) * n) of `w`.  Null: one weight matrix for all rows.
     const int* tile_group;
 };
+// n / d for d >= 1 (or NaN), rounded from a quotient in double: the reciprocal's approximation (some 20 bits, of double's range)
+// after a step of Newton's iteration.  Of 2.7e8 gates and denominators 186 differ from the division operator, by one place.
+// For epilogues that nothing runs beside: a thread has up to 256 quotients, and with the operator, which may branch, each waited for
+// the one before.  us, gated products of one round of tiles with the operator and so: 200 rows of 28672 x 4096 90 and 72,
+// of 16384 x 2048 49 and 33, of 3072 x 576 14 and 10.  Beside another tile's products the operator is the better one (2048 rows of
+// 28672 x 4096: 304 and 368; double costs power that the tensor cores want).
+__device__ __forceinline__ float quotient(float n, float d) {
+    const double dd = d;
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(dd));
+    const double e = d < INFINITY ? fma(-dd, r, 1.0) : 0.0;              // an infinite d has the reciprocal 0
+    return (float)((double)n * fma(r, e, r));
+}
 // 32 floats -> 32 bfloat16 (64 bytes) at dst; `count` of them are valid
 __device__ __forceinline__ void store_bf16x32(bf16* dst, const float (&v)[32], int count) {
     if (count >= 32 && ((uintptr_t)dst & 15) == 0) {
@@ -94,7 +107,8 @@ __device__ __forceinline__ void unit_columns(const Epilogue& ep, int unit, int& 
 // (feature); load(column, v) gives 32 columns of the row's sums (called by whole warps).
 // `pos`, `page` (ROPE): the row's position and the cache page it is written to, looked up by the caller while the tile
 // was still being accumulated (-1: a padding row, or a row beyond the step).
-template <int BN, int EPI, typename Load>
+// ALONE: nothing runs beside this epilogue.
+template <int BN, int EPI, bool ALONE, typename Load>
 __device__ __forceinline__ void epilogue_tile(const Epilogue& ep, Load load, int u0, int u1, int row, int m, int n, int n0, int pos, int page) {
 #pragma unroll 1
     for (int unit = u0; unit < u1; ++unit) {
@@ -142,19 +156,17 @@ __device__ __forceinline__ void epilogue_tile(const Epilogue& ep, Load load, int
             }
             if (row < m && n0 + lo_col < n) store_bf16x32(ep.out_bf16 + (size_t)row * n + n0 + lo_col, act, n - (n0 + lo_col));
         } else if (paired_rows(EPI)) {
-            // The divisions go without the ordinary one's second path (2^-22 and less, beside the 2^-9 that act is rounded to):
-            // with it the 64 quotients of a thread ran one after the other, 10 us of a launch of few rows.  Denominators above
-            // 2^126 give 0, where the quotient is at most 2^-119.
             uint32_t u[32];
             load(hi_col, u);
             float act[32];
+            const auto over = [](float a, float b) { return ALONE ? quotient(a, b) : a / b; };
             if (EPI == EPI_GATED) {
                 // the clamped gated activation of stacked gate and up rows, as bfloat16 [m, inter]
                 const float limit = ep.limit, alpha = ep.alpha;
 #pragma unroll
                 for (int j = 0; j < 32; ++j) {
                     const float gv = fminf(__uint_as_float(v[j]), limit), uv = fminf(fmaxf(__uint_as_float(u[j]), -limit), limit);
-                    act[j] = __fdividef(gv, 1.f + expf(-alpha * gv)) * (uv + 1.f);
+                    act[j] = over(gv, 1.f + expf(-alpha * gv)) * (uv + 1.f);
                 }
             } else {
                 // silu(z) = z / (1 + exp(-z)) and gelu(z) = z / (1 + exp(-2 sqrt(2 / pi) (z + 0.044715 z^3))) differ in the exponent only
@@ -162,7 +174,7 @@ __device__ __forceinline__ void epilogue_tile(const Epilogue& ep, Load load, int
 #pragma unroll
                 for (int j = 0; j < 32; ++j) {
                     const float gv = __uint_as_float(v[j]);
-                    act[j] = __fdividef(gv, 1.f + expf(-lin * (gv + cub * gv * gv * gv))) * __uint_as_float(u[j]);
+                    act[j] = over(gv, 1.f + expf(-lin * (gv + cub * gv * gv * gv))) * __uint_as_float(u[j]);
                 }
             }
             if (row < m && n0 + lo_col < ep.inter)
@@ -350,7 +362,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             if (!ok) break;
             tcgen05_fence_after();
             const uint32_t lane_base = tmem_base + (uint32_t)(acc * BN) + ((uint32_t)(quarter * 32) << 16);
-            epilogue_tile<BN, EPI>(ep, [&](int c, uint32_t (&v)[32]) { tmem_load32(lane_base + (uint32_t)c, v); }, 0, epilogue_units<BN, EPI>(), row, m, n, n0, pos, page);
+            epilogue_tile<BN, EPI, false>(ep, [&](int c, uint32_t (&v)[32]) { tmem_load32(lane_base + (uint32_t)c, v); }, 0, epilogue_units<BN, EPI>(), row, m, n, n0, pos, page);
             tcgen05_fence_before();
             __syncwarp();
             if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(acc_empty + acc)) : "memory");
@@ -541,7 +553,7 @@ gemm_tcgen05_split_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
             ok = mbar_wait(inbox_full, 0) && ok;
             if (__all_sync(0xffffffffu, ok)) {
                 const float* next = inbox + row_in;                            // loads come in the order unit, side
-                epilogue_tile<BN, EPI>(ep, [&](int c, uint32_t (&v)[32]) {
+                epilogue_tile<BN, EPI, true>(ep, [&](int c, uint32_t (&v)[32]) {
                     const float* from = next;
                     next += 32 * BM;
 #pragma unroll
@@ -568,7 +580,7 @@ gemm_tcgen05_split_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
 #pragma unroll
         for (int t = 0; t < MT; ++t) {
             const uint32_t lane_base = tmem_base + lanes + (uint32_t)(t * BN);
-            epilogue_tile<BN, EPI>(ep, [&](int c, uint32_t (&v)[32]) { tmem_load32(lane_base + (uint32_t)c, v); }, 0, UNITS,
+            epilogue_tile<BN, EPI, true>(ep, [&](int c, uint32_t (&v)[32]) { tmem_load32(lane_base + (uint32_t)c, v); }, 0, UNITS,
                                    m0 + t * BM + quarter * 32 + lane, m, n, n0, pos[t], page[t]);
         }
     }

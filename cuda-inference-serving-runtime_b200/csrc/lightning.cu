@@ -229,9 +229,6 @@ __global__ void lightning_output_kernel(const float* __restrict__ o, const float
 // The same, four columns an access and the row and its gates in registers, all requested before the sum: bound by memory (2048
 // tokens of 2048: 42 MB, 6.4 us), where single columns asked for one float a thread and the gates only after the sum:
 // 18.4 us, now 10.5.
-// The sigmoid's division without the ordinary one's second path where the result is rounded to bfloat16 (2^-22 beside 2^-9).
-template <typename CT> __device__ __forceinline__ float sigmoid_of(float g) { return 1.f / (1.f + expf(-g)); }
-template <> __device__ __forceinline__ float sigmoid_of<__nv_bfloat16>(float g) { return __fdividef(1.f, 1.f + expf(-g)); }
 __device__ __forceinline__ void store4(float* to, const float (&v)[4]) { *reinterpret_cast<float4*>(to) = make_float4(v[0], v[1], v[2], v[3]); }
 __device__ __forceinline__ void store4(__nv_bfloat16* to, const float (&v)[4]) {
     __nv_bfloat162 pair[2] = {__floats2bfloat162_rn(v[0], v[1]), __floats2bfloat162_rn(v[2], v[3])};
@@ -269,7 +266,7 @@ lightning_output_runs_kernel(const float* __restrict__ o, const float* __restric
         const float4 w = *reinterpret_cast<const float4*>(norm_w + j);
         const float ww[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
-        for (int e = 0; e < 4; ++e) v[r][e] = v[r][e] * unit * ww[e] * sigmoid_of<CT>(g[r][e]);
+        for (int e = 0; e < 4; ++e) v[r][e] = v[r][e] * unit * ww[e] * (1.f / (1.f + expf(-g[r][e])));
         store4(out + t * out_stride + j, v[r]);
     }
 }

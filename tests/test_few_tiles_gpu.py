@@ -70,3 +70,23 @@ def test_rotated(m, hq, hkv, dim, kk):
     for got, want in ((q, turned[:, :hq]), *((cache.transpose(1, 2).reshape(-1, hkv, dim)[order.long()], turned[:, at:at + hkv])
                                              for cache, at in zip(caches, (hq, hq + hkv)))):
         assert ((got.double() - want).abs() <= 1e-3 + 2 ** -8 * want.abs()).all()
+
+
+@pytest.mark.parametrize("gate,x,up", [("silu", -88.0, 1e30), ("silu", -87.5, 1e30), ("gelu_tanh", -10.0, 1e30), ("gated_clamp", -51.75, 3.0)])
+def test_quotients_of_large_denominators(gate, x, up):
+    """1 + exp(.) above 2^126: the gate is small and not zero."""
+    from cisr_b200.ops import kernels
+    m, inter, kk = 130, 200, 64
+    a, w = torch.zeros(m, kk, device="cuda", dtype=torch.bfloat16), torch.zeros(2 * inter, kk, device="cuda", dtype=torch.bfloat16)
+    a[:, 0] = 1
+    w[:inter, 0], w[inter:, 0] = x, up
+    z, u = (torch.tensor(v).bfloat16().double() for v in (x, up))
+    if gate == "gelu_tanh":
+        want = z / (1 + torch.exp(-2 * 0.7978845608028654 * (z + 0.044715 * z ** 3))) * u
+    else:
+        want = z * torch.sigmoid(1.702 * z) * (u + 1) if gate == "gated_clamp" else z * torch.sigmoid(z) * u
+    out = torch.full((m, inter), float("nan"), device="cuda", dtype=torch.bfloat16)
+    kernels.gemm_tcgen05_swiglu(a, w, out, gate, 7.0 if gate == "gated_clamp" else None)
+    kernels.raise_if_kernel_gave_up()
+    # the exponential carries a few 2^-24 of its argument of 88 (1e-4 with room), the result bfloat16's rounding of eight bits, 2^-8
+    assert ((out.double() - want).abs() <= (2 ** -8 + 1e-4) * want.abs()).all()

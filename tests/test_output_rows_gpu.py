@@ -36,3 +36,23 @@ def test_heads(out_dtype, tokens, heads, dv):
     o = y.double().view(tokens, heads, dv) / (torch.maximum(yn.double().abs(), torch.exp(-m.double())) + 1e-6)[..., None]
     want = gated((o * torch.rsqrt((o ** 2).mean(-1, keepdim=True) + 1e-3)).view(tokens, -1), gate[:, 4:4 + heads * dv], w)
     assert ((out.double() - want).abs() <= TOLERANCE[out_dtype] * want.abs() + 1e-30).all()
+
+
+@pytest.mark.parametrize("out_dtype", [torch.float32, torch.bfloat16])
+def test_gates_of_large_denominators(out_dtype):
+    """1 + exp(-gate) above 2^126: the gate is small and not zero."""
+    from cisr_b200.ops import kernels
+    tokens, heads, dv = 3, 4, 128
+    width = heads * dv
+    (o,) = drawn(1, (tokens, width))
+    gate, w = torch.full((tokens, width), -88.0, device="cuda"), torch.full((width,), 1e30, device="cuda")
+    out = torch.empty(tokens, width, dtype=out_dtype, device="cuda")
+    kernels.lightning_output(o, gate, 0, w, 1e-5, out)
+    want = gated(o.double() * torch.rsqrt((o.double() ** 2).mean(-1, keepdim=True) + 1e-5), gate, w)
+    tolerance = TOLERANCE[out_dtype] + 1e-5                              # and 2^-24 of the exponent 88
+    assert ((out.double() - want).abs() <= tolerance * want.abs()).all()
+    yn, m = torch.full((tokens, heads), 2.0, device="cuda"), torch.zeros(tokens, heads, device="cuda")
+    kernels.exp_output(o.view(tokens, heads, dv), yn, m, gate, 0, w, 1e-5, out)
+    v = o.double().view(tokens, heads, dv) / (2 + 1e-6)
+    want = gated((v * torch.rsqrt((v ** 2).mean(-1, keepdim=True) + 1e-5)).view(tokens, width), gate, w)
+    assert ((out.double() - want).abs() <= tolerance * want.abs()).all()
