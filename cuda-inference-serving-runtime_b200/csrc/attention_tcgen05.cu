@@ -159,7 +159,11 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     const int n_kept = (window > 0 && keep_first > 0) ? min((keep_first + BN - 1) / BN, k_begin / BN) : 0;
     const int n_tiles = n_kept + (k_end - k_begin + BN - 1) / BN;
     const int count0 = shared ? (n_tiles + 1) / 2 : n_kept + (qpos0 + BM - k_begin + BN - 1) / BN;      // tiles of stream 0
-    const int count1 = shared ? n_tiles / 2 : n_tiles;
+    // Stream 1's window begins one tile later, unless both begin with the sequence's first key: the tile that the window of
+    // stream 0 begins in is none of stream 1's, which lets it go unread.
+    const bool passes = !shared && window > 0 && qpos0 - window + 1 >= 0 && keep_first <= k_begin;
+    const int count1 = shared ? n_tiles / 2 : n_tiles - passes;
+    auto tile_of = [&](int stream, int i) { return shared ? 2 * i + stream : i + (stream && passes && i >= n_kept); };
     // a value tile's place in its ring, and the parity of its turn there
     auto v_slot = [&](int j) { return shared ? j % value_slots(true) : j % value_slots(false); };
     auto v_turn = [&](int j) { return (uint32_t)(shared ? j / value_slots(true) : j / value_slots(false)) & 1; };
@@ -262,9 +266,16 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         const bool clean_last = tile_k0(n_tiles - 1) + BN > k_end;
         // descriptor addresses count 16 bytes; every tile lies below 256 KB, so the sums stay inside the field
         const uint64_t desc_q0 = umma_desc(Qs), desc_q1 = umma_desc(Qs1), desc_k0 = umma_desc(Kring), desc_v0 = umma_desc_mn_major(Vring, KV_SUB);
-        auto tile_of = [&](int stream, int i) { return shared ? 2 * i + stream : i; };
+        // a tile that stream 1 passes over: once it has landed (its slot's turn has come) it is free as far as stream 1 goes
+        auto pass_over = [&](uint64_t* full, uint64_t* empty, int slot, uint32_t turn) -> bool {
+            if (!warp_wait(full + slot, turn)) return false;
+            if (lane == 0) mbar_arrive(empty + slot);
+            __syncwarp();
+            return true;
+        };
         // S = Q K(j)^T of a stream's i-th tile
         auto score_product = [&](int stream, int i) -> bool {
+            if (stream && passes && i == n_kept && !pass_over(k_full, k_empty, n_kept % K_STAGES, (n_kept / K_STAGES) & 1)) return false;
             const int j = tile_of(stream, i), s = j % K_STAGES;
             if (!warp_wait(k_full + s, (j / K_STAGES) & 1)) return false;
             tcgen05_fence_after();
@@ -279,6 +290,7 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         };
         // O += P V(j), half a tile's keys at a time, as their P arrives
         auto output_product = [&](int stream, int i) -> bool {
+            if (stream && passes && i == n_kept && !pass_over(v_full, v_empty, v_slot(n_kept), v_turn(n_kept))) return false;
             const int j = tile_of(stream, i), s = v_slot(j);
             if (!warp_wait(v_full + s, v_turn(j))) return false;
             if (clean_last && j == n_tiles - 1 && !warp_wait(v_clean, 0)) return false;
@@ -336,7 +348,7 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         float m_used = bounded ? 0.f : -INFINITY, l = 0.f;
         bool ok = true;
         for (int i = 0; i < count; ++i) {
-            const int kt = tile_k0(shared ? 2 * i + stream : i);    // the tile's first key
+            const int kt = tile_k0(tile_of(stream, i));             // the tile's first key
             ok = warp_wait(s_full + stream, i & 1);
             if (!ok) break;
             tcgen05_fence_after();

@@ -27,8 +27,9 @@ def plain(q, k, v, window, keep_first, sink, cap):
     return out
 
 
-def run(portions, d, hq, hkv, span, window=0, keep_first=0, sink=None, cap=None, sharp=1.0):
-    """portions: (queries, keys before them) per request; cache rows that no request wrote hold NaN."""
+def run(portions, d, hq, hkv, span, window=0, keep_first=0, sink=None, cap=None, sharp=1.0, spoiled=None):
+    """portions: (queries, keys before them) per request; cache rows that no request wrote hold NaN, and so does the first
+    request's key `spoiled`."""
     from cisr_b200.ops import kernels
     g = torch.Generator().manual_seed(7 + d + len(portions))
     pages = sum(-(-(n + b) // PAGE) for n, b in portions) + 2
@@ -47,6 +48,9 @@ def run(portions, d, hq, hkv, span, window=0, keep_first=0, sink=None, cap=None,
             rows = min(PAGE, total - i * PAGE)
             k_cache[page, :, :rows] = k[i * PAGE:i * PAGE + rows].transpose(0, 1)
             v_cache[page, :, :rows] = v[i * PAGE:i * PAGE + rows].transpose(0, 1)
+        if spoiled is not None and r == 0:
+            for cache in (k_cache, v_cache):
+                cache[table[0, spoiled // PAGE], :, spoiled % PAGE] = float("nan")
         qs.append(q)
         want.append(plain(q.double(), k.double(), v.double(), window, keep_first, sink, cap))
     dev = lambda a: torch.as_tensor(np.asarray(a, dtype=np.int32), device="cuda")
@@ -91,3 +95,18 @@ def test_bent_scores(cap, span):
 @pytest.mark.parametrize("d", [64, 128])
 def test_a_max_that_moves_rescales_the_rows_before_it(d, span):
     check(*run([(256, 512), (90, 900)], d, 2, 2, span, sharp=12.0))
+
+
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("keep_first", [0, 5, 128, 150, 300])
+@pytest.mark.parametrize("n,before,window", [(256, 300, 128), (200, 300, 100), (512, 40, 128), (300, 700, 257), (256, 127, 128), (256, 128, 130)])
+def test_windows_of_both_streams(d, keep_first, n, before, window):
+    check(*run([(n, before)], d, 2, 1, 256, window=window, keep_first=keep_first))
+
+
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("key", [173, 200, 255])
+def test_a_key_before_the_second_streams_window_does_not_reach_it(d, key):
+    """Queries 428 to 555 see keys from 301 on; the tile of keys 128 to 255 belongs to the queries before them."""
+    out, want = run([(256, 300)], d, 2, 1, 256, window=128, spoiled=key)
+    check(out[128:], want[128:])
