@@ -160,14 +160,14 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     const int n_tiles = n_kept + (k_end - k_begin + BN - 1) / BN;
     const int count0 = shared ? (n_tiles + 1) / 2 : n_kept + (qpos0 + BM - k_begin + BN - 1) / BN;      // tiles of stream 0
     // Stream 1's window begins one tile later, unless both begin with the sequence's first key: the tile that the window of
-    // stream 0 begins in is none of stream 1's, which lets it go unread.
-    const bool passes = !shared && window > 0 && qpos0 - window + 1 >= 0 && keep_first <= k_begin;
+    // stream 0 begins in is none of stream 1's, which lets it go unread.  It comes first then, before the kept keys' tiles.
+    const int passes = !shared && window > 0 && qpos0 - window + 1 >= 0 && keep_first <= k_begin;
     const int count1 = shared ? n_tiles / 2 : n_tiles - passes;
-    auto tile_of = [&](int stream, int i) { return shared ? 2 * i + stream : i + (stream && passes && i >= n_kept); };
+    auto tile_of = [&](int stream, int i) { return shared ? 2 * i + stream : i + (stream & passes); };
     // a value tile's place in its ring, and the parity of its turn there
     auto v_slot = [&](int j) { return shared ? j % value_slots(true) : j % value_slots(false); };
     auto v_turn = [&](int j) { return (uint32_t)(shared ? j / value_slots(true) : j / value_slots(false)) & 1; };
-    auto tile_k0 = [&](int j) { return j < n_kept ? j * BN : k_begin + (j - n_kept) * BN; };
+    auto tile_k0 = [&](int j) { return j < n_kept + passes && j >= passes ? (j - passes) * BN : k_begin + (j < passes ? 0 : j - n_kept) * BN; };
     if (tid == 0) {
         // a tile is free when both streams' products are done; the tiles that stream 0 no longer sees are never waited for
         for (int s = 0; s < K_STAGES; ++s) { mbar_init(k_full + s, 1); mbar_init(k_empty + s, shared ? 1 : 2); }
@@ -266,16 +266,16 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         const bool clean_last = tile_k0(n_tiles - 1) + BN > k_end;
         // descriptor addresses count 16 bytes; every tile lies below 256 KB, so the sums stay inside the field
         const uint64_t desc_q0 = umma_desc(Qs), desc_q1 = umma_desc(Qs1), desc_k0 = umma_desc(Kring), desc_v0 = umma_desc_mn_major(Vring, KV_SUB);
-        // a tile that stream 1 passes over: once it has landed (its slot's turn has come) it is free as far as stream 1 goes
-        auto pass_over = [&](uint64_t* full, uint64_t* empty, int slot, uint32_t turn) -> bool {
-            if (!warp_wait(full + slot, turn)) return false;
-            if (lane == 0) mbar_arrive(empty + slot);
+        // the first tile, where stream 1 passes it over: once it has landed it is free as far as stream 1 goes
+        auto pass_over = [&](uint64_t* full, uint64_t* empty) -> bool {
+            if (!passes) return true;
+            if (!warp_wait(full, 0)) return false;
+            if (lane == 0) mbar_arrive(empty);
             __syncwarp();
             return true;
         };
         // S = Q K(j)^T of a stream's i-th tile
         auto score_product = [&](int stream, int i) -> bool {
-            if (stream && passes && i == n_kept && !pass_over(k_full, k_empty, n_kept % K_STAGES, (n_kept / K_STAGES) & 1)) return false;
             const int j = tile_of(stream, i), s = j % K_STAGES;
             if (!warp_wait(k_full + s, (j / K_STAGES) & 1)) return false;
             tcgen05_fence_after();
@@ -290,7 +290,6 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         };
         // O += P V(j), half a tile's keys at a time, as their P arrives
         auto output_product = [&](int stream, int i) -> bool {
-            if (stream && passes && i == n_kept && !pass_over(v_full, v_empty, v_slot(n_kept), v_turn(n_kept))) return false;
             const int j = tile_of(stream, i), s = v_slot(j);
             if (!warp_wait(v_full + s, v_turn(j))) return false;
             if (clean_last && j == n_tiles - 1 && !warp_wait(v_clean, 0)) return false;
@@ -311,7 +310,10 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         if (OWN_P) {
             // a warp per stream
             const int stream = warp >> 1, count = stream ? count1 : count0;
-            bool ok = count > 0 && warp_wait(q_full + (shared ? 0 : stream), 0) && score_product(stream, 0);
+            bool ok = count > 0 && warp_wait(q_full + (shared ? 0 : stream), 0);
+            if (stream) ok = ok && pass_over(k_full, k_empty);
+            ok = ok && score_product(stream, 0);
+            if (stream) ok = ok && pass_over(v_full, v_empty);
             for (int i = 0; i < count && ok; ++i) {
                 if (i + 1 < count) ok = warp_wait(s_free + stream, i & 1) && score_product(stream, i + 1);
                 ok = ok && output_product(stream, i);
@@ -321,7 +323,7 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __g
             // warp each the streams fell into step: 188 us against 164 for 4096 queries of 32 heads).  Products run in the
             // order they are issued, so a stream's next scores are written over its P after it was read.
             bool ok = warp_wait(q_full, 0) && score_product(0, 0);
-            if (ok && count1 > 0) ok = (shared || warp_wait(q_full + 1, 0)) && score_product(1, 0);
+            if (ok && count1 > 0) ok = (shared || warp_wait(q_full + 1, 0)) && pass_over(k_full, k_empty) && score_product(1, 0) && pass_over(v_full, v_empty);
             for (int i = 0; i < max(count0, count1) && ok; ++i)
                 for (int stream = 0; stream < 2 && ok; ++stream) {
                     const int count = stream ? count1 : count0;
