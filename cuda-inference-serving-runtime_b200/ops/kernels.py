@@ -70,6 +70,18 @@ def _need(t: torch.Tensor, dtype, name: str, dims: Optional[int] = None) -> None
         raise KernelError(f"{name} must have {dims} dimensions, got shape {tuple(t.shape)}")
 
 
+_sm_counts = {}
+
+
+def sm_count(device) -> int:
+    """Streaming multiprocessors of a CUDA device."""
+    index = torch.device(device).index
+    index = torch.cuda.current_device() if index is None else index
+    if index not in _sm_counts:
+        _sm_counts[index] = torch.cuda.get_device_properties(index).multi_processor_count
+    return _sm_counts[index]
+
+
 # ------------------------------------------------------------------ elementwise library
 def _elementwise():
     lib = load_library("elementwise.cu")

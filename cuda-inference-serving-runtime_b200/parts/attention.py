@@ -7,7 +7,7 @@ by construction).  q_proj, k_proj and v_proj are stacked into one matrix at load
 """
 from __future__ import annotations
 
-from typing import Dict
+from typing import Dict, Optional
 
 import numpy as np
 import torch
@@ -121,7 +121,7 @@ class GQAAttention(Mixer):
         out = torch.empty((tokens, hq, dim), dtype=self.dtype, device=device)
         plan = ctx.plan_for(self)
         if plan.info["n_tiles"] and kernels.attn_prefill_wide_ok(q, cache.k, cache.page_size):
-            tiles, span = wide_tiles(plan, hq)
+            tiles, span = wide_tiles(plan, ctx, hq, self.window)
             kernels.attn_prefill_wide(q, out, cache.k, cache.v, ctx.req_slot, cache.block_table, *tiles, ctx.q_start, ctx.q_len,
                                       ctx.ctx_len, hq, hkv, cache.page_size, self.scale, self.window, span=span)
         elif plan.info["n_tiles"]:
@@ -160,16 +160,55 @@ def decode_ranges(longest_context: int) -> int:
     return n
 
 
-WIDE_CTAS = 148            # CTAs of the tcgen05 prompt attention that run at once: one per SM
+# The tcgen05 prompt attention runs a CTA per tile and head and one CTA per SM.  In units of a key tile's time in a CTA of 128
+# queries that has the chip to itself: a CTA's start and end; a key tile in a CTA of more than 128 queries; a key tile in CTAs of
+# 128 queries while all SMs are busy (they copy every key tile for half as many queries, and their last round is less even).
+WIDE_START, WIDE_PAIR_COST, WIDE_BUSY_COST = 3.0, 1.5, 1.3
 
 
-def wide_tiles(plan, heads: int) -> tuple:
-    """The tile list for the tcgen05 prompt attention, and its queries per tile.  A CTA does most work per copy with 256
-    queries; where CTAs of 128 all run at once, twice as many of half the length end sooner (2048 queries, 9 heads of 64: 26
-    us against 36; 300 queries, 32 heads of 128: 14.5 against 15.6; 512 CTAs of 128 queries: 72 against 57)."""
-    if plan.info["n_wide"] * heads <= WIDE_CTAS:
-        return (plan["wide_req"], plan["wide_q0"]), kernels.WIDE_TILE
-    return (plan["pair_req"], plan["pair_q0"]), kernels.WIDE_PAIR
+def wide_span(q_len, ctx_len, heads: int, window: Optional[int], keep_first: int, sms: int) -> int:
+    """How many queries a tile of the tcgen05 prompt attention has, 128 or 256, for portions of `q_len` tokens that end at
+    `ctx_len`: the form whose estimate is shorter, and an estimate is the longest CTA or all CTAs' work over the SMs,
+    whichever is more.  Tiles of 256 do most work per copy; those of 128 are twice as many CTAs of two thirds the length, which
+    ends sooner while the longest CTA sets the time.  us with 128 and 256 (in brackets: the kernel whose tiles had 128 queries and
+    one stream): 2176 tokens, 9 heads of 64 31 and 37 (33), 4096 55 and 62 (79), 6144 106 and 89 (136); 2560 tokens, 8 heads of 128
+    41 and 55 (41); 1000 tokens behind 2000, 16 heads of 128 46 and 66 (48); 2048 tokens, 32 heads of 128 74 and 57 (88).  The
+    three constants were fitted to 190 such steps of 6 kinds of layers: none comes out slower than that kernel, and the sum is
+    0.5 % above the better form's of each."""
+    best = None
+    for span, cost, busy in ((kernels.WIDE_TILE, 1.0, WIDE_BUSY_COST), (kernels.WIDE_PAIR, WIDE_PAIR_COST, 1.0)):
+        longest = total = 0.0
+        ctas = 0
+        for n, end in zip(q_len, ctx_len):
+            if n <= 1:
+                continue
+            reach = (window + keep_first + span) if window else end          # most keys that a tile sees
+            full, rest = divmod(n, span)
+            if rest:                                                         # the last tile; up to 128 queries share both streams
+                c = (cost if rest > kernels.WIDE_TILE else 1.0) * min(end, reach)
+                longest, total = max(longest, c), total + c
+            if full:
+                first, last = end - n + span, end - rest
+                ramp = min(full, max(0, -(-(reach - first) // span)))        # tiles that see fewer than `reach`
+                total += cost * ((full - ramp) * reach + ramp * (first + min(last, first + (ramp - 1) * span)) / 2)
+                longest = max(longest, cost * min(last, reach))
+            ctas += full + (rest > 0)
+        estimate = max(WIDE_START + longest / 128, busy * (WIDE_START * ctas + total / 128) * heads / sms)
+        if best is None or estimate < best[0]:
+            best = (estimate, span)
+    return best[1]
+
+
+def wide_tiles(plan, ctx, heads: int, window: Optional[int], keep_first: int = 0) -> tuple:
+    """The tile list for the tcgen05 prompt attention, and its queries per tile (`wide_span`, once per step and kind of layer).
+    Either list serves any contexts, so a captured step stays right when it is replayed with others."""
+    key = ("wide_span", heads, window, keep_first)
+    span = ctx.shared.get(key)
+    if span is None:
+        span = ctx.shared[key] = wide_span(ctx.host.q_len, ctx.host.ctx_len, heads, window, keep_first, kernels.sm_count(ctx.device))
+    if span == kernels.WIDE_TILE:
+        return (plan["wide_req"], plan["wide_q0"]), span
+    return (plan["pair_req"], plan["pair_q0"]), span
 
 
 ATTENTION_PLAN_KEY = ("paged_attention", kernels.PREFILL_TILE, kernels.WIDE_TILE, DECODE_RANGE)
@@ -183,7 +222,7 @@ def attention_step_plan(host):
     the paged attention kernels shares this plan (`ATTENTION_PLAN_KEY`)."""
     from ..engine.batch import StepPlan
 
-    tile_req, tile_q0, wide_req, wide_q0, pair_req, pair_q0, dec_req = [], [], [], [], [], [], []
+    tile_req, tile_q0, wide_req, wide_q0, pairs, small, dec_req = [], [], [], [], [], [], []
     longest = 0
     for r, n in enumerate(host.q_len):
         if n == 1:
@@ -197,10 +236,11 @@ def attention_step_plan(host):
                 wide_req.append(r)
                 wide_q0.append(q0)
             for q0 in reversed(range(0, n, kernels.WIDE_PAIR)):
-                pair_req.append(r)
-                pair_q0.append(q0)
+                # 128 queries or fewer take half the time of more: such tiles go last
+                (pairs if n - q0 > kernels.WIDE_TILE else small).append((r, q0))
     if dec_req and host.ctx_bound:
         longest = max(longest, host.ctx_bound)
+    pair_req, pair_q0 = [r for r, _ in pairs + small], [q0 for _, q0 in pairs + small]
     as_i32 = lambda values: np.asarray(values, dtype=np.int32)
     return StepPlan(
         arrays={"tile_req": as_i32(tile_req), "tile_q0": as_i32(tile_q0), "wide_req": as_i32(wide_req),
@@ -219,7 +259,7 @@ def paged_attention(plan, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, cac
     tokens, _, dim = q.shape
     out = torch.empty_like(q)
     if plan.info["n_tiles"] and kernels.attn_prefill_wide_ok(q, k, cache.page_size):
-        tiles, span = wide_tiles(plan, hq)
+        tiles, span = wide_tiles(plan, ctx, hq, window, keep_first)
         kernels.attn_prefill_wide(q, out, k, v, ctx.req_slot, cache.block_table, *tiles, ctx.q_start, ctx.q_len, ctx.ctx_len, hq, hkv,
                                   cache.page_size, scale, window, sink=sink, keep_first=keep_first, softcap=softcap, span=span)
     elif plan.info["n_tiles"]:

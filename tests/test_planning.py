@@ -100,3 +100,24 @@ def test_which_tokens_counts_take_the_tcgen05_product():
     assert not k.tcgen05_ok(torch.zeros(256, 60, dtype=torch.bfloat16), w[:, :60])     # rows that are no multiple of 16 bytes
     assert k.tcgen05_rope_ok(64, 32, False) and k.tcgen05_rope_ok(128, 64, False)
     assert not k.tcgen05_rope_ok(64, 16, False) and not k.tcgen05_rope_ok(64, 32, True) and not k.tcgen05_rope_ok(48, 24, False)
+
+
+@pytest.mark.parametrize("heads,window,portions,span", [
+    # measured (us, 128 / 256 queries per tile): the form with 256 is the longer one although its CTAs do not all run at once
+    (9, None, [(2176, 0)], 128), (9, None, [(4096, 0)], 128),                                        # 31 / 37, 55 / 62
+    (8, None, [(2560, 0)], 128), (8, None, [(3072, 0)], 128),                                        # 41 / 55, 47 / 64
+    (8, None, [(256, 2000), (700, 0), (1300, 300)], 128), (16, None, [(1000, 2000)], 128),            # 39 / 53, 46 / 66
+    (9, None, [(2048, 0)], 128), (32, None, [(512, 3584)], 128), (32, None, [(300, 0)], 128),        # 29 / 38, 47 / 64, 14.5 / 15.6
+    # and the shorter one
+    (9, None, [(6144, 0)], 256), (16, None, [(4096, 0)], 256), (32, None, [(2048, 0)], 256),         # 106 / 89, 88 / 66, 57 / 43
+    (32, None, [(4096, 0)], 256), (32, None, [(130, 4000)] * 4, 256), (32, 128, [(4096, 0)], 256),   # 159 / 121, 91 / 71, 62 / 58
+    (32, None, [(1, 5000)] * 60 + [(700, 300)] * 4, 256)])                                           # single tokens have no tiles
+def test_queries_per_tile_of_the_prompt_attention(heads, window, portions, span):
+    from cisr_b200.parts.attention import wide_span
+    q_len, ctx_len = [n for n, _ in portions], [n + before for n, before in portions]
+    assert wide_span(q_len, ctx_len, heads, window, 0, 148) == span
+
+
+def test_queries_per_tile_follow_the_device():
+    from cisr_b200.parts.attention import wide_span
+    assert wide_span([2048], [2048], 12, None, 0, 296) == 128 and wide_span([4096], [4096], 12, None, 0, 37) == 256
