@@ -655,14 +655,19 @@ int launch_split(const void* a, const void* w, const Epilogue& ep, int m, int n,
 //   rows 63 and 56; gated 3584 x 4096, 1024 rows 45 and 28.
 // - more rows or columns: the persistent kernel, whose epilogues run beside the next tile's products (2048 x 2048, 2048 rows: 19
 //   us; 24 here).
+// A plain product of at most 64 columns (a router's few outputs) is a column of row tiles of its own kind: a long K is cut in two
+// where the tiles leave room for it; a short one, or more row tiles, go to the persistent kernel with tiles of 64 columns.
 struct SplitChoice { int bn, mt, shares; };
-SplitChoice split_choice(int m, int cols64, int k, int max64, int max128) {
-    static int sms = 0, on = -1;
-    if (!sms) { int device = 0; cudaGetDevice(&device); cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device); }
+SplitChoice split_choice(int m, int cols64, int k, int max64, int max128, int sms) {
+    static int on = -1;
     if (on < 0) { const char* e = getenv("CISR_GEMM_DEEP"); on = !(e && e[0] == '0'); }
     const int blocks = (k + BK - 1) / BK, cols128 = (cols64 + 1) / 2;
     const long long tiles_m = (m + BM - 1) / BM, tiles64 = tiles_m * cols64, tiles128 = tiles_m * cols128;
     if (!on) return {0, 0, 0};
+    if (cols64 == 1 && max64 >= 2) {
+        if (k >= 32 * BK && 2 * tiles64 <= sms) return {64, 1, 2};
+        return {0, 0, 0};
+    }
     if (max64 && blocks <= 32 && tiles64 <= sms) return {64, 1, max64 >= 2 && blocks >= 24 && 2 * tiles64 <= sms ? 2 : 1};
     if (tiles128 <= sms) {
         int shares = 1;
@@ -672,6 +677,11 @@ SplitChoice split_choice(int m, int cols64, int k, int max64, int max128) {
     if (tiles_m * ((cols128 + 1) / 2) <= sms) return {256, 1, 1};
     if (tiles_m == 2 && (cols128 + 1) / 2 <= sms) return {256, 2, 1};
     return {0, 0, 0};
+}
+SplitChoice split_choice(int m, int cols64, int k, int max64, int max128) {
+    static int sms = 0;
+    if (!sms) { int device = 0; cudaGetDevice(&device); cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device); }
+    return split_choice(m, cols64, k, max64, max128, sms);
 }
 template <int EPI>
 int launch_split_choice(SplitChoice c, const void* a, const void* w, const Epilogue& ep, int m, int n, int k, cudaStream_t s) {
@@ -694,6 +704,13 @@ CISR_EXPORT int cisr_gemm_tcgen05_init(int* error_flag) {
 
 CISR_EXPORT void cisr_gemm_tcgen05_set_pdl(int on) { g_pdl = on != 0; }
 
+// How the plain product of these sizes is made on a device of `sms` SMs: 0 by the persistent kernel, else the columns of a tile x 100
+// + its row tiles x 10 + the shares of K.
+CISR_EXPORT int cisr_gemm_tcgen05_plain_choice(int m, int n, int k, int sms) {
+    const SplitChoice c = split_choice(m, (n + 63) / 64, k, 2, 4, sms);
+    return c.bn * 100 + c.mt * 10 + c.shares;
+}
+
 // How many tensor maps the library remembers before it empties its cache (tests lower it to force evictions).
 CISR_EXPORT void cisr_gemm_tcgen05_set_map_cache_limit(int entries) { g_map_cache_limit = entries < 1 ? 1 : (size_t)entries; }
 
@@ -710,13 +727,8 @@ CISR_EXPORT int cisr_gemm_tcgen05(const void* a, const void* w, float* out, int 
     Epilogue ep = {};
     ep.out_f32 = out; ep.accumulate = accumulate != 0; ep.out_mult = out_mult == 1.f ? 0.f : out_mult;
     cudaStream_t s = (cudaStream_t)stream;
-    if (n <= 64) {
-        // a router's few outputs: a column of row tiles, K cut in two where it is long (uncut, 16 CTAs wait for all of K one after another)
-        const int shares = k >= 2048 && (m + BM - 1) / BM <= 74 ? 2 : 1;
-        if (shares == 2) return launch_split<64, 1, 8, EPI_PLAIN>(a, w, ep, m, n, k, 2, s);
-        return launch<64, 8, EPI_PLAIN>(a, w, ep, m, n, k, 1, s);
-    }
     if (const SplitChoice c = split_choice(m, (n + 63) / 64, k, 2, 4); c.mt) return launch_split_choice<EPI_PLAIN>(c, a, w, ep, m, n, k, s);
+    if (n <= 64) return launch<64, 8, EPI_PLAIN>(a, w, ep, m, n, k, 1, s);
     if (wide_tiles(m, (n + 255) / 256)) return launch<256, 4, EPI_PLAIN>(a, w, ep, m, n, k, (n + 255) / 256, s);
     return launch<128, 3, EPI_PLAIN>(a, w, ep, m, n, k, (n + 127) / 128, s);
 }
