@@ -1158,11 +1158,12 @@ CISR_EXPORT int cisr_delta_recurrence(const float* qkv, const float* beta, const
 }
 
 CISR_EXPORT int cisr_delta_chunk_tokens() { return CHUNK; }
-CISR_EXPORT long long cisr_delta_chunk_table_floats() { return FORM_FLOATS; }        // enough for either form's scratch
+// Floats of scratch per (chunk, head) for heads of these sizes: the forms, or the tables T and P and the decays of the wider heads' walk.
+CISR_EXPORT long long cisr_delta_chunk_table_floats(int dk, int dv) { return dk <= CHUNK && dv <= CHUNK ? FORM_FLOATS : 2 * CHUNK * CHUNK + CHUNK; }
 
 // The recurrence for the requests of the step that bring at least `least` tokens, chunk by chunk.  chunk_req / chunk_t0:
 // per chunk its request and first token inside the portion; req_chunk0: per request the index of its first chunk (requests
-// below `least` have none); tables: float scratch [n_chunks][heads][cisr_delta_chunk_table_floats()].
+// below `least` have none); tables: float scratch [n_chunks][heads][cisr_delta_chunk_table_floats(dk, dv)].
 CISR_EXPORT int cisr_delta_chunks(const float* qkv, const float* beta, const float* decay, const int* chunk_req, const int* chunk_t0,
                                   int n_chunks, const int* req_chunk0, float* tables, float* state, long long state_stride,
                                   const int* req_slot, const int* q_start, const int* q_len, float* out, int heads, int kvh, int dk,

@@ -892,7 +892,6 @@ def bias_add(out: torch.Tensor, bias: torch.Tensor) -> torch.Tensor:
 _delta_state = {}
 DELTA_MAX_KEY_DIM = 256
 DELTA_CHUNK = 64                                       # tokens per chunk of the chunked recurrence
-DELTA_CHUNK_TABLE = 7 * DELTA_CHUNK * DELTA_CHUNK // 2 + 4       # floats of scratch per (chunk, head)
 
 
 def _delta():
@@ -904,7 +903,6 @@ def _delta():
             getattr(lib, name).restype = ctypes.c_int
         lib.cisr_delta_chunk_table_floats.restype = ctypes.c_longlong
         assert lib.cisr_delta_max_key_dim() == DELTA_MAX_KEY_DIM and lib.cisr_delta_chunk_tokens() == DELTA_CHUNK
-        assert lib.cisr_delta_chunk_table_floats() == DELTA_CHUNK_TABLE
         lib.cisr_delta_set_pdl(int(_pdl_state["on"]))
         _delta_state["lib"] = lib
     return lib
@@ -939,7 +937,7 @@ def delta_chunks(qkv, beta, decay, chunk_req, chunk_t0, n_chunks, req_chunk0, st
         _need(t, torch.int32, name, 1)
     if chunk_req.numel() < n_chunks or chunk_t0.numel() < n_chunks or req_chunk0.numel() < n_req:
         raise KernelError("delta_chunks: the chunk lists are too short")
-    tables = torch.empty((n_chunks, heads, DELTA_CHUNK_TABLE), dtype=torch.float32, device=qkv.device)
+    tables = torch.empty((n_chunks, heads, _delta().cisr_delta_chunk_table_floats(key_dim, value_dim)), dtype=torch.float32, device=qkv.device)
     _check(_delta().cisr_delta_chunks(_p(qkv), _p(beta), _p(decay), _p(chunk_req), _p(chunk_t0), n_chunks, _p(req_chunk0), _p(tables),
                                       _p(state), ctypes.c_longlong(state.shape[1]), _p(req_slot), _p(q_start), _p(q_len), _p(o), heads,
                                       kv_heads, key_dim, value_dim, n_req, int(least), _stream()), "delta_chunks",
