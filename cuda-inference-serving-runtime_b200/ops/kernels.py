@@ -1887,6 +1887,13 @@ def _at(t: Optional[torch.Tensor]) -> int:
     return 0 if t is None else t.data_ptr()
 
 
+def _skinny_call(*values) -> bytes:
+    try:
+        return _SKINNY_CALL.pack(*values)
+    except struct.error as err:          # a number that is missing, or beyond what the kernels take
+        raise KernelError(f"skinny_gemm: {err}") from err
+
+
 def skinny_gemm(w: torch.Tensor, tokens: int, *, act: Optional[torch.Tensor] = None, x: Optional[torch.Tensor] = None,
                 delta: Optional[torch.Tensor] = None, norm_w: Optional[torch.Tensor] = None, eps: float = 0.0,
                 x_out: Optional[torch.Tensor] = None, rows: Optional[torch.Tensor] = None, epilogue: int = EPI_PLAIN,
@@ -1943,7 +1950,7 @@ def skinny_gemm(w: torch.Tensor, tokens: int, *, act: Optional[torch.Tensor] = N
             _need(r["cos"], torch.float32, "cos", 2); _need(r["sin"], torch.float32, "sin", 2)
     gate_act, _ = _gate(gate, gate_limit)
     get = r.get
-    args = _SKINNY_CALL.pack(
+    args = _skinny_call(
         w.data_ptr(), _at(act), _at(x), _at(delta), _at(norm_w), _at(x_out), _at(rows), _at(out_f32), _at(out_b16), _at(get("cos")),
         _at(get("sin")), _at(get("q_out")), _at(get("k_cache")), _at(get("v_cache")), _at(get("positions")), _at(get("token_req")),
         _at(get("req_slot")), _at(get("block_table")), _stream().value or 0, eps, out_mult, gate_limit or 0.0, n, k,
