@@ -208,10 +208,6 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     };
     auto warp_wait = [&](uint64_t* bar, uint32_t parity) { return (bool)__all_sync(0xffffffffu, wait(bar, parity)); };
 
-#ifdef REGS
-    if (warp < FIRST_SOFTMAX_WARP) asm volatile("setmaxnreg.dec.sync.aligned.u32 80;");
-    else asm volatile("setmaxnreg.inc.sync.aligned.u32 208;");
-#endif
     if (warp == 0 || warp == 2) {
         // ------------------------------------------------------------ producers: warp 0 the queries and the keys, warp 2 the values
         const bool values = warp == 2;

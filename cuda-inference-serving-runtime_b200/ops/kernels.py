@@ -1027,14 +1027,14 @@ def lightning_jobs():
 
 def lightning_recurrence(proj: torch.Tensor, q_col: int, k_col: int, v_col: int, decay: torch.Tensor, state: torch.Tensor,
                          req_slot: torch.Tensor, q_start: torch.Tensor, q_len: torch.Tensor, n_req: int, o: torch.Tensor, heads: int,
-                         key_dim: int, value_dim: int, least: int = 0, n_short: int = 0, chunks=None, columns_per_cta: int = 0) -> torch.Tensor:
+                         key_dim: int, value_dim: int, least: int = 0, n_short: int = 0, chunks=None) -> torch.Tensor:
     """Per head S <- decay S + silu(k) silu(v)^T, o = S^T silu(q) over each request's tokens in order.  proj float
     [tokens, columns] holds the projections' sums (q and k: heads x key_dim from `q_col` / `k_col`; v: heads x value_dim
     from `v_col`); state float [slots, heads * value_dim * key_dim] is read and advanced; o float [tokens, heads *
     value_dim].  `least` > 0 with `chunks` = (chunk_req, chunk_t0, req_chunk0, n_chunks): the requests that bring at least
     that many tokens run chunk by chunk (per chunk of LIGHTNING_CHUNK tokens its request and its first token inside the
     portion, per request the index of its first chunk: int32 on the device), the `n_short` others token by token; 0: all
-    token by token.  `columns_per_cta` is accepted and changes nothing: a CTA of the chunked form takes 64 value columns."""
+    token by token."""
     _need(proj, torch.float32, "proj", 2); _need(decay, torch.float32, "decay", 1); _need(state, torch.float32, "state", 2)
     _need(o, torch.float32, "o", 2)
     for name, t in (("req_slot", req_slot), ("q_start", q_start), ("q_len", q_len)):

@@ -85,9 +85,9 @@ def dev(a):
 
 
 # ------------------------------------------------------------------ each mechanism alone: kernels
-@pytest.mark.parametrize("heads, dk, dv, columns", [(3, 20, 12, 0), (2, 64, 64, 16), (1, 10, 7, 0), (2, 100, 40, 32), (1, 160, 24, 0),
-                                                    (2, 32, 128, 64), (1, 256, 16, 0)])
-def test_recurrence_token_by_token_and_chunk_by_chunk(heads, dk, dv, columns):
+@pytest.mark.parametrize("heads, dk, dv", [(3, 20, 12), (2, 64, 64), (1, 10, 7), (2, 100, 40), (1, 160, 24), (2, 32, 128), (1, 256, 16),
+                                           (1, 32, 63), (1, 32, 65), (1, 32, 132)])          # a CTA takes 64 value columns
+def test_recurrence_token_by_token_and_chunk_by_chunk(heads, dk, dv):
     """Two requests in portions of every kind (one token, a few, a whole chunk, several chunks with a tail), rows of a step
     not in slot order, slots that held another request's state before, both forms side by side in one step: read-outs
     and the state left behind against the plain recurrence in float64."""
@@ -126,8 +126,7 @@ def test_recurrence_token_by_token_and_chunk_by_chunk(heads, dk, dv, columns):
         o = torch.full((proj.shape[0], nv), 7.0, device="cuda")
         kernels.lightning_recurrence(proj, 0, nqk, 2 * nqk, decay.cuda(), state, dev([slot[r] for r in batch]), dev(q_start), dev(sizes),
                                      len(batch), o, heads, dk, dv, least=kernels.LIGHTNING_CHUNK if chunk_req else 0, n_short=n_short,
-                                     chunks=(dev(chunk_req), dev(chunk_t0), dev(req_chunk0), len(chunk_req)) if chunk_req else None,
-                                     columns_per_cta=columns)
+                                     chunks=(dev(chunk_req), dev(chunk_t0), dev(req_chunk0), len(chunk_req)) if chunk_req else None)
         for i, (r, n) in enumerate(zip(batch, sizes)):
             got[r].append(o[q_start[i]:q_start[i] + n].double().cpu())
             at[r] += n
