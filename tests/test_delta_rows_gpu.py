@@ -47,3 +47,22 @@ def test_prepare(heads, kvh, dk, dv, taps, lens):
     assert ((beta.double() - want_beta).abs() <= 1e-6 * want_beta).all()
     # an exponential carries the error of its argument
     assert ((decay.double() - want_decay).abs() <= 1e-6 * (2 - want_decay.log()) * want_decay + 1e-37).all()
+
+
+# 8, 16 and 32 lanes share a (token, head), also where its values do not fill them; other widths and strides go to the older kernel
+@pytest.mark.parametrize("out_dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("tokens,heads,dv,gate_col,pad", [(1, 1, 4, 0, 0), (5, 3, 20, 4, 8), (33, 2, 32, 0, 0), (7, 5, 36, 8, 4), (9, 2, 64, 4, 0), (3, 3, 100, 0, 4),
+                                                           (17, 2, 128, 4, 0), (3, 2, 132, 4, 0), (4, 2, 33, 4, 0), (4, 2, 64, 2, 0), (4, 2, 64, 4, 2)])
+def test_output(out_dtype, tokens, heads, dv, gate_col, pad):
+    from cisr_b200.ops import kernels
+    g = torch.Generator(device="cuda").manual_seed(tokens + dv)
+    rand = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    o, proj, w = rand(tokens, heads, dv), rand(tokens, gate_col + heads * dv + 12 - gate_col % 4), rand(dv)
+    out = torch.full((tokens, heads * dv + pad), 5.0, dtype=out_dtype, device="cuda")
+    kernels.delta_output(o, proj, gate_col, w, 1e-5, out, heads, dv)
+    gate = proj[:, gate_col:gate_col + heads * dv].double().view(tokens, heads, dv)
+    unit = o.double() * torch.rsqrt((o.double() ** 2).mean(-1, keepdim=True) + 1e-5)
+    want = (unit * w.double() * gate * torch.sigmoid(gate)).view(tokens, -1)
+    # some twenty roundings of 2^-24; bfloat16's 2^-8 on top
+    tolerance = 3e-6 + (2 ** -8 if out_dtype == torch.bfloat16 else 0.0)
+    assert ((out[:, :heads * dv].double() - want).abs() <= tolerance * want.abs() + 1e-30).all() and (out[:, heads * dv:] == 5.0).all()
