@@ -4,22 +4,24 @@
 // a decay in (0, 1):
 //     S <- decay * S;   u = beta * (v - S^T k);   S <- S + k u^T;   o = S^T q          (o reads this token's write)
 //
-// Three kernels around the step's one stacked projection proj [T, cols] = h W^T (float):
-//   delta_prepare    per token: the short causal convolution over time of the q, k and v channels (taps weights per
+// Kernels around the step's one stacked projection proj [T, cols] = h W^T (float):
+//   delta_prepare    per token (many tokens and four taps: four tokens per CTA, delta_prepare_tile): the short causal convolution over time of the q, k and v channels (taps weights per
 //                    channel, the last one the current token's; inputs before the portion come from the request's
 //                    kept inputs, zeros before the sequence), silu, unit norm of q and k per head
 //                    (x / sqrt(sum x^2 + norm_eps), q times key_dim^-1/2), beta = sigmoid(.), and
 //                    decay = exp(-exp(A_log) * softplus(a + dt_bias)).
 //   delta_keep       per request: the last taps - 1 convolution inputs become the request's kept inputs.
-//   delta_recurrence per (request, head, a few value columns): one warp walks the portion's tokens in order.  A column of
+//   delta_recurrence single tokens and short portions, per (request, head, a few value columns): one warp walks the tokens in order.  A column of
 //                    S evolves on its own, so 4 to 32 lanes share a column (each holds its share of the rows in
 //                    registers) and the two dot products are finished by shuffles.  The tokens' operands are staged
 //                    through shared memory a block of tokens ahead.
+//   portions of 64 tokens and more go chunk by chunk, CHUNK tokens at a time: heads of up to 64 x 64 by delta_chunk_forms, _states and
+//                    _reads (the chunks as affine maps of the state, made at once), wider ones by delta_chunk_tables and _walk.
 //   delta_output     per (token, head): o / sqrt(mean(o^2) + eps) * norm_w * silu(gate), rounded to the operand type of
 //                    the output projection.
 // A request's row of the state tensor holds [heads][key_dim][value_dim] and then [taps - 1][conv channels], all float.
-// A portion of a prompt and a single decoded token take the same path, so a position's result does not depend on
-// how the sequence was cut.  Everything that enters the recurrence is float.
+// The forms are the same recurrence and differ by rounding only, so beyond that a position's result does not depend on how the
+// sequence was cut.  Everything that enters the recurrence is float.
 #include "split_mma.cuh"
 
 static bool g_pdl = false;

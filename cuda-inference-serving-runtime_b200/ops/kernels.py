@@ -1990,7 +1990,9 @@ def _stream_lib():
 
 # ------------------------------------------------------------------ tcgen05 + TMA matrix product
 _tcgen05_state = {}
-TCGEN05_MIN_TOKENS = int(os.environ.get("CISR_TCGEN05_MIN_TOKENS", "128"))   # below one 128-row tile the weight-streaming kernels or the library serve better
+# Below one 128-row tile: the weight-streaming kernels, and from 17 tokens the library (the line was drawn against the persistent kernel of
+# 128-row tiles; the kernel for few tiles has not been compared with the library there).
+TCGEN05_MIN_TOKENS = int(os.environ.get("CISR_TCGEN05_MIN_TOKENS", "128"))
 
 
 def _tcgen05():
