@@ -200,15 +200,19 @@ def wide_span(q_len, ctx_len, heads: int, window: Optional[int], keep_first: int
 
 
 def wide_tiles(plan, ctx, heads: int, window: Optional[int], keep_first: int = 0) -> tuple:
-    """The tile list for the tcgen05 prompt attention, and its queries per tile (`wide_span`, once per step and kind of layer).
-    Either list serves any contexts, so a captured step stays right when it is replayed with others."""
+    """The tile list for the tcgen05 prompt attention, and its queries per tile: 128 where their CTAs all run at once, else by
+    `wide_span`, once per step and kind of layer (3 to 12 us of Python, which small steps would wait for).  Either list serves
+    any contexts, so a captured step stays right when it is replayed with others."""
+    sms = kernels.sm_count(ctx.device)
+    if plan.info["n_wide"] * heads <= sms:         # all at once: nothing is gained by fewer and longer ones
+        return (plan["wide_req"], plan["wide_q0"]), kernels.WIDE_TILE
     key = ("wide_span", heads, window, keep_first)
     span = ctx.shared.get(key)
     if span is None:
-        span = ctx.shared[key] = wide_span(ctx.host.q_len, ctx.host.ctx_len, heads, window, keep_first, kernels.sm_count(ctx.device))
+        span = ctx.shared[key] = wide_span(ctx.host.q_len, ctx.host.ctx_len, heads, window, keep_first, sms)
     if span == kernels.WIDE_TILE:
         return (plan["wide_req"], plan["wide_q0"]), span
-    return (plan["pair_req"], plan["pair_q0"]), span
+    return plan["pairs"].chunk(2), span
 
 
 ATTENTION_PLAN_KEY = ("paged_attention", kernels.PREFILL_TILE, kernels.WIDE_TILE, DECODE_RANGE)
@@ -216,35 +220,39 @@ ATTENTION_PLAN_KEY = ("paged_attention", kernels.PREFILL_TILE, kernels.WIDE_TILE
 
 def attention_step_plan(host):
     """Which CTAs the attention kernels launch for a step: portions of more than one token are cut into query
-    tiles (request, first query), once per tile size of the prompt kernels, a portion's last tile first (it
-    has the longest key loop); single tokens are listed for the split kernel, whose number of key ranges comes
-    from the longest context among them (or from the bound a captured graph was made for).  Every mixer that runs
-    the paged attention kernels shares this plan (`ATTENTION_PLAN_KEY`)."""
+    tiles (request, first query), once per tile size of the prompt kernels (`pairs`, those of 256 queries: all requests and then
+    all first queries), a portion's last tile first (it has the longest key loop); single tokens are listed for the split
+    kernel, whose number of key ranges comes from the longest context among them (or from the bound a captured graph was
+    made for).  Every mixer that runs the paged attention kernels shares this plan (`ATTENTION_PLAN_KEY`)."""
     from ..engine.batch import StepPlan
 
-    tile_req, tile_q0, wide_req, wide_q0, pairs, small, dec_req = [], [], [], [], [], [], []
+    tile_req, tile_q0, wide_req, wide_q0, pair_req, pair_q0, small_req, small_q0, dec_req = [], [], [], [], [], [], [], [], []
+    tile, wide, pair = kernels.PREFILL_TILE, kernels.WIDE_TILE, kernels.WIDE_PAIR
     longest = 0
     for r, n in enumerate(host.q_len):
         if n == 1:
             dec_req.append(r)
             longest = max(longest, host.ctx_len[r])
-        else:
-            for q0 in reversed(range(0, n, kernels.PREFILL_TILE)):
-                tile_req.append(r)
-                tile_q0.append(q0)
-            for q0 in reversed(range(0, n, kernels.WIDE_TILE)):
-                wide_req.append(r)
-                wide_q0.append(q0)
-            for q0 in reversed(range(0, n, kernels.WIDE_PAIR)):
-                # 128 queries or fewer take half the time of more: such tiles go last
-                (pairs if n - q0 > kernels.WIDE_TILE else small).append((r, q0))
+        elif n > 1:
+            q0 = range((n - 1) // tile * tile, -1, -tile)
+            tile_q0 += q0
+            tile_req += [r] * len(q0)
+            q0 = range((n - 1) // wide * wide, -1, -wide)
+            wide_q0 += q0
+            wide_req += [r] * len(q0)
+            q0 = range((n - 1) // pair * pair, -1, -pair)
+            if n - q0[0] <= wide:         # 128 queries or fewer take half the time of more: such tiles go last
+                small_req.append(r)
+                small_q0.append(q0[0])
+                q0 = q0[1:]
+            pair_q0 += q0
+            pair_req += [r] * len(q0)
     if dec_req and host.ctx_bound:
         longest = max(longest, host.ctx_bound)
-    pair_req, pair_q0 = [r for r, _ in pairs + small], [q0 for _, q0 in pairs + small]
-    as_i32 = lambda values: np.asarray(values, dtype=np.int32)
+    as_i32 = lambda values: np.array(values, np.int32)
     return StepPlan(
-        arrays={"tile_req": as_i32(tile_req), "tile_q0": as_i32(tile_q0), "wide_req": as_i32(wide_req),
-                "wide_q0": as_i32(wide_q0), "pair_req": as_i32(pair_req), "pair_q0": as_i32(pair_q0), "dec_req": as_i32(dec_req)},
+        arrays={"tile_req": as_i32(tile_req), "tile_q0": as_i32(tile_q0), "wide_req": as_i32(wide_req), "wide_q0": as_i32(wide_q0),
+                "pairs": as_i32(pair_req + small_req + pair_q0 + small_q0), "dec_req": as_i32(dec_req)},
         info={"n_tiles": len(tile_req), "n_wide": len(wide_req), "n_decode": len(dec_req),
               "n_splits": decode_ranges(longest)})
 

@@ -121,3 +121,21 @@ def test_queries_per_tile_of_the_prompt_attention(heads, window, portions, span)
 def test_queries_per_tile_follow_the_device():
     from cisr_b200.parts.attention import wide_span
     assert wide_span([2048], [2048], 12, None, 0, 296) == 128 and wide_span([4096], [4096], 12, None, 0, 37) == 256
+
+
+def test_tiles_of_256_queries():
+    """All requests, then all first queries; tiles of 128 queries or fewer behind the others."""
+    pairs = attention().step_plan(host_batch([300, 1, 2, 600, 256, 513], [300, 40, 12, 900, 256, 513])).arrays["pairs"].reshape(2, -1)
+    assert list(zip(*pairs.tolist())) == [(0, 0), (3, 256), (3, 0), (4, 0), (5, 256), (5, 0), (0, 256), (2, 0), (3, 512), (5, 512)]
+
+
+def test_small_steps_take_tiles_of_128_queries_without_an_estimate(monkeypatch):
+    from types import SimpleNamespace
+    from cisr_b200.parts import attention as module
+    monkeypatch.setattr(module.kernels, "sm_count", lambda device: 148)
+    host = host_batch([2048], [2048])
+    plan = type("Plan", (), {"info": attention().step_plan(host).info, "__getitem__": lambda self, name: name})()
+    ctx = SimpleNamespace(device="cuda", host=None, shared={})                       # no look at the portions
+    assert module.wide_tiles(plan, ctx, 9, None) == (("wide_req", "wide_q0"), kernels.WIDE_TILE)
+    with pytest.raises(AttributeError):
+        module.wide_tiles(plan, ctx, 10, None)
