@@ -581,7 +581,7 @@ delta_chunk_walk_kernel(const float* __restrict__ qkv, const float* __restrict__
 //                       tensor cores with S in the registers of its result; G's place receives the state before its chunk
 //   delta_chunk_reads   a CTA per (chunk, head): out += R S0
 // The walk over a chunk's own products in order took 256 us for 2048 tokens of 32 heads, and the tables before it 120, most
-// of it the inversion row by row; these three take 110, 41 and 26 us. Error of outputs and
+// of it the inversion row by row; these three take 114, 41 and 26 us. Error of outputs and
 // states against 64 bits 1.0e-7 to 1.6e-7, where the walk has 1.7e-7 to 8.8e-7.
 constexpr int FORM_THREADS = 256;
 constexpr int FORM_G = 3 * CHUNK * CHUNK / 2, FORM_R = FORM_G + CHUNK * CHUNK, FORM_C = FORM_R + CHUNK * CHUNK;

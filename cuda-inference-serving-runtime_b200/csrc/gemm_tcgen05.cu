@@ -655,8 +655,9 @@ int launch_split(const void* a, const void* w, const Epilogue& ep, int m, int n,
 //   rows 63 and 56; gated 3584 x 4096, 1024 rows 45 and 28.
 // - more rows or columns: the persistent kernel, whose epilogues run beside the next tile's products (2048 x 2048, 2048 rows: 19
 //   us; 24 here).
-// A plain product of at most 64 columns (a router's few outputs) is a column of row tiles of its own kind: a long K is cut in two
-// where the tiles leave room for it; a short one, or more row tiles, go to the persistent kernel with tiles of 64 columns.
+// A plain product of at most 64 columns (a router's few outputs) is a column of row tiles: a long K is cut in two where the tiles
+// leave room for it (us, 2048 rows of K 2048 12.6 in the persistent kernel and 7.5, of K 4096 21.0 and 10.3; 9472 rows 13.0 and 8.3,
+// 21.5 and 11.3); a shorter one, or more row tiles, go to the persistent kernel with tiles of 64 columns (K 1024: 8.3).
 struct SplitChoice { int bn, mt, shares; };
 SplitChoice split_choice(int m, int cols64, int k, int max64, int max128, int sms) {
     static int on = -1;

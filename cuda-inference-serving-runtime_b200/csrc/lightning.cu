@@ -228,7 +228,7 @@ __global__ void lightning_output_kernel(const float* __restrict__ o, const float
 
 // The same, four columns an access and the row and its gates in registers, all requested before the sum: bound by memory (2048
 // tokens of 2048: 42 MB, 6.4 us), where single columns asked for one float a thread and the gates only after the sum:
-// 18.4 us, now 10.5.
+// 18.4 us, now 11.8.
 __device__ __forceinline__ void store4(float* to, const float (&v)[4]) { *reinterpret_cast<float4*>(to) = make_float4(v[0], v[1], v[2], v[3]); }
 __device__ __forceinline__ void store4(__nv_bfloat16* to, const float (&v)[4]) {
     __nv_bfloat162 pair[2] = {__floats2bfloat162_rn(v[0], v[1]), __floats2bfloat162_rn(v[2], v[3])};

@@ -1990,8 +1990,9 @@ def _stream_lib():
 
 # ------------------------------------------------------------------ tcgen05 + TMA matrix product
 _tcgen05_state = {}
-# Below one 128-row tile: the weight-streaming kernels, and from 17 tokens the library (the line was drawn against the persistent kernel of
-# 128-row tiles; the kernel for few tiles has not been compared with the library there).
+# Below one 128-row tile: the weight-streaming kernels, and from 17 tokens the library.  us in a graph, library and tcgen05, 17 / 64
+# / 96 tokens: 3072 x 576 3.3 / 3.4 / 3.5 and 4.9 / 5.3 / 5.6; 2048 x 2048 4.9 / 5.0 / 5.1 and 9.9 / 7.5 / 7.7; 4096 x 4096 7.4 / 7.6 / 7.8 and
+# 11.4 / 11.6 / 11.6; 28672 x 4096 41 / 44 / 50 and 44 / 47 / 49; 4096 x 14336 24.1 / 24.3 / 24.9 and 27.1 / 27.5 / 27.7.
 TCGEN05_MIN_TOKENS = int(os.environ.get("CISR_TCGEN05_MIN_TOKENS", "128"))
 
 
