@@ -48,8 +48,8 @@ struct Epilogue {                       // what the epilogue variants need beyon
 };
 // n / d for d >= 1 (or NaN), rounded from a quotient in double: the reciprocal's approximation (some 20 bits, of double's range)
 // after a step of Newton's iteration.  Of 2.7e8 gates and denominators 186 differ from the division operator, by one place.
-// For epilogues that nothing runs beside: a thread has up to 256 quotients, and with the operator, which may branch, each waited for
-// the one before.  us, gated products of one round of tiles with the operator and so: 200 rows of 28672 x 4096 90 and 72,
+// For epilogues that nothing runs beside: a thread has up to 256 quotients, and with the operator one came 160 cycles after the
+// other.  us, gated products of one round of tiles with the operator and so: 200 rows of 28672 x 4096 90 and 72,
 // of 16384 x 2048 49 and 33, of 3072 x 576 14 and 10.  Beside another tile's products the operator is the better one (2048 rows of
 // 28672 x 4096: 304 and 368; double costs power that the tensor cores want).
 __device__ __forceinline__ float quotient(float n, float d) {
