@@ -224,8 +224,9 @@ __device__ __forceinline__ void epilogue_tile(const Epilogue& ep, Load load, int
 }
 
 // Persistent: a CTA walks output tiles blockIdx.x, blockIdx.x + gridDim.x, ...; the accumulator is double-buffered in
-// tensor memory, so the MMA thread fills one buffer while the epilogue warps drain the other.
-template <int BN, int STAGES, int EPI>
+// tensor memory, so the MMA thread fills one buffer while the epilogue warps drain the other.  EXPOSED: K is so short that the epilogue
+// sets the time (SHORT_K).
+template <int BN, int STAGES, int EPI, bool EXPOSED>
 __global__ void __launch_bounds__(192)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
                     const Epilogue ep, int m, int n, int k, int tiles_m, int tiles_n, int* __restrict__ error) {
@@ -362,7 +363,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             if (!ok) break;
             tcgen05_fence_after();
             const uint32_t lane_base = tmem_base + (uint32_t)(acc * BN) + ((uint32_t)(quarter * 32) << 16);
-            epilogue_tile<BN, EPI, false>(ep, [&](int c, uint32_t (&v)[32]) { tmem_load32(lane_base + (uint32_t)c, v); }, 0, epilogue_units<BN, EPI>(), row, m, n, n0, pos, page);
+            epilogue_tile<BN, EPI, EXPOSED>(ep, [&](int c, uint32_t (&v)[32]) { tmem_load32(lane_base + (uint32_t)c, v); }, 0, epilogue_units<BN, EPI>(), row, m, n, n0, pos, page);
             tcgen05_fence_before();
             __syncwarp();
             if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(acc_empty + acc)) : "memory");
@@ -594,8 +595,15 @@ gemm_tcgen05_split_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
 bool g_pdl = false;
 int* g_error = nullptr;          // device flag, owned by the caller (see cisr_gemm_tcgen05_init)
 
-template <int BN, int STAGES, int EPI>
+// Gated products of at most this K make their quotients in double (`quotient`): with the operator a tile's epilogue takes longer than
+// the next tile's products.  us with the operator and so, silu / tanh form of gelu / clamped: 2048 rows of 3072 x 576 20.5 / 20.9 / 23.9 and 16.2 /
+// 19.7 / 18.5, 4096 rows 47 / 48 / 45 and 36 / 44 / 34; 2048 rows of 3072 x 1024 22.9 / 23.1 / 26.5 and 20.1 / 23.5 / 23.0, of 16384 x
+// 1024 80 / 82 / 75 and 75 / 92 / 72, of 16384 x 1536 86 / 88 / 83 and 93 / 110 / 91: one is the better for every gate up to 768.
+constexpr int SHORT_K = 768;
+
+template <int BN, int STAGES, int EPI, bool EXPOSED = false>
 int launch(const void* a, const void* w, const Epilogue& ep, int m, int n, int k, int tiles_n, cudaStream_t s, int groups = 1) {
+    if (paired_rows(EPI) && !EXPOSED && k <= SHORT_K) return launch<BN, STAGES, EPI, paired_rows(EPI)>(a, w, ep, m, n, k, tiles_n, s, groups);
     CUtensorMap map_a, map_w;
     int status = cached_map(&map_a, a, m, k, BM);
     if (status) return status;
@@ -603,7 +611,7 @@ int launch(const void* a, const void* w, const Epilogue& ep, int m, int n, int k
     typedef Smem<BN, STAGES> S;
     static bool configured = false;
     if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_kernel<BN, STAGES, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::TOTAL);
+        cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_kernel<BN, STAGES, EPI, EXPOSED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::TOTAL);
         if (e != cudaSuccess) return (int)e;
         configured = true;
     }
@@ -612,13 +620,13 @@ int launch(const void* a, const void* w, const Epilogue& ep, int m, int n, int k
         int device = 0, sms = 0, per_sm = 0;
         cudaGetDevice(&device);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gemm_tcgen05_kernel<BN, STAGES, EPI>, 192, S::TOTAL);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gemm_tcgen05_kernel<BN, STAGES, EPI, EXPOSED>, 192, S::TOTAL);
         per_sm = per_sm < 1 ? 1 : per_sm;
         if (per_sm * tmem_columns(BN) > 512) per_sm = 512 / tmem_columns(BN);      // tensor memory: 512 columns per SM
         slots = sms * per_sm;
     }
     const int tiles_m = (m + BM - 1) / BM, total = tiles_m * tiles_n;
-    return launch_kernel(gemm_tcgen05_kernel<BN, STAGES, EPI>, dim3(total < slots ? total : slots), dim3(192), S::TOTAL, s, g_pdl,
+    return launch_kernel(gemm_tcgen05_kernel<BN, STAGES, EPI, EXPOSED>, dim3(total < slots ? total : slots), dim3(192), S::TOTAL, s, g_pdl,
                          map_a, map_w, ep, m, n, k, tiles_m, tiles_n, g_error);
 }
 

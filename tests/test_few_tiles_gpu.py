@@ -29,7 +29,8 @@ def test_plain(m, n, kk, accumulate):
     near(out, 0.5 * want + accumulate, kk)
 
 
-@pytest.mark.parametrize("m,inter,kk", [(200, 1500, 576), (64, 2368, 1536), (128, 2000, 4096), (200, 4800, 520), (900, 2300, 200), (100, 9500, 520), (256, 9500, 136)])
+@pytest.mark.parametrize("m,inter,kk", [(200, 1500, 576), (64, 2368, 1536), (128, 2000, 4096), (200, 4800, 520), (900, 2300, 200), (100, 9500, 520), (256, 9500, 136),
+                                       (1000, 4800, 520), (1000, 4800, 768), (1000, 4800, 776), (2100, 700, 576)])       # more than one round: K to 768 and beyond
 @pytest.mark.parametrize("gate", ["silu", "gelu_tanh", "gated_clamp"])
 def test_gated(m, inter, kk, gate):
     from cisr_b200.ops import kernels
@@ -72,11 +73,11 @@ def test_rotated(m, hq, hkv, dim, kk):
         assert ((got.double() - want).abs() <= 1e-3 + 2 ** -8 * want.abs()).all()
 
 
+@pytest.mark.parametrize("m,inter,kk", [(130, 200, 64), (1000, 4800, 64), (1000, 4800, 2056)])
 @pytest.mark.parametrize("gate,x,up", [("silu", -88.0, 1e30), ("silu", -87.5, 1e30), ("gelu_tanh", -10.0, 1e30), ("gated_clamp", -51.75, 3.0)])
-def test_quotients_of_large_denominators(gate, x, up):
+def test_quotients_of_large_denominators(gate, x, up, m, inter, kk):
     """1 + exp(.) above 2^126: the gate is small and not zero."""
     from cisr_b200.ops import kernels
-    m, inter, kk = 130, 200, 64
     a, w = torch.zeros(m, kk, device="cuda", dtype=torch.bfloat16), torch.zeros(2 * inter, kk, device="cuda", dtype=torch.bfloat16)
     a[:, 0] = 1
     w[:inter, 0], w[inter:, 0] = x, up
