@@ -33,7 +33,7 @@ struct ChunkArgs {
     int heads, groups, N, dv, least;
 };
 
-__device__ __forceinline__ float chunk_silu(float z) { return z / (1.f + expf(-z)); }
+__device__ __forceinline__ float chunk_silu(float z) { return quotient(z, 1.f + expf(-z)); }
 
 // Rows [0, nr) x columns [0, nc) of src (row stride `stride`), zeros elsewhere: asked for, and later put into a tile, so that
 // several tiles' loads are on their way together.  put: silu of each where asked, then each row times weight(row).

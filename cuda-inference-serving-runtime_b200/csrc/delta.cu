@@ -28,7 +28,7 @@ static bool g_pdl = false;
 CISR_EXPORT void cisr_delta_set_pdl(int on) { g_pdl = on != 0; }
 
 namespace {
-__device__ __forceinline__ float silu(float z) { return z / (1.f + expf(-z)); }
+__device__ __forceinline__ float silu(float z) { return quotient(z, 1.f + expf(-z)); }
 __device__ __forceinline__ float softplus(float z) { return z > 20.f ? z : log1pf(expf(z)); }
 
 // conv channels: [q: kvh * dk][k: kvh * dk][v: heads * dv]; proj columns: the same, then gate [heads * dv], b [heads], a [heads]
@@ -72,7 +72,7 @@ delta_prepare_kernel(const float* __restrict__ proj, int row_stride, const float
     const float* row = proj + (size_t)t * row_stride;
     const int b_col = channels + heads * dv, a_col = b_col + heads;
     for (int hd = threadIdx.x; hd < heads; hd += blockDim.x) {
-        beta[(size_t)t * heads + hd] = 1.f / (1.f + expf(-row[b_col + hd]));
+        beta[(size_t)t * heads + hd] = quotient(1.f, 1.f + expf(-row[b_col + hd]));
         decay[(size_t)t * heads + hd] = expf(-expf(a_log[hd]) * softplus(row[a_col + hd] + dt_bias[hd]));
     }
 }
@@ -153,7 +153,7 @@ delta_prepare_tile_kernel(const float* __restrict__ proj, int row_stride, const 
     for (int e = threadIdx.x; e < count * heads; e += blockDim.x) {
         const int i = e / heads, hd = e - i * heads;
         const float* row = proj + (size_t)(t0 + i) * row_stride;
-        beta[(size_t)(t0 + i) * heads + hd] = 1.f / (1.f + expf(-row[b_col + hd]));
+        beta[(size_t)(t0 + i) * heads + hd] = quotient(1.f, 1.f + expf(-row[b_col + hd]));
         decay[(size_t)(t0 + i) * heads + hd] = expf(-expf(a_log[hd]) * softplus(row[a_col + hd] + dt_bias[hd]));
     }
 }

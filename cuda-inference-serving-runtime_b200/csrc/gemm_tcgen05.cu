@@ -46,19 +46,6 @@ struct Epilogue {                       // what the epilogue variants need beyon
     // rows [g * n, (g + 1) * n) of `w`.  Null: one weight matrix for all rows.
     const int* tile_group;
 };
-// n / d for d >= 1 (or NaN), rounded from a quotient in double: the reciprocal's approximation (some 20 bits, of double's range)
-// after a step of Newton's iteration.  Of 2.7e8 gates and denominators 186 differ from the division operator, by one place.
-// For epilogues that nothing runs beside: a thread has up to 256 quotients, and with the operator one came 160 cycles after the
-// other.  us, gated products of one round of tiles with the operator and so: 200 rows of 28672 x 4096 90 and 72,
-// of 16384 x 2048 49 and 33, of 3072 x 576 14 and 10.  Beside another tile's products the operator is the better one (2048 rows of
-// 28672 x 4096: 304 and 368; double costs power that the tensor cores want).
-__device__ __forceinline__ float quotient(float n, float d) {
-    const double dd = d;
-    double r;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(dd));
-    const double e = d < INFINITY ? fma(-dd, r, 1.0) : 0.0;              // an infinite d has the reciprocal 0
-    return (float)((double)n * fma(r, e, r));
-}
 // 32 floats -> 32 bfloat16 (64 bytes) at dst; `count` of them are valid
 __device__ __forceinline__ void store_bf16x32(bf16* dst, const float (&v)[32], int count) {
     if (count >= 32 && ((uintptr_t)dst & 15) == 0) {
@@ -107,8 +94,7 @@ __device__ __forceinline__ void unit_columns(const Epilogue& ep, int unit, int& 
 // (feature); load(column, v) gives 32 columns of the row's sums (called by whole warps).
 // `pos`, `page` (ROPE): the row's position and the cache page it is written to, looked up by the caller while the tile
 // was still being accumulated (-1: a padding row, or a row beyond the step).
-// ALONE: nothing runs beside this epilogue.
-template <int BN, int EPI, bool ALONE, typename Load>
+template <int BN, int EPI, typename Load>
 __device__ __forceinline__ void epilogue_tile(const Epilogue& ep, Load load, int u0, int u1, int row, int m, int n, int n0, int pos, int page) {
 #pragma unroll 1
     for (int unit = u0; unit < u1; ++unit) {
@@ -159,14 +145,13 @@ __device__ __forceinline__ void epilogue_tile(const Epilogue& ep, Load load, int
             uint32_t u[32];
             load(hi_col, u);
             float act[32];
-            const auto over = [](float a, float b) { return ALONE ? quotient(a, b) : a / b; };
             if (EPI == EPI_GATED) {
                 // the clamped gated activation of stacked gate and up rows, as bfloat16 [m, inter]
                 const float limit = ep.limit, alpha = ep.alpha;
 #pragma unroll
                 for (int j = 0; j < 32; ++j) {
                     const float gv = fminf(__uint_as_float(v[j]), limit), uv = fminf(fmaxf(__uint_as_float(u[j]), -limit), limit);
-                    act[j] = over(gv, 1.f + expf(-alpha * gv)) * (uv + 1.f);
+                    act[j] = quotient(gv, 1.f + expf(-alpha * gv)) * (uv + 1.f);
                 }
             } else {
                 // silu(z) = z / (1 + exp(-z)) and gelu(z) = z / (1 + exp(-2 sqrt(2 / pi) (z + 0.044715 z^3))) differ in the exponent only
@@ -174,7 +159,7 @@ __device__ __forceinline__ void epilogue_tile(const Epilogue& ep, Load load, int
 #pragma unroll
                 for (int j = 0; j < 32; ++j) {
                     const float gv = __uint_as_float(v[j]);
-                    act[j] = over(gv, 1.f + expf(-lin * (gv + cub * gv * gv * gv))) * __uint_as_float(u[j]);
+                    act[j] = quotient(gv, 1.f + expf(-lin * (gv + cub * gv * gv * gv))) * __uint_as_float(u[j]);
                 }
             }
             if (row < m && n0 + lo_col < ep.inter)
@@ -224,9 +209,8 @@ __device__ __forceinline__ void epilogue_tile(const Epilogue& ep, Load load, int
 }
 
 // Persistent: a CTA walks output tiles blockIdx.x, blockIdx.x + gridDim.x, ...; the accumulator is double-buffered in
-// tensor memory, so the MMA thread fills one buffer while the epilogue warps drain the other.  EXPOSED: K is so short that the epilogue
-// sets the time (SHORT_K).
-template <int BN, int STAGES, int EPI, bool EXPOSED>
+// tensor memory, so the MMA thread fills one buffer while the epilogue warps drain the other.
+template <int BN, int STAGES, int EPI>
 __global__ void __launch_bounds__(192)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
                     const Epilogue ep, int m, int n, int k, int tiles_m, int tiles_n, int* __restrict__ error) {
@@ -363,7 +347,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             if (!ok) break;
             tcgen05_fence_after();
             const uint32_t lane_base = tmem_base + (uint32_t)(acc * BN) + ((uint32_t)(quarter * 32) << 16);
-            epilogue_tile<BN, EPI, EXPOSED>(ep, [&](int c, uint32_t (&v)[32]) { tmem_load32(lane_base + (uint32_t)c, v); }, 0, epilogue_units<BN, EPI>(), row, m, n, n0, pos, page);
+            epilogue_tile<BN, EPI>(ep, [&](int c, uint32_t (&v)[32]) { tmem_load32(lane_base + (uint32_t)c, v); }, 0, epilogue_units<BN, EPI>(), row, m, n, n0, pos, page);
             tcgen05_fence_before();
             __syncwarp();
             if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(acc_empty + acc)) : "memory");
@@ -554,7 +538,7 @@ gemm_tcgen05_split_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
             ok = mbar_wait(inbox_full, 0) && ok;
             if (__all_sync(0xffffffffu, ok)) {
                 const float* next = inbox + row_in;                            // loads come in the order unit, side
-                epilogue_tile<BN, EPI, true>(ep, [&](int c, uint32_t (&v)[32]) {
+                epilogue_tile<BN, EPI>(ep, [&](int c, uint32_t (&v)[32]) {
                     const float* from = next;
                     next += 32 * BM;
 #pragma unroll
@@ -581,7 +565,7 @@ gemm_tcgen05_split_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
 #pragma unroll
         for (int t = 0; t < MT; ++t) {
             const uint32_t lane_base = tmem_base + lanes + (uint32_t)(t * BN);
-            epilogue_tile<BN, EPI, true>(ep, [&](int c, uint32_t (&v)[32]) { tmem_load32(lane_base + (uint32_t)c, v); }, 0, UNITS,
+            epilogue_tile<BN, EPI>(ep, [&](int c, uint32_t (&v)[32]) { tmem_load32(lane_base + (uint32_t)c, v); }, 0, UNITS,
                                    m0 + t * BM + quarter * 32 + lane, m, n, n0, pos[t], page[t]);
         }
     }
@@ -595,15 +579,8 @@ gemm_tcgen05_split_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
 bool g_pdl = false;
 int* g_error = nullptr;          // device flag, owned by the caller (see cisr_gemm_tcgen05_init)
 
-// Gated products of at most this K make their quotients in double (`quotient`): with the operator a tile's epilogue takes longer than
-// the next tile's products.  us with the operator and so, silu / tanh form of gelu / clamped: 2048 rows of 3072 x 576 20.5 / 20.9 / 23.9 and 16.2 /
-// 19.7 / 18.5, 4096 rows 47 / 48 / 45 and 36 / 44 / 34; 2048 rows of 3072 x 1024 22.9 / 23.1 / 26.5 and 20.1 / 23.5 / 23.0, of 16384 x
-// 1024 80 / 82 / 75 and 75 / 92 / 72, of 16384 x 1536 86 / 88 / 83 and 93 / 110 / 91: one is the better for every gate up to 768.
-constexpr int SHORT_K = 768;
-
-template <int BN, int STAGES, int EPI, bool EXPOSED = false>
+template <int BN, int STAGES, int EPI>
 int launch(const void* a, const void* w, const Epilogue& ep, int m, int n, int k, int tiles_n, cudaStream_t s, int groups = 1) {
-    if (paired_rows(EPI) && !EXPOSED && k <= SHORT_K) return launch<BN, STAGES, EPI, paired_rows(EPI)>(a, w, ep, m, n, k, tiles_n, s, groups);
     CUtensorMap map_a, map_w;
     int status = cached_map(&map_a, a, m, k, BM);
     if (status) return status;
@@ -611,7 +588,7 @@ int launch(const void* a, const void* w, const Epilogue& ep, int m, int n, int k
     typedef Smem<BN, STAGES> S;
     static bool configured = false;
     if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_kernel<BN, STAGES, EPI, EXPOSED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::TOTAL);
+        cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_kernel<BN, STAGES, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::TOTAL);
         if (e != cudaSuccess) return (int)e;
         configured = true;
     }
@@ -620,13 +597,13 @@ int launch(const void* a, const void* w, const Epilogue& ep, int m, int n, int k
         int device = 0, sms = 0, per_sm = 0;
         cudaGetDevice(&device);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gemm_tcgen05_kernel<BN, STAGES, EPI, EXPOSED>, 192, S::TOTAL);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gemm_tcgen05_kernel<BN, STAGES, EPI>, 192, S::TOTAL);
         per_sm = per_sm < 1 ? 1 : per_sm;
         if (per_sm * tmem_columns(BN) > 512) per_sm = 512 / tmem_columns(BN);      // tensor memory: 512 columns per SM
         slots = sms * per_sm;
     }
     const int tiles_m = (m + BM - 1) / BM, total = tiles_m * tiles_n;
-    return launch_kernel(gemm_tcgen05_kernel<BN, STAGES, EPI, EXPOSED>, dim3(total < slots ? total : slots), dim3(192), S::TOTAL, s, g_pdl,
+    return launch_kernel(gemm_tcgen05_kernel<BN, STAGES, EPI>, dim3(total < slots ? total : slots), dim3(192), S::TOTAL, s, g_pdl,
                          map_a, map_w, ep, m, n, k, tiles_m, tiles_n, g_error);
 }
 

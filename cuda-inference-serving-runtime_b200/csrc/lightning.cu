@@ -223,7 +223,7 @@ __global__ void lightning_output_kernel(const float* __restrict__ o, const float
     const float unit = rsqrtf(block_sum(sq, scratch) / (float)width + eps);
     const float* g = gate + (size_t)t * gate_stride + gate_col;
     for (int j = threadIdx.x; j < width; j += blockDim.x)
-        out[(size_t)t * out_stride + j] = from_float<CT>(row[j] * unit * norm_w[j] * (1.f / (1.f + expf(-g[j]))));
+        out[(size_t)t * out_stride + j] = from_float<CT>(row[j] * unit * norm_w[j] * quotient(1.f, 1.f + expf(-g[j])));
 }
 
 // The same, four columns an access and the row and its gates in registers, all requested before the sum: bound by memory (2048
@@ -266,7 +266,7 @@ lightning_output_runs_kernel(const float* __restrict__ o, const float* __restric
         const float4 w = *reinterpret_cast<const float4*>(norm_w + j);
         const float ww[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
-        for (int e = 0; e < 4; ++e) v[r][e] = v[r][e] * unit * ww[e] * (1.f / (1.f + expf(-g[r][e])));
+        for (int e = 0; e < 4; ++e) v[r][e] = v[r][e] * unit * ww[e] * quotient(1.f, 1.f + expf(-g[r][e]));
         store4(out + t * out_stride + j, v[r]);
     }
 }

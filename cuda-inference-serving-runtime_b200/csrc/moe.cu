@@ -200,7 +200,7 @@ moe_up_rows_kernel(const T* __restrict__ h, const T* __restrict__ w_up, const in
         const T* w = w_up + (size_t)e * 2 * ff * hidden;
         const float g = fminf(warp_dot(w + (size_t)f * hidden, x, hidden, lane), limit);
         const float u = fminf(fmaxf(warp_dot(w + (size_t)(ff + f) * hidden, x, hidden, lane), -limit), limit);
-        if (lane == 0) act[(size_t)pair * ff + f] = from_float<T>(g / (1.f + expf(-GATE_ALPHA * g)) * (u + 1.f));
+        if (lane == 0) act[(size_t)pair * ff + f] = from_float<T>(quotient(g, 1.f + expf(-GATE_ALPHA * g)) * (u + 1.f));
         return;
     }
     const float z = warp_dot(w_up + ((size_t)e * ff + f) * hidden, x, hidden, lane);

@@ -7,8 +7,8 @@ static bool g_pdl = false;
 CISR_EXPORT void cisr_recurrent_rows_set_pdl(int on) { g_pdl = on != 0; }
 
 namespace {
-__device__ __forceinline__ float sigmoid_f(float z) { return 1.f / (1.f + expf(-z)); }
-__device__ __forceinline__ float silu_f(float z) { return z / (1.f + expf(-z)); }
+__device__ __forceinline__ float sigmoid_f(float z) { return quotient(1.f, 1.f + expf(-z)); }
+__device__ __forceinline__ float silu_f(float z) { return quotient(z, 1.f + expf(-z)); }
 __device__ __forceinline__ float softplus_f(float z) { return fmaxf(z, 0.f) + log1pf(expf(-fabsf(z))); }
 
 // ------------------------------------------------------------------ short convolution over time
