@@ -2,10 +2,12 @@
 // operands, float accumulation in tensor memory.  Used for steps with more tokens than the weight-streaming
 // kernels take (prompt portions, large decode batches).
 //
-//   * products of one round of tiles have a kernel of their own (gemm_tcgen05_split_kernel, further down); the others
-//     go to persistent CTAs, each walking output tiles of 128 x BN (BN = 256, 192, 128 or 64, chosen from the number of
-//     tiles: see the launchers), with two accumulators of BN columns in tensor memory so that the epilogue of
-//     one tile runs under the products of the next
+//   * few tiles: gemm_tcgen05_split_kernel, a tile per CTA, K cut over a cluster
+//   * more: gemm_tcgen05_pair_kernel, persistent, tiles of 256 rows on two SMs
+//   * grouped products, and narrow ones with many rows: gemm_tcgen05_kernel, persistent CTAs that walk output tiles of 128 x BN
+//     (BN = 256, 128 or 64) with two accumulators of BN columns in tensor memory, so that the epilogue of one tile runs under the
+//     products of the next
+// All three have the same roles (here those of gemm_tcgen05_kernel):
 //   * warp 0: one thread issues TMA loads (cp.async.bulk.tensor.2d, 128-byte swizzle) of the A tile
 //     [128 rows x 64 k] and the B tile [BN rows x 64 k] into a STAGES-deep ring of shared memory (3 to 8
 //     stages), each load completing on the stage's "full" mbarrier
@@ -65,6 +67,38 @@ __device__ __forceinline__ void store_bf16x32(bf16* dst, const float (&v)[32], i
     }
 }
 
+// A warp's results leave by way of a patch of shared memory (STAGE_BYTES, 16-byte units of a row exchanged among eight rows against
+// bank conflicts): in registers a lane has a row, and stores of 16 bytes each to 32 rows reach L2 as half-filled sectors; from the patch
+// four to eight rows leave as whole runs.  us, persistent kernel, without and with: 2533 rows of 6144 x 2048 67 and 58, 4096 rows of 8192 x
+// 2048 116 and 106; few tiles, 2048 rows of 2048 x 2048 19.0 and 17.8.  Gated results, half as many bytes, go straight out of the kernel
+// for few tiles (200 rows of 4096 x 1024 8.4 us, 8.8 through the patch); in the pair kernel there is no difference.
+constexpr size_t STAGE_BYTES = 4096;
+// 32 bfloat16 per lane and row to dst + 32-column runs: `to(r)` is where row r of the warp's 32 goes (null: nowhere); units of eight
+// columns, `units` of them valid
+template <typename To>
+__device__ __forceinline__ void store_rows_bf16(unsigned char* patch, const float (&v)[32], To to, int units) {
+    const int lane = threadIdx.x & 31;
+    __syncwarp();                                        // the run before has been read
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        uint32_t w[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const __nv_bfloat162 p = __floats2bfloat162_rn(v[8 * u + 2 * e], v[8 * u + 2 * e + 1]);
+            w[e] = *reinterpret_cast<const uint32_t*>(&p);
+        }
+        *reinterpret_cast<uint4*>(patch + lane * 64 + ((u ^ (lane >> 1)) & 3) * 16) = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int r = 8 * i + (lane >> 2), u = lane & 3;
+        bf16* dst = to(r);
+        const uint4 w = *reinterpret_cast<const uint4*>(patch + r * 64 + ((u ^ (r >> 1)) & 3) * 16);
+        if (dst && u < units) *reinterpret_cast<uint4*>(dst + 8 * u) = w;
+    }
+}
+
 // Columns of tensor memory for two accumulators of `bn` columns: allocations are powers of two.
 __host__ __device__ constexpr int tmem_columns(int bn) { return 2 * bn <= 32 ? 32 : 2 * bn <= 64 ? 64 : 2 * bn <= 128 ? 128 : 2 * bn <= 256 ? 256 : 512; }
 
@@ -73,33 +107,48 @@ struct Smem {
     static constexpr size_t A_BYTES = (size_t)BM * BK * sizeof(bf16);
     static constexpr size_t B_BYTES = (size_t)BN * BK * sizeof(bf16);
     static constexpr size_t TILES = STAGES * (A_BYTES + B_BYTES);
-    static constexpr size_t TOTAL = TILES + 1024 /* alignment slack */ + 256 /* barriers */;
+    static constexpr bool PATCHES = BN != 128;      // tiles of 128 columns: two CTAs share an SM, which leaves no room for them
+    static constexpr size_t TOTAL = TILES + 1024 /* alignment slack */ + 256 /* barriers */ + (PATCHES ? 4 * STAGE_BYTES : 0);
 };
 
+// 32 activations per lane and row into out [m, width] at column `col`
+__device__ __forceinline__ void store_activations(bf16* out, int width, int col, const float (&act)[32], unsigned char* patch, int row, int m) {
+    if (col >= width) return;
+    if (patch && (width & 7) == 0 && ((uintptr_t)out & 15) == 0) {
+        const int row0 = row - (int)(threadIdx.x & 31);
+        store_rows_bf16(patch, act, [&](int r) { return row0 + r < m ? out + (size_t)(row0 + r) * width + col : nullptr; }, (width - col) >> 3);
+    } else if (row < m) store_bf16x32(out + (size_t)row * width + col, act, width - col);
+}
+
 // A tile's result is taken 32 columns at a time: in units of 32 columns (PLAIN, RELU2), of 32 gate and the 32 up columns of
-// the same features (SWIGLU, GATED), or of 32 rotation pairs of a head (ROPE: columns c and c + dim / 2).
-template <int BN, int EPI>
-__device__ __forceinline__ constexpr int epilogue_units() { return EPI == EPI_PLAIN || EPI == EPI_RELU2 ? BN / 32 : BN / 64; }
-template <int BN, int EPI>
-__device__ __forceinline__ void unit_columns(const Epilogue& ep, int unit, int& lo, int& hi) {
+// the same features (SWIGLU, GATED; where half the tile is no multiple of 32 the last unit begins early and makes some columns a
+// second time), or of 32 rotation pairs of a head (ROPE: columns c and c + dim / 2).
+template <int EPI>
+__device__ __forceinline__ constexpr int epilogue_units(int bn) {
+    return EPI == EPI_PLAIN || EPI == EPI_RELU2 ? bn / 32 : paired_rows(EPI) ? (bn / 2 + 31) / 32 : bn / 64;
+}
+template <int EPI>
+__device__ __forceinline__ void unit_columns(const Epilogue& ep, int bn, int unit, int& lo, int& hi) {
     lo = 32 * unit; hi = 0;
-    if (paired_rows(EPI)) hi = BN / 2 + lo;
+    if (paired_rows(EPI)) { lo = min(lo, bn / 2 - 32); hi = bn / 2 + lo; }
     if (EPI == EPI_ROPE) {
         const int per_head = ep.dim / 64;
         lo = (unit / per_head) * ep.dim + (unit % per_head) * 32;
         hi = lo + ep.dim / 2;
     }
 }
-// The epilogue of units [u0, u1) of an output tile for one thread: `row` is the thread's output row, n0 the tile's first column
+// The epilogue of units [u0, u1) of an output tile of `bn` columns for one thread: `row` is the thread's output row, n0 the tile's first column
 // (feature); load(column, v) gives 32 columns of the row's sums (called by whole warps).
 // `pos`, `page` (ROPE): the row's position and the cache page it is written to, looked up by the caller while the tile
 // was still being accumulated (-1: a padding row, or a row beyond the step).
-template <int BN, int EPI, typename Load>
-__device__ __forceinline__ void epilogue_tile(const Epilogue& ep, Load load, int u0, int u1, int row, int m, int n, int n0, int pos, int page) {
+template <int EPI, typename Load>
+__device__ __forceinline__ void epilogue_tile(const Epilogue& ep, int bn, Load load, int u0, int u1, int row, int m, int n, int n0, int pos, int page,
+                                              unsigned char* patch) {
+    const int lane = threadIdx.x & 31, row0 = row - lane;
 #pragma unroll 1
     for (int unit = u0; unit < u1; ++unit) {
         int lo_col, hi_col;
-        unit_columns<BN, EPI>(ep, unit, lo_col, hi_col);
+        unit_columns<EPI>(ep, bn, unit, lo_col, hi_col);
         uint32_t v[32];
         load(lo_col, v);
         if (EPI == EPI_PLAIN) {
@@ -108,13 +157,28 @@ __device__ __forceinline__ void epilogue_tile(const Epilogue& ep, Load load, int
                 for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) * ep.out_mult);
             }
             const int c = lo_col;
-            if (row < m) {
+            if (patch && (n & 3) == 0) {
+                __syncwarp();                            // the run before has been read
+#pragma unroll
+                for (int u = 0; u < 8; ++u)
+                    *reinterpret_cast<uint4*>(patch + lane * 128 + ((u ^ lane) & 7) * 16) = make_uint4(v[4 * u], v[4 * u + 1], v[4 * u + 2], v[4 * u + 3]);
+                __syncwarp();
+                const int u = lane & 7, col = n0 + c + 4 * u;
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const int r = 4 * i + (lane >> 3);
+                    const float4 x = *reinterpret_cast<const float4*>(patch + r * 128 + ((u ^ r) & 7) * 16);
+                    if (row0 + r >= m || col >= n) continue;
+                    float* dst = ep.out_f32 + (size_t)(row0 + r) * n + col;
+                    // The add is done where the element lives (a reduction in L2), so the epilogue does not wait for a load: every
+                    // element belongs to this thread alone, and one float add in round-to-nearest is the same sum wherever it is made.
+                    if (ep.accumulate) asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst), "f"(x.x), "f"(x.y), "f"(x.z), "f"(x.w) : "memory");
+                    else *reinterpret_cast<float4*>(dst) = x;
+                }
+            } else if (row < m) {
                 float* dst = ep.out_f32 + (size_t)row * n + n0 + c;
                 if (n0 + c + 32 <= n && (n & 3) == 0) {
                     if (ep.accumulate) {
-                        // The add is done where the element lives (a reduction in L2), so the epilogue does not wait for
-                        // a load: every element belongs to this thread alone, and one float add in round-to-nearest is
-                        // the same sum wherever it is made.
 #pragma unroll
                         for (int j = 0; j < 32; j += 4)
                             asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst + j), "f"(__uint_as_float(v[j])),
@@ -140,7 +204,7 @@ __device__ __forceinline__ void epilogue_tile(const Epilogue& ep, Load load, int
                 const float z = __uint_as_float(v[j]), r = fmaxf(z, 0.f);
                 act[j] = gelu ? 0.5f * z * (1.f + erff(z * 0.70710678118654752f)) : r * r;
             }
-            if (row < m && n0 + lo_col < n) store_bf16x32(ep.out_bf16 + (size_t)row * n + n0 + lo_col, act, n - (n0 + lo_col));
+            store_activations(ep.out_bf16, n, n0 + lo_col, act, patch, row, m);
         } else if (paired_rows(EPI)) {
             uint32_t u[32];
             load(hi_col, u);
@@ -162,8 +226,7 @@ __device__ __forceinline__ void epilogue_tile(const Epilogue& ep, Load load, int
                     act[j] = quotient(gv, 1.f + expf(-lin * (gv + cub * gv * gv * gv))) * __uint_as_float(u[j]);
                 }
             }
-            if (row < m && n0 + lo_col < ep.inter)
-                store_bf16x32(ep.out_bf16 + (size_t)row * ep.inter + n0 + lo_col, act, ep.inter - (n0 + lo_col));
+            store_activations(ep.out_bf16, ep.inter, n0 + lo_col, act, patch, row, m);
         } else {
             // whole heads of the stacked q, k, v projection: BN / dim heads per tile, rotation pairs (i, i + dim / 2)
             const int dim = ep.dim, half = dim / 2;
@@ -200,7 +263,11 @@ __device__ __forceinline__ void epilogue_tile(const Epilogue& ep, Load load, int
 #pragma unroll
                 for (int j = 0; j < 32; ++j) { first[j] = __uint_as_float(v[j]); second[j] = __uint_as_float(hi[j]); }
             }
-            if (dst) {
+            if (patch && !(((uintptr_t)ep.q_out | (uintptr_t)ep.k_cache | (uintptr_t)ep.v_cache) & 15)) {      // heads are 128 bytes and more
+                const auto place = [&](int r) { return reinterpret_cast<bf16*>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(dst), r)); };
+                store_rows_bf16(patch, first, [&](int r) { bf16* p = place(r); return p ? p + c : p; }, 4);
+                store_rows_bf16(patch, second, [&](int r) { bf16* p = place(r); return p ? p + half + c : p; }, 4);
+            } else if (dst) {
                 store_bf16x32(dst + c, first, 32);
                 store_bf16x32(dst + half + c, second, 32);
             }
@@ -347,7 +414,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             if (!ok) break;
             tcgen05_fence_after();
             const uint32_t lane_base = tmem_base + (uint32_t)(acc * BN) + ((uint32_t)(quarter * 32) << 16);
-            epilogue_tile<BN, EPI>(ep, [&](int c, uint32_t (&v)[32]) { tmem_load32(lane_base + (uint32_t)c, v); }, 0, epilogue_units<BN, EPI>(), row, m, n, n0, pos, page);
+            epilogue_tile<EPI>(ep, BN, [&](int c, uint32_t (&v)[32]) { tmem_load32(lane_base + (uint32_t)c, v); }, 0, epilogue_units<EPI>(BN), row, m, n, n0, pos, page,
+                                        S::PATCHES && EPI == EPI_PLAIN ? tiles + S::TILES + 256 + (warp - 2) * STAGE_BYTES : nullptr);
             tcgen05_fence_before();
             __syncwarp();
             if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(acc_empty + acc)) : "memory");
@@ -381,7 +449,8 @@ struct SplitSmem {
     static constexpr size_t TOTAL = TILES + 1024 /* alignment slack */ + 256 /* barriers */;
     // what a CTA sends away and what it receives, (shares - 1) / shares of the tile each, lie side by side in the ring
     static constexpr bool CAN_SPLIT = MT == 1 && BN <= 128;
-    static_assert(!CAN_SPLIT || 2 * (size_t)BN * BM * sizeof(float) * 3 / 4 <= TILES, "the runs of four shares");
+    static constexpr size_t PATCHES = TILES - 4 * STAGE_BYTES;      // the ring is free by then, but for the runs
+    static_assert(!CAN_SPLIT || 2 * (size_t)BN * BM * sizeof(float) * 3 / 4 <= PATCHES, "the runs of four shares");
 };
 
 __device__ __forceinline__ void cluster_meet() {
@@ -493,7 +562,8 @@ gemm_tcgen05_split_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
         tcgen05_fence_after();
     }
     const uint32_t lanes = (uint32_t)(quarter * 32) << 16;
-    constexpr int UNITS = epilogue_units<BN, EPI>();
+    unsigned char* patch = paired_rows(EPI) ? nullptr : tiles + S::PATCHES + quarter * STAGE_BYTES;
+    constexpr int UNITS = epilogue_units<EPI>(BN);
     if (S::CAN_SPLIT && shares > 1) {
         // every thread meets the barriers, also where a wait ran out (its sums are then not written)
         __syncwarp();
@@ -508,7 +578,7 @@ gemm_tcgen05_split_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
                 float* box = outbox + (size_t)(to < rank ? to : to - 1) * run + row_in;
                 for (int u = 0; u < per_cta; ++u) {
                     int lo, hi;
-                    unit_columns<BN, EPI>(ep, to * per_cta + u, lo, hi);
+                    unit_columns<EPI>(ep, BN, to * per_cta + u, lo, hi);
                     for (int side = 0; side < sides; ++side) {
                         uint32_t v[32];
                         tmem_load32(tmem_base + lanes + (uint32_t)(side ? hi : lo), v);
@@ -538,7 +608,7 @@ gemm_tcgen05_split_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
             ok = mbar_wait(inbox_full, 0) && ok;
             if (__all_sync(0xffffffffu, ok)) {
                 const float* next = inbox + row_in;                            // loads come in the order unit, side
-                epilogue_tile<BN, EPI>(ep, [&](int c, uint32_t (&v)[32]) {
+                epilogue_tile<EPI>(ep, BN, [&](int c, uint32_t (&v)[32]) {
                     const float* from = next;
                     next += 32 * BM;
 #pragma unroll
@@ -556,7 +626,7 @@ gemm_tcgen05_split_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
 #pragma unroll
                         for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) + __uint_as_float(share[j]));
                     }
-                }, rank * per_cta, (rank + 1) * per_cta, m0 + row_in, m, n, n0, pos[0], page[0]);
+                }, rank * per_cta, (rank + 1) * per_cta, m0 + row_in, m, n, n0, pos[0], page[0], patch);
             }
         }
         __syncwarp();
@@ -565,14 +635,157 @@ gemm_tcgen05_split_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
 #pragma unroll
         for (int t = 0; t < MT; ++t) {
             const uint32_t lane_base = tmem_base + lanes + (uint32_t)(t * BN);
-            epilogue_tile<BN, EPI>(ep, [&](int c, uint32_t (&v)[32]) { tmem_load32(lane_base + (uint32_t)c, v); }, 0, UNITS,
-                                   m0 + t * BM + quarter * 32 + lane, m, n, n0, pos[t], page[t]);
+            epilogue_tile<EPI>(ep, BN, [&](int c, uint32_t (&v)[32]) { tmem_load32(lane_base + (uint32_t)c, v); }, 0, UNITS,
+                                   m0 + t * BM + quarter * 32 + lane, m, n, n0, pos[t], page[t], patch);
         }
     }
     if (!ok && lane == 0) atomicExch(error, 1);
     tcgen05_fence_before();
     __syncthreads();
     if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(COLUMNS) : "memory");
+}
+
+// ---------------------------------------------------------------- large products: a tile on two SMs
+// Tiles of 256 rows x bn columns (bn a multiple of 32 up to 256, chosen by pair_choice), one per pair of CTAs that share a TPC.  Each
+// CTA brings its 128 rows of A and half of the weight rows into its own shared memory; the products (tcgen05.mma.cta_group::2, M = 256)
+// are issued by the pair's first CTA and read both halves, and each CTA's tensor memory receives its own 128 rows by all columns, so
+// the epilogue is the one of a 128-row tile.  Persistent, two accumulators per CTA, eight epilogue warps (four per half of the columns).
+//
+// Barriers: `full` (in the first CTA) counts both CTAs' copies; `empty` and `acc_full` are in both and told by commits that reach both;
+// `acc_empty` (in the first CTA) hears the epilogue warps of both.
+//
+// What bounds it: an SM brings 110 to 150 B/ns from L2, and a 128 x 256 tile on one SM wants 48 KB per 64 of K (512 cycles of products);
+// a pair's 256 x 256 tile wants 32 KB per SM.  From there on the tensor cores, at the clock that the power leaves them (a block of K of a 256
+// x 256 tile 0.29 us on an idle chip, 0.38 on a busy one), and the last round.  us, 128 x 256 tiles on one SM each and so: gated 14336 x 4096,
+// 2048 rows 330 and 315, 1000 rows 201 and 157, 512 rows 111 and 90; gated 8192 x 2048, 2048 rows 100 and 90; plain 6144 x 2048, 2533 rows 67 and
+// 50; 8192 x 2048, 2048 rows 65 and 52; 4096 x 14336, 2048 rows 184 and 166.
+constexpr int PAIR_STAGES = 6, PAIR_THREADS = 320, PAIR_BN = 256;
+struct PairSmem {
+    static constexpr size_t A_BYTES = (size_t)BM * BK * sizeof(bf16), B_BYTES = (size_t)PAIR_BN / 2 * BK * sizeof(bf16);
+    static constexpr size_t STAGE = A_BYTES + B_BYTES, TILES = PAIR_STAGES * STAGE;
+    static constexpr size_t TOTAL = TILES + 1024 /* alignment slack */ + 256 /* barriers */ + 8 * STAGE_BYTES;
+};
+
+template <int EPI>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
+gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
+                         const Epilogue ep, int m, int n, int k, int bn, int tiles_m, int tiles_n, int* __restrict__ error) {
+    CISR_TRACE_SCOPE(TRACE_GEMM_TCGEN05);
+    extern __shared__ unsigned char smem_raw[];
+    typedef PairSmem S;
+    unsigned char* tiles = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    uint64_t* full_bar = reinterpret_cast<uint64_t*>(tiles + S::TILES);
+    uint64_t* empty_bar = full_bar + PAIR_STAGES;
+    uint64_t* acc_full = empty_bar + PAIR_STAGES;
+    uint64_t* acc_empty = acc_full + 2;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+    const int rank = (int)blockIdx.x & 1, pair = (int)blockIdx.x >> 1, pairs = (int)gridDim.x >> 1;
+    const int k_blocks = (k + BK - 1) / BK, total_tiles = tiles_m * tiles_n;
+    const int tile_n = paired_rows(EPI) ? bn / 2 : bn;
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < PAIR_STAGES; ++s) { mbar_init(full_bar + s, 1); mbar_init(empty_bar + s, 1); }
+        for (int b = 0; b < 2; ++b) { mbar_init(acc_full + b, 1); mbar_init(acc_empty + b, 16); }
+        mbar_init_fence();
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(2 * PAIR_BN) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    }
+    tcgen05_fence_before();
+    cluster_meet();                      // both CTAs' barriers are there before either is told anything
+    tcgen05_fence_after();
+    const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+    bool ok = true;
+    pdl_trigger();
+
+    if (warp == 0) {
+        if (lane == 0) {
+            const uint32_t full_first = in_cluster(full_bar, 0);
+            const uint32_t stage_bytes = 2 * (uint32_t)(S::A_BYTES + (size_t)bn / 2 * BK * sizeof(bf16));       // of both CTAs
+            // this CTA's half of the weight rows: of a tile's columns, or (paired) the gate rows here and the up rows there
+            const int w_off = paired_rows(EPI) ? rank * ep.inter : rank * (bn / 2);
+            auto load_b = [&](int s, int kb, int n0) { tma_load_2d_pair(tiles + s * S::STAGE + S::A_BYTES, &map_w, kb * BK, n0 + w_off, full_first + 8 * s); };
+            auto load_a = [&](int s, int kb, int m0) { tma_load_2d_pair(tiles + s * S::STAGE, &map_a, kb * BK, m0 + rank * BM, full_first + 8 * s); };
+            // the first stages' weights are requested before the wait on the kernel before, the activations after it
+            const int early = pair < total_tiles ? min(k_blocks, PAIR_STAGES) : 0;
+            for (int kb = 0; kb < early; ++kb) {
+                if (rank == 0) mbar_expect_tx(full_bar + kb, stage_bytes);
+                load_b(kb, kb, pair / tiles_m * tile_n);
+            }
+            pdl_wait();
+            CISR_TRACE_WAITED();
+            int kbg = 0;
+            for (int tile = pair; tile < total_tiles && ok; tile += pairs) {
+                const int m0 = tile % tiles_m * 2 * BM, n0 = tile / tiles_m * tile_n;
+                for (int kb = 0; kb < k_blocks; ++kb, ++kbg) {
+                    const int s = kbg % PAIR_STAGES;
+                    if (kbg >= early) {
+                        ok = mbar_wait(empty_bar + s, ((kbg / PAIR_STAGES) & 1) ^ 1);
+                        if (!ok) break;
+                        if (rank == 0) mbar_expect_tx(full_bar + s, stage_bytes);
+                        load_b(s, kb, n0);
+                    }
+                    load_a(s, kb, m0);
+                }
+            }
+        }
+    } else if (warp == 1) {
+        if (rank == 0) {
+            const uint32_t idesc = umma_idesc_pair(bn);
+            const uint64_t desc_a = umma_desc(tiles), desc_b = umma_desc(tiles + S::A_BYTES);
+            int kbg = 0, it = 0;
+            for (int tile = pair; tile < total_tiles && ok; tile += pairs, ++it) {
+                const int acc = it & 1;
+                ok = __all_sync(0xffffffffu, mbar_wait(acc_empty + acc, ((it >> 1) & 1) ^ 1));
+                if (!ok) break;
+                tcgen05_fence_after();
+                const uint32_t tmem_acc = tmem_base + (uint32_t)(acc * PAIR_BN);
+                for (int kb = 0; kb < k_blocks; ++kb, ++kbg) {
+                    const int s = kbg % PAIR_STAGES;
+                    ok = __all_sync(0xffffffffu, mbar_wait(full_bar + s, (kbg / PAIR_STAGES) & 1));
+                    if (!ok) break;
+                    tcgen05_fence_after();
+                    const uint64_t at = (uint64_t)s * (S::STAGE >> 4);
+#pragma unroll
+                    for (int kk = 0; kk < BK / UMMA_K; ++kk) umma_bf16_pair_elect(tmem_acc, desc_a + at + 2 * kk, desc_b + at + 2 * kk, idesc, (kb | kk) != 0);
+                    umma_commit_pair_elect(empty_bar + s);
+                }
+                if (ok) umma_commit_pair_elect(acc_full + acc);
+            }
+        }
+    } else {
+        const int quarter = warp & 3, half = (warp - 2) >> 2;                  // the 32 lanes this warp may read; its half of the columns
+        const int units = epilogue_units<EPI>(bn), u0 = half ? (units + 1) / 2 : 0, u1 = half ? units : (units + 1) / 2;
+        int it = 0;
+        pdl_wait();      // outputs may alias what the kernel before still reads; step metadata is older than that kernel
+        for (int tile = pair; tile < total_tiles && ok; tile += pairs, ++it) {
+            const int acc = it & 1;
+            const int m0 = tile % tiles_m * 2 * BM + rank * BM, n0 = tile / tiles_m * tile_n;
+            const int row = m0 + quarter * 32 + lane;
+            int pos = 0, page = -1;
+            if (EPI == EPI_ROPE && row < m) {
+                pos = ep.positions[row];
+                page = ep.block_table[(size_t)ep.req_slot[ep.token_req[row]] * ep.table_width + pos / ep.page_size];
+            }
+            ok = __all_sync(0xffffffffu, mbar_wait(acc_full + acc, (it >> 1) & 1));
+            if (!ok) break;
+            tcgen05_fence_after();
+            const uint32_t lane_base = tmem_base + (uint32_t)(acc * PAIR_BN) + ((uint32_t)(quarter * 32) << 16);
+            epilogue_tile<EPI>(ep, bn, [&](int c, uint32_t (&v)[32]) { tmem_load32(lane_base + (uint32_t)c, v); }, u0, u1, row, m, n, n0, pos, page,
+                                        tiles + S::TILES + 256 + (warp - 2) * STAGE_BYTES);
+            tcgen05_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(in_cluster(acc_empty + acc, 0));
+        }
+    }
+    if (!ok && lane == 0) atomicExch(error, 1);
+    __syncwarp();
+    tcgen05_fence_before();
+    cluster_meet();                      // neither CTA leaves while the other's products read its tiles or its barriers are told
+    if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(2 * PAIR_BN) : "memory");
 }
 
 // ---------------------------------------------------------------- host side
@@ -607,8 +820,9 @@ int launch(const void* a, const void* w, const Epilogue& ep, int m, int n, int k
                          map_a, map_w, ep, m, n, k, tiles_m, tiles_n, g_error);
 }
 
-// 128 x 256 tiles read a third less from L2 per flop than 128 x 128; worth it once there are enough of them to
-// occupy most of the device (one CTA per SM at that size).
+// Grouped products: 128 x 256 tiles read a third less from L2 per flop than 128 x 128; worth it once there are enough of them to occupy
+// most of the device (one CTA per SM at that size).  Three stages of 128 x 128 tiles keep a CTA near 100 KB of shared memory, so that two share an SM
+// and one's epilogue overlaps the other's main loop.
 bool wide_tiles(int m, int tiles_n256) { return (long long)((m + BM - 1) / BM) * tiles_n256 >= 120; }
 
 template <int BN, int MT, int STAGES, int EPI>
@@ -630,16 +844,15 @@ int launch_split(const void* a, const void* w, const Epilogue& ep, int m, int n,
 }
 
 // How the kernel for few tiles takes a product of m rows and cols64 tiles of 64 columns, max64 and max128 the shares of K that tiles
-// of 64 and 128 columns can be cut in (0: no such tiles); mt 0: not at all, the persistent kernel is better (or CISR_GEMM_DEEP=0).
+// of 64 and 128 columns can be cut in (0: no such tiles); mt 0: not at all, the pair kernel is better (or CISR_GEMM_DEEP=0).
 // - K to 2048 and tiles of 64 columns fit the SMs at one each: those, cut in two from 24 blocks of K on where there is room.  us,
 //   64 and 128 columns wide: 576 x 576, 200 rows 6.0 and 7.6; 2048 x 2048, 64 rows 7.6 and 8.7; 512 rows 9.9 and 10.4.
 // - tiles of 128 columns fit: K cut in as many shares as fit, of at least eight blocks each.  A longer K wants the wider tiles,
 //   which read the activations half as often: 2048 x 8192, 64 rows, 64 CTAs either way: 14 us, 17 with 64 columns.
-// - tiles of 256 columns fit, or do for two row tiles that share them: those.  us, in the persistent kernel (whose 128 x 128 tiles
-//   read half as much again) and here: 4096 x 14336, 800 rows 170 and 88; 6144 x 4096, 512 rows 46 and 34; gated 28672 x 4096, 200
-//   rows 63 and 56; gated 3584 x 4096, 1024 rows 45 and 28.
-// - more rows or columns: the persistent kernel, whose epilogues run beside the next tile's products (2048 x 2048, 2048 rows: 19
-//   us; 24 here).
+// - K to 1024 and tiles of 256 columns fit, or do for two row tiles that share them: those, which are done before a pair of CTAs has met.
+//   us, here and in the pair kernel: gated 1536 x 576, 1400 rows 9.5 and 10.7; gated 3072 x 1024, 700 rows 12.0 and 12.6; a longer K
+//   is the pairs': gated 14336 x 4096, 200 rows 57 and 53.
+// - more rows or columns: the pair kernel (2048 x 2048, 700 rows 11.3 here and 13.2 there, 1400 rows 17.2 and 14.9).
 // A plain product of at most 64 columns (a router's few outputs) is a column of row tiles: a long K is cut in two where the tiles
 // leave room for it (us, 2048 rows of K 2048 12.6 in the persistent kernel and 7.5, of K 4096 21.0 and 10.3; 9472 rows 13.0 and 8.3,
 // 21.5 and 11.3); a shorter one, or more row tiles, go to the persistent kernel with tiles of 64 columns (K 1024: 8.3).
@@ -660,6 +873,7 @@ SplitChoice split_choice(int m, int cols64, int k, int max64, int max128, int sm
         while (2 * shares <= max128 && 2 * shares * tiles128 <= sms && blocks >= 16 * shares) shares *= 2;
         return {128, 1, shares};
     }
+    if (blocks > 16) return {0, 0, 0};
     if (tiles_m * ((cols128 + 1) / 2) <= sms) return {256, 1, 1};
     if (tiles_m == 2 && (cols128 + 1) / 2 <= sms) return {256, 2, 1};
     return {0, 0, 0};
@@ -676,6 +890,50 @@ int launch_split_choice(SplitChoice c, const void* a, const void* w, const Epilo
     return c.mt == 1 ? launch_split<256, 1, 4, EPI>(a, w, ep, m, n, k, 1, s) : launch_split<256, 2, 3, EPI>(a, w, ep, m, n, k, 1, s);
 }
 
+// The tile width of the pair kernel for m rows and `cols` output columns (features of a gated product), of the first `widths` bits'
+// widths: the one with the least estimate, 3.9 + bn / 76 + c b (r + 0.4 t) us with b blocks of K,
+// r rounds and t rounds' worth of tiles over the pairs (a busy chip runs at a lower clock) and c below.  The constants were fitted to 407 plain
+// products of 11 sizes and 11 numbers of rows, within 2.8 %; the width they pick is the best of five but for 0.3 % on the average of 118
+// products, plain and gated.
+int pair_width(int m, int cols, int k, bool paired, unsigned widths, int pairs) {
+    static const struct { int bn; double block; } WIDTHS[] = {{256, .262}, {224, .2318}, {192, .204}, {160, .1929}, {128, .1881}};
+    const long long tiles_m = (m + 2 * BM - 1) / (2 * BM);
+    int best = 0;
+    double least = 0.;
+    for (int i = 0; i < 5; ++i) {
+        if (!(widths >> i & 1)) continue;
+        const int bn = WIDTHS[i].bn, tile = paired ? bn / 2 : bn;
+        const long long tiles = tiles_m * ((cols + tile - 1) / tile), rounds = (tiles + pairs - 1) / pairs;
+        const double us = 3.9 + 3.36 / 256 * bn + WIDTHS[i].block * ((k + BK - 1) / BK) * (rounds + .4 * tiles / pairs);
+        if (!best || us < least) { best = bn; least = us; }
+    }
+    return best;
+}
+// rotated: whole heads per tile, 256, 192 or 128 columns, at head size 128 not 192
+unsigned pair_widths(int dim) { return dim == 0 ? 0x1f : dim == 64 ? 0x15 : 0x11; }
+int device_pairs() {
+    static int pairs = 0;
+    if (!pairs) { int device = 0, sms = 0; cudaGetDevice(&device); cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device); pairs = sms / 2; }
+    return pairs;
+}
+template <int EPI>
+int launch_pair(const void* a, const void* w, const Epilogue& ep, int m, int n, int k, int bn, cudaStream_t s) {
+    CUtensorMap map_a, map_w;
+    int status = cached_map(&map_a, a, m, k, BM);
+    if (status) return status;
+    if ((status = cached_map(&map_w, w, n, k, bn / 2))) return status;
+    static bool configured = false;
+    if (!configured) {
+        cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_pair_kernel<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PairSmem::TOTAL);
+        if (e != cudaSuccess) return (int)e;
+        configured = true;
+    }
+    const int tile_n = paired_rows(EPI) ? bn / 2 : bn, cols = paired_rows(EPI) ? n / 2 : n;
+    const int tiles_m = (m + 2 * BM - 1) / (2 * BM), tiles_n = (cols + tile_n - 1) / tile_n, total = tiles_m * tiles_n, pairs = device_pairs();
+    return launch_kernel(gemm_tcgen05_pair_kernel<EPI>, dim3(2 * (total < pairs ? total : pairs)), dim3(PAIR_THREADS), PairSmem::TOTAL, s,
+                         g_pdl, map_a, map_w, ep, m, n, k, bn, tiles_m, tiles_n, g_error);
+}
+
 bool operands_ok(const void* a, const void* w, int k) {
     return g_encode && g_error && k > 0 && k % 8 == 0 && !(((uintptr_t)a | (uintptr_t)w) & 15);
 }
@@ -690,18 +948,22 @@ CISR_EXPORT int cisr_gemm_tcgen05_init(int* error_flag) {
 
 CISR_EXPORT void cisr_gemm_tcgen05_set_pdl(int on) { g_pdl = on != 0; }
 
-// How the plain product of these sizes is made on a device of `sms` SMs: 0 by the persistent kernel, else the columns of a tile x 100
+// How the plain product of these sizes is made on a device of `sms` SMs: 0 by a persistent kernel, else the columns of a tile x 100
 // + its row tiles x 10 + the shares of K.
 CISR_EXPORT int cisr_gemm_tcgen05_plain_choice(int m, int n, int k, int sms) {
     const SplitChoice c = split_choice(m, (n + 63) / 64, k, 2, 4, sms);
     return c.bn * 100 + c.mt * 10 + c.shares;
 }
 
+// The columns of the pair kernel's tiles on a device of `sms` SMs; paired: of a gated product of `cols` features; dim: of the rotated projection with
+// heads of that size, else 0.
+CISR_EXPORT int cisr_gemm_tcgen05_pair_width(int m, int cols, int k, int paired, int dim, int sms) {
+    return pair_width(m, cols, k, paired != 0, pair_widths(dim), sms / 2);
+}
+
 // How many tensor maps the library remembers before it empties its cache (tests lower it to force evictions).
 CISR_EXPORT void cisr_gemm_tcgen05_set_map_cache_limit(int entries) { g_map_cache_limit = entries < 1 ? 1 : (size_t)entries; }
 
-// Three pipeline stages keep a CTA near 100 KB of shared memory, so two CTAs share an SM and one's epilogue overlaps
-// the other's main loop.
 // accumulate != 0: out += a w^T (each output element is read, added to in float and written by the one thread that
 // owns it: what the residual add of a layer does, without a pass of its own).  out_mult: the product is multiplied by it
 // before it is written or added (1: as it is).
@@ -715,8 +977,7 @@ CISR_EXPORT int cisr_gemm_tcgen05(const void* a, const void* w, float* out, int 
     cudaStream_t s = (cudaStream_t)stream;
     if (const SplitChoice c = split_choice(m, (n + 63) / 64, k, 2, 4); c.mt) return launch_split_choice<EPI_PLAIN>(c, a, w, ep, m, n, k, s);
     if (n <= 64) return launch<64, 8, EPI_PLAIN>(a, w, ep, m, n, k, 1, s);
-    if (wide_tiles(m, (n + 255) / 256)) return launch<256, 4, EPI_PLAIN>(a, w, ep, m, n, k, (n + 255) / 256, s);
-    return launch<128, 3, EPI_PLAIN>(a, w, ep, m, n, k, (n + 127) / 128, s);
+    return launch_pair<EPI_PLAIN>(a, w, ep, m, n, k, pair_width(m, n, k, false, pair_widths(0), device_pairs()), s);
 }
 
 // w stacks gate rows [0, inter) over up rows [inter, 2 * inter); out (bfloat16 [m, inter]) = act(a gate^T) * (a up^T), act silu (gate_act 0)
@@ -729,26 +990,14 @@ CISR_EXPORT int cisr_gemm_tcgen05_swiglu(const void* a, const void* w, void* out
     Epilogue ep = {};
     ep.out_bf16 = (bf16*)out; ep.inter = inter; ep.act = gate_act;
     const SplitChoice few = split_choice(m, (inter + 31) / 32, k, 1, 2);
+    const int bn = pair_width(m, inter, k, true, pair_widths(0), device_pairs());
     if (gate_act == 2) {
         ep.limit = gate_limit; ep.alpha = 1.702f;
         if (few.mt) return launch_split_choice<EPI_GATED>(few, a, w, ep, m, 2 * inter, k, (cudaStream_t)stream);
-        if (wide_tiles(m, (inter + 127) / 128))
-            return launch<256, 4, EPI_GATED>(a, w, ep, m, 2 * inter, k, (inter + 127) / 128, (cudaStream_t)stream);
-        return launch<128, 3, EPI_GATED>(a, w, ep, m, 2 * inter, k, (inter + 63) / 64, (cudaStream_t)stream);
+        return launch_pair<EPI_GATED>(a, w, ep, m, 2 * inter, k, bn, (cudaStream_t)stream);
     }
     if (few.mt) return launch_split_choice<EPI_SWIGLU>(few, a, w, ep, m, 2 * inter, k, (cudaStream_t)stream);
-    if (wide_tiles(m, (inter + 127) / 128)) {
-        // 128 x 256 tiles, or 128 x 192 where their last round would be much emptier: 192 tiles of 256 columns on 148 SMs
-        // are two rounds for 1.3 rounds of work, 256 tiles of 192 columns are two rounds of three quarters the length
-        static int sms = 0;
-        if (!sms) { int device = 0; cudaGetDevice(&device); cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device); if (sms <= 0) sms = 148; }
-        const long long tiles_m = (m + BM - 1) / BM;
-        const long long rounds256 = (tiles_m * ((inter + 127) / 128) + sms - 1) / sms, rounds192 = (tiles_m * ((inter + 95) / 96) + sms - 1) / sms;
-        if (rounds192 * 192 * 10 <= rounds256 * 256 * 9)
-            return launch<192, 4, EPI_SWIGLU>(a, w, ep, m, 2 * inter, k, (inter + 95) / 96, (cudaStream_t)stream);
-        return launch<256, 4, EPI_SWIGLU>(a, w, ep, m, 2 * inter, k, (inter + 127) / 128, (cudaStream_t)stream);
-    }
-    return launch<128, 3, EPI_SWIGLU>(a, w, ep, m, 2 * inter, k, (inter + 63) / 64, (cudaStream_t)stream);
+    return launch_pair<EPI_SWIGLU>(a, w, ep, m, 2 * inter, k, bn, (cudaStream_t)stream);
 }
 
 // w stacks the q, k and v heads; q and k heads are rotated (pairs (i, i + dim / 2), cos/sin [m, dim / 2]); q goes to
@@ -767,8 +1016,7 @@ CISR_EXPORT int cisr_gemm_tcgen05_rope(const void* a, const void* w, int m, int 
     ep.table_width = table_width; ep.page_size = page_size; ep.hq = hq; ep.hkv = hkv; ep.dim = dim;
     const int n = (hq + 2 * hkv) * dim;
     if (const SplitChoice c = split_choice(m, (n + 63) / 64, k, dim == 64 ? 1 : 0, 2); c.mt) return launch_split_choice<EPI_ROPE>(c, a, w, ep, m, n, k, (cudaStream_t)stream);
-    if (wide_tiles(m, (n + 255) / 256)) return launch<256, 4, EPI_ROPE>(a, w, ep, m, n, k, (n + 255) / 256, (cudaStream_t)stream);
-    return launch<128, 3, EPI_ROPE>(a, w, ep, m, n, k, (n + 127) / 128, (cudaStream_t)stream);
+    return launch_pair<EPI_ROPE>(a, w, ep, m, n, k, pair_width(m, n, k, false, pair_widths(dim), device_pairs()), (cudaStream_t)stream);
 }
 
 // The product of rows sorted by group with each group's own weight matrix: a [m, k] with every group's rows padded to
