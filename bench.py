@@ -568,11 +568,11 @@ DESIGN_SIZES = {"1024": (1024, 8, 16, 2048, 16, 4), "2048": (2048, 8, 32, 4096, 
 KERNEL_KIND = {   # which kernels of the two designs are alike
     "gemm_tcgen05": "product, many tokens", "gemm_library": "product, many tokens", "gemm_tcgen05_swiglu": "feed-forward product, many tokens",
     "gemm_tcgen05_rope": "product, many tokens", "gemm_tcgen05_grouped": "feed-forward product, many tokens",
-    "gemm_tcgen05_grouped_gated": "feed-forward product, many tokens", "skinny_gemm": "product, few tokens",
+    "gemm_tcgen05_experts": "feed-forward product, many tokens", "skinny_gemm": "product, few tokens",
     "moe_rows": "feed-forward product, few tokens", "gemm_heads": "product per head", "attn_prefill_wide": "prompt attention", "attn_prefill": "prompt attention",
     "attn_decode": "decode attention", "merge_out_proj": "product, few tokens", "add_rmsnorm": "norm", "embedding": "row kernels", "embedding_pairs": "row kernels", "rope_store": "row kernels",
     "latent_rows": "row kernels", "latent_query": "row kernels", "latent_gate": "row kernels", "latent_absorb": "product per head",
-    "latent_values": "product per head", "moe_select": "row kernels", "moe_gather": "row kernels",
+    "latent_values": "product per head", "moe_select": "row kernels", "moe_scatter": "row kernels",
     "moe_combine": "row kernels", "moe_sort": "bookkeeping", "stream_add": "row kernels", "swiglu": "row kernels",
     "hyper_mix_norm": "norm", "attention_rows": "row kernels", "activation": "row kernels", "delta_prepare": "row kernels",
     "delta_output": "row kernels", "delta_keep": "bookkeeping", "delta_recurrence": "recurrence", "delta_chunks": "recurrence",
@@ -593,9 +593,9 @@ def generic_need(name: str, shape: tuple, cache_tokens: int, causal: int):
     if name == "gemm_tcgen05_grouped":
         m, groups, n, k, relu2 = shape
         return (m * k + groups * n * k) * 2 + m * n * (2 if relu2 else 4), 2.0 * m * n * k
-    if name == "gemm_tcgen05_grouped_gated":
-        m, groups, n2, k = shape
-        return (m * k + groups * n2 * k) * 2 + m * (n2 // 2) * 2, 2.0 * m * n2 * k
+    if name == "gemm_tcgen05_experts":
+        m, groups, n, k, act = shape          # act 0: float out, 1: activated, 2: gated
+        return (m * k + groups * n * k) * 2 + m * (n * 4 if act == 0 else n * 2 // act), 2.0 * m * n * k
     if name == "gemm_heads":
         m, heads, a, b = shape
         return heads * a * b * 2 + m * heads * (a + b) * 2, 2.0 * m * heads * a * b
@@ -704,7 +704,7 @@ def generic_need(name: str, shape: tuple, cache_tokens: int, causal: int):
         return shape[0] * shape[1] * 6, 0.0
     if name == "latent_gate":
         return shape[0] * shape[1] * 10, 0.0
-    if name == "moe_gather":
+    if name == "moe_scatter":
         return shape[0] * shape[1] * 4, 0.0
     if name == "moe_combine":
         tokens, top, hidden = shape

@@ -26,6 +26,8 @@
 // frees its tensor memory and returns, and the host reports the failure.
 //
 // Parity: this is the product runtime/blas.py:41-56 of the reference hands to cuBLAS (C^T = W * X^T).
+#include <limits.h>
+
 #include "tcgen05.cuh"
 
 namespace {
@@ -34,6 +36,12 @@ enum : int { EPI_PLAIN = 0, EPI_SWIGLU = 1, EPI_ROPE = 2, EPI_RELU2 = 3, EPI_GAT
 // SWIGLU and GATED: the B tile is BN / 2 gate rows and the BN / 2 up rows of the same features
 __host__ __device__ constexpr bool paired_rows(int epi) { return epi == EPI_SWIGLU || epi == EPI_GATED; }
 constexpr int BK = 64, UMMA_K = 16;     // BM = 128 (tcgen05.cuh)
+
+// Where a role is in a ring of `stages`: the stage, and the parity of the turn it is on.
+struct RingAt {
+    int stage = 0; uint32_t turn = 0;
+    __device__ __forceinline__ void next(int stages) { if (++stage == stages) { stage = 0; turn ^= 1u; } }
+};
 
 struct Epilogue {                       // what the epilogue variants need beyond the accumulator
     float* out_f32; bf16* out_bf16; int inter;
@@ -495,53 +503,51 @@ gemm_tcgen05_split_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
     pdl_trigger();
 
     if (warp == 0) {
-        if (lane == 0) {
-            auto load_b = [&](int s, int kb) {
-                unsigned char* b_tile = tiles + s * S::STAGE + S::A_BYTES;
-                if (paired_rows(EPI)) {       // two boxes of BN/2 rows: gate rows n0.., up rows inter + n0..
-                    tma_load_2d(b_tile, &map_w, (kb0 + kb) * BK, n0, full_bar + s);
-                    tma_load_2d(b_tile + S::B_BYTES / 2, &map_w, (kb0 + kb) * BK, ep.inter + n0, full_bar + s);
-                } else {
-                    tma_load_2d(b_tile, &map_w, (kb0 + kb) * BK, n0, full_bar + s);
-                }
-            };
-            auto load_a = [&](int s, int kb) {
+        auto load_b = [&](int s, int kb) {
+            unsigned char* b_tile = tiles + s * S::STAGE + S::A_BYTES;
+            if (paired_rows(EPI)) {       // two boxes of BN/2 rows: gate rows n0.., up rows inter + n0..
+                tma_load_2d_elect(b_tile, &map_w, (kb0 + kb) * BK, n0, full_bar + s);
+                tma_load_2d_elect(b_tile + S::B_BYTES / 2, &map_w, (kb0 + kb) * BK, ep.inter + n0, full_bar + s);
+            } else {
+                tma_load_2d_elect(b_tile, &map_w, (kb0 + kb) * BK, n0, full_bar + s);
+            }
+        };
+        auto load_a = [&](int s, int kb) {
 #pragma unroll
-                for (int t = 0; t < MT; ++t) tma_load_2d(tiles + s * S::STAGE + t * (S::A_BYTES / MT), &map_a, (kb0 + kb) * BK, m0 + t * BM, full_bar + s);
-            };
-            // the weights do not come from the kernel before: the first stages' tiles of them are requested before the wait on it
-            const int early = k_blocks < STAGES ? k_blocks : STAGES;
-            for (int kb = 0; kb < early; ++kb) {
-                mbar_expect_tx(full_bar + kb, (uint32_t)S::STAGE);
-                load_b(kb, kb);
-            }
-            pdl_wait();
-            CISR_TRACE_WAITED();
-            for (int kb = 0; kb < early; ++kb) load_a(kb, kb);
-            for (int kb = early; kb < k_blocks; ++kb) {
-                const int s = kb % STAGES;
-                ok = mbar_wait(empty_bar + s, ((kb / STAGES) & 1) ^ 1);
-                if (!ok) break;
-                mbar_expect_tx(full_bar + s, (uint32_t)S::STAGE);
-                load_a(s, kb);
-                load_b(s, kb);
-            }
+            for (int t = 0; t < MT; ++t) tma_load_2d_elect(tiles + s * S::STAGE + t * (S::A_BYTES / MT), &map_a, (kb0 + kb) * BK, m0 + t * BM, full_bar + s);
+        };
+        // the weights do not come from the kernel before: the first stages' tiles of them are requested before the wait on it
+        const int early = k_blocks < STAGES ? k_blocks : STAGES;
+        for (int kb = 0; kb < early; ++kb) {
+            mbar_expect_tx_elect(full_bar + kb, (uint32_t)S::STAGE);
+            load_b(kb, kb);
+        }
+        pdl_wait();
+        CISR_TRACE_WAITED();
+        for (int kb = 0; kb < early; ++kb) load_a(kb, kb);
+        RingAt at{0, 1u};                                    // the second turn
+        for (int kb = early; kb < k_blocks; ++kb, at.next(STAGES)) {
+            ok = __all_sync(0xffffffffu, mbar_wait(empty_bar + at.stage, at.turn ^ 1));
+            if (!ok) break;
+            mbar_expect_tx_elect(full_bar + at.stage, (uint32_t)S::STAGE);
+            load_a(at.stage, kb);
+            load_b(at.stage, kb);
         }
     } else if (warp == 1) {
         constexpr uint32_t idesc = umma_idesc(BN);
         const uint64_t desc_a = umma_desc(tiles), desc_b = umma_desc(tiles + S::A_BYTES);      // addresses below 256 KB: sums stay in the field
-        for (int kb = 0; kb < k_blocks; ++kb) {
-            const int s = kb % STAGES;
-            ok = __all_sync(0xffffffffu, mbar_wait(full_bar + s, (kb / STAGES) & 1));
+        RingAt ring;
+        for (int kb = 0; kb < k_blocks; ++kb, ring.next(STAGES)) {
+            ok = __all_sync(0xffffffffu, mbar_wait(full_bar + ring.stage, ring.turn));
             if (!ok) break;
             tcgen05_fence_after();
-            const uint64_t at = (uint64_t)s * (S::STAGE >> 4);
+            const uint64_t at = (uint64_t)ring.stage * (S::STAGE >> 4);
 #pragma unroll
             for (int t = 0; t < MT; ++t)
 #pragma unroll
                 for (int kk = 0; kk < BK / UMMA_K; ++kk)
                     umma_bf16_elect(tmem_base + (uint32_t)(t * BN), desc_a + at + t * (S::A_BYTES / MT >> 4) + 2 * kk, desc_b + at + 2 * kk, idesc, (kb | kk) != 0);
-            umma_commit_elect(empty_bar + s);
+            umma_commit_elect(empty_bar + ring.stage);
         }
         if (ok) umma_commit_elect(acc_full);
     }
@@ -659,7 +665,7 @@ gemm_tcgen05_split_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
 // x 256 tile 0.29 us on an idle chip, 0.38 on a busy one), and the last round.  us, 128 x 256 tiles on one SM each and so: gated 14336 x 4096,
 // 2048 rows 330 and 315, 1000 rows 201 and 157, 512 rows 111 and 90; gated 8192 x 2048, 2048 rows 100 and 90; plain 6144 x 2048, 2533 rows 67 and
 // 50; 8192 x 2048, 2048 rows 65 and 52; 4096 x 14336, 2048 rows 184 and 166.
-constexpr int PAIR_STAGES = 6, PAIR_THREADS = 320, PAIR_BN = 256;
+constexpr int PAIR_STAGES = 6, PAIR_THREADS = 320, PAIR_BN = 256;      // stages of one block of K; half as many of two
 struct PairSmem {
     static constexpr size_t A_BYTES = (size_t)BM * BK * sizeof(bf16), B_BYTES = (size_t)PAIR_BN / 2 * BK * sizeof(bf16);
     static constexpr size_t STAGE = A_BYTES + B_BYTES, TILES = PAIR_STAGES * STAGE;
@@ -669,7 +675,7 @@ struct PairSmem {
 template <int EPI>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
 gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
-                         const Epilogue ep, int m, int n, int k, int bn, int tiles_m, int tiles_n, int* __restrict__ error) {
+                         const Epilogue ep, int m, int n, int k, int bn, int tiles_m, int tiles_n, int per, int* __restrict__ error) {
     CISR_TRACE_SCOPE(TRACE_GEMM_TCGEN05);
     extern __shared__ unsigned char smem_raw[];
     typedef PairSmem S;
@@ -682,7 +688,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
 
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const int rank = (int)blockIdx.x & 1, pair = (int)blockIdx.x >> 1, pairs = (int)gridDim.x >> 1;
-    const int k_blocks = (k + BK - 1) / BK, total_tiles = tiles_m * tiles_n;
+    const int stages = PAIR_STAGES / per, k_blocks = (k + per * BK - 1) / (per * BK), total_tiles = tiles_m * tiles_n;
     const int tile_n = paired_rows(EPI) ? bn / 2 : bn;
 
     if (threadIdx.x == 0) {
@@ -702,56 +708,62 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     pdl_trigger();
 
     if (warp == 0) {
-        if (lane == 0) {
-            const uint32_t full_first = in_cluster(full_bar, 0);
-            const uint32_t stage_bytes = 2 * (uint32_t)(S::A_BYTES + (size_t)bn / 2 * BK * sizeof(bf16));       // of both CTAs
-            // this CTA's half of the weight rows: of a tile's columns, or (paired) the gate rows here and the up rows there
-            const int w_off = paired_rows(EPI) ? rank * ep.inter : rank * (bn / 2);
-            auto load_b = [&](int s, int kb, int n0) { tma_load_2d_pair(tiles + s * S::STAGE + S::A_BYTES, &map_w, kb * BK, n0 + w_off, full_first + 8 * s); };
-            auto load_a = [&](int s, int kb, int m0) { tma_load_2d_pair(tiles + s * S::STAGE, &map_a, kb * BK, m0 + rank * BM, full_first + 8 * s); };
-            // the first stages' weights are requested before the wait on the kernel before, the activations after it
-            const int early = pair < total_tiles ? min(k_blocks, PAIR_STAGES) : 0;
-            for (int kb = 0; kb < early; ++kb) {
-                if (rank == 0) mbar_expect_tx(full_bar + kb, stage_bytes);
-                load_b(kb, kb, pair / tiles_m * tile_n);
-            }
-            pdl_wait();
-            CISR_TRACE_WAITED();
-            int kbg = 0;
-            for (int tile = pair; tile < total_tiles && ok; tile += pairs) {
-                const int m0 = tile % tiles_m * 2 * BM, n0 = tile / tiles_m * tile_n;
-                for (int kb = 0; kb < k_blocks; ++kb, ++kbg) {
-                    const int s = kbg % PAIR_STAGES;
-                    if (kbg >= early) {
-                        ok = mbar_wait(empty_bar + s, ((kbg / PAIR_STAGES) & 1) ^ 1);
-                        if (!ok) break;
-                        if (rank == 0) mbar_expect_tx(full_bar + s, stage_bytes);
-                        load_b(s, kb, n0);
-                    }
-                    load_a(s, kb, m0);
+        const uint32_t full_first = in_cluster(full_bar, 0);
+        const uint32_t stage_bytes = 2 * per * (uint32_t)(S::A_BYTES + (size_t)bn / 2 * BK * sizeof(bf16));       // of both CTAs
+        // this CTA's half of the weight rows: of a tile's columns, or (paired) the gate rows here and the up rows there
+        const int w_off = paired_rows(EPI) ? rank * ep.inter : rank * (bn / 2);
+        auto load = [&](unsigned char* to, const CUtensorMap* map, int kb, int row, uint32_t bar) {
+            if (per == 2) tma_load_3d_pair(to, map, 0, row, 2 * kb, bar);
+            else tma_load_2d_pair(to, map, kb * BK, row, bar);
+        };
+        auto load_b = [&](int s, int kb, int n0) { load(tiles + per * (s * S::STAGE + S::A_BYTES), &map_w, kb, n0 + w_off, full_first + 8 * s); };
+        auto load_a = [&](int s, int kb, int m0) { load(tiles + per * s * S::STAGE, &map_a, kb, m0 + rank * BM, full_first + 8 * s); };
+        // the first stages' weights are requested before the wait on the kernel before, the activations after it
+        const int early = pair < total_tiles ? min(k_blocks, stages) : 0;
+        for (int kb = 0; kb < early; ++kb) {
+            if (rank == 0) mbar_expect_tx_elect(full_bar + kb, stage_bytes);
+            load_b(kb, kb, pair / tiles_m * tile_n);
+        }
+        pdl_wait();
+        CISR_TRACE_WAITED();
+        int asked = early;                                       // blocks of the first tile whose weights are on their way
+        RingAt at;
+        for (int tile = pair; tile < total_tiles && ok; tile += pairs) {
+            const int m0 = tile % tiles_m * 2 * BM, n0 = tile / tiles_m * tile_n;
+            for (int kb = 0; kb < k_blocks; ++kb, at.next(stages)) {
+                if (asked) --asked;
+                else {
+                    ok = __all_sync(0xffffffffu, mbar_wait(empty_bar + at.stage, at.turn ^ 1));
+                    if (!ok) break;
+                    if (rank == 0) mbar_expect_tx_elect(full_bar + at.stage, stage_bytes);
+                    load_b(at.stage, kb, n0);
                 }
+                load_a(at.stage, kb, m0);
             }
         }
     } else if (warp == 1) {
         if (rank == 0) {
             const uint32_t idesc = umma_idesc_pair(bn);
-            const uint64_t desc_a = umma_desc(tiles), desc_b = umma_desc(tiles + S::A_BYTES);
-            int kbg = 0, it = 0;
+            const uint64_t desc_a = umma_desc(tiles), desc_b = umma_desc(tiles + per * S::A_BYTES);
+            const uint32_t b_group = (uint32_t)bn / 2 * BK * sizeof(bf16) >> 4;
+            RingAt ring;
+            int it = 0;
             for (int tile = pair; tile < total_tiles && ok; tile += pairs, ++it) {
                 const int acc = it & 1;
                 ok = __all_sync(0xffffffffu, mbar_wait(acc_empty + acc, ((it >> 1) & 1) ^ 1));
                 if (!ok) break;
                 tcgen05_fence_after();
                 const uint32_t tmem_acc = tmem_base + (uint32_t)(acc * PAIR_BN);
-                for (int kb = 0; kb < k_blocks; ++kb, ++kbg) {
-                    const int s = kbg % PAIR_STAGES;
-                    ok = __all_sync(0xffffffffu, mbar_wait(full_bar + s, (kbg / PAIR_STAGES) & 1));
+                for (int kb = 0; kb < k_blocks; ++kb, ring.next(stages)) {
+                    ok = __all_sync(0xffffffffu, mbar_wait(full_bar + ring.stage, ring.turn));
                     if (!ok) break;
                     tcgen05_fence_after();
-                    const uint64_t at = (uint64_t)s * (S::STAGE >> 4);
+                    const uint64_t at = (uint64_t)ring.stage * per * (S::STAGE >> 4);
+                    for (int g = 0; g < per; ++g)
 #pragma unroll
-                    for (int kk = 0; kk < BK / UMMA_K; ++kk) umma_bf16_pair_elect(tmem_acc, desc_a + at + 2 * kk, desc_b + at + 2 * kk, idesc, (kb | kk) != 0);
-                    umma_commit_pair_elect(empty_bar + s);
+                        for (int kk = 0; kk < BK / UMMA_K; ++kk)
+                            umma_bf16_pair_elect(tmem_acc, desc_a + at + g * (S::A_BYTES >> 4) + 2 * kk, desc_b + at + g * b_group + 2 * kk, idesc, (kb | g | kk) != 0);
+                    umma_commit_pair_elect(empty_bar + ring.stage);
                 }
                 if (ok) umma_commit_pair_elect(acc_full + acc);
             }
@@ -785,6 +797,207 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     __syncwarp();
     tcgen05_fence_before();
     cluster_meet();                      // neither CTA leaves while the other's products read its tiles or its barriers are told
+    if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(2 * PAIR_BN) : "memory");
+}
+
+// two warps that exchange values meet at a named barrier; both_ok: and whether both are
+__device__ __forceinline__ void meet_two(int barrier) { asm volatile("bar.sync %0, 64;" ::"r"(barrier) : "memory"); }
+__device__ __forceinline__ bool both_ok(int barrier, bool ok) {
+    uint32_t all;
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %1, 0;\n\tbar.red.and.pred q, %2, 64, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+                 : "=r"(all) : "r"((uint32_t)ok), "r"(barrier) : "memory");
+    return all != 0;
+}
+// A lane has feature f of the tokens row0, row0 + 1, ...: neighbours put their features together, a lane of two writes every other
+// token's.  `left` tokens are there; width (features per row) is even.
+template <int TOKENS>
+__device__ __forceinline__ void store_columns_bf16(bf16* out, int width, int row0, int left, int f, const float (&act)[TOKENS]) {
+    const bool odd = threadIdx.x & 1;
+    bf16* dst = out + (size_t)(row0 + odd) * width + (f & ~1);
+#pragma unroll
+    for (int j = 0; j < TOKENS; j += 2) {
+        const float other = __shfl_xor_sync(0xffffffffu, odd ? act[j] : act[j + 1], 1);
+        const __nv_bfloat162 p = odd ? __floats2bfloat162_rn(other, act[j + 1]) : __floats2bfloat162_rn(act[j], other);
+        if (f < width && j + odd < left) *reinterpret_cast<__nv_bfloat162*>(dst + (size_t)j * width) = p;
+    }
+}
+
+// ---------------------------------------------------------------- experts: weight rows on the lanes, tokens as columns
+// The products of rows sorted by expert (moe_sort), each expert's with its own matrix.  Where the rows are the 128 lanes of a tile an expert's
+// rows are padded to whole tiles, a quarter of all products for 256 rows an expert; here a pair of CTAs has 256 weight rows (A) and up to
+// 256 of an expert's rows as the columns (B), in steps of 32: tiles [i] = (expert, first row, rows, -), rows 0 from the last one on.  An expert's
+// further tiles follow one another, so its weights come from memory once.  Ring, barriers and accumulators as in the pair kernel.
+//   PLAIN   out float [rows, n]
+//   RELU2   out bfloat16 [rows, n], an activation of the product
+//   GATED   w has an expert's gate rows and then its up rows; a CTA's 128 lanes are 64 gate rows and the 64 up rows of the same features,
+//           and two epilogue warps exchange halves of their columns, so that each has both for 16 of 32 tokens; out bfloat16 [rows, n / 2]
+// us, 2048 tokens, 64 experts of which each token has eight, on rows padded to 128 and so: gated 1792 x 4096 253 and 229, 4096 x 896 165
+// and 145 (of which 113 are the bytes at the rate of memory, the float rows most of them).
+struct ExpertMaps { CUtensorMap w, rows[8]; };          // rows[i]: boxes of 16 (i + 1) of the sorted rows
+template <int EPI>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
+gemm_tcgen05_experts_kernel(const __grid_constant__ ExpertMaps maps, const Epilogue ep, int n, int k, const int4* __restrict__ tiles_list, int max_tiles,
+                            int per, int* __restrict__ error) {
+    CISR_TRACE_SCOPE(TRACE_GEMM_TCGEN05);
+    extern __shared__ unsigned char smem_raw[];
+    typedef PairSmem S;
+    unsigned char* tiles = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    uint64_t* full_bar = reinterpret_cast<uint64_t*>(tiles + S::TILES);
+    uint64_t* empty_bar = full_bar + PAIR_STAGES;
+    uint64_t* acc_full = empty_bar + PAIR_STAGES;
+    uint64_t* acc_empty = acc_full + 2;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+    const int rank = (int)blockIdx.x & 1, pair = (int)blockIdx.x >> 1, pairs = (int)gridDim.x >> 1;
+    const int stages = PAIR_STAGES / per, k_blocks = (k + per * BK - 1) / (per * BK);
+    const int cols = EPI == EPI_GATED ? n / 2 : n, tile_cols = EPI == EPI_GATED ? BM : 2 * BM, tiles_n = (cols + tile_cols - 1) / tile_cols;
+    const int total = max_tiles * tiles_n;
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < PAIR_STAGES; ++s) { mbar_init(full_bar + s, 1); mbar_init(empty_bar + s, 1); }
+        for (int b = 0; b < 2; ++b) { mbar_init(acc_full + b, 1); mbar_init(acc_empty + b, 16); }
+        mbar_init_fence();
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(2 * PAIR_BN) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    }
+    tcgen05_fence_before();
+    cluster_meet();
+    tcgen05_fence_after();
+    const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+    bool ok = true;
+    pdl_trigger();
+    pdl_wait();                          // the tiles come from a kernel before
+    // item i: the rows of tiles_list[i / tiles_n] with column tile i % tiles_n; every role walks the same items, and asks for the next one's rows early
+    const auto rows_of = [&](int item) { return item < total ? tiles_list[item / tiles_n] : make_int4(0, 0, 0, 0); };
+
+    if (warp == 0) {
+        const uint32_t full_first = in_cluster(full_bar, 0);
+        RingAt at;
+        int4 t = rows_of(pair), next;
+        for (int item = pair; t.z && ok; item += pairs, t = next) {
+            next = rows_of(item + pairs);
+            const int f0 = item % tiles_n * tile_cols, half = (t.z + 31) / 32 * 16;      // rows of the tile that each CTA brings
+            const int row0 = t.y + rank * half, w_row = t.x * n + f0 + rank * BM, side = f0 + rank * (BM / 2);
+            const uint32_t stage_bytes = 2 * per * (uint32_t)(S::A_BYTES + half * BK * sizeof(bf16));
+            const CUtensorMap* rows = &maps.rows[half / 16 - 1];
+            for (int kb = 0; kb < k_blocks; ++kb, at.next(stages)) {
+                unsigned char* stage = tiles + per * at.stage * S::STAGE;
+                ok = __all_sync(0xffffffffu, mbar_wait(empty_bar + at.stage, at.turn ^ 1));
+                if (!ok) break;
+                if (rank == 0) mbar_expect_tx_elect(full_bar + at.stage, stage_bytes);
+                const uint32_t bar = full_first + 8 * at.stage;
+                if (per == 2) {
+                    if (EPI == EPI_GATED) tma_load_4d_pair(stage, &maps.w, 0, side, 2 * t.x, 2 * kb, bar);
+                    else tma_load_3d_pair(stage, &maps.w, 0, w_row, 2 * kb, bar);
+                    tma_load_3d_pair(stage + 2 * S::A_BYTES, rows, 0, row0, 2 * kb, bar);
+                } else {
+                    if (EPI == EPI_GATED) {
+                        tma_load_2d_pair(stage, &maps.w, kb * BK, t.x * n + side, bar);
+                        tma_load_2d_pair(stage + S::A_BYTES / 2, &maps.w, kb * BK, t.x * n + cols + side, bar);
+                    } else {
+                        tma_load_2d_pair(stage, &maps.w, kb * BK, w_row, bar);
+                    }
+                    tma_load_2d_pair(stage + S::A_BYTES, rows, kb * BK, row0, bar);
+                }
+            }
+        }
+    } else if (warp == 1) {
+        if (rank == 0) {
+            const uint64_t desc_a = umma_desc(tiles), desc_b = umma_desc(tiles + per * S::A_BYTES);
+            RingAt ring;
+            int it = 0;
+            int4 t = rows_of(pair), next;
+            for (int item = pair; t.z && ok; item += pairs, ++it, t = next) {
+                next = rows_of(item + pairs);
+                const int acc = it & 1;
+                const uint32_t idesc = umma_idesc_pair((t.z + 31) / 32 * 32), b_group = (uint32_t)((t.z + 31) / 32 * 16) * BK * sizeof(bf16) >> 4;
+                ok = __all_sync(0xffffffffu, mbar_wait(acc_empty + acc, ((it >> 1) & 1) ^ 1));
+                if (!ok) break;
+                tcgen05_fence_after();
+                const uint32_t tmem_acc = tmem_base + (uint32_t)(acc * PAIR_BN);
+                for (int kb = 0; kb < k_blocks; ++kb, ring.next(stages)) {
+                    ok = __all_sync(0xffffffffu, mbar_wait(full_bar + ring.stage, ring.turn));
+                    if (!ok) break;
+                    tcgen05_fence_after();
+                    const uint64_t at = (uint64_t)ring.stage * per * (S::STAGE >> 4);
+                    for (int g = 0; g < per; ++g)
+#pragma unroll
+                        for (int kk = 0; kk < BK / UMMA_K; ++kk)
+                            umma_bf16_pair_elect(tmem_acc, desc_a + at + g * (S::A_BYTES >> 4) + 2 * kk, desc_b + at + g * b_group + 2 * kk, idesc, (kb | g | kk) != 0);
+                    umma_commit_pair_elect(empty_bar + ring.stage);
+                }
+                if (ok) umma_commit_pair_elect(acc_full + acc);
+            }
+        }
+    } else {
+        const int quarter = warp & 3, half = (warp - 2) >> 2;
+        unsigned char* patches = tiles + S::TILES + 256;
+        float* mine = reinterpret_cast<float*>(patches + (warp - 2) * STAGE_BYTES);      // [2][16 tokens][32 features]: GATED
+        const float* theirs = reinterpret_cast<const float*>(patches + ((warp - 2) ^ 2) * STAGE_BYTES);
+        const bool up = EPI == EPI_GATED && quarter >= 2;
+        const int meeting = 1 + half * 2 + (quarter & 1);                      // the named barrier of two warps that exchange
+        int it = 0, turn = 0;
+        int4 t = rows_of(pair), next;
+        for (int item = pair; t.z && ok; item += pairs, ++it, t = next) {
+            next = rows_of(item + pairs);
+            const int acc = it & 1, count = t.z, units = (count + 31) / 32;
+            const int u0 = half ? (units + 1) / 2 : 0, u1 = half ? units : (units + 1) / 2;
+            const int lane_feature = EPI == EPI_GATED ? rank * (BM / 2) + (quarter & 1) * 32 + lane : rank * BM + quarter * 32 + lane;
+            const int f = item % tiles_n * tile_cols + lane_feature;
+            ok = __all_sync(0xffffffffu, mbar_wait(acc_full + acc, (it >> 1) & 1));
+            if (EPI == EPI_GATED) ok = both_ok(meeting, ok);                   // or the one would wait for the other
+            if (!ok) break;
+            tcgen05_fence_after();
+            const uint32_t lane_base = tmem_base + (uint32_t)(acc * PAIR_BN) + ((uint32_t)(quarter * 32) << 16);
+            for (int u = u0; u < u1; ++u) {
+                uint32_t v[32];
+                tmem_load32(lane_base + 32 * u, v);
+                if (EPI == EPI_PLAIN) {
+                    float* dst = ep.out_f32 + (size_t)(t.y + 32 * u) * n + f;
+                    const int left = f < n ? count - 32 * u : 0;
+#pragma unroll
+                    for (int j = 0; j < 32; ++j)
+                        if (j < left) dst[(size_t)j * n] = __uint_as_float(v[j]);
+                } else if (EPI == EPI_RELU2) {
+                    const bool gelu = ep.act == 1;
+                    float act[32];
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) {
+                        const float z = __uint_as_float(v[j]), r = fmaxf(z, 0.f);
+                        act[j] = gelu ? 0.5f * z * (1.f + erff(z * 0.70710678118654752f)) : r * r;
+                    }
+                    store_columns_bf16(ep.out_bf16, n, t.y + 32 * u, count - 32 * u, f, act);
+                } else {
+                    // the gate warp keeps tokens 0..15 and sends the gates of 16..31, the up warp the other way round
+                    float* box = mine + turn * 512;
+                    const float* from = theirs + turn * 512;
+                    turn ^= 1;
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) box[j * 32 + lane] = __uint_as_float(up ? v[j] : v[16 + j]);
+                    meet_two(meeting);
+                    float act[16];
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) {
+                        const float own = __uint_as_float(up ? v[16 + j] : v[j]), other = from[j * 32 + lane];
+                        const float gv = fminf(up ? other : own, ep.limit), uv = fminf(fmaxf(up ? own : other, -ep.limit), ep.limit);
+                        act[j] = quotient(gv, 1.f + expf(-ep.alpha * gv)) * (uv + 1.f);
+                    }
+                    const int j0 = 32 * u + (up ? 16 : 0);
+                    store_columns_bf16(ep.out_bf16, cols, t.y + j0, count - j0, f, act);
+                }
+            }
+            tcgen05_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(in_cluster(acc_empty + acc, 0));
+        }
+    }
+    if (!ok && lane == 0) atomicExch(error, 1);
+    __syncwarp();
+    tcgen05_fence_before();
+    cluster_meet();
     if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(2 * PAIR_BN) : "memory");
 }
 
@@ -891,12 +1104,12 @@ int launch_split_choice(SplitChoice c, const void* a, const void* w, const Epilo
 }
 
 // The tile width of the pair kernel for m rows and `cols` output columns (features of a gated product), of the first `widths` bits'
-// widths: the one with the least estimate, 3.9 + bn / 76 + c b (r + 0.4 t) us with b blocks of K,
-// r rounds and t rounds' worth of tiles over the pairs (a busy chip runs at a lower clock) and c below.  The constants were fitted to 407 plain
-// products of 11 sizes and 11 numbers of rows, within 2.8 %; the width they pick is the best of five but for 0.3 % on the average of 118
-// products, plain and gated.
+// widths: the one with the least estimate, 3.7 + bn / 59 + c b (r + 0.45 t) us with b blocks of K,
+// r rounds and t rounds' worth of tiles over the pairs (a busy chip runs at a lower clock) and c below.  The constants were fitted to 620 plain
+// products of 11 sizes and 11 numbers of rows (4.5 %); the width they pick is behind the best of five by 0.2 % on the average of 173 products, plain and
+// gated.
 int pair_width(int m, int cols, int k, bool paired, unsigned widths, int pairs) {
-    static const struct { int bn; double block; } WIDTHS[] = {{256, .262}, {224, .2318}, {192, .204}, {160, .1929}, {128, .1881}};
+    static const struct { int bn; double block; } WIDTHS[] = {{256, .254}, {224, .2255}, {192, .199}, {160, .183}, {128, .162}};
     const long long tiles_m = (m + 2 * BM - 1) / (2 * BM);
     int best = 0;
     double least = 0.;
@@ -904,7 +1117,7 @@ int pair_width(int m, int cols, int k, bool paired, unsigned widths, int pairs) 
         if (!(widths >> i & 1)) continue;
         const int bn = WIDTHS[i].bn, tile = paired ? bn / 2 : bn;
         const long long tiles = tiles_m * ((cols + tile - 1) / tile), rounds = (tiles + pairs - 1) / pairs;
-        const double us = 3.9 + 3.36 / 256 * bn + WIDTHS[i].block * ((k + BK - 1) / BK) * (rounds + .4 * tiles / pairs);
+        const double us = 3.7 + bn / 59. + WIDTHS[i].block * ((k + BK - 1) / BK) * (rounds + .45 * tiles / pairs);
         if (!best || us < least) { best = bn; least = us; }
     }
     return best;
@@ -918,10 +1131,13 @@ int device_pairs() {
 }
 template <int EPI>
 int launch_pair(const void* a, const void* w, const Epilogue& ep, int m, int n, int k, int bn, cudaStream_t s) {
+    // Two blocks of K per stage, a box of each operand for both, in the narrowest tiles, whose boxes are small and whose products are done before the next
+    // two boxes are on their way: a block of K 0.16 us on an idle chip, 0.21 with a box for each.  Wider ones want the finer ring (3 % at 192).
+    const int per = bn < 160 && k % BK == 0 ? 2 : 1;
     CUtensorMap map_a, map_w;
-    int status = cached_map(&map_a, a, m, k, BM);
+    int status = cached_map(&map_a, a, m, k, BM, per * BK);
     if (status) return status;
-    if ((status = cached_map(&map_w, w, n, k, bn / 2))) return status;
+    if ((status = cached_map(&map_w, w, n, k, bn / 2, per * BK))) return status;
     static bool configured = false;
     if (!configured) {
         cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_pair_kernel<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PairSmem::TOTAL);
@@ -931,7 +1147,20 @@ int launch_pair(const void* a, const void* w, const Epilogue& ep, int m, int n, 
     const int tile_n = paired_rows(EPI) ? bn / 2 : bn, cols = paired_rows(EPI) ? n / 2 : n;
     const int tiles_m = (m + 2 * BM - 1) / (2 * BM), tiles_n = (cols + tile_n - 1) / tile_n, total = tiles_m * tiles_n, pairs = device_pairs();
     return launch_kernel(gemm_tcgen05_pair_kernel<EPI>, dim3(2 * (total < pairs ? total : pairs)), dim3(PAIR_THREADS), PairSmem::TOTAL, s,
-                         g_pdl, map_a, map_w, ep, m, n, k, bn, tiles_m, tiles_n, g_error);
+                         g_pdl, map_a, map_w, ep, m, n, k, bn, tiles_m, tiles_n, per, g_error);
+}
+
+template <int EPI>
+int launch_experts(const ExpertMaps& maps, const Epilogue& ep, int n, int k, const int4* tiles, int max_tiles, int items, cudaStream_t s) {
+    static bool configured = false;
+    if (!configured) {
+        const cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_experts_kernel<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PairSmem::TOTAL);
+        if (e != cudaSuccess) return (int)e;
+        configured = true;
+    }
+    const int pairs = device_pairs();
+    return launch_kernel(gemm_tcgen05_experts_kernel<EPI>, dim3(2 * (items < pairs ? items : pairs)), dim3(PAIR_THREADS), PairSmem::TOTAL, s, g_pdl, maps,
+                         ep, n, k, tiles, max_tiles, k % BK ? 1 : 2, g_error);
 }
 
 bool operands_ok(const void* a, const void* w, int k) {
@@ -1043,22 +1272,24 @@ CISR_EXPORT int cisr_gemm_tcgen05_grouped(const void* a, const void* w, void* ou
     return launch<128, 3, EPI_PLAIN>(a, w, ep, m, n, k, (n + 127) / 128, s, groups);
 }
 
-// The grouped product of gated experts with the activation as its epilogue: w [groups * 2 * inter, k] holds, per group,
-// inter gate rows and then inter up rows; out is bfloat16 [m, inter] = g' sigmoid(alpha g') (u' + 1) with
-// g' = min(gate, limit), u' = clamp(up, -limit, limit).  Rows and tile_group as for the grouped product above.
-CISR_EXPORT int cisr_gemm_tcgen05_grouped_gated(const void* a, const void* w, void* out, int m, int inter, int k, int groups,
-                                                const int* tile_group, float limit, float alpha, void* stream) {
-    if (m <= 0 || inter <= 0) return 0;
+// The products of rows sorted by expert: a [m, k], w [experts * n, k], tiles int4 [max_tiles] = (expert, first row, rows (at most 256), -), compact: rows 0
+// from the first unused one on.  act < 0: out float [m, n] = a_e w_e^T; 0, 1: out bfloat16 [m, n] = max(z, 0)^2 or the exact gelu;
+// 2: w holds an expert's n / 2 gate and then its n / 2 up rows, out bfloat16 [m, n / 2] = g' sigmoid(alpha g') (u' + 1).
+CISR_EXPORT int cisr_gemm_tcgen05_experts(const void* a, const void* w, void* out, int m, int n, int k, int experts, const int* tiles, int max_tiles,
+                                          int act, float limit, float alpha, void* stream) {
+    if (m <= 0 || n <= 0 || max_tiles <= 0) return 0;
     if (!g_encode || !g_error) return -13;
-    if (!operands_ok(a, w, k) || ((uintptr_t)out & 15) || m % BM || !tile_group || groups <= 0) return -2;
+    if (!operands_ok(a, w, k) || (((uintptr_t)out | (uintptr_t)tiles) & 15) || !tiles || experts <= 0 || n % 4) return -2;
     Epilogue ep = {};
-    ep.tile_group = tile_group;
-    ep.out_bf16 = (bf16*)out;
-    ep.inter = inter;
-    ep.limit = limit;
-    ep.alpha = alpha;
-    cudaStream_t s = (cudaStream_t)stream;
-    if (wide_tiles(m, (inter + 127) / 128))
-        return launch<256, 4, EPI_GATED>(a, w, ep, m, 2 * inter, k, (inter + 127) / 128, s, groups);
-    return launch<128, 3, EPI_GATED>(a, w, ep, m, 2 * inter, k, (inter + 63) / 64, s, groups);
+    ep.out_f32 = (float*)out; ep.out_bf16 = (bf16*)out; ep.act = act; ep.limit = limit; ep.alpha = alpha;
+    const bool gated = act == 2;
+    const int box_cols = k % BK ? BK : 2 * BK;
+    ExpertMaps maps;
+    int status = cached_map(&maps.w, w, (long long)experts * n, k, gated ? BM / 2 : BM, box_cols, gated && box_cols > BK ? 2 * experts : 1, 2);
+    for (int i = 0; i < 8 && !status; ++i) status = cached_map(&maps.rows[i], a, m, k, 16 * (i + 1), box_cols);
+    if (status) return status;
+    const long long items = (long long)max_tiles * ((n + 2 * BM - 1) / (2 * BM));
+    if (items > INT_MAX) return -2;
+    const auto go = act < 0 ? launch_experts<EPI_PLAIN> : act == 2 ? launch_experts<EPI_GATED> : launch_experts<EPI_RELU2>;
+    return go(maps, ep, n, k, (const int4*)tiles, max_tiles, (int)items, (cudaStream_t)stream);
 }

@@ -15,8 +15,8 @@
 //
 // Two shapes of the expert products.  Few tokens (and the float path): a warp per output feature, each chosen expert's
 // rows streamed once per token that chose it (moe_up_rows / moe_down_rows).  Many tokens in bfloat16: the pairs are
-// sorted by expert on the device (moe_sort), the activations gathered into that order (moe_gather), the two products run
-// as grouped tcgen05 products (gemm_tcgen05.cu, the first with the activation as its epilogue), and each token's rows
+// sorted by expert on the device (moe_sort), the activations copied into that order (moe_scatter), the two products run
+// with the experts' matrices (gemm_tcgen05.cu, the first with the activation as its epilogue), and each token's rows
 // are summed with the router's weights (moe_combine).
 #include "common.cuh"
 
@@ -255,25 +255,29 @@ CISR_EXPORT int cisr_moe_rows(const void* h, const void* w_up, const void* w_dow
 //   row_of[pair]        the row of pair t * top + k in the sorted layout
 //   src_token[row]      the token whose activations row `row` holds, -1 for padding (and for rows beyond the last tile used)
 //   tile_group[i]       the expert of row tile i, -1 for tiles beyond the last one used
+//   tiles[i]            (where asked for; src_token and tile_group may then be absent) (expert, first row, rows, 0): every expert's rows cut into
+//                       equal runs of up to `run` rows, in steps of 16, expert by expert; rows 0 beyond the last one
 // Pairs whose expert has no matrices (chosen >= n_experts: an identity expert) get row_of = -1 and no row.
-// One CTA; shared memory: 3 * n_experts ints.  Which row inside its expert's block a pair gets depends on the order the
+// One CTA; shared memory: 4 * n_experts ints.  Which row inside its expert's block a pair gets depends on the order the
 // atomics happen to run in; every row is computed by itself and a token's experts are summed in the router's order, so
 // the result does not.
 // The pairs are read SORT_BATCH per thread at a time, all on their way together: with one at a time the kernel waited for
-// memory once per 1024 pairs, twice over (16,384 pairs: 21 us, now 14).
+// memory once per 1024 pairs, twice over (16,384 pairs: 21 us, then 14; 6.5 without src_token, which only the layout's other readers ask for).
 constexpr int SORT_THREADS = 1024, SORT_BATCH = 16;
 __global__ void __launch_bounds__(SORT_THREADS)
 moe_sort_kernel(const int* __restrict__ chosen, int n_pairs, int top, int n_experts, int tile, int max_rows,
-                int* __restrict__ row_of, int* __restrict__ src_token, int* __restrict__ tile_group) {
+                int* __restrict__ row_of, int* __restrict__ src_token, int* __restrict__ tile_group, int4* __restrict__ tiles, int max_tiles, int run) {
     extern __shared__ int sort_smem[];
     int* count = sort_smem;
     int* offset = sort_smem + n_experts;
     int* fill = sort_smem + 2 * n_experts;
+    int* first_tile = sort_smem + 3 * n_experts;
     pdl_trigger();
     pdl_wait();
     for (int e = threadIdx.x; e < n_experts; e += SORT_THREADS) { count[e] = 0; fill[e] = 0; }
-    for (int r = threadIdx.x; r < max_rows; r += SORT_THREADS) src_token[r] = -1;
-    for (int i = threadIdx.x; i < max_rows / tile; i += SORT_THREADS) tile_group[i] = -1;
+    if (src_token) for (int r = threadIdx.x; r < max_rows; r += SORT_THREADS) src_token[r] = -1;
+    if (tile_group) for (int i = threadIdx.x; i < max_rows / tile; i += SORT_THREADS) tile_group[i] = -1;
+    if (tiles) for (int i = threadIdx.x; i < max_tiles; i += SORT_THREADS) tiles[i] = make_int4(0, 0, 0, 0);
     int e[SORT_BATCH];
     auto fetch = [&](int base) {
 #pragma unroll
@@ -292,21 +296,27 @@ moe_sort_kernel(const int* __restrict__ chosen, int n_pairs, int top, int n_expe
     }
     __syncthreads();
     if (threadIdx.x < 32) {                        // the experts' first rows: a running sum of whole tiles, 32 experts at a time
-        int at = 0;
+        int at = 0, runs_at = 0;
         for (int x0 = 0; x0 < n_experts; x0 += 32) {
             const int x = x0 + threadIdx.x, rows = x < n_experts ? (count[x] + tile - 1) / tile * tile : 0;
-            int sum = rows;
+            const int runs = x < n_experts && tiles ? (count[x] + run - 1) / run : 0;
+            int sum = rows, runs_sum = runs;
 #pragma unroll
             for (int off = 1; off < 32; off <<= 1) {
-                const int before = __shfl_up_sync(0xffffffffu, sum, off);
-                if ((int)threadIdx.x >= off) sum += before;
+                const int before = __shfl_up_sync(0xffffffffu, sum, off), runs_before = __shfl_up_sync(0xffffffffu, runs_sum, off);
+                if ((int)threadIdx.x >= off) { sum += before; runs_sum += runs_before; }
             }
-            if (x < n_experts) offset[x] = at + sum - rows;
+            if (x < n_experts) { offset[x] = at + sum - rows; first_tile[x] = runs_at + runs_sum - runs; }
             at += __shfl_sync(0xffffffffu, sum, 31);
+            runs_at += __shfl_sync(0xffffffffu, runs_sum, 31);
         }
     }
     __syncthreads();
-    for (int x = threadIdx.x; x < n_experts; x += SORT_THREADS)
+    for (int x = threadIdx.x; x < n_experts && tiles; x += SORT_THREADS) {
+        const int runs = (count[x] + run - 1) / run, each = runs ? ((count[x] + runs - 1) / runs + 15) / 16 * 16 : 0;
+        for (int i = 0; i < runs; ++i) tiles[first_tile[x] + i] = make_int4(x, offset[x] + i * each, max(0, min(each, count[x] - i * each)), 0);
+    }
+    for (int x = threadIdx.x; x < n_experts && tile_group; x += SORT_THREADS)
         for (int i = offset[x] / tile; i < (offset[x] + count[x] + tile - 1) / tile; ++i) tile_group[i] = x;
     for (int base = 0; base < n_pairs; base += SORT_BATCH * SORT_THREADS) {
         if (n_pairs > SORT_BATCH * SORT_THREADS) fetch(base);      // else they are still at hand
@@ -317,32 +327,28 @@ moe_sort_kernel(const int* __restrict__ chosen, int n_pairs, int top, int n_expe
             if (e[u] >= n_experts) { row_of[p] = -1; continue; }
             const int row = offset[e[u]] + atomicAdd(&fill[e[u]], 1);
             row_of[p] = row;
-            src_token[row] = p / top;
+            if (src_token) src_token[row] = p / top;
         }
     }
 }
 
-// sorted[row, :] = h[src_token[row], :]; a padding row (src_token < 0) gets zeros where `fill`, and else keeps what it holds: a row
-// of a product depends on its own row of the operand alone, and no one reads a padding row's.  16-byte copies (hidden * 2
-// bytes % 16 == 0).
-__global__ void __launch_bounds__(128)
-moe_gather_kernel(const uint4* __restrict__ h, const int* __restrict__ src_token, uint4* __restrict__ sorted, int row_vec, int fill) {
+// sorted[row_of[t * top + k], :] = h[t, :] for each of a token's `top` pairs that has a row: a token's row is read once for all of them (2048 rows of
+// 4096, eight experts each: 27 us where every sorted row fetched its token's, now 24, at the rate of memory).
+constexpr int SCATTER_THREADS = 256, SCATTER_ROWS = 8;       // rows asked for together
+__global__ void __launch_bounds__(SCATTER_THREADS)
+moe_scatter_kernel(const uint4* __restrict__ h, const int* __restrict__ row_of, uint4* __restrict__ sorted, int row_vec, int top) {
     pdl_trigger();
     pdl_wait();
-    const int row = blockIdx.x, src = src_token[row];
-    if (src < 0) {
-        if (fill)
-            for (int i = threadIdx.x; i < row_vec; i += 128) sorted[(size_t)row * row_vec + i] = make_uint4(0, 0, 0, 0);
-        return;
-    }
-    const uint4* from = h + (size_t)src * row_vec;
-    uint4* to = sorted + (size_t)row * row_vec;
-    for (int i = threadIdx.x; i < row_vec; i += 4 * 128) {      // four on their way together
-        uint4 v[4];
+    const int t = blockIdx.x, i = blockIdx.y * SCATTER_THREADS + threadIdx.x;
+    if (i >= row_vec) return;
+    const uint4 v = h[(size_t)t * row_vec + i];
+    for (int k0 = 0; k0 < top; k0 += SCATTER_ROWS) {
+        int row[SCATTER_ROWS];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) if (i + u * 128 < row_vec) v[u] = from[i + u * 128];
+        for (int u = 0; u < SCATTER_ROWS; ++u) row[u] = k0 + u < top ? row_of[(size_t)t * top + k0 + u] : -1;
 #pragma unroll
-        for (int u = 0; u < 4; ++u) if (i + u * 128 < row_vec) to[i + u * 128] = v[u];
+        for (int u = 0; u < SCATTER_ROWS; ++u)
+            if (row[u] >= 0) sorted[(size_t)row[u] * row_vec + i] = v;
     }
 }
 
@@ -404,22 +410,26 @@ moe_combine_runs_kernel(const float* __restrict__ sorted_out, const int* __restr
 }
 
 CISR_EXPORT int cisr_moe_sort(const int* chosen, int tokens, int top, int n_experts, int tile, int max_rows, int* row_of,
-                              int* src_token, int* tile_group, void* stream) {
+                              int* src_token, int* tile_group, int* tiles, int max_tiles, int run, void* stream) {
     if (tokens <= 0) return 0;
     // the padded blocks of all experts together: at most pairs + (experts in use) * (tile - 1) rows, in whole tiles
     const long long pairs = (long long)tokens * top, in_use = pairs < n_experts ? pairs : n_experts;
     if (tile <= 0 || max_rows % tile || max_rows < (pairs + in_use * (tile - 1)) / tile * tile) return -2;
-    const size_t smem = (size_t)3 * n_experts * sizeof(int);
+    // every expert in use has one run that is not full, and one more where its equal runs are rounded up
+    if (tiles && (run < 16 || run % 16 || max_tiles < pairs / run + in_use || ((uintptr_t)tiles & 15))) return -2;
+    if (!tiles && (!src_token || !tile_group)) return -2;
+    const size_t smem = (size_t)4 * n_experts * sizeof(int);
     if (smem > 48 * 1024) return -3;
     return launch_kernel(moe_sort_kernel, dim3(1), dim3(SORT_THREADS), smem, (cudaStream_t)stream, g_pdl, chosen, tokens * top, top, n_experts, tile,
-                         max_rows, row_of, src_token, tile_group);
+                         max_rows, row_of, src_token, tile_group, (int4*)tiles, max_tiles, run);
 }
 
-CISR_EXPORT int cisr_moe_gather(const void* h, const int* src_token, void* sorted, int rows, int hidden, int fill, void* stream) {
-    if (rows <= 0) return 0;
+CISR_EXPORT int cisr_moe_scatter(const void* h, const int* row_of, void* sorted, int tokens, int top, int hidden, void* stream) {
+    if (tokens <= 0) return 0;
     if ((hidden * 2) % 16 || (((uintptr_t)h | (uintptr_t)sorted) & 15)) return -2;
-    return launch_kernel(moe_gather_kernel, dim3(rows), dim3(128), 0, (cudaStream_t)stream, g_pdl, (const uint4*)h, src_token, (uint4*)sorted,
-                         hidden * 2 / 16, fill);
+    const int row_vec = hidden * 2 / 16;
+    return launch_kernel(moe_scatter_kernel, dim3(tokens, (row_vec + SCATTER_THREADS - 1) / SCATTER_THREADS), dim3(SCATTER_THREADS), 0, (cudaStream_t)stream, g_pdl, (const uint4*)h, row_of, (uint4*)sorted,
+                         row_vec, top);
 }
 
 CISR_EXPORT int cisr_moe_combine(const float* sorted_out, const int* row_of, const float* weight, int tokens, int top, int hidden,

@@ -77,10 +77,33 @@ __device__ __forceinline__ uint32_t in_cluster(const void* p, int rank) {
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
-// a copy into this CTA that completes on a barrier of either CTA of the pair
+// Copies called by a whole converged warp of which one lane issues, with operands that are the same in every lane: issued from a branch of a
+// single lane each took about a hundred cycles, as the products did.  The _pair forms complete on a barrier of either CTA of a pair
+// (in_cluster).
+#define TMA_ELECT(DIM, GROUP) "{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t@q cp.async.bulk.tensor." DIM GROUP ".shared::cluster.global.mbarrier::complete_tx::bytes "
+__device__ __forceinline__ void tma_load_2d_elect(void* dst, const CUtensorMap* map, int c0, int c1, uint64_t* bar) {
+    asm volatile(TMA_ELECT("2d", "") "[%0], [%1, {%2, %3}], [%4];\n\t}" ::"r"(smem_u32(dst)), "l"(map), "r"(c0), "r"(c1), "r"(smem_u32(bar)) : "memory");
+}
+__device__ __forceinline__ void tma_load_3d_elect(void* dst, const CUtensorMap* map, int c0, int c1, int c2, uint64_t* bar) {
+    asm volatile(TMA_ELECT("3d", "") "[%0], [%1, {%2, %3, %4}], [%5];\n\t}" ::"r"(smem_u32(dst)), "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(smem_u32(bar)) : "memory");
+}
+__device__ __forceinline__ void tma_load_4d_elect(void* dst, const CUtensorMap* map, int c0, int c1, int c2, int c3, uint64_t* bar) {
+    asm volatile(TMA_ELECT("4d", "") "[%0], [%1, {%2, %3, %4, %5}], [%6];\n\t}"
+                 ::"r"(smem_u32(dst)), "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(smem_u32(bar)) : "memory");
+}
 __device__ __forceinline__ void tma_load_2d_pair(void* dst, const CUtensorMap* map, int c0, int c1, uint32_t bar) {
-    asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-                 ::"r"(smem_u32(dst)), "l"(map), "r"(c0), "r"(c1), "r"(bar) : "memory");
+    asm volatile(TMA_ELECT("2d", ".cta_group::2") "[%0], [%1, {%2, %3}], [%4];\n\t}" ::"r"(smem_u32(dst)), "l"(map), "r"(c0), "r"(c1), "r"(bar) : "memory");
+}
+__device__ __forceinline__ void tma_load_3d_pair(void* dst, const CUtensorMap* map, int c0, int c1, int c2, uint32_t bar) {
+    asm volatile(TMA_ELECT("3d", ".cta_group::2") "[%0], [%1, {%2, %3, %4}], [%5];\n\t}" ::"r"(smem_u32(dst)), "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(bar) : "memory");
+}
+__device__ __forceinline__ void tma_load_4d_pair(void* dst, const CUtensorMap* map, int c0, int c1, int c2, int c3, uint32_t bar) {
+    asm volatile(TMA_ELECT("4d", ".cta_group::2") "[%0], [%1, {%2, %3, %4, %5}], [%6];\n\t}"
+                 ::"r"(smem_u32(dst)), "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(bar) : "memory");
+}
+#undef TMA_ELECT
+__device__ __forceinline__ void mbar_expect_tx_elect(uint64_t* bar, uint32_t bytes) {
+    asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t@q mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n\t}" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
 }
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");

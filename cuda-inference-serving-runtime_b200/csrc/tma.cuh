@@ -107,16 +107,31 @@ int make_map_nd(CUtensorMap* map, const void* base, int rank, const cuuint64_t* 
     return r == CUDA_SUCCESS ? 0 : -20 - (int)r;
 }
 
+// A row-major bfloat16 matrix [rows, cols], cols a multiple of 64, as [64][rows][cols / 64] (or [64][rows / halves][halves][cols / 64]: the rows in
+// `halves` equal runs), read in boxes of 64 columns x box_rows (of each of box_halves neighbouring runs) x two groups of columns, which land one
+// group after the other.
+int make_map_groups(CUtensorMap* map, const void* base, long long rows, int cols, int box_rows, long long halves, int box_halves) {
+    const cuuint64_t row = (cuuint64_t)cols * sizeof(__nv_bfloat16), groups = (cuuint64_t)(cols / 64);
+    if (halves <= 1) {
+        const cuuint64_t dims[3] = {64, (cuuint64_t)rows, groups}, strides[2] = {row, 128};
+        const cuuint32_t box[3] = {64, (cuuint32_t)box_rows, 2};
+        return make_map_nd(map, base, 3, dims, strides, box);
+    }
+    const cuuint64_t per = (cuuint64_t)(rows / halves), dims[4] = {64, per, (cuuint64_t)halves, groups}, strides[3] = {row, per * row, 128};
+    const cuuint32_t box[4] = {64, (cuuint32_t)box_rows, (cuuint32_t)box_halves, 2};
+    return make_map_nd(map, base, 4, dims, strides, box);
+}
+
 struct MapKey {
-    const void* base; long long rows; int cols, box_rows, box_cols;
+    const void* base; long long rows; int cols, box_rows, box_cols; long long halves;      // box_cols 128: two groups of 64, rows in `halves` runs
     bool operator==(const MapKey& o) const {
-        return base == o.base && rows == o.rows && cols == o.cols && box_rows == o.box_rows && box_cols == o.box_cols;
+        return base == o.base && rows == o.rows && cols == o.cols && box_rows == o.box_rows && box_cols == o.box_cols && halves == o.halves;
     }
 };
 struct MapKeyHash {
     size_t operator()(const MapKey& k) const {
         return std::hash<const void*>()(k.base) ^ ((size_t)k.rows * 1000003u) ^ ((size_t)k.cols * 7919u) ^
-               ((size_t)k.box_rows << 8) ^ (size_t)k.box_cols;
+               ((size_t)k.box_rows << 8) ^ (size_t)k.box_cols ^ ((size_t)k.halves << 20);
     }
 };
 std::unordered_map<MapKey, CUtensorMap, MapKeyHash> g_maps;     // a map describes geometry only, so it stays right while the address does
@@ -125,13 +140,13 @@ size_t g_map_cache_limit = 4096;                                // entries kept 
 // The tensor map for (base, shape, box), encoded once and then found again.  The map is COPIED into the caller's
 // storage: a launcher asks for several maps in a row, and a later call may empty the cache, so nothing may keep a
 // pointer into it.
-int cached_map(CUtensorMap* out, const void* base, long long rows, int cols, int box_rows, int box_cols = 64) {
-    const MapKey key{base, rows, cols, box_rows, box_cols};
+int cached_map(CUtensorMap* out, const void* base, long long rows, int cols, int box_rows, int box_cols = 64, long long halves = 1, int box_halves = 1) {
+    const MapKey key{base, rows, cols, box_rows, box_cols, halves};
     auto it = g_maps.find(key);
     if (it == g_maps.end()) {
         if (g_maps.size() >= g_map_cache_limit) g_maps.clear();
         CUtensorMap map;
-        const int status = make_map(&map, base, rows, cols, box_rows, box_cols);
+        const int status = box_cols == 128 ? make_map_groups(&map, base, rows, cols, box_rows, halves, box_halves) : make_map(&map, base, rows, cols, box_rows, box_cols);
         if (status) return status;
         it = g_maps.emplace(key, map).first;
     }

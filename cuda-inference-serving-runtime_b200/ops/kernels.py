@@ -1518,7 +1518,7 @@ def _moe():
     lib = _moe_state.get("lib")
     if lib is None:
         lib = load_library("moe.cu")
-        for name in ("cisr_moe_select", "cisr_moe_rows", "cisr_moe_sort", "cisr_moe_gather", "cisr_moe_combine"):
+        for name in ("cisr_moe_select", "cisr_moe_rows", "cisr_moe_sort", "cisr_moe_scatter", "cisr_moe_combine"):
             getattr(lib, name).restype = ctypes.c_int
         lib.cisr_moe_set_pdl(int(_pdl_state["on"]))
         _moe_state["lib"] = lib
@@ -1587,17 +1587,28 @@ def moe_rows(h: torch.Tensor, w_up: torch.Tensor, w_down: torch.Tensor, chosen: 
 
 EXPERT_ACTIVATIONS = {"relu_squared": 0, "gelu": 1}      # ungated expert activations as the kernels number them
 MOE_TILE = 128                   # rows per tile of the grouped product: each expert's rows are padded to whole tiles
-MOE_GROUPED_MIN_ROWS = 64        # (token, expert) pairs per expert, on average, from which sorting and the grouped product pay
+MOE_RUN = 256                    # most rows of a run of one expert's rows that the tensor-core products take as one tile
+MOE_GROUPED_MIN_ROWS = 64        # (token, expert) pairs per expert, on average, from which sorting and the products by expert pay for any width
+# Below that: `moe_rows` brings an expert's matrices once per pair (8 TB/s: mostly from L2), the products by expert once per expert in use (5 TB/s); they
+# are taken where that saves this many us, since they are three launches more.  us, rows and by expert: 16 experts of 768 + 1024 x 384 x 2 bytes, 4 per
+# token, 32 / 64 / 400 tokens 67 / 127 / 744 and 25 / 25 / 29; 64 experts of 1792 + 4096 x 896, 8 per token, 4 / 16 / 100 tokens 147 / 431 / 2194 and
+# 117 / 227 / 259.
+MOE_GROUPED_MIN_SAVED = 40.0
 
 
 def moe_grouped_ok(h: torch.Tensor, w_up: torch.Tensor, top: int, gated: bool = False) -> bool:
-    """Whether a step's experts run as grouped tcgen05 products: bfloat16, widths whose rows are 16-byte multiples, and
-    enough pairs per expert that whole 128-row tiles are mostly real rows."""
+    """Whether a step's experts run as tcgen05 products of rows sorted by expert: bfloat16, widths whose rows are 16-byte multiples, and enough
+    (token, expert) pairs."""
     experts, ff, hidden = w_up.shape
     if gated:
         ff //= 2
-    return (h.dtype == torch.bfloat16 and hidden % 8 == 0 and ff % 8 == 0 and h.shape[0] * top >= MOE_GROUPED_MIN_ROWS * experts
-            and h.shape[0] >= TCGEN05_MIN_TOKENS)
+    if h.dtype != torch.bfloat16 or hidden % 8 or ff % 8:
+        return False
+    pairs = h.shape[0] * top
+    if pairs >= MOE_GROUPED_MIN_ROWS * experts and h.shape[0] >= TCGEN05_MIN_TOKENS:
+        return True
+    matrices = (3 if gated else 2) * ff * hidden * 2
+    return pairs * matrices / 8e6 - min(pairs, experts) * matrices / 5e6 >= MOE_GROUPED_MIN_SAVED
 
 
 def moe_sorted_rows(tokens: int, top: int, experts: int) -> int:
@@ -1606,27 +1617,40 @@ def moe_sorted_rows(tokens: int, top: int, experts: int) -> int:
     return max(MOE_TILE, (pairs + min(pairs, experts) * (MOE_TILE - 1)) // MOE_TILE * MOE_TILE)
 
 
-def moe_sort(chosen: torch.Tensor, experts: int, row_of: torch.Tensor, src_token: torch.Tensor, tile_group: torch.Tensor) -> None:
+def moe_tiles(tokens: int, top: int, experts: int) -> int:
+    """Most runs of up to MOE_RUN rows that the experts' rows are cut into."""
+    return tokens * top // MOE_RUN + min(tokens * top, experts)
+
+
+def moe_sort(chosen: torch.Tensor, experts: int, row_of: torch.Tensor, src_token: Optional[torch.Tensor], tile_group: Optional[torch.Tensor],
+             tiles: Optional[torch.Tensor] = None, rows: Optional[int] = None) -> None:
     """Lay the (token, chosen expert) pairs out expert by expert, each expert's rows padded to whole tiles of MOE_TILE:
-    row_of[pair] = its row, src_token[row] = the token of that row (-1: padding), tile_group[tile] = its expert (-1: unused)."""
-    _need(chosen, torch.int32, "chosen", 2)
-    for name, t in (("row_of", row_of), ("src_token", src_token), ("tile_group", tile_group)):
-        _need(t, torch.int32, name, 1)
+    row_of[pair] = its row, src_token[row] = the token of that row (-1: padding), tile_group[tile] = its expert (-1: unused).
+    `tiles` int32 [moe_tiles, 4] (src_token and tile_group may then be None, `rows` the layout's rows): (expert, first row, rows, 0) of each run of up to
+    MOE_RUN rows, rows 0 beyond the last."""
+    _need(chosen, torch.int32, "chosen", 2); _need(row_of, torch.int32, "row_of", 1)
+    for name, t in (("src_token", src_token), ("tile_group", tile_group)):
+        if t is not None or tiles is None:
+            _need(t, torch.int32, name, 1)
     tokens, top = chosen.shape
-    rows = src_token.numel()
-    if row_of.numel() != tokens * top or rows % MOE_TILE or tile_group.numel() != rows // MOE_TILE:
+    rows = src_token.numel() if src_token is not None else rows
+    if (rows is None or row_of.numel() != tokens * top or rows % MOE_TILE or (tile_group is not None and tile_group.numel() != rows // MOE_TILE)):
         raise KernelError("moe_sort: shapes disagree")
-    _check(_moe().cisr_moe_sort(_p(chosen), tokens, top, experts, MOE_TILE, rows, _p(row_of), _p(src_token), _p(tile_group), _stream()),
-           "moe_sort")
+    if tiles is not None:
+        _need(tiles, torch.int32, "tiles", 2)
+        if tiles.shape[1] != 4:
+            raise KernelError("moe_sort: tiles must be [n, 4]")
+    _check(_moe().cisr_moe_sort(_p(chosen), tokens, top, experts, MOE_TILE, rows, _p(row_of), _p(src_token), _p(tile_group), _p(tiles),
+                                0 if tiles is None else tiles.shape[0], MOE_RUN, _stream()), "moe_sort")
 
 
-def moe_gather(h: torch.Tensor, src_token: torch.Tensor, sorted_h: torch.Tensor, fill: bool = True) -> torch.Tensor:
-    """sorted_h[row] = h[src_token[row]] (bfloat16 rows of 16-byte multiples); where src_token[row] < 0 zeros, or with
-    `fill` False whatever the row holds."""
-    _need(h, torch.bfloat16, "h", 2); _need(sorted_h, torch.bfloat16, "sorted_h", 2); _need(src_token, torch.int32, "src_token", 1)
-    if sorted_h.shape != (src_token.numel(), h.shape[1]):
-        raise KernelError("moe_gather: shapes disagree")
-    _check(_moe().cisr_moe_gather(_p(h), _p(src_token), _p(sorted_h), sorted_h.shape[0], h.shape[1], int(fill), _stream()), "moe_gather")
+def moe_scatter(h: torch.Tensor, row_of: torch.Tensor, sorted_h: torch.Tensor) -> torch.Tensor:
+    """sorted_h[row_of[t * top + k]] = h[t] for every pair that has a row (bfloat16 rows of 16-byte multiples); other rows keep what they hold."""
+    _need(h, torch.bfloat16, "h", 2); _need(sorted_h, torch.bfloat16, "sorted_h", 2); _need(row_of, torch.int32, "row_of", 1)
+    tokens, hidden = h.shape
+    if sorted_h.shape[1] != hidden or row_of.numel() % max(1, tokens):
+        raise KernelError("moe_scatter: shapes disagree")
+    _check(_moe().cisr_moe_scatter(_p(h), _p(row_of), _p(sorted_h), tokens, row_of.numel() // max(1, tokens), hidden, _stream()), "moe_scatter")
     return sorted_h
 
 
@@ -1650,8 +1674,8 @@ def moe_combine(sorted_out: torch.Tensor, row_of: torch.Tensor, weight: torch.Te
 def moe_grouped(h: torch.Tensor, w_up: torch.Tensor, w_down: torch.Tensor, chosen: torch.Tensor, weight: torch.Tensor,
                 out: torch.Tensor, out_scale: Optional[torch.Tensor] = None, gate_limit: Optional[float] = None,
                 activation: str = "relu_squared") -> torch.Tensor:
-    """The same sum as `moe_rows` for many tokens: pairs sorted by expert on the device, activations gathered into that
-    order, both products as grouped tcgen05 products (the activation, relu^2 or the clamped gated form over the stacked
+    """The same sum as `moe_rows` for many tokens: pairs sorted by expert on the device, activations copied into that
+    order, both products on the tensor cores with each expert's matrix (the activation, relu^2 or the clamped gated form over the stacked
     gate and up rows, as the first one's epilogue), rows summed per token with the router's weights in the router's
     order.  Nothing is read back to the host."""
     _need(w_up, torch.bfloat16, "w_up", 3); _need(w_down, torch.bfloat16, "w_down", 3)
@@ -1665,18 +1689,12 @@ def moe_grouped(h: torch.Tensor, w_up: torch.Tensor, w_down: torch.Tensor, chose
     rows = moe_sorted_rows(tokens, top, experts)
     device = h.device
     row_of = torch.empty(tokens * top, dtype=torch.int32, device=device)
-    src_token = torch.empty(rows, dtype=torch.int32, device=device)
-    tile_group = torch.empty(rows // MOE_TILE, dtype=torch.int32, device=device)
-    moe_sort(chosen, experts, row_of, src_token, tile_group)
-    # a padding row's products are read by no one, and a row's depend on it alone: the padding is not filled
-    sorted_h = moe_gather(h, src_token, torch.empty((rows, hidden), dtype=torch.bfloat16, device=device), fill=False)
-    if gate_limit is None:
-        act = gemm_tcgen05_grouped(sorted_h, w_up, torch.empty((rows, ff), dtype=torch.bfloat16, device=device), tile_group, tokens * top,
-                                   activation=activation)
-    else:
-        act = gemm_tcgen05_grouped_gated(sorted_h, w_up, torch.empty((rows, ff), dtype=torch.bfloat16, device=device), tile_group,
-                                         gate_limit, tokens * top)
-    sorted_out = gemm_tcgen05_grouped(act, w_down, torch.empty((rows, hidden), dtype=torch.float32, device=device), tile_group, tokens * top)
+    tiles = torch.empty((moe_tiles(tokens, top, experts), 4), dtype=torch.int32, device=device)
+    moe_sort(chosen, experts, row_of, None, None, tiles, rows)
+    # a padding row's products are made by no one: the padding is not filled
+    sorted_h = moe_scatter(h, row_of, torch.empty((rows, hidden), dtype=torch.bfloat16, device=device))
+    act = gemm_tcgen05_experts(sorted_h, w_up, torch.empty((rows, ff), dtype=torch.bfloat16, device=device), tiles, tokens * top, activation, gate_limit)
+    sorted_out = gemm_tcgen05_experts(act, w_down, torch.empty((rows, hidden), dtype=torch.float32, device=device), tiles, tokens * top)
     return moe_combine(sorted_out, row_of, weight, out, out_scale, h=h)
 
 
@@ -2005,7 +2023,7 @@ def _tcgen05():
         lib.cisr_gemm_tcgen05_swiglu.restype = ctypes.c_int
         lib.cisr_gemm_tcgen05_rope.restype = ctypes.c_int
         lib.cisr_gemm_tcgen05_grouped.restype = ctypes.c_int
-        lib.cisr_gemm_tcgen05_grouped_gated.restype = ctypes.c_int
+        lib.cisr_gemm_tcgen05_experts.restype = ctypes.c_int
         _check(lib.cisr_gemm_tcgen05_init(_p(_error_flag())), "tcgen05 gemm init", own=0)
         lib.cisr_gemm_tcgen05_set_pdl(int(_pdl_state["on"]))
         _tcgen05_state["lib"] = lib
@@ -2074,19 +2092,22 @@ def tcgen05_rope_ok(dim: int, rot_half: int, interleaved: bool) -> bool:
     return dim in (64, 128) and 2 * rot_half == dim and not interleaved
 
 
-def gemm_tcgen05_grouped_gated(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, tile_group: torch.Tensor, limit: float,
-                               rows_in_use: Optional[int] = None) -> torch.Tensor:
-    """The grouped product of gated experts with the activation as its epilogue: rows of `a` as for `gemm_tcgen05_grouped`,
-    w bfloat16 [groups, 2 ff, K] (a group's gate rows, then its up rows), out bfloat16 [M, ff] =
-    g' sigmoid(1.702 g') (u' + 1) with g' = min(gate, limit), u' = clamp(up, -limit, limit) from the float sums."""
-    _need(a, torch.bfloat16, "a", 2); _need(w, torch.bfloat16, "w", 3); _need(out, torch.bfloat16, "out", 2); _need(tile_group, torch.int32, "tile_group", 1)
+def gemm_tcgen05_experts(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, tiles: torch.Tensor, rows_in_use: Optional[int] = None,
+                         activation: str = "relu_squared", gate_limit: Optional[float] = None) -> torch.Tensor:
+    """Runs of rows of `a` (bfloat16 [M, K]), each with its expert's matrix (w bfloat16 [experts, N, K]); tiles int32 [n, 4] as `moe_sort` makes
+    them.  out float [M, N]: the products; out bfloat16 [M, N]: the activation of the products; with `gate_limit` (w an expert's gate rows, then its up
+    rows) out bfloat16 [M, N / 2] = g' sigmoid(1.702 g') (u' + 1) with g' = min(gate, limit), u' = clamp(up, -limit, limit) from the float
+    sums.  Rows outside the runs are not written.  `rows_in_use` only labels measurements."""
+    _need(a, torch.bfloat16, "a", 2); _need(w, torch.bfloat16, "w", 3); _need(tiles, torch.int32, "tiles", 2)
+    _need(out, None if gate_limit is None else torch.bfloat16, "out", 2)
     m, k = a.shape
-    groups, n2, _ = w.shape
-    ff = out.shape[1]
-    if w.shape[2] != k or n2 != 2 * ff or out.shape[0] != m or m % 128 or tile_group.numel() != m // 128:
-        raise KernelError(f"gemm grouped gated: shapes a{tuple(a.shape)} w{tuple(w.shape)} out{tuple(out.shape)} disagree")
-    _check(_tcgen05().cisr_gemm_tcgen05_grouped_gated(_p(a), _p(w), _p(out), m, ff, k, groups, _p(tile_group), ctypes.c_float(limit),
-                                                      ctypes.c_float(GATE_ALPHA), _stream()), "gemm_tcgen05_grouped_gated")
+    experts, n, _ = w.shape
+    if (w.shape[2] != k or out.shape != (m, n if gate_limit is None else n // 2) or n % 4 or tiles.shape[1] != 4
+            or out.dtype not in (torch.float32, torch.bfloat16)):
+        raise KernelError(f"gemm experts: shapes a{tuple(a.shape)} w{tuple(w.shape)} out{tuple(out.shape)} disagree")
+    act = 2 if gate_limit is not None else EXPERT_ACTIVATIONS[activation] if out.dtype == torch.bfloat16 else -1
+    _check(_tcgen05().cisr_gemm_tcgen05_experts(_p(a), _p(w), _p(out), m, n, k, experts, _p(tiles), tiles.shape[0], act,
+                                                ctypes.c_float(gate_limit or 0.0), ctypes.c_float(GATE_ALPHA), _stream()), "gemm_tcgen05_experts")
     return out
 
 
@@ -2187,12 +2208,12 @@ _DESCRIBE = {
     "moe_select": lambda logits, *a, **kw: (int(logits.shape[0]), int(logits.shape[1])),
     "moe_rows": lambda h, w_up, w_down, chosen, *a, **kw: (int(h.shape[0]), int(w_up.shape[0]), int(w_up.shape[1]), int(w_up.shape[2]), int(chosen.shape[1])),
     "moe_sort": lambda chosen, experts, *a: (int(chosen.shape[0]), int(chosen.shape[1]), int(experts)),
-    "moe_gather": lambda h, src_token, sorted_h, fill=True: (int(sorted_h.shape[0]), int(sorted_h.shape[1])),
+    "moe_scatter": lambda h, row_of, sorted_h: (int(row_of.numel()), int(sorted_h.shape[1])),
     "moe_combine": lambda sorted_out, row_of, weight, out, out_scale=None, h=None: (int(out.shape[0]), int(weight.shape[1]), int(out.shape[1])),
     "gemm_tcgen05_grouped": lambda a, w, out, tile_group, rows_in_use=None, activation="relu_squared":
         (int(rows_in_use or a.shape[0]), int(w.shape[0]), int(w.shape[1]), int(w.shape[2]), out.dtype == torch.bfloat16),
-    "gemm_tcgen05_grouped_gated": lambda a, w, out, tile_group, limit, rows_in_use=None:
-        (int(rows_in_use or a.shape[0]), int(w.shape[0]), int(w.shape[1]), int(w.shape[2])),
+    "gemm_tcgen05_experts": lambda a, w, out, tiles, rows_in_use=None, activation="relu_squared", gate_limit=None:
+        (int(rows_in_use or a.shape[0]), int(w.shape[0]), int(w.shape[1]), int(w.shape[2]), 2 if gate_limit is not None else int(out.dtype == torch.bfloat16)),
     "gemm_heads": lambda a, w, out, w_is_nk: (int(a.shape[0]), int(w.shape[0]), int(w.shape[1]), int(w.shape[2])),
     "swiglu": lambda gate_up, out, gate="silu", limit=None: (int(out.shape[0]), int(out.shape[1])),
     "rotary_tables": lambda positions, inv_freq, cos, sin, magnitude=1.0: (int(cos.shape[0]), int(cos.shape[1])),

@@ -3,7 +3,7 @@ import pytest
 import torch
 
 SIZES = [(257, 9000, 1096), (1400, 5184, 1096), (600, 9000, 264), (1400, 4000, 1032), (2533, 2052, 1032), (300, 37001, 72), (2049, 5184, 136), (511, 22222, 200), (4000, 700, 1096)]
-GATED = [(1000, 2052, 1096), (1000, 4804, 1096), (513, 9001, 136), (2533, 700, 1096), (2100, 2056, 72), (300, 8192, 1096), (1281, 3000, 264)]
+GATED = [(1000, 2052, 1096), (2049, 5184, 1096), (2049, 5184, 136), (1000, 4804, 1096), (513, 9001, 136), (2533, 700, 1096), (2100, 2056, 72), (300, 8192, 1096), (1281, 3000, 264)]
 ROTATED = [(700, 64, 16, 64, 264), (2533, 32, 32, 64, 136), (1500, 32, 8, 128, 72), (300, 66, 40, 128, 1096), (520, 64, 64, 64, 1096)]
 
 
