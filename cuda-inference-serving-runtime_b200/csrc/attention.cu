@@ -41,9 +41,6 @@ typedef __nv_bfloat16 st_t;
 typedef float st_t;
 #endif
 
-// float tensors with heads of up to 128: products of split floats on the tensor cores (attention_split.cuh)
-#define SPLIT_PREFILL (!STORAGE_BF16 && HEAD_DIM <= 128)
-
 namespace {
 constexpr int D = HEAD_DIM;
 constexpr int VEC = 16 / sizeof(st_t);  // elements per 16-byte load
@@ -63,7 +60,6 @@ __device__ __forceinline__ void load_vec(const st_t* p, float* out) {
 
 // ------------------------------------------------------------------ prefill
 constexpr int BM = 64;
-#if !SPLIT_PREFILL
 constexpr int BN = (D <= 128) ? 64 : (D <= 256) ? 32 : 16;
 constexpr int NJ = BN / 16;  // score columns per thread
 constexpr int ND = D / 16;   // output columns per thread
@@ -227,8 +223,6 @@ attn_prefill_kernel(const st_t* __restrict__ q, st_t* __restrict__ out, const st
         for (int j = 0; j < ND; ++j) dst[tx + 16 * j] = from_float<st_t>(o[i][j] * inv);
     }
 }
-
-#endif
 
 // ------------------------------------------------------------------ decode (split over key ranges)
 constexpr int DEC_THREADS = 128;
@@ -404,9 +398,6 @@ __global__ void attn_merge_kernel(const float* __restrict__ partial, const float
     }
 }
 }  // namespace
-#if SPLIT_PREFILL
-#include "attention_split.cuh"
-#endif
 
 CISR_EXPORT int cisr_attn_head_dim() { return D; }
 CISR_EXPORT int cisr_attn_storage_bf16() { return STORAGE_BF16; }
@@ -420,24 +411,6 @@ CISR_EXPORT int cisr_attn_prefill(const void* q, void* out, const void* k_cache,
     if (n_tiles <= 0) return 0;
     if (hq % hkv || (SOFTCAP ? !(softcap > 0.f) : softcap != 0.f)) return -2;
     static bool configured = false;
-#if SPLIT_PREFILL
-    static int sms = 0;
-    if (!configured) {
-        const cudaError_t e = cudaFuncSetAttribute(attn_prefill_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SPLIT_SMEM);
-        if (e != cudaSuccess) return (int)e;
-        int device = 0;
-        cudaGetDevice(&device);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-        configured = true;
-    }
-    const int ctas = hq * n_tiles * (BM / SPLIT_ROWS);
-    SplitAttention a = {};
-    a.q = (const float*)q; a.out = (float*)out; a.k_cache = (const float*)k_cache; a.v_cache = (const float*)v_cache;
-    a.req_slot = req_slot; a.block_table = block_table; a.table_width = table_width; a.tile_req = tile_req; a.tile_q0 = tile_q0;
-    a.q_start = q_start; a.q_len = q_len; a.ctx_len = ctx_len; a.sink_heads = sink_heads; a.hq = hq; a.hkv = hkv; a.page_size = page_size;
-    a.window = window; a.keep_first = keep_first; a.scale = scale; a.softcap = softcap; a.sink = sink; a.one_round = ctas > sms && ctas <= 2 * sms ? sms : 0;
-    attn_prefill_split_kernel<<<dim3(ctas), SPLIT_THREADS, SPLIT_SMEM, (cudaStream_t)stream>>>(a);
-#else
     if (!configured) {
         cudaError_t e = cudaFuncSetAttribute(attn_prefill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PREFILL_SMEM);
         if (e != cudaSuccess) return (int)e;
@@ -446,7 +419,6 @@ CISR_EXPORT int cisr_attn_prefill(const void* q, void* out, const void* k_cache,
     attn_prefill_kernel<<<dim3(n_tiles, hq), PREFILL_THREADS, PREFILL_SMEM, (cudaStream_t)stream>>>(
         (const st_t*)q, (st_t*)out, (const st_t*)k_cache, (const st_t*)v_cache, req_slot, block_table, table_width, tile_req,
         tile_q0, q_start, q_len, ctx_len, hq, hkv, page_size, scale, softcap, window, keep_first, sink, sink_heads);
-#endif
     return launch_status();
 }
 

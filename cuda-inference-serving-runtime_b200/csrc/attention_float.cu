@@ -12,10 +12,19 @@
 //
 // Scores or outputs that are not finite (an infinity among the inputs, or a float that rounds to a bfloat16 infinity, has NaN among its
 // parts) send the CTA through plain_rows, which has float multiply-adds only.
-#pragma once
+//
+// Compiled once per HEAD_DIM, a multiple of 16 up to 128; with -DSOFTCAP=1 a score becomes cap tanh(score / cap) before the softmax.  Wider heads,
+// and single tokens, are attention.cu's, whose formulas these are.
 #include "split_mma.cuh"
+#include "softcap.cuh"
+
+#if !defined(HEAD_DIM) || (HEAD_DIM % 16) || (HEAD_DIM > 128) || (HEAD_DIM < 16)
+#error "compile with -DHEAD_DIM=<multiple of 16 between 16 and 128>"
+#endif
 
 namespace {
+constexpr int D = HEAD_DIM;
+constexpr int TILE = 64;                            // queries of a listed tile
 constexpr int SPLIT_ROWS = 32, WARP_KEYS = 16, KEYS = D <= 64 ? 64 : 32, SHARES = KEYS / WARP_KEYS;
 constexpr int SPLIT_THREADS = 2 * 32 * SHARES;
 constexpr int PLD = D + 8;                          // row stride of a plane: an odd number of 16-byte units, eight rows in different banks
@@ -306,3 +315,33 @@ attn_prefill_split_kernel(const __grid_constant__ SplitAttention a) {
     }
 }
 }  // namespace
+
+CISR_EXPORT int cisr_attn_float_head_dim() { return D; }
+CISR_EXPORT int cisr_attn_float_tile() { return TILE; }
+
+CISR_EXPORT int cisr_attn_prefill_float(const void* q, void* out, const void* k_cache, const void* v_cache,
+                                        const int* req_slot, const int* block_table, int table_width, const int* tile_req, const int* tile_q0,
+                                        int n_tiles, const int* q_start, const int* q_len, const int* ctx_len, int hq,
+                                        int hkv, int page_size, float scale, float softcap, int window, int keep_first, float sink,
+                                        const float* sink_heads, void* stream) {
+    if (n_tiles <= 0) return 0;
+    if (hq % hkv || (SOFTCAP ? !(softcap > 0.f) : softcap != 0.f)) return -2;
+    static bool configured = false;
+    static int sms = 0;
+    if (!configured) {
+        const cudaError_t e = cudaFuncSetAttribute(attn_prefill_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SPLIT_SMEM);
+        if (e != cudaSuccess) return (int)e;
+        int device = 0;
+        cudaGetDevice(&device);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+        configured = true;
+    }
+    const int ctas = hq * n_tiles * (TILE / SPLIT_ROWS);
+    SplitAttention a = {};
+    a.q = (const float*)q; a.out = (float*)out; a.k_cache = (const float*)k_cache; a.v_cache = (const float*)v_cache;
+    a.req_slot = req_slot; a.block_table = block_table; a.table_width = table_width; a.tile_req = tile_req; a.tile_q0 = tile_q0;
+    a.q_start = q_start; a.q_len = q_len; a.ctx_len = ctx_len; a.sink_heads = sink_heads; a.hq = hq; a.hkv = hkv; a.page_size = page_size;
+    a.window = window; a.keep_first = keep_first; a.scale = scale; a.softcap = softcap; a.sink = sink; a.one_round = ctas > sms && ctas <= 2 * sms ? sms : 0;
+    attn_prefill_split_kernel<<<dim3(ctas), SPLIT_THREADS, SPLIT_SMEM, (cudaStream_t)stream>>>(a);
+    return launch_status();
+}

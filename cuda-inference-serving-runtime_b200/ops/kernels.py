@@ -361,7 +361,9 @@ def attention_jobs(head_dim: int, dtype: torch.dtype, softcap: bool = False):
 
 
 def attention_tcgen05_jobs(head_dim: int, dtype: torch.dtype, softcap: bool = False):
-    """The build jobs of the tcgen05 prompt attention, where this head size and storage type have one."""
+    """The build jobs of the prompt attention on the tensor cores, where this head size and storage type have one of their own."""
+    if dtype == torch.float32 and head_dim <= FLOAT_PREFILL_MAX_HEAD_DIM and head_dim % 16 == 0:
+        return [("attention_float.cu", {"HEAD_DIM": head_dim, **({"SOFTCAP": 1} if softcap else {})}, ())]
     if dtype == torch.bfloat16 and head_dim in TCGEN05_HEAD_DIMS:
         return [("attention_tcgen05.cu", {"HEAD_DIM": head_dim, **({"SOFTCAP": 1} if softcap else {})}, ())]
     return []
@@ -370,6 +372,21 @@ def attention_tcgen05_jobs(head_dim: int, dtype: torch.dtype, softcap: bool = Fa
 TCGEN05_HEAD_DIMS = (64, 128)
 WIDE_TILE = 128                  # queries per tile of the tcgen05 prompt attention
 WIDE_PAIR = 2 * WIDE_TILE        # the same where a CTA takes two tiles
+FLOAT_PREFILL_MAX_HEAD_DIM = 128       # wider float heads stay on the CUDA cores
+_attention_float_libs = {}
+
+
+def _attention_float(head_dim: int, softcap: bool = False):
+    lib = _attention_float_libs.get((head_dim, softcap))
+    if lib is None:
+        if head_dim % 16:
+            raise KernelError(f"attention kernels take head sizes that are multiples of 16, not {head_dim}")
+        lib = load_library("attention_float.cu", {"HEAD_DIM": head_dim, **({"SOFTCAP": 1} if softcap else {})})
+        assert lib.cisr_attn_float_head_dim() == head_dim and lib.cisr_attn_float_tile() == PREFILL_TILE
+        _attention_float_libs[(head_dim, softcap)] = lib
+    return lib
+
+
 _attention_tcgen05_libs = {}
 
 
@@ -441,8 +458,11 @@ def attn_prefill(q, out, k_cache, v_cache, req_slot, block_table, tile_req, tile
     for name, t in (("req_slot", req_slot), ("block_table", block_table), ("tile_req", tile_req), ("tile_q0", tile_q0), ("q_start", q_start),
                     ("q_len", q_len), ("ctx_len", ctx_len)):
         _need(t, torch.int32, name)
-    lib = attention_library(dim, k_cache.dtype, kind, softcap is not None)
-    _check(lib.cisr_attn_prefill(_p(q), _p(out), _p(k_cache), _p(v_cache), _p(req_slot), _p(block_table), block_table.shape[1],
+    if kind == "auto" and k_cache.dtype == torch.float32 and dim <= FLOAT_PREFILL_MAX_HEAD_DIM:
+        launch = _attention_float(dim, softcap is not None).cisr_attn_prefill_float
+    else:
+        launch = attention_library(dim, k_cache.dtype, kind, softcap is not None).cisr_attn_prefill
+    _check(launch(_p(q), _p(out), _p(k_cache), _p(v_cache), _p(req_slot), _p(block_table), block_table.shape[1],
                                  _p(tile_req), _p(tile_q0), tile_req.numel(), _p(q_start), _p(q_len), _p(ctx_len),
                                  hq, hkv, page_size, ctypes.c_float(scale), _softcap(softcap), int(window or 0), int(keep_first or 0),
                                  *_sink(sink, hq), _stream()), "attn_prefill")
