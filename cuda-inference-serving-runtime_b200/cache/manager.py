@@ -75,6 +75,7 @@ class PageGroup:
             # [entries, key|value, pages, kv_heads, page_size, head_dim]; one plane where a row serves as both
             self.storage = torch.zeros((len(entries), use.planes, n_pages, use.kv_heads, page_size, use.head_dim), dtype=dtype,
                                        device=device)
+            self.planes = [(s[0], s[use.planes - 1]) for s in self.storage]      # each entry's keys and values
             self.device_table = torch.full((max_slots + 1, width), -1, dtype=torch.int32, device=device)   # last row: the null slot
         self.host_table = np.full((max_slots, width), -1, dtype=np.int32)
         self.updates: List[Tuple[int, int]] = []   # (flat index into the table, page id)
@@ -96,6 +97,7 @@ class StateGroup:
         if device is not None:
             self.storage = torch.zeros((len(entries), max_slots + 1) + tuple(use.state_shape),
                                        dtype=getattr(torch, use.state_dtype), device=device)
+            self.states = list(self.storage)                                     # each entry's [slots, ...]
 
 
 class CacheManager:
@@ -315,16 +317,16 @@ class CacheManager:
         kind, gi = kind_group
         if kind == "pages":
             g = self.page_groups[gi]
-            e = g.entry_slot[source]
-            return PagedBinding(g.storage[e, 0], g.storage[e, g.use.planes - 1], g.device_table, g.page_size,
+            k, v = g.planes[g.entry_slot[source]]
+            return PagedBinding(k, v, g.device_table, g.page_size,
                                 write=reads_from is None, window=g.use.window, keep_first=g.use.keep_first, state=self.side_state(entry))
         g = self.state_groups[gi]
-        return StateBinding(g.storage[g.entry_slot[source]])
+        return StateBinding(g.states[g.entry_slot[source]])
 
     def side_state(self, place: int) -> Optional[torch.Tensor]:
         """The side state [slots, ...] asked for at `place` of `side_states`, or None."""
         side = self.entry_side.get(place)
-        return None if side is None else self.state_groups[side[0]].storage[side[1]]
+        return None if side is None else self.state_groups[side[0]].states[side[1]]
 
     # ---------------------------------------------------------------- checks and reports
     def check(self) -> None:

@@ -28,8 +28,8 @@ ARCH_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a"]
 BASE_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "--shared", "-Xcompiler", "-fPIC,-fvisibility=hidden",
               "--expt-relaxed-constexpr"]
 
-_loaded: Dict[str, ctypes.CDLL] = {}
-_plain: Dict[str, ctypes.CDLL] = {}      # those without definitions, by source name
+_loaded: Dict[str, "KernelLibrary"] = {}
+_plain: Dict[str, "KernelLibrary"] = {}      # those without definitions, by source name
 _lock = threading.Lock()
 
 
@@ -175,7 +175,52 @@ def _drop_superseded(target: Path) -> None:
                 pass
 
 
-def load_library(source_name: str, defines: Optional[Mapping[str, object]] = None, extra: Sequence[str] = ()) -> ctypes.CDLL:
+_EXPORT = re.compile(r"^CISR_EXPORT\s+(int|void|float|long long)\s+(\w+)\(([^)]*)\)", re.MULTILINE)
+
+
+def _ctype(declaration: str):
+    if "*" in declaration:
+        return ctypes.c_void_p
+    words = declaration.split()
+    if "float" in words or "double" in words:
+        return ctypes.c_float if "float" in words else ctypes.c_double
+    if words.count("long") == 2:
+        return ctypes.c_longlong
+    if words[0] != "int" or len(words) != 2:
+        raise BuildError(f"an exported function has a parameter of a type that calls are not made with: {declaration.strip()!r}")
+    return ctypes.c_int
+
+
+def exported_signatures(source: Path) -> dict:
+    """name -> (result type, parameter types) of the functions that a source and the files it includes export, as they are declared there."""
+    out = {}
+    for path in source_closure(source):
+        for result, name, parameters in _EXPORT.findall(path.read_text()):
+            out[name] = (None if result == "void" else ctypes.c_float if result == "float" else ctypes.c_longlong if result == "long long" else ctypes.c_int,
+                         [_ctype(d) for d in parameters.split(",")] if parameters.strip() else [])
+    return out
+
+
+class KernelLibrary(ctypes.CDLL):
+    """A built library whose functions have the types they are declared with: an address, a number or a handle is then passed as
+    it is (a third of a launch's time in Python went to wrapping each argument), and a call with too few or wrong ones fails.  A function that is
+    not declared in the sources is refused: called without types it would lose half of every address."""
+
+    def __init__(self, path: Path, signatures: dict):
+        super().__init__(str(path))
+        self._signatures = signatures
+
+    def __getattr__(self, name: str):
+        if name.startswith("_"):
+            raise AttributeError(name)
+        if name not in self._signatures:
+            raise AttributeError(f"{name} is not declared in the sources of {self._name}")
+        fn = ctypes.CDLL.__getattr__(self, name)
+        fn.restype, fn.argtypes = self._signatures[name]
+        return fn
+
+
+def load_library(source_name: str, defines: Optional[Mapping[str, object]] = None, extra: Sequence[str] = ()) -> KernelLibrary:
     if not defines and not extra and source_name in _plain:        # the usual call, one per launch
         return _plain[source_name]
     key = repr((source_name, sorted((defines or {}).items()), list(extra)))
@@ -184,7 +229,7 @@ def load_library(source_name: str, defines: Optional[Mapping[str, object]] = Non
         if lib is None:
             path = compile_library(source_name, defines, extra)
             try:
-                lib = ctypes.CDLL(str(path))
+                lib = KernelLibrary(path, exported_signatures(CSRC / source_name))
             except OSError as err:
                 raise BuildError(f"could not load {path}: {err}") from err
             _loaded[key] = lib

@@ -55,7 +55,7 @@ def gated_product(h, gate_up: torch.Tensor, activation: str, limit=None) -> torc
     """act(h W_gate^T, h W_up^T) for the stacked matrices gate_up [2I, H], [tokens, I] in their type; `h` a tensor or a
     pending norm."""
     tokens = h.x.shape[0] if not isinstance(h, torch.Tensor) else h.shape[0]
-    act = torch.empty((tokens, gate_up.shape[0] // 2), dtype=gate_up.dtype, device=gate_up.device)
+    act = gate_up.new_empty((tokens, gate_up.shape[0] // 2))
     if kernels.skinny_ok(tokens, gate_up):
         # few tokens: (norm,) gate and up products and the activation in one launch
         gate = dict(epilogue=kernels.EPI_SWIGLU, out=act, gate=activation, gate_limit=limit)

@@ -13,11 +13,12 @@ from ..ops import kernels
 
 def linear(a: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
     """Few tokens (a decode step): the weight-streaming kernel; otherwise the library product."""
-    out = torch.empty((a.shape[0], w.shape[0]), dtype=torch.float32, device=a.device)
-    if a.shape[0] == 0:
+    tokens = a.shape[0]
+    out = a.new_empty((tokens, w.shape[0]), dtype=torch.float32)
+    if tokens == 0:
         return out
-    if kernels.skinny_ok(a.shape[0], w) and a.dtype == torch.bfloat16:
-        kernels.skinny_gemm(w, a.shape[0], act=a, epilogue=kernels.EPI_PLAIN, out=out)
+    if kernels.skinny_ok(tokens, w) and a.dtype == torch.bfloat16:
+        kernels.skinny_gemm(w, tokens, act=a, epilogue=kernels.EPI_PLAIN, out=out)
         return out
     return kernels.gemm(a, w, out)
 
@@ -54,6 +55,8 @@ def linear_add(a: torch.Tensor, w: torch.Tensor, into: torch.Tensor) -> torch.Te
 
 def norm_fusable(h, tokens: int, w: torch.Tensor) -> bool:
     """Whether `h` is a pending norm that this product can compute in its own prologue."""
+    if isinstance(h, torch.Tensor):
+        return False
     from .base import PendingNorm
     if not (isinstance(h, PendingNorm) and h.fusable() and tokens <= kernels.SKINNY_NORM_MAX_TOKENS
             and kernels.skinny_ok(tokens, w)):
@@ -77,14 +80,15 @@ def linear_normed(h, w: torch.Tensor, tokens: int) -> torch.Tensor:
 
 
 def as_tensor(h) -> torch.Tensor:
-    from .base import PendingNorm
-    return h.materialize_once() if isinstance(h, PendingNorm) else h
+    return h if isinstance(h, torch.Tensor) else h.materialize_once()
 
 
 def stream_target(h, tokens: int, width: int):
     """The residual stream's own tensor, when a product may add its result to it in place: `h` is the part's input as a
     `PendingNorm` that is resolved by now (the norm has run, here or inside a product, so `h.stream.x` holds x + the
     output before and nothing is pending), float, contiguous and [tokens, width].  Otherwise None."""
+    if isinstance(h, torch.Tensor):
+        return None
     from .base import PendingNorm
     if not (isinstance(h, PendingNorm) and h.resolved and h.in_place_ok and h.stream.pending is None):
         return None
