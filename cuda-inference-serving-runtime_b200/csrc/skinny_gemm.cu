@@ -565,3 +565,11 @@ CISR_EXPORT int cisr_skinny_gemm(const SkinnyCall* call) {
     if (m <= 32) return launch<4>(a, epilogue, s);
     return launch<8>(a, epilogue, s);
 }
+
+// Several products, each with what the one before it wrote: one call from the host for all of them (a call's way through the interpreter takes longer
+// than these kernels run).
+CISR_EXPORT int cisr_skinny_chain(const SkinnyCall* calls, int n) {
+    int status = 0;
+    for (int i = 0; i < n && !status; ++i) status = cisr_skinny_gemm(calls + i);
+    return status;
+}

@@ -2009,6 +2009,40 @@ def skinny_gemm(w: torch.Tensor, tokens: int, *, act: Optional[torch.Tensor] = N
     _check(_skinny().cisr_skinny_gemm(args), "skinny_gemm")
 
 
+def skinny_mlp_ok(h: torch.Tensor, gate_up: torch.Tensor, down: torch.Tensor) -> bool:
+    """Whether `skinny_mlp` takes these: few bfloat16 tokens, matrices for the latency kernels."""
+    tokens = h.shape[0]
+    return (skinny_ok(tokens, gate_up) and skinny_ok(tokens, down) and h.dtype == torch.bfloat16
+            and max(gate_up.numel(), down.numel()) * 2 < STREAM_MIN_BYTES)
+
+
+# two SkinnyCalls in a row
+_SKINNY_PAIR = struct.Struct("@19P3d15i4x19P3d15i4x")
+
+
+def skinny_mlp(h: torch.Tensor, gate_up: torch.Tensor, down: torch.Tensor, gate: str = "silu", gate_limit: Optional[float] = None) -> torch.Tensor:
+    """down(act(h W_gate^T, h W_up^T)), float [tokens, N], for the stacked matrices gate_up [2 I, K] and down [N, I]: what two `skinny_gemm` calls
+    make (SWIGLU, then PLAIN), launched by one call."""
+    _need(h, torch.bfloat16, "h", 2); _need(gate_up, torch.bfloat16, "gate_up", 2); _need(down, torch.bfloat16, "down", 2)
+    tokens, k = h.shape
+    n2, k1 = gate_up.shape
+    n, inter = down.shape
+    if k != k1 or n2 != 2 * inter:
+        raise KernelError("skinny_mlp: shapes of h, gate_up and down disagree")
+    act, out = h.new_empty((tokens, inter)), h.new_empty((tokens, n), dtype=torch.float32)
+    gate_act, limit = _gate(gate, gate_limit)
+    stream, act_at = _stream(), act.data_ptr()
+    try:
+        args = _SKINNY_PAIR.pack(gate_up.data_ptr(), h.data_ptr(), 0, 0, 0, 0, 0, 0, act_at, 0, 0, 0, 0, 0, 0, 0, 0, 0, stream, 0.0, 1.0, limit,
+                                 n2, k, 0, tokens, EPI_SWIGLU, inter, 0, 0, 0, 0, 0, 0, 0, 0, gate_act,
+                                 down.data_ptr(), act_at, 0, 0, 0, 0, 0, out.data_ptr(), 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, stream, 0.0, 1.0, 0.0,
+                                 n, inter, 0, tokens, EPI_PLAIN, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0)
+    except struct.error as err:
+        raise KernelError(f"skinny_mlp: {err}") from err
+    _check(_skinny().cisr_skinny_chain(args, 2), "skinny_mlp", own=2)
+    return out
+
+
 STREAM_MAX_TOKENS = 16
 STREAM_MIN_BYTES = 8 << 20       # smaller weight matrices are latency-bound: the kernels of skinny_gemm.cu serve them better
 _stream_state = {}

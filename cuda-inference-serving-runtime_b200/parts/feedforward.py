@@ -48,6 +48,8 @@ class SwiGLU(FeedForward):
                 + (kernels.skinny_jobs() if self.dtype == torch.bfloat16 else []))
 
     def forward(self, h, ctx):
+        if isinstance(h, torch.Tensor) and kernels.skinny_mlp_ok(h, self.gate_up, self.down):
+            return kernels.skinny_mlp(h, self.gate_up, self.down, self.activation, self.limit)
         return linear_to_stream(gated_product(h, self.gate_up, self.activation, self.limit), self.down, h)
 
 
