@@ -352,11 +352,12 @@ def kernel_need(name: str, shape: tuple, cfg: dict, dtype_bytes: int, cache_toke
         tokens, n, k, epilogue, normed = shape
         label = f"weight-streaming product {EPILOGUE_NAMES[epilogue]}{' +norm' if normed else ''} [{tokens}x{k}]x[{n}x{k}]"
         return n * k * 2 + tokens * k * (8 if normed else 2), 2.0 * tokens * n * k, label
-    if name in ("gemm_tcgen05", "gemm_tcgen05_swiglu", "gemm_tcgen05_rope", "gemm_library"):
+    if name in ("gemm_tcgen05", "gemm_tcgen05_swiglu", "gemm_tcgen05_rope", "gemm_library", "gemm_float"):
         m, n, k = shape
-        out_bytes = m * n * (4 if name in ("gemm_tcgen05", "gemm_library") else 2)
+        out_bytes = m * n * (4 if name in ("gemm_tcgen05", "gemm_library", "gemm_float") else 2)
         label = {"gemm_tcgen05": "tcgen05 product", "gemm_tcgen05_swiglu": "tcgen05 product + SwiGLU",
-                 "gemm_tcgen05_rope": "tcgen05 product + rotation + cache write", "gemm_library": "library product"}[name]
+                 "gemm_tcgen05_rope": "tcgen05 product + rotation + cache write", "gemm_library": "library product",
+                 "gemm_float": "split-float product"}[name]
         return (m * k + n * k) * dtype_bytes + out_bytes, 2.0 * m * n * k, f"{label} [{m}x{k}]x[{n}x{k}]"
     if name == "attn_decode":
         n_dec = shape[0]
@@ -587,9 +588,9 @@ def generic_need(name: str, shape: tuple, cache_tokens: int, causal: int):
     if name == "skinny_gemm":
         tokens, n, k, epilogue, normed = shape
         return n * k * 2 + tokens * k * (8 if normed else 2), 2.0 * tokens * n * k
-    if name in ("gemm_tcgen05", "gemm_tcgen05_swiglu", "gemm_tcgen05_rope", "gemm_library"):
+    if name in ("gemm_tcgen05", "gemm_tcgen05_swiglu", "gemm_tcgen05_rope", "gemm_library", "gemm_float"):
         m, n, k = shape
-        return (m * k + n * k) * 2 + m * n * (4 if name in ("gemm_tcgen05", "gemm_library") else 2), 2.0 * m * n * k
+        return (m * k + n * k) * 2 + m * n * (4 if name in ("gemm_tcgen05", "gemm_library", "gemm_float") else 2), 2.0 * m * n * k
     if name == "gemm_tcgen05_grouped":
         m, groups, n, k, relu2 = shape
         return (m * k + groups * n * k) * 2 + m * n * (2 if relu2 else 4), 2.0 * m * n * k

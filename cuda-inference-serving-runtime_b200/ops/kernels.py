@@ -1823,20 +1823,58 @@ def gemm_heads(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, w_is_nk: boo
 
 def gemm_jobs(dtype: torch.dtype):
     """Build jobs of the libraries `gemm` may launch for operands of this dtype."""
-    jobs = [("gemm_library.cu", {}, ("-lcublas",))]
-    if dtype == torch.bfloat16:
-        jobs.append(("gemm_tcgen05.cu", {}, ()))
-    return jobs
+    return [("gemm_library.cu", {}, ("-lcublas",)), ("gemm_tcgen05.cu" if dtype == torch.bfloat16 else "gemm_float.cu", {}, ())]
 
 
 def gemm(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
     """out[M, N] (float) = a[M, K] @ w[N, K]^T; picks the kernel for the shape and dtype.
 
-    bfloat16 with at least one 128-row tile of tokens: this package's tcgen05 + TMA kernel; float (true 32-bit),
-    and shapes that kernel does not take: the vendor library."""
+    bfloat16 with at least one 128-row tile of tokens: this package's tcgen05 + TMA kernel; float (true 32-bit) where it is estimated to
+    be faster: products of split floats (`gemm_float`); the other shapes: the vendor library."""
     if tcgen05_ok(a, w):
         return gemm_tcgen05(a, w, out)
+    if a.dtype == torch.float32 and w.dtype == torch.float32 and out.dtype == torch.float32:
+        width = float_tile(a.shape[0], w.shape[0], a.shape[1], sm_count(a.device))
+        if width and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0:
+            return gemm_float(a, w, out, narrow=width == 64)
     return gemm_library(a, w, out)
+
+
+_gemm_float_state = {}
+
+
+def float_tile(m: int, n: int, k: int, sms: int) -> int:
+    """The columns of `gemm_float`'s tiles for a float product, 0 where the library is estimated to be faster.  Per tile 5.5 us and, per 64 of K, 1.45 us
+    with 128 columns and 1.07 with 64, 0.25 more where all SMs are busy; the library 3 us, 56 TFLOP/s and 3 us per 1000 of K, a little less than it takes: where it
+    is behind, products of split floats are the more exact too (error against 64 bits 1.0e-7 to 2.9e-7, the library's 1.6e-7 to 1.1e-6; a few rows, at
+    1.1e-7, stay with it).  us, library and here: 1000 rows of 960 x 576 29 and 15, of 576 x 576 19 and 15; 128 rows of 4096 x 4096 123 and 72, of
+    8192 -> 2048 109 and 135; 512 rows of 16384 x 2048 624 and 236, of 4096 x 14336 1065 and 348."""
+    if m < 64 or k % 4:
+        return 0
+    blocks, rows = -(-k // 64), -(-m // 128)
+    best, least = 0, 3.0 + 2.0 * m * n * k / 56e6 + 0.003 * k
+    for width, block in ((128, 1.45), (64, 1.07)):
+        tiles = rows * -(-n // width)
+        us = 5.5 + blocks * (block * -(-tiles // sms) + 0.25 * tiles / sms)
+        if us < least:
+            best, least = width, us
+    return best
+
+
+def gemm_float(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, narrow: bool = False) -> torch.Tensor:
+    """out[M, N] = a[M, K] @ w[N, K]^T, all float, on the tensor cores by products of split floats (csrc/gemm_float.cu); `narrow`: tiles of 64 columns."""
+    _need(a, torch.float32, "a", 2); _need(w, torch.float32, "w", 2); _need(out, torch.float32, "out", 2)
+    m, k = a.shape
+    n = w.shape[0]
+    if w.shape[1] != k or out.shape != (m, n):
+        raise KernelError("gemm_float: shapes disagree")
+    lib = _gemm_float_state.get("lib")
+    if lib is None:
+        lib = load_library("gemm_float.cu")
+        _check(lib.cisr_gemm_float_init(_p(_error_flag())), "float gemm init", own=0)
+        _gemm_float_state["lib"] = lib
+    _check(lib.cisr_gemm_float(_p(a), _p(w), _p(out), m, n, k, int(narrow), _stream()), "gemm_float")
+    return out
 
 
 # ------------------------------------------------------------------ weight-streaming products for few tokens
@@ -2269,6 +2307,7 @@ _DESCRIBE = {
     "moe_combine": lambda sorted_out, row_of, weight, out, out_scale=None, h=None: (int(out.shape[0]), int(weight.shape[1]), int(out.shape[1])),
     "gemm_tcgen05_grouped": lambda a, w, out, tile_group, rows_in_use=None, activation="relu_squared":
         (int(rows_in_use or a.shape[0]), int(w.shape[0]), int(w.shape[1]), int(w.shape[2]), out.dtype == torch.bfloat16),
+    "gemm_float": _describe_gemm,
     "gemm_tcgen05_experts": lambda a, w, out, tiles, rows_in_use=None, activation="relu_squared", gate_limit=None:
         (int(rows_in_use or a.shape[0]), int(w.shape[0]), int(w.shape[1]), int(w.shape[2]), 2 if gate_limit is not None else int(out.dtype == torch.bfloat16)),
     "gemm_heads": lambda a, w, out, w_is_nk: (int(a.shape[0]), int(w.shape[0]), int(w.shape[1]), int(w.shape[2])),
