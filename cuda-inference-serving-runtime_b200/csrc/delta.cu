@@ -581,7 +581,7 @@ delta_chunk_walk_kernel(const float* __restrict__ qkv, const float* __restrict__
 //                       tensor cores with S in the registers of its result; G's place receives the state before its chunk
 //   delta_chunk_reads   a CTA per (chunk, head): out += R S0
 // The walk over a chunk's own products in order took 256 us for 2048 tokens of 32 heads, and the tables before it 120, most
-// of it the inversion row by row; these three take 114, 41 and 26 us. Error of outputs and
+// of it the inversion row by row; these three take 102, 30 and 26 us. Error of outputs and
 // states against 64 bits 1.0e-7 to 1.6e-7, where the walk has 1.7e-7 to 8.8e-7.
 constexpr int FORM_THREADS = 256;
 constexpr int FORM_G = 3 * CHUNK * CHUNK / 2, FORM_R = FORM_G + CHUNK * CHUNK, FORM_C = FORM_R + CHUNK * CHUNK;
@@ -625,6 +625,37 @@ __device__ __forceinline__ void for_pairs(const float (&acc)[4][4], int m0, int 
 
 // T = (I + A)^-1 for the strictly lower triangle A [64][AF_LD] (its upper triangle is scratch): the diagonal blocks of 16 by
 // substitution, a column per lane; then twice the block below the diagonal, -T22 (A21 T11), from blocks of half the size.
+template <int HALF, bool BOUNDED>
+__device__ __forceinline__ void invert_level(float* __restrict__ A, float* __restrict__ T) {
+    // pairs of blocks at 2 HALF p; runs of four columns: r inside the block below, c inside the block beside
+    constexpr int RUNS = HALF / 4, PER_PAIR = HALF * RUNS, TOTAL = PER_PAIR * (CHUNK / (2 * HALF));
+    const int i = threadIdx.x, p = i / PER_PAIR, e = i - p * PER_PAIR, r = e / RUNS, c = 4 * (e - r * RUNS), base = 2 * HALF * p;
+    static_assert(TOTAL <= FORM_THREADS, "a run per thread");
+    if (i < TOTAL) {
+        float4 y = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 16
+        for (int k = 0; k < HALF; ++k) {
+            const float a = A[(base + HALF + r) * AF_LD + base + k];
+            const float4 t = *reinterpret_cast<const float4*>(T + (base + k) * AF_LD + base + c);
+            y.x = fmaf(a, t.x, y.x); y.y = fmaf(a, t.y, y.y); y.z = fmaf(a, t.z, y.z); y.w = fmaf(a, t.w, y.w);
+        }
+        *reinterpret_cast<float4*>(A + (base + r) * AF_LD + base + HALF + c) = y;      // the block above the diagonal is free
+    }
+    __syncthreads();
+    if (i < TOTAL) {
+        float4 y = make_float4(0.f, 0.f, 0.f, 0.f);
+        // T22 holds nothing right of its diagonal.  BOUNDED: nor does a NaN below meet those zeros; elsewhere it may, and is seen in the results
+#pragma unroll 16
+        for (int k = 0; k < (BOUNDED ? r + 1 : HALF); ++k) {
+            const float a = -T[(base + HALF + r) * AF_LD + base + HALF + k];
+            const float4 t = *reinterpret_cast<const float4*>(A + (base + k) * AF_LD + base + HALF + c);
+            y.x = fmaf(a, t.x, y.x); y.y = fmaf(a, t.y, y.y); y.z = fmaf(a, t.z, y.z); y.w = fmaf(a, t.w, y.w);
+        }
+        *reinterpret_cast<float4*>(T + (base + HALF + r) * AF_LD + base + c) = y;
+    }
+    __syncthreads();
+}
+template <bool BOUNDED>
 __device__ __forceinline__ void invert_unit_lower(float* __restrict__ A, float* __restrict__ T) {
     const int tid = threadIdx.x;
     for (int i = tid; i < CHUNK * CHUNK; i += FORM_THREADS) {
@@ -636,41 +667,19 @@ __device__ __forceinline__ void invert_unit_lower(float* __restrict__ A, float* 
         float x[16];
 #pragma unroll
         for (int t = 0; t < 16; ++t) {
-            float v = t == c ? 1.f : 0.f;
+            float v = t == c ? 1.f : 0.f, u = 0.f;         // two sums side by side: half the chain
 #pragma unroll
-            for (int i = 0; i < t; ++i) v = fmaf(-A[(b + t) * AF_LD + b + i], x[i], v);
-            x[t] = v;                                       // zero above the diagonal: every term before it is
-            T[(b + t) * AF_LD + b + c] = v;
+            for (int i = 0; i < t; ++i) {
+                const float a = -A[(b + t) * AF_LD + b + i];
+                if (i & 1) u = fmaf(a, x[i], u); else v = fmaf(a, x[i], v);
+            }
+            x[t] = v + u;                                   // zero above the diagonal: every term before it is
+            T[(b + t) * AF_LD + b + c] = x[t];
         }
     }
     __syncthreads();
-#pragma unroll 1
-    for (int half = 16; half < CHUNK; half *= 2) {
-        // pairs of blocks at 2 half p; runs of four columns: r inside the block below, c inside the block beside
-        const int runs = half / 4, per_pair = half * runs, total = per_pair * (CHUNK / (2 * half));
-        for (int i = tid; i < total; i += FORM_THREADS) {
-            const int p = i / per_pair, e = i - p * per_pair, r = e / runs, c = 4 * (e - r * runs), base = 2 * half * p;
-            float4 y = make_float4(0.f, 0.f, 0.f, 0.f);
-            for (int k = 0; k < half; ++k) {
-                const float a = A[(base + half + r) * AF_LD + base + k];
-                const float4 t = *reinterpret_cast<const float4*>(T + (base + k) * AF_LD + base + c);
-                y.x = fmaf(a, t.x, y.x); y.y = fmaf(a, t.y, y.y); y.z = fmaf(a, t.z, y.z); y.w = fmaf(a, t.w, y.w);
-            }
-            *reinterpret_cast<float4*>(A + (base + r) * AF_LD + base + half + c) = y;      // the block above the diagonal is free
-        }
-        __syncthreads();
-        for (int i = tid; i < total; i += FORM_THREADS) {
-            const int p = i / per_pair, e = i - p * per_pair, r = e / runs, c = 4 * (e - r * runs), base = 2 * half * p;
-            float4 y = make_float4(0.f, 0.f, 0.f, 0.f);
-            for (int k = 0; k <= r; ++k) {                 // T22 holds nothing right of its diagonal, and a NaN below must not meet it
-                const float a = -T[(base + half + r) * AF_LD + base + half + k];
-                const float4 t = *reinterpret_cast<const float4*>(A + (base + k) * AF_LD + base + half + c);
-                y.x = fmaf(a, t.x, y.x); y.y = fmaf(a, t.y, y.y); y.z = fmaf(a, t.z, y.z); y.w = fmaf(a, t.w, y.w);
-            }
-            *reinterpret_cast<float4*>(T + (base + half + r) * AF_LD + base + c) = y;
-        }
-        __syncthreads();
-    }
+    invert_level<16, BOUNDED>(A, T);
+    invert_level<32, BOUNDED>(A, T);
 }
 
 struct FormArgs {
@@ -731,16 +740,20 @@ __device__ __forceinline__ int forms_pass(const FormArgs& a, FormShared& sh) {
         }
         fetch_form<VEC>(raw, v, channels, count, dv);      // wanted after the inversion
         __syncthreads();                                   // Q has been read: P takes its place
-        for_pairs(kk, m0, n0, [&](int t, int i, float x, float y) {
-            const float r0 = i < t ? expf((float)(L[t] - L[i])) : 0.f, r1 = i + 1 < t ? expf((float)(L[t] - L[i + 1])) : 0.f;
-            *reinterpret_cast<float2*>(Af + t * AF_LD + i) = make_float2(bt[t] * r0 * x, bt[t] * r1 * y);
-        });
-        for_pairs(qk, m0, n0, [&](int t, int i, float x, float y) {
-            tile_store2<PLAIN>(tile[1], t, i, i <= t ? expf((float)(L[t] - L[i])) * x : 0.f, i + 1 <= t ? expf((float)(L[t] - L[i + 1])) * y : 0.f);
-        });
+        const int lane = tid & 31;
+#pragma unroll
+        for (int half = 0; half < 2; ++half)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int t = m0 + 8 * half + (lane >> 2), i = n0 + 8 * j + 2 * (lane & 3);
+                // the decay from each of the two tokens to t (none from a later one)
+                const float r0 = i <= t ? expf((float)(L[t] - L[i])) : 0.f, r1 = i + 1 <= t ? expf((float)(L[t] - L[i + 1])) : 0.f;
+                *reinterpret_cast<float2*>(Af + t * AF_LD + i) = make_float2(i < t ? bt[t] * r0 * kk[j][2 * half] : 0.f, i + 1 < t ? bt[t] * r1 * kk[j][2 * half + 1] : 0.f);
+                tile_store2<PLAIN>(tile[1], t, i, i <= t ? r0 * qk[j][2 * half] : 0.f, i + 1 <= t ? r1 * qk[j][2 * half + 1] : 0.f);
+            }
     }
     __syncthreads();
-    invert_unit_lower(Af, Tf);
+    invert_unit_lower<PLAIN>(Af, Tf);
     {
         float4 t4[4];
 #pragma unroll
@@ -786,13 +799,27 @@ __device__ __forceinline__ int forms_pass(const FormArgs& a, FormShared& sh) {
         for_pairs(acc, m0, n0, [&](int r, int c, float x, float y) { *reinterpret_cast<float2*>(G + r * CHUNK + c) = make_float2(x, y); });
     }
     {
+        const int lane = tid & 31;
+        float2 qv[2][4];                                   // of this thread's elements: asked for before the product, which they wait beside
+#pragma unroll
+        for (int half = 0; half < 2; ++half)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int t = m0 + 8 * half + (lane >> 2), d = n0 + 8 * j + 2 * (lane & 3);
+                const float* at = q + (size_t)t * channels + d;
+                if (VEC) qv[half][j] = t < count && d < dk ? *reinterpret_cast<const float2*>(at) : make_float2(0.f, 0.f);
+                else qv[half][j] = make_float2(t < count && d < dk ? at[0] : 0.f, t < count && d + 1 < dk ? at[1] : 0.f);
+            }
         float acc[4][4] = {};
         tile_product<PLAIN, false, true, true>(acc, tile[1], tile[3], m0, n0, m0 / 16 + 1);
         bad |= not_finite(acc);
-        for_pairs(acc, m0, n0, [&](int t, int d, float x, float y) {
-            const float q0 = t < count && d < dk ? q[(size_t)t * channels + d] : 0.f, q1 = t < count && d + 1 < dk ? q[(size_t)t * channels + d + 1] : 0.f;
-            *reinterpret_cast<float2*>(R + t * CHUNK + d) = make_float2(fmaf(ct[t], q0, -x), fmaf(ct[t], q1, -y));
-        });
+#pragma unroll
+        for (int half = 0; half < 2; ++half)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int t = m0 + 8 * half + (lane >> 2), d = n0 + 8 * j + 2 * (lane & 3);
+                *reinterpret_cast<float2*>(R + t * CHUNK + d) = make_float2(fmaf(ct[t], qv[half][j].x, -acc[j][2 * half]), fmaf(ct[t], qv[half][j].y, -acc[j][2 * half + 1]));
+            }
     }
     {
         float acc[4][4] = {};
@@ -817,13 +844,15 @@ delta_chunk_forms_kernel(const __grid_constant__ FormArgs a) {
     if (__syncthreads_or(forms_pass<VEC, false>(a, sh))) forms_plain<VEC>(a, sh);
 }
 
-constexpr int STATE_COLS = 16, STATE_STAGES = 3, STATE_THREADS = 128;
+constexpr int STATE_COLS = 16, STATE_STAGES = 3, STATE_THREADS = 128, STATE_COPIERS = 64;
 constexpr int STATE_LD = 24;                               // row stride of S's parts: 48 bytes, eight rows in different banks
 struct StateParts { __nv_bfloat16 part[3][CHUNK][STATE_LD]; };
 struct StateStage { SplitTile n; float g[CHUNK][STATE_COLS]; };
 constexpr size_t STATES_SMEM = STATE_STAGES * sizeof(StateStage) + 2 * sizeof(StateParts);
 
-__global__ void __launch_bounds__(STATE_THREADS)
+// Four warps carry the state and two more bring the chunks' N and G in front of them: issued by the warps that carry it, a chunk's copies took
+// 1,100 of its 2,550 cycles (41 us for 32 chunks, 30 so).
+__global__ void __launch_bounds__(STATE_THREADS + STATE_COPIERS)
 delta_chunk_states_kernel(float* __restrict__ scratch, const int* __restrict__ req_chunk0, float* __restrict__ state, long long state_stride,
                           const int* __restrict__ req_slot, const int* __restrict__ q_len, int heads, int dk, int dv, int least) {
     extern __shared__ __align__(16) unsigned char form_smem[];
@@ -838,25 +867,34 @@ delta_chunk_states_kernel(float* __restrict__ scratch, const int* __restrict__ r
     if (n < least) return;
     float* forms = scratch + ((size_t)req_chunk0[req] * heads + head) * FORM_FLOATS;
     const size_t step = (size_t)heads * FORM_FLOATS;
-    auto fetch = [&](int chunk) {                          // N and G of a chunk into their stage; an empty group beyond the last
-        if (chunk < n_chunks) {
-            StateStage& to = stage[chunk % STATE_STAGES];
-            const float* from = forms + chunk * step;
+    if (tid >= STATE_THREADS) {
+        const int mine = tid - STATE_THREADS;
+        auto fetch = [&](int chunk) {                      // N and G of a chunk into their stage; an empty group beyond the last
+            if (chunk < n_chunks) {
+                StateStage& to = stage[chunk % STATE_STAGES];
+                const float* from = forms + chunk * step;
+#pragma unroll 8
+                for (int u = 0; u < 3 * CHUNK * 8 / STATE_COPIERS; ++u) {
+                    const int i = mine + u * STATE_COPIERS, r = (i >> 3) & 63, k = (i & 7) * 8;
+                    copy16(reinterpret_cast<float*>(&to.n.part[i >> 9][r][k]), from + (i >> 9) * (CHUNK * CHUNK / 2) + ((r * CHUNK + k) >> 1));
+                }
 #pragma unroll
-            for (int u = 0; u < 3 * CHUNK * 8 / STATE_THREADS; ++u) {
-                const int i = tid + u * STATE_THREADS, r = (i >> 3) & 63, k = (i & 7) * 8;
-                copy16(reinterpret_cast<float*>(&to.n.part[i >> 9][r][k]), from + (i >> 9) * (CHUNK * CHUNK / 2) + ((r * CHUNK + k) >> 1));
+                for (int u = 0; u < CHUNK * 4 / STATE_COPIERS; ++u) {
+                    const int i = mine + u * STATE_COPIERS, r = i >> 2, c = 4 * (i & 3);
+                    copy16(&to.g[r][c], from + FORM_G + r * CHUNK + col0 + c);
+                }
             }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        };
 #pragma unroll
-            for (int u = 0; u < CHUNK * 4 / STATE_THREADS; ++u) {
-                const int i = tid + u * STATE_THREADS, r = i >> 2, c = 4 * (i & 3);
-                copy16(&to.g[r][c], from + FORM_G + r * CHUNK + col0 + c);
-            }
+        for (int s = 0; s < STATE_STAGES - 1; ++s) fetch(s);
+        for (int chunk = 0; chunk < n_chunks; ++chunk) {
+            asm volatile("cp.async.wait_group %0;" ::"n"(STATE_STAGES - 2) : "memory");
+            __syncthreads();                               // N and G have landed, and the stage before this one is free
+            fetch(chunk + STATE_STAGES - 1);
         }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    };
-#pragma unroll
-    for (int s = 0; s < STATE_STAGES - 1; ++s) fetch(s);
+        return;
+    }
     float now[2][4];                                       // as a result of the tensor core has it: [columns 8 j ..][row, row + 8]
 #pragma unroll
     for (int j = 0; j < 2; ++j)
@@ -879,9 +917,7 @@ delta_chunk_states_kernel(float* __restrict__ scratch, const int* __restrict__ r
 #pragma unroll
                 for (int i = 0; i < 3; ++i) *reinterpret_cast<uint32_t*>(&Sp.part[i][row + 8 * half][8 * j + col]) = p[i];
             }
-        asm volatile("cp.async.wait_group %0;" ::"n"(STATE_STAGES - 2) : "memory");
-        __syncthreads();                                   // S is whole, N and G have landed, and the stage before this one is free
-        fetch(chunk + STATE_STAGES - 1);
+        __syncthreads();                                   // S is whole, N and G have landed
         const float f = keep;
         if (chunk + 1 < n_chunks) keep = forms[(chunk + 1) * step + FORM_C];
         float sum[2][4];
@@ -984,7 +1020,7 @@ int launch_forms(const float* qkv, const float* beta, const float* decay, const 
     int st = launch_kernel(delta_chunk_forms_kernel<VEC>, dim3(n_chunks, heads), dim3(FORM_THREADS), FORMS_SMEM, s, g_pdl,
                            FormArgs{qkv, beta, decay, chunk_req, chunk_t0, q_start, q_len, scratch, out, heads, kvh, dk, dv});
     if (st) return st;
-    st = launch_kernel(delta_chunk_states_kernel, dim3(n_req, heads, (dv + STATE_COLS - 1) / STATE_COLS), dim3(STATE_THREADS), STATES_SMEM, s, g_pdl, scratch,
+    st = launch_kernel(delta_chunk_states_kernel, dim3(n_req, heads, (dv + STATE_COLS - 1) / STATE_COLS), dim3(STATE_THREADS + STATE_COPIERS), STATES_SMEM, s, g_pdl, scratch,
                        req_chunk0, state, state_stride, req_slot, q_len, heads, dk, dv, least);
     if (st) return st;
     return launch_kernel(delta_chunk_reads_kernel<VEC>, dim3(n_chunks, heads), dim3(FORM_THREADS), 2 * sizeof(SplitTile), s, g_pdl,
