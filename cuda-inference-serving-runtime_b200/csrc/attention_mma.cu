@@ -649,11 +649,14 @@ __device__ __forceinline__ void stamp(int i) {
 
 // cluster: CTAs per cluster along the key ranges (1: none).  n_parts = n_splits / cluster partial sums per query head
 // remain; with one, the first CTA writes the finished rows to `out`, otherwise partial sums for the merge kernel.
+// DIRECT: the launch has one key range and no cluster: a CTA writes its finished rows to `out`, the very numbers that the merge kernel would make of
+// its one partial sum, and neither that kernel nor a merge in front of the output projection runs (8 requests of up to 256 keys, 135m shape: the
+// layer's merge and projection took 5.0 us behind the attention, the projection alone 2.5).
 // STAGES: tiles a warp has on the way at once (each in its own 16 KB stage).  With one, a warp whose share is two tiles
 // (ranges of 256 keys at head size 128) requests the second only after the first is used; with two, both are requested
 // before the wait on the kernel before, at twice the shared memory: for launches of no more CTAs than the device has
 // SMs, where that memory is idle anyway.  The sums are the same either way.
-template <int STAGES>
+template <int STAGES, bool DIRECT>
 __global__ void __launch_bounds__(DEC_THREADS, STAGES == 1 ? 3 : 1)
 attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
                        const bf16* __restrict__ q, bf16* __restrict__ out, const bf16* __restrict__ k_cache,
@@ -661,7 +664,7 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
                        const int* __restrict__ block_table, int table_width, const int* __restrict__ dec_req,
                        const int* __restrict__ q_start, const int* __restrict__ ctx_len, float* __restrict__ partial,
                        float* __restrict__ stats, int hq, int hkv, int page_size, float scale, float softcap, int window,
-                       int keep_first, int split_size, int cluster, int n_parts, int row0, int* __restrict__ error) {
+                       int keep_first, int split_size, int cluster, int n_parts, int row0, float sink_all, const float* __restrict__ sink_heads, int* __restrict__ error) {
     CISR_TRACE_SCOPE(TRACE_ATTN_DECODE_TMA);
     extern __shared__ unsigned char smem_raw[];
     unsigned char* ring = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);   // swizzle atoms are 1024-byte aligned
@@ -689,6 +692,10 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
     const bool empty = lo >= hi;              // nothing in this range (the same for every thread)
     if (empty && cluster == 1) {              // the merge skips a zero denominator
         pdl_wait();
+        if (DIRECT) {                         // a padding row
+            for (int e = tid; e < rows * D; e += DEC_THREADS) out[((size_t)tok * hq + kvh * group + row0) * D + e] = __float2bfloat16_rn(0.f);
+            return;
+        }
         for (int g = tid; g < rows; g += DEC_THREADS) {
             const size_t p = part_base + (size_t)g * n_parts + split;
             stats[2 * p] = -INFINITY; stats[2 * p + 1] = 0.f;
@@ -874,6 +881,19 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
     CISR_TRACE_MARK(2);
     if (cluster == 1) {
         if (*failed) return;  // a copy never arrived; the host reads the error flag
+        if (DIRECT) {
+            warps_to_merge_area(merge, o, m_run, l_run, warp, lane, rows);
+            __syncthreads();
+            for (int e = tid; e < rows * D; e += DEC_THREADS) {
+                const int g = e / D, d = e - g * D, head = kvh * group + row0 + g;
+                const float sink = sink_heads ? sink_heads[head] : sink_all;
+                float m, den;
+                const float num = merged_element(merge, g, d, m, den);
+                if (den > 0.f && sink > -INFINITY) den += expf(sink - m * LN2);      // the sink: one more term of the denominator, no value
+                out[((size_t)tok * hq + head) * D + d] = __float2bfloat16_rn(den > 0.f ? num / den : 0.f);
+            }
+            return;
+        }
         decode_finish(merge, o, m_run, l_run, partial, stats, part_base, rows, n_parts, split, tid);
         STAMP(7);
         return;
@@ -1067,7 +1087,7 @@ CISR_EXPORT int cisr_attn_tma_init(int* error_flag) {
 
 // As cisr_attn_decode, for caches of `n_pages` pages whose address is 16-byte aligned.  Key ranges are grouped into
 // thread-block clusters of up to 16 where the device can hold such clusters; when one cluster covers all ranges
-// the finished rows go straight to `out` and no merge kernel runs.
+// the finished rows go straight to `out` and no merge kernel runs; nor does it where there is one range.
 CISR_EXPORT int cisr_attn_decode_tma(const void* q, void* out, const void* k_cache, const void* v_cache, int n_pages,
                                      const int* req_slot, const int* block_table, int table_width, const int* dec_req,
                                      int n_dec, const int* q_start, const int* ctx_len, float* partial, float* stats,
@@ -1093,11 +1113,12 @@ CISR_EXPORT int cisr_attn_decode_tma(const void* q, void* out, const void* k_cac
     static bool configured = false;
     static int sms = 0;
     if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(attn_decode_tma_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_CAP);
+        cudaError_t e = cudaFuncSetAttribute(attn_decode_tma_kernel<1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_CAP);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(attn_decode_tma_kernel<1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_CAP);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(attn_decode_tma_kernel<2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_CAP_DEEP);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(attn_decode_tma_kernel<2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_CAP_DEEP);
         if (e != cudaSuccess) return (int)e;
-        e = cudaFuncSetAttribute(attn_decode_tma_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_CAP_DEEP);
-        if (e != cudaSuccess) return (int)e;
-        cudaFuncSetAttribute(attn_decode_tma_kernel<1>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);   // clusters of more than 8
+        cudaFuncSetAttribute(attn_decode_tma_kernel<1, false>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);   // clusters of more than 8
         cudaGetLastError();
         int device = 0;
         if (cudaGetDevice(&device) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) sms = 0;
@@ -1119,7 +1140,7 @@ CISR_EXPORT int cisr_attn_decode_tma(const void* q, void* out, const void* k_cac
             attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = (unsigned)c;
             config.attrs = attr; config.numAttrs = 1;
             int n = 0;
-            const cudaError_t e = cudaOccupancyMaxActiveClusters(&n, attn_decode_tma_kernel<1>, &config);
+            const cudaError_t e = cudaOccupancyMaxActiveClusters(&n, attn_decode_tma_kernel<1, false>, &config);
             cudaGetLastError();
             resident[c] = (e == cudaSuccess && n >= 1) ? 1 : -1;
         }
@@ -1130,26 +1151,22 @@ CISR_EXPORT int cisr_attn_decode_tma(const void* q, void* out, const void* k_cac
     }
     const int n_parts = n_splits / cluster;
     cudaStream_t s = (cudaStream_t)stream;
-    g_last_launches = (group + 15) / 16 + (((n_parts == 1 && cluster > 1) || !merge) ? 0 : 1);
+    const bool direct = merge && n_splits == 1;      // cluster is 1 then
+    g_last_launches = (group + 15) / 16 + ((n_parts == 1 && cluster > 1) || direct || !merge ? 0 : 1);
     // a warp's share of a range is more than one tile, and the launch leaves most of the device's shared memory idle
     const size_t smem_deep = smem + 4 * (size_t)TMA_TILE_BYTES;
     const bool deep = cluster == 1 && split_size > 4 * TK && (long long)n_dec * hkv * n_splits <= sms && smem_deep <= SMEM_CAP_DEEP;
     for (int row0 = 0; row0 < group; row0 += 16) {
-        if (deep)
-            status = launch_kernel_cluster(attn_decode_tma_kernel<2>, dim3(n_dec, hkv, n_splits), dim3(DEC_THREADS), smem_deep, s, g_pdl, 1,
-                                           map_k, map_v, (const bf16*)q, (bf16*)out, (const bf16*)k_cache, (const bf16*)v_cache,
-                                           (int)cache_rows, req_slot, block_table, table_width,
-                                           dec_req, q_start, ctx_len, partial, stats, hq, hkv, page_size, scale, softcap, window, keep_first, split_size,
-                                           1, n_parts, row0, g_error);
-        else
-            status = launch_kernel_cluster(attn_decode_tma_kernel<1>, dim3(n_dec, hkv, n_splits), dim3(DEC_THREADS), smem, s, g_pdl, cluster,
-                                           map_k, map_v, (const bf16*)q, (bf16*)out, (const bf16*)k_cache, (const bf16*)v_cache,
-                                           (int)cache_rows, req_slot, block_table, table_width,
-                                           dec_req, q_start, ctx_len, partial, stats, hq, hkv, page_size, scale, softcap, window, keep_first, split_size,
-                                           cluster, n_parts, row0, g_error);
+        const auto kernel = deep ? (direct ? attn_decode_tma_kernel<2, true> : attn_decode_tma_kernel<2, false>)
+                                 : (direct ? attn_decode_tma_kernel<1, true> : attn_decode_tma_kernel<1, false>);
+        status = launch_kernel_cluster(kernel, dim3(n_dec, hkv, n_splits), dim3(DEC_THREADS), deep ? smem_deep : smem, s, g_pdl, cluster,
+                                       map_k, map_v, (const bf16*)q, (bf16*)out, (const bf16*)k_cache, (const bf16*)v_cache,
+                                       (int)cache_rows, req_slot, block_table, table_width,
+                                       dec_req, q_start, ctx_len, partial, stats, hq, hkv, page_size, scale, softcap, window, keep_first, split_size,
+                                       cluster, n_parts, row0, sink, sink_heads, g_error);
         if (status) return status;
     }
-    if ((n_parts == 1 && cluster > 1) || !merge) return 0;
+    if ((n_parts == 1 && cluster > 1) || direct || !merge) return 0;
     return launch_kernel(attn_merge_kernel, dim3(n_dec, hq), dim3(D <= 64 ? 64 : 128), sizeof(float) * 2 * (size_t)n_parts, s, g_pdl,
                          (const float*)partial, (const float*)stats, (bf16*)out, dec_req, q_start, hq, n_parts, sink, sink_heads);
 }

@@ -470,6 +470,17 @@ def attn_prefill(q, out, k_cache, v_cache, req_slot, block_table, tile_req, tile
                   int(keep_first or 0), *_sink(sink, hq), _stream()), "attn_prefill")
 
 
+def _decode_by_tensor_maps(lib, k_cache, v_cache, page_size: int, split_size: int) -> bool:
+    return bool(lib._tensor_maps and lib.cisr_attn_decode_tma_ok(page_size, split_size) and k_cache.is_contiguous()
+                and v_cache.is_contiguous() and k_cache.data_ptr() % 16 == 0 and v_cache.data_ptr() % 16 == 0
+                and k_cache.shape[0] * k_cache.shape[1] * page_size < 2 ** 31)
+
+
+def attn_decode_finishes(k_cache, v_cache, page_size: int, split_size: int, n_splits: int) -> bool:
+    """Whether `attn_decode` with one key range writes the finished rows itself (the tensor-map kernel), so that nothing is left to merge."""
+    return n_splits == 1 and _decode_by_tensor_maps(attention_library(k_cache.shape[-1], k_cache.dtype), k_cache, v_cache, page_size, split_size)
+
+
 def attn_decode(q, out, k_cache, v_cache, req_slot, block_table, dec_req, n_dec, q_start, ctx_len, partial, stats, hq, hkv,
                 page_size, scale, window, split_size, n_splits, kind: str = "auto", staging: str = "auto", merge: bool = True,
                 sink=None, keep_first: int = 0, softcap: Optional[float] = None) -> None:
@@ -503,9 +514,7 @@ def attn_decode(q, out, k_cache, v_cache, req_slot, block_table, dec_req, n_dec,
     tail.append(_stream())
     if staging not in ("auto", "tensor_map", "gather"):
         raise KernelError(f"unknown staging {staging!r}")
-    tensor_maps = (lib._tensor_maps and lib.cisr_attn_decode_tma_ok(page_size, split_size) and k_cache.is_contiguous()
-                   and v_cache.is_contiguous() and k_cache.data_ptr() % 16 == 0 and v_cache.data_ptr() % 16 == 0
-                   and k_cache.shape[0] * hkv * page_size < 2 ** 31)
+    tensor_maps = _decode_by_tensor_maps(lib, k_cache, v_cache, page_size, split_size)
     if staging == "tensor_map" and not tensor_maps:
         raise KernelError("attn_decode: tensor-map staging does not take this head size, page size, range size or cache")
     if tensor_maps and staging != "gather":

@@ -133,8 +133,10 @@ class GQAAttention(Mixer):
             partial = torch.empty((n_decode, hq, n_splits, dim), dtype=torch.float32, device=device)
             stats = torch.empty((n_decode, hq, n_splits, 2), dtype=torch.float32, device=device)
             # a step of single tokens only, with a small output projection: the merge of the key ranges is the prologue
-            # of that projection (one launch of a thread-block cluster instead of the merge kernel and the product)
+            # of that projection (one launch of a thread-block cluster instead of the merge kernel and the product); where
+            # the attention kernel finishes its rows there is nothing to merge
             fused = (n_decode == tokens and self.dtype == torch.bfloat16 and dim <= kernels.TENSOR_CORE_MAX_HEAD_DIM
+                     and not kernels.attn_decode_finishes(cache.k, cache.v, cache.page_size, DECODE_RANGE, n_splits)
                      and kernels.merge_out_proj_ok(n_decode, hq, dim, self.o))
             kernels.attn_decode(q, out, cache.k, cache.v, ctx.req_slot, cache.block_table, plan["dec_req"], n_decode, ctx.q_start,
                                 ctx.ctx_len, partial, stats, hq, hkv, cache.page_size, self.scale, self.window,
