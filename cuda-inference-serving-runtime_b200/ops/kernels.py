@@ -1908,6 +1908,8 @@ def set_pdl(on: bool) -> None:
         _stream_state["lib"].cisr_stream_set_pdl(int(on))
     for lib in _attention_tcgen05_libs.values():
         lib.cisr_attn_tcgen05_set_pdl(int(on))
+    if "lib" in _few_state:
+        _few_state["lib"].cisr_few_set_pdl(int(on))
     if "lib" in _merge_proj_state:
         _merge_proj_state["lib"].cisr_merge_proj_set_pdl(int(on))
     _elementwise().cisr_elementwise_set_pdl(int(on))
@@ -1942,11 +1944,11 @@ def set_pdl(on: bool) -> None:
 
 
 def skinny_jobs():
-    return [("skinny_gemm.cu", {}, ()), ("stream_gemm.cu", {}, ())]
+    return [("skinny_gemm.cu", {}, ()), ("stream_gemm.cu", {}, ()), ("few_gemm.cu", {}, ())]
 
 
 def stream_takes(tokens: int, w: torch.Tensor) -> bool:
-    """Whether skinny_gemm(kind="auto") hands this product to the persistent streaming kernel (stream_gemm.cu): a large
+    """Whether the persistent streaming kernel (stream_gemm.cu), which skinny_gemm(kind="auto") tries after few_gemm.cu, takes this product: a large
     bfloat16 weight matrix, at most 16 tokens, the tokens and at least three 16 KB stages in shared memory.  (The
     epilogues add their own conditions; where they fail the latency kernels take over.)"""
     if w.dtype != torch.bfloat16 or not 0 < tokens <= STREAM_MAX_TOKENS or w.shape[1] % 8 or w.numel() * 2 < STREAM_MIN_BYTES:
@@ -1956,16 +1958,24 @@ def stream_takes(tokens: int, w: torch.Tensor) -> bool:
     return fixed + 3 * (16384 + 16) <= 224 * 1024 - 8192          # 8 KB kept for the rotation tables of the ROPE epilogue
 
 
-def skinny_ok(tokens: int, w: torch.Tensor) -> bool:
-    """Shapes the weight-streaming kernels take: bfloat16 weights, at most 16 tokens, K a multiple of 8."""
+def few_takes(tokens: int, w: torch.Tensor, turn: Optional[tuple] = None) -> bool:
+    """Whether skinny_gemm(kind="auto") hands this product of finished activations to the tcgen05 kernel of few tokens (few_gemm.cu): a large
+    bfloat16 weight matrix with K in whole groups of 64, at most 16 tokens.  `turn` for the ROPE epilogue: (head dimension, rot_half, interleaved)."""
+    return (w.dtype == torch.bfloat16 and 0 < tokens <= STREAM_MAX_TOKENS and w.shape[1] > 0 and w.shape[1] % 64 == 0
+            and w.numel() * 2 >= STREAM_MIN_BYTES and w.data_ptr() % 16 == 0
+            and (turn is None or (turn[0] in (64, 128) and 2 * turn[1] == turn[0] and not turn[2])))
+
+
+def skinny_ok(tokens: int, w: torch.Tensor, turn: Optional[tuple] = None) -> bool:
+    """Shapes the weight-streaming kernels take: bfloat16 weights, at most 16 tokens, K a multiple of 8.  `turn` as for `few_takes`."""
     if not 0 < tokens <= SKINNY_MAX_TOKENS or w.dtype != torch.bfloat16:
         return False
     k = w.shape[1]
     if k % 8:
         return False
     padded = -(-tokens // 8) * 8
-    # the tokens and the partial sums fit in shared memory, or the streaming kernel takes the shape
-    return padded * (k + 8) * 2 + 64 * padded * 4 * 2 <= 200 * 1024 or stream_takes(tokens, w)
+    # the tokens and the partial sums fit in shared memory, or one of the kernels for large matrices takes the shape
+    return padded * (k + 8) * 2 + 64 * padded * 4 * 2 <= 200 * 1024 or stream_takes(tokens, w) or few_takes(tokens, w, turn)
 
 
 # struct SkinnyCall of csrc/skinny_call.cuh: 19 addresses, three doubles, 15 ints
@@ -1984,11 +1994,12 @@ def skinny_gemm(w: torch.Tensor, tokens: int, *, act: Optional[torch.Tensor] = N
                 x_out: Optional[torch.Tensor] = None, rows: Optional[torch.Tensor] = None, epilogue: int = EPI_PLAIN,
                 out: Optional[torch.Tensor] = None, rope: Optional[dict] = None, kind: str = "auto",
                 accumulate: bool = False, out_mult: float = 1.0, gate: str = "silu", gate_limit: Optional[float] = None) -> None:
-    """out = prologue(input) @ w^T with a fused epilogue; see csrc/skinny_gemm.cu and csrc/stream_gemm.cu.
+    """out = prologue(input) @ w^T with a fused epilogue; see csrc/skinny_gemm.cu, csrc/few_gemm.cu and csrc/stream_gemm.cu.
 
-    `kind`: "latency" (skinny_gemm.cu: a CTA per 16 output rows, weights straight to registers), "stream"
-    (stream_gemm.cu: persistent CTAs, weights through a ring of tensor-map copies; up to 16 tokens), or "auto": the
-    streaming kernel for weight matrices of 8 MB and more where it takes the shape.
+    `kind`: "latency" (skinny_gemm.cu: a CTA per 16 output rows, weights straight to registers), "few" (few_gemm.cu: the
+    weight rows as the rows of tcgen05 products, K split over clusters; up to 16 tokens, `act` only), "stream"
+    (stream_gemm.cu: persistent CTAs, weights through a ring of tensor-map copies; up to 16 tokens), or "auto": for weight
+    matrices of 8 MB and more "few" where it takes the call, else "stream" where that does.
 
     Input is either `act` (bfloat16 [tokens, K]) or the norm prologue (`x`, optional `delta`, `norm_w`, `eps`,
     optional `x_out` receiving x + delta, optional `rows` picking rows of x).  PLAIN writes float `out`
@@ -2004,6 +2015,8 @@ def skinny_gemm(w: torch.Tensor, tokens: int, *, act: Optional[torch.Tensor] = N
         rows_in, width = act.shape
         if rows_in < tokens or width != k:
             raise KernelError("skinny_gemm: act must be [tokens, K]")
+        if act.data_ptr() % 16:           # the kernels read rows by 16 bytes
+            act = act.clone()
     else:
         _need(x, torch.float32, "x", 2); _need(norm_w, None, "norm_w", 1)
         if x.shape[1] != k or norm_w.numel() != k:
@@ -2044,8 +2057,15 @@ def skinny_gemm(w: torch.Tensor, tokens: int, *, act: Optional[torch.Tensor] = N
                             r["block_table"].shape[1], int(r["page_size"]), int(r["hq"]), int(r["hkv"]), int(r["dim"]), int(bool(accumulate)), gate_act)
     if (accumulate or out_mult != 1.0) and epilogue != EPI_PLAIN:
         raise KernelError("skinny_gemm: only the plain epilogue adds into its output or multiplies it")
-    if kind not in ("auto", "latency", "stream"):
+    if kind not in ("auto", "latency", "few", "stream"):
         raise KernelError(f"unknown kind {kind!r}")
+    if kind == "few" or (kind == "auto" and act is not None and tokens <= STREAM_MAX_TOKENS and w.numel() * 2 >= STREAM_MIN_BYTES):
+        status = _few_lib().cisr_few_gemm(args, 0)
+        if status != -2:                  # -2: not a call for the tcgen05 kernel of few tokens
+            _check(status, "few_gemm")
+            return
+        if kind == "few":
+            raise KernelError("few_gemm does not take this call")
     if kind == "stream" or (kind == "auto" and tokens <= STREAM_MAX_TOKENS and w.numel() * 2 >= STREAM_MIN_BYTES):
         status = _stream_lib().cisr_stream_gemm(args)
         if status != -2:                  # -2: not a shape for the streaming kernel
@@ -2104,6 +2124,19 @@ def _stream_lib():
         _check(lib.cisr_stream_init(_p(_error_flag())), "stream gemm init", own=0)
         lib.cisr_stream_set_pdl(int(_pdl_state["on"]))
         _stream_state["lib"] = lib
+    return lib
+
+
+_few_state = {}
+
+
+def _few_lib():
+    lib = _few_state.get("lib")
+    if lib is None:
+        lib = load_library("few_gemm.cu")
+        _check(lib.cisr_few_init(_p(_error_flag())), "few gemm init", own=0)
+        lib.cisr_few_set_pdl(int(_pdl_state["on"]))
+        _few_state["lib"] = lib
     return lib
 
 

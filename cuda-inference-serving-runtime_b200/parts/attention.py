@@ -86,13 +86,14 @@ class GQAAttention(Mixer):
         device = ctx.device
         rot = self.position.rotation(ctx)
         q = torch.empty((tokens, hq, dim), dtype=self.dtype, device=device)
-        if cache.write and kernels.skinny_ok(tokens, self.qkv):
+        turn = (dim, rot.rot_half, rot.interleaved) if rot else (dim, 0, False)
+        if cache.write and kernels.skinny_ok(tokens, self.qkv, turn):
             # few tokens: one launch computes (the norm,) the projection, the rotation and the cache write
             rope = dict(cos=rot.cos if rot else None, sin=rot.sin if rot else None, rot_half=rot.rot_half if rot else 0,
                         interleaved=rot.interleaved if rot else False, q_out=q, k_cache=cache.k, v_cache=cache.v,
                         positions=ctx.positions, token_req=ctx.token_req, req_slot=ctx.req_slot,
                         block_table=cache.block_table, page_size=cache.page_size, hq=hq, hkv=hkv, dim=dim)
-            if norm_fusable(h, tokens, self.qkv):
+            if norm_fusable(h, tokens, self.qkv, turn):
                 x_out = h.new_stream_buffer()
                 kernels.skinny_gemm(self.qkv, tokens, x=h.x, delta=h.delta, norm_w=h.weight, eps=h.eps, x_out=x_out,
                                     epilogue=kernels.EPI_ROPE, rope=rope)

@@ -53,14 +53,23 @@ def linear_add(a: torch.Tensor, w: torch.Tensor, into: torch.Tensor) -> torch.Te
     return into
 
 
-def norm_fusable(h, tokens: int, w: torch.Tensor) -> bool:
-    """Whether `h` is a pending norm that this product can compute in its own prologue."""
+FEW_NORM_APART_BYTES = 24 << 20      # a larger matrix hides the launch of the norm's own kernel
+
+
+def norm_fusable(h, tokens: int, w: torch.Tensor, turn=None) -> bool:
+    """Whether `h` is a pending norm that this product can compute in its own prologue; `turn` (head dimension, rot_half, interleaved) where the
+    rotation is its epilogue."""
     if isinstance(h, torch.Tensor):
         return False
     from .base import PendingNorm
     if not (isinstance(h, PendingNorm) and h.fusable() and tokens <= kernels.SKINNY_NORM_MAX_TOKENS
-            and kernels.skinny_ok(tokens, w)):
+            and kernels.skinny_ok(tokens, w, turn)):
         return False
+    # The tcgen05 kernel of few tokens takes finished activations only.  With the norm's kernel in front of it, against the persistent streaming
+    # kernel with the norm in its prologue, us in a graph: 1 token 3072 x 2048 6.5 / 5.9, 6144 x 2048 8.4 / 8.5, 16384 x 2048 14.3 / 15.1,
+    # 28672 x 4096 39.6 / 45.3; 2 tokens 6.6 / 7.1, 8.5 / 10.1, 14.4 / 16.3, 40.8 / 47.1.
+    if kernels.few_takes(tokens, w, turn):
+        return tokens == 1 and w.numel() * 2 < FEW_NORM_APART_BYTES and kernels.stream_takes(tokens, w)
     # The persistent streaming kernel would redo the norm of every token in each of its CTAs, in front of a full ring
     # of weights: beyond two tokens the norm kernel, once, and the activation prologue are faster.
     return not (kernels.stream_takes(tokens, w) and tokens > 2)
