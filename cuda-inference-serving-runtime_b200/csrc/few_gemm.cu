@@ -10,9 +10,11 @@
 // Two CTAs share an SM: one streams while the other starts or ends.
 //
 // What bounds it: the weights at the rate of memory.  The persistent kernel of stream_gemm.cu, whose warps multiply by mma.sync, takes longer with
-// every token and splits no K.  us in a graph with 1, 4 and 16 tokens, that kernel and this one (floor at 6.55 TB/s): 28672 x 4096 gated 43.7, 46.5,
-// 85.2 and 37.0, 37.1, 39.1 (35.9); 4096 x 4096 9.1, 10.6, 17.8 and 7.5, 7.6, 8.2 (5.1); 2048 x 8192 13.7, 16.3, - and 8.4, 8.6, 8.9 (5.1);
-// 49152 x 576 17.0, 18.0, 26.8 and 12.0, 12.5, 15.8 (8.6).  Smaller matrices are the latency kernel's (skinny_gemm.cu): 960 x 2560 3.2 there, 3.7 here.
+// every token and splits no K.  us in a graph with 1, 8 and 16 tokens, that kernel and this one (floor at 6.55 TB/s): 28672 x 4096 gated 43.7, 50.8,
+// 85.2 and 37.5, 38.3, 39.1 (35.9); 4096 x 4096 9.1, 11.7, 17.8 and 7.5, 7.8, 8.1 (5.1); 2048 x 8192 13.7, 24.6, - and 8.6, 8.8, 9.0 (5.1);
+// 49152 x 576 17.0, 19.3, 26.8 and 12.0, 12.4, 12.5 (8.6).  Smaller matrices are the latency kernel's (skinny_gemm.cu): 960 x 2560 3.2 there, 3.7 here.
+// A share that is all of K writes its sums from tensor memory: through shared memory 49152 x 576 takes 15.8 at 16 tokens, 128256 x 4096 161 (159).
+// With 32 or 64 columns it is no longer the better one: 49152 x 576 17.4 and 22.6, the library 12.8 and 13.4.
 // Every wait is bounded; one that runs out sets the error flag (code 4), and what the call wrote is not to be used.
 #include "skinny_call.cuh"
 #include "tcgen05.cuh"
@@ -80,6 +82,11 @@ few_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     int issued = 0;                                        // warp 0: blocks of K requested
     pdl_trigger();
 
+    const bool whole = EPI == EPI_PLAIN && shares == 1;    // sums that are the results: from tensor memory to the output
+    const auto put = [&](int j, int col, float v) {        // one thread owns an element
+        float* dst = a.out_f32 + (size_t)j * a.n + col;
+        *dst = a.accumulate ? *dst + v * a.out_mult : v * a.out_mult;
+    };
     if (warp == 0) {
         const auto load_w = [&](int s, int kb) {
             if (EPI == EPI_SWIGLU) tma_load_4d_elect(ring + s * STAGE, &map_w, 0, 64 * block, 0, 2 * (kb0 + kb), full + s);
@@ -126,18 +133,25 @@ few_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     } else {
         const int quarter = warp & 3;
         pdl_wait();      // outputs may alias what the kernel before still reads
-        if (EPI == EPI_ROPE && warp == 2 && lane < a.m) {
-            const int pos = a.positions[lane], page = a.block_table[(size_t)a.req_slot[a.token_req[lane]] * a.table_width + pos / a.page_size];
-            cache_row[lane] = page < 0 ? -1 : (long long)page * a.hkv * a.page_size + pos % a.page_size;
+        const int token = threadIdx.x - (THREADS - EPI_THREADS);
+        if (EPI == EPI_ROPE && token < a.m) {
+            const int pos = a.positions[token], page = a.block_table[(size_t)a.req_slot[a.token_req[token]] * a.table_width + pos / a.page_size];
+            cache_row[token] = page < 0 ? -1 : (long long)page * a.hkv * a.page_size + pos % a.page_size;
         }
         __syncwarp();
         ok = __all_sync(0xffffffffu, mbar_wait(acc_full, 0));
         tcgen05_fence_after();
+        const int col = block * BM + quarter * 32 + lane;
         if (ok) {
-            uint32_t v[16];
+            uint32_t v[TN];
             tmem_load16(tmem + ((uint32_t)(quarter * 32) << 16), v);
+            if (whole) {
 #pragma unroll
-            for (int j = 0; j < TN; ++j) part[j * BM + quarter * 32 + lane] = __uint_as_float(v[j]);
+                for (int j = 0; j < TN; ++j) if (j < a.m && col < a.n) put(j, col, __uint_as_float(v[j]));
+            } else {
+#pragma unroll
+                for (int j = 0; j < TN; ++j) part[j * BM + quarter * 32 + lane] = __uint_as_float(v[j]);
+            }
         }
     }
     __syncwarp();
@@ -151,12 +165,13 @@ few_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     }
     __syncwarp();
     if (shares > 1) cluster_meet();                        // every share's sums lie in its shared memory
-    if (warp >= 2 && ok) {
+    if (warp >= 2 && ok && !whole) {
         const int tid = threadIdx.x - (THREADS - EPI_THREADS);
         uint32_t from[8];
 #pragma unroll
         for (int q = 0; q < 8; ++q) from[q] = in_cluster(part, q < shares ? q : 0);
         const auto sum = [&](int j, int row) {             // over the shares, in the order of K
+            if (shares == 1) return part[j * BM + row];
             const uint32_t at = (uint32_t)(j * BM + row) * 4u;
             float v[8];
 #pragma unroll
@@ -166,41 +181,39 @@ few_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
             for (int q = 1; q < 8; ++q) if (q < shares) s += v[q];
             return s;
         };
-        const int rows = (EPI == EPI_PLAIN ? BM : BM / 2) / shares, row0 = share * rows;      // this CTA's rows (or pairs of rows) of the block
-        for (int e = tid; e < a.m * rows; e += EPI_THREADS) {
-            const int j = e / rows, r = row0 + e - j * rows;
-            if (EPI == EPI_PLAIN) {
-                const int col = block * BM + r;
-                if (col >= a.n) continue;
-                float* dst = a.out_f32 + (size_t)j * a.n + col;
-                const float there = a.accumulate ? *dst : 0.f;      // one thread owns the element
-                const float v = sum(j, r) * a.out_mult;
-                *dst = a.accumulate ? there + v : v;
-            } else if (EPI == EPI_SWIGLU) {
-                const int f = block * 64 + r, inter = a.n / 2;
-                const float g = sum(j, r), u = sum(j, 64 + r);
-                if (f < inter) a.out_bf16[(size_t)j * inter + f] = __float2bfloat16_rn(gated_product(g, u, a.gate_act, a.gate_limit));
-            } else {
-                const int half = a.dim / 2, in_block = r / half, d = r - in_block * half, hh = block * (BM / a.dim) + in_block, lo = in_block * a.dim + d;
-                const float x = sum(j, lo), y = sum(j, lo + half);
-                if (hh >= a.hq + 2 * a.hkv) continue;
-                const bool is_q = hh < a.hq, is_k = !is_q && hh < a.hq + a.hkv;
-                float first = x, second = y;
-                if (is_q || is_k) {
-                    const float c = a.cos_t[(size_t)j * half + d], s = a.sin_t[(size_t)j * half + d];
-                    first = x * c - y * s;
-                    second = y * c + x * s;
+        const int rows = (EPI == EPI_PLAIN ? BM : BM / 2) / shares, r = share * rows + (tid & (rows - 1));    // this CTA's rows (or pairs of rows) of the block
+        const int j0 = tid >> (31 - __clz(rows)), step = EPI_THREADS >> (31 - __clz(rows));
+        if (EPI == EPI_PLAIN) {
+            const int col = block * BM + r;
+            if (col < a.n)
+#pragma unroll 1
+                for (int j = j0; j < a.m; j += step) put(j, col, sum(j, r));
+        } else if (EPI == EPI_SWIGLU) {
+            const int f = block * 64 + r, inter = a.n / 2;
+            if (f < inter)
+#pragma unroll 1
+                for (int j = j0; j < a.m; j += step)
+                    a.out_bf16[(size_t)j * inter + f] = __float2bfloat16_rn(gated_product(sum(j, r), sum(j, 64 + r), a.gate_act, a.gate_limit));
+        } else {
+            const int half = a.dim / 2, in_block = r / half, d = r - in_block * half, hh = block * (BM / a.dim) + in_block, lo = in_block * a.dim + d;
+            const bool is_q = hh < a.hq, is_k = !is_q && hh < a.hq + a.hkv;
+            const int kvh = is_k ? hh - a.hq : hh - a.hq - a.hkv;
+            if (hh < a.hq + 2 * a.hkv)
+#pragma unroll 1
+                for (int j = j0; j < a.m; j += step) {
+                    const float x = sum(j, lo), y = sum(j, lo + half);
+                    float turned = x, second = y;
+                    if (is_q || is_k) {
+                        const float c = a.cos_t[(size_t)j * half + d], s = a.sin_t[(size_t)j * half + d];
+                        turned = x * c - y * s;
+                        second = y * c + x * s;
+                    }
+                    if (!is_q && cache_row[j] < 0) continue;        // a padding row: its slot holds no pages
+                    bf16* dst = is_q ? a.q_out + ((size_t)j * a.hq + hh) * a.dim + d
+                                     : (is_k ? a.k_cache : a.v_cache) + ((size_t)cache_row[j] + (size_t)kvh * a.page_size) * a.dim + d;
+                    dst[0] = __float2bfloat16_rn(turned);
+                    dst[half] = __float2bfloat16_rn(second);
                 }
-                bf16* dst;
-                if (is_q) dst = a.q_out + ((size_t)j * a.hq + hh) * a.dim + d;
-                else {
-                    if (cache_row[j] < 0) continue;        // a padding row: its slot holds no pages
-                    const int kvh = is_k ? hh - a.hq : hh - a.hq - a.hkv;
-                    dst = (is_k ? a.k_cache : a.v_cache) + ((size_t)cache_row[j] + (size_t)kvh * a.page_size) * a.dim + d;
-                }
-                dst[0] = __float2bfloat16_rn(first);
-                dst[half] = __float2bfloat16_rn(second);
-            }
         }
     }
     __syncwarp();
@@ -214,7 +227,7 @@ int device_sms() {
 }
 // Shares of K for `blocks` blocks of rows and blocks_k blocks of 128 of K: the most of 1, 2, 4, 8 whose CTAs are on the chip at once, two an SM, with
 // two blocks of K each.  us alone with 1, 2, 4, 8 shares, 4 tokens: 2048 x 2048
-// 7.8, 6.7, 5.5, 5.5; 4096 x 14336 45.8, 28.8, 23.4, 21.9; 6144 x 2048 (48 blocks) 10.2, 9.5, 8.3, 11.3; 16384 x 2048 gated (256 blocks) 14.1, 14.2,
+// 7.8, 6.7, 5.5, 5.5; 4096 x 14336 45.8, 28.8, 23.4, 21.9; 6144 x 2048 (48 blocks) 10.2, 9.5, 8.3, 11.3; 16384 x 2048 gated (128 blocks) 14.1, 14.2,
 // 17.2, 22.1.
 int few_shares(int blocks, int blocks_k, int sms) {
     int shares = 1;
@@ -265,6 +278,6 @@ CISR_EXPORT int cisr_few_gemm(const SkinnyCall* call, int shares) {
     const int rows = c.epilogue == EPI_SWIGLU ? c.inter : c.n, per = c.epilogue == EPI_SWIGLU ? BM / 2 : BM, blocks = (rows + per - 1) / per;
     if (!shares) shares = few_shares(blocks, a.blocks_k, device_sms());
     if (shares > a.blocks_k) return -2;
-    return c.epilogue == EPI_PLAIN ? launch<EPI_PLAIN>(c, a, blocks, shares) : c.epilogue == EPI_SWIGLU ? launch<EPI_SWIGLU>(c, a, blocks, shares)
-                                                                                                       : launch<EPI_ROPE>(c, a, blocks, shares);
+    return c.epilogue == EPI_PLAIN ? launch<EPI_PLAIN>(c, a, blocks, shares) : c.epilogue == EPI_SWIGLU
+        ? launch<EPI_SWIGLU>(c, a, blocks, shares) : launch<EPI_ROPE>(c, a, blocks, shares);
 }
