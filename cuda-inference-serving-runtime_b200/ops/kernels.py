@@ -2179,6 +2179,20 @@ def tcgen05_ok(a: torch.Tensor, w: torch.Tensor, fused: bool = False) -> bool:
             and a.shape[1] % 8 == 0 and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
 
 
+# The gated product replaces two launches as well.  us in a graph, library and activation kernel against fused, 17 / 32 / 64 / 120 tokens: 3072 x 576
+# 4.9 / 4.8 / 5.1 / 5.6 and 4.1 / 3.7 / 3.7 / 3.7; 5120 x 960 7.1 / 7.1 / 7.3 / 8.1 and 6.5 / 6.7 / 6.3 / 5.4; 16384 x 2048 15.0 / 15.2 / 16.7 / 19.2 and
+# 18.7 / 13.3 / 13.4 / 13.8; 28672 x 4096 43.1 / 44.6 / 47.7 / 57.2 and 44.6 / 45.4 / 46.3 / 47.7, and of the largest the library is ahead where the
+# kernel before hides no start: a feed-forward of 4096, 14336 and 40 tokens outside a graph 75 and 83.
+TCGEN05_GATED_MIN_TOKENS, TCGEN05_GATED_SMALL_BYTES, TCGEN05_GATED_LARGE_BYTES = 32, 16 << 20, 80 << 20
+
+
+def tcgen05_gated_ok(a: torch.Tensor, w: torch.Tensor) -> bool:
+    """Whether the gated product of `a` with the stacked `w` is better one launch of the tcgen05 kernel."""
+    size = w.numel() * 2
+    least = 0 if size < TCGEN05_GATED_SMALL_BYTES else TCGEN05_GATED_MIN_TOKENS if size < TCGEN05_GATED_LARGE_BYTES else TCGEN05_MIN_TOKENS
+    return tcgen05_ok(a, w, fused=True) and a.shape[0] >= min(TCGEN05_MIN_TOKENS, least)
+
+
 def gemm_tcgen05(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, accumulate: bool = False, out_mult: float = 1.0) -> torch.Tensor:
     """out[M, N] (float) = a[M, K] @ w[N, K]^T on tcgen05 tensor cores fed by TMA (bfloat16 operands); with
     `accumulate`, out += the product (the residual add as the product's epilogue); `out_mult`: the product is multiplied

@@ -69,8 +69,8 @@ def gated_product(h, gate_up: torch.Tensor, activation: str, limit=None) -> torc
             kernels.skinny_gemm(gate_up, tokens, act=as_tensor(h), **gate)
     else:
         hn = as_tensor(h)
-        if kernels.tcgen05_ok(hn, gate_up):
-            kernels.gemm_tcgen05_swiglu(hn, gate_up, act, gate=activation, limit=limit)      # many tokens: the activation is the product's epilogue
+        if kernels.tcgen05_gated_ok(hn, gate_up):
+            kernels.gemm_tcgen05_swiglu(hn, gate_up, act, gate=activation, limit=limit)      # more tokens: the activation is the product's epilogue
         else:
             kernels.swiglu(linear(hn, gate_up), act, gate=activation, limit=limit)
     return act
