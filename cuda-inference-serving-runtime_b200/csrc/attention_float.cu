@@ -3,12 +3,13 @@
 //
 // A CTA has 32 queries of one head and walks tiles of KEYS keys (64, or 32 beyond head size 64): a warp has 16 queries and 16 of
 // every tile's keys, with a running softmax of its own, and the shares are merged at the end.  A tile's keys and values arrive as
-// floats by cp.async while the tile before is multiplied, and are split into parts once for all four warps; the probabilities are split
+// floats by cp.async while the tile before is multiplied, and are split into parts once for all warps; the probabilities are split
 // in the registers in which the scores came out, which are the operand's.
 //
 // What bounds it: products at the rate of mma.sync (six where float has one: 91 TFLOP/s), the splitting beside them, and the longest
 // row of key tiles: tiles of 32 queries make 288 CTAs of 1000 tokens x 9 heads, two per SM, the longest first.
-// With four warps a CTA, each for 32 keys of a tile: 73.  On the CUDA cores (64 queries a CTA, transposed operands in shared memory): 1000 tokens, 9 heads of 64: 137 us; as here 41.
+// 1000 tokens, 9 heads of 64: 41 us; with four warps a CTA, each for 32 keys of a tile, 73; on the CUDA cores (64 queries a CTA, transposed
+// operands in shared memory) 137.
 //
 // Scores or outputs that are not finite (an infinity among the inputs, or a float that rounds to a bfloat16 infinity, has NaN among its
 // parts) send the CTA through plain_rows, which has float multiply-adds only.

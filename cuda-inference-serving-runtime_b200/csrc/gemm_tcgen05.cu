@@ -4,10 +4,11 @@
 //
 //   * few tiles: gemm_tcgen05_split_kernel, a tile per CTA, K cut over a cluster
 //   * more: gemm_tcgen05_pair_kernel, persistent, tiles of 256 rows on two SMs
+//   * routed experts: gemm_tcgen05_experts_kernel, weight rows as the rows of a tile, an expert's tokens as its columns
 //   * grouped products, and narrow ones with many rows: gemm_tcgen05_kernel, persistent CTAs that walk output tiles of 128 x BN
 //     (BN = 256, 128 or 64) with two accumulators of BN columns in tensor memory, so that the epilogue of one tile runs under the
 //     products of the next
-// All three have the same roles (here those of gemm_tcgen05_kernel):
+// All of them have the same roles (here those of gemm_tcgen05_kernel):
 //   * warp 0: one thread issues TMA loads (cp.async.bulk.tensor.2d, 128-byte swizzle) of the A tile
 //     [128 rows x 64 k] and the B tile [BN rows x 64 k] into a STAGES-deep ring of shared memory (3 to 8
 //     stages), each load completing on the stage's "full" mbarrier

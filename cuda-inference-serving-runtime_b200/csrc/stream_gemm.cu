@@ -1,7 +1,8 @@
 // Weight-streaming matrix product for steps with few tokens and large weight matrices (decode of wide models, and
 // the vocabulary head of any model): out[M, N] = a[M, K] * w[N, K]^T, M <= 16, bfloat16 operands, float accumulation.
 // The same prologues and epilogues as skinny_gemm.cu (activation or residual add + RMSNorm in; float out, SwiGLU,
-// rotation + cache write out), built for bandwidth instead of latency:
+// rotation + cache write out), built for bandwidth instead of latency.  Products of finished activations with K in whole
+// groups of 64 are few_gemm.cu's; here are the norm as a prologue, other K and other rotations:
 //
 //   * persistent: one CTA per SM walks "row blocks" (32, 64 or 128 weight rows by all of K); the tokens are staged
 //     (and normalised) once per CTA, not once per 16 rows
