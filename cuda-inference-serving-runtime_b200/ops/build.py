@@ -204,7 +204,8 @@ def exported_signatures(source: Path) -> dict:
 class KernelLibrary(ctypes.CDLL):
     """A built library whose functions have the types they are declared with: an address, a number or a handle is then passed as
     it is (a third of a launch's time in Python went to wrapping each argument), and a call with too few or wrong ones fails.  A function that is
-    not declared in the sources is refused: called without types it would lose half of every address."""
+    not declared in the sources is refused: called without types it would lose half of every address.  For the same reason a function is kept
+    on the library, where other threads find it, only once it has its types (`CDLL.__getattr__` keeps it before)."""
 
     def __init__(self, path: Path, signatures: dict):
         super().__init__(str(path))
@@ -215,8 +216,9 @@ class KernelLibrary(ctypes.CDLL):
             raise AttributeError(name)
         if name not in self._signatures:
             raise AttributeError(f"{name} is not declared in the sources of {self._name}")
-        fn = ctypes.CDLL.__getattr__(self, name)
+        fn = self[name]
         fn.restype, fn.argtypes = self._signatures[name]
+        self.__dict__[name] = fn
         return fn
 
 

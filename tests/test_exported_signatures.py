@@ -32,3 +32,17 @@ def test_an_address_is_passed_whole_and_undeclared_functions_are_refused():
         lib.cisr_not_there
     with pytest.raises(ctypes.ArgumentError):
         lib.cisr_gemm_tcgen05(0.5, 0, 0, 0, 8, 8, 0, 1.0, 0)
+
+
+def test_other_threads_find_a_function_only_with_its_types():
+    path = build.load_library("gemm_tcgen05.cu")._name
+    found = []
+
+    class Watched(dict):
+        def __getitem__(self, name):                     # what another thread would find while this one looks the types up
+            found.append(vars(lib).get(name))
+            return dict.__getitem__(self, name)
+
+    lib = build.KernelLibrary(path, Watched(build.exported_signatures(build.CSRC / "gemm_tcgen05.cu")))
+    fn = lib.cisr_gemm_tcgen05
+    assert found == [None] and vars(lib)["cisr_gemm_tcgen05"] is fn and fn.argtypes[0] is ctypes.c_void_p and lib.cisr_gemm_tcgen05 is fn
