@@ -551,6 +551,7 @@ CISR_EXPORT int cisr_skinny_gemm(const SkinnyCall* call) {
     if (m > 64 || k % 8 || k <= 0 || n <= 0) return -2;
     if (epilogue == EPI_ROPE && (dim % 16 || dim > 256 || dim < 16 || n != (hq + 2 * hkv) * dim || 2 * rot_half > dim)) return -2;
     if (epilogue == EPI_SWIGLU && n != 2 * inter) return -2;
+    if (((uintptr_t)w | (uintptr_t)act | (uintptr_t)x | (uintptr_t)delta | (uintptr_t)x_out) & 15) return -2;      // rows are read and written by 16 bytes
     SkinnyArgs a;
     a.w = (const bf16*)w; a.n = n; a.k = k; a.act = (const bf16*)act; a.x = x; a.delta = delta; a.norm_w = norm_w;
     a.norm_w_bf16 = norm_w_dtype == CISR_BF16; a.eps = eps; a.x_out = x_out; a.rows = rows; a.m = m; a.rt = 1; a.ks = 1;

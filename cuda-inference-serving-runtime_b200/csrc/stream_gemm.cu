@@ -502,8 +502,8 @@ CISR_EXPORT int cisr_stream_init(int* error_flag) {
 }
 
 // The arguments of cisr_skinny_gemm.  Returns -2 for shapes it does not take (more than 16 tokens, K not a
-// multiple of 8, rows too long for shared memory, a rotation that does not pair d with d + dim / 2): the caller then
-// uses the other kernels.
+// multiple of 8, rows too long for shared memory, a rotation that does not pair d with d + dim / 2, operands that do not start on
+// 16 bytes): the caller then uses the other kernels.
 CISR_EXPORT int cisr_stream_gemm(const SkinnyCall* call) {
     const void *w = call->w, *act = call->act, *norm_w = call->norm_w;
     const float *x = (const float*)call->x, *delta = (const float*)call->delta, *cos_t = (const float*)call->cos_t, *sin_t = (const float*)call->sin_t;
@@ -517,7 +517,8 @@ CISR_EXPORT int cisr_stream_gemm(const SkinnyCall* call) {
     const int hq = call->hq, hkv = call->hkv, dim = call->dim, accumulate = call->accumulate, gate_act = call->gate_act;
     if (m <= 0) return 0;
     if (!g_encode || !g_error) return -13;
-    if (m > 16 || k % 8 || k <= 0 || n <= 0 || ((uintptr_t)w & 15)) return -2;
+    if (m > 16 || k % 8 || k <= 0 || n <= 0) return -2;
+    if (((uintptr_t)w | (uintptr_t)act | (uintptr_t)x | (uintptr_t)delta | (uintptr_t)x_out | (norm_w_dtype == CISR_BF16 ? 0 : (uintptr_t)norm_w)) & 15) return -2;
     if (epilogue == EPI_ROPE) {
         if (dim % 32 || dim > 256 || dim < 32 || n != (hq + 2 * hkv) * dim) return -2;
         if (2 * rot_half != dim) return -2;      // the whole head rotates: pairs (d, d + dim / 2), or neighbours when interleaved

@@ -2096,6 +2096,8 @@ def skinny_mlp(h: torch.Tensor, gate_up: torch.Tensor, down: torch.Tensor, gate:
     n, inter = down.shape
     if k != k1 or n2 != 2 * inter:
         raise KernelError("skinny_mlp: shapes of h, gate_up and down disagree")
+    if h.data_ptr() % 16:                 # the kernels read rows by 16 bytes
+        h = h.clone()
     act, out = h.new_empty((tokens, inter)), h.new_empty((tokens, n), dtype=torch.float32)
     gate_act, limit = _gate(gate, gate_limit)
     stream, act_at = _stream(), act.data_ptr()

@@ -29,3 +29,12 @@ def test_what_it_leaves_to_others():
         kernels.skinny_mlp(h, gate_up, down[:, :1528].contiguous())
     with pytest.raises(kernels.KernelError):
         kernels.skinny_mlp(h, gate_up, down, "gated_clamp")
+
+
+def test_activations_off_a_16_byte_boundary():
+    from cisr_b200.ops import kernels
+    g = torch.Generator(device="cuda").manual_seed(3)
+    flat, gate_up, down = ((torch.randn(*s, generator=g, device="cuda") * 576 ** -0.5).bfloat16() for s in ((4 * 576 + 8,), (3072, 576), (576, 1536)))
+    for start in (1, 4, 7):
+        h = flat[start:start + 4 * 576].view(4, 576)
+        assert h.data_ptr() % 16 and torch.equal(kernels.skinny_mlp(h, gate_up, down), kernels.skinny_mlp(h.clone(), gate_up, down))
