@@ -15,7 +15,7 @@
 // parts) send the CTA through plain_rows, which has float multiply-adds only.
 //
 // Compiled once per HEAD_DIM, a multiple of 16 up to 128; with -DSOFTCAP=1 a score becomes cap tanh(score / cap) before the softmax.  Wider heads,
-// and single tokens, are attention.cu's, whose formulas these are.
+// single tokens and buffers that do not start on 16 bytes are attention.cu's, whose formulas these are.
 #include "split_mma.cuh"
 #include "softcap.cuh"
 
@@ -327,6 +327,7 @@ CISR_EXPORT int cisr_attn_prefill_float(const void* q, void* out, const void* k_
                                         const float* sink_heads, void* stream) {
     if (n_tiles <= 0) return 0;
     if (hq % hkv || (SOFTCAP ? !(softcap > 0.f) : softcap != 0.f)) return -2;
+    if (((uintptr_t)q | (uintptr_t)k_cache | (uintptr_t)v_cache) & 15) return -2;      // rows are read by 16 bytes
     static bool configured = false;
     static int sms = 0;
     if (!configured) {
