@@ -2052,9 +2052,9 @@ def skinny_gemm(w: torch.Tensor, tokens: int, *, act: Optional[torch.Tensor] = N
             _need(r[name], torch.int32, name)
         if r["rot_half"]:
             _need(r["cos"], torch.float32, "cos", 2); _need(r["sin"], torch.float32, "sin", 2)
-        args = _skinny_call(w.data_ptr(), act_at, x_at, delta_at, norm_at, x_out_at, rows_at, 0, 0, _p(r["cos"]), _p(r["sin"]), _p(r["q_out"]),
+        args = _skinny_call(w.data_ptr(), act_at, x_at, delta_at, norm_at, x_out_at, rows_at, 0, 0, _p(r.get("cos")), _p(r.get("sin")), _p(r["q_out"]),
                             _p(r["k_cache"]), _p(r["v_cache"]), _p(r["positions"]), _p(r["token_req"]), _p(r["req_slot"]), _p(r["block_table"]), _stream(),
-                            eps, out_mult, gate_limit, n, k, norm_code, tokens, epilogue, 0, int(r["rot_half"]), int(bool(r["interleaved"])),
+                            eps, out_mult, gate_limit, n, k, norm_code, tokens, epilogue, 0, int(r["rot_half"]), int(bool(r.get("interleaved"))),
                             r["block_table"].shape[1], int(r["page_size"]), int(r["hq"]), int(r["hkv"]), int(r["dim"]), int(bool(accumulate)), gate_act)
     if (accumulate or out_mult != 1.0) and epilogue != EPI_PLAIN:
         raise KernelError("skinny_gemm: only the plain epilogue adds into its output or multiplies it")

@@ -1,4 +1,4 @@
-"""Rows of the weight-streaming products are read by 16 bytes: what does not start there is copied or refused, never launched (no GPU needed)."""
+"""What the weight-streaming products are handed: rows, read by 16 bytes, that do not start there; rotations without tables (no GPU needed)."""
 import pytest
 import torch
 
@@ -35,3 +35,21 @@ def test_feed_forward_copies_activations_that_start_off_a_boundary(monkeypatch):
         h = off_by(n, 4, 16)
         kernels.skinny_mlp(h, gate_up, down)
         assert seen[-1] % 16 == 0 and (n or seen[-1] == h.data_ptr())
+
+
+def test_rotation_without_tables_or_pairing(monkeypatch):
+    """A head without rotation needs neither tables nor the order of its pairs."""
+    seen = []
+
+    class Library:
+        def cisr_skinny_gemm(self, args):
+            seen.append(kernels._SKINNY_CALL.unpack(args))
+            return 0
+
+    monkeypatch.setattr(kernels, "_need", lambda *a, **kw: None)
+    monkeypatch.setattr(kernels, "_skinny", Library)
+    monkeypatch.setattr(kernels, "_stream", lambda: 0)
+    ints, cache = torch.zeros(2, 3, dtype=torch.int32), off_by(0, 4, 32)
+    rope = dict(rot_half=0, q_out=cache, k_cache=cache, v_cache=cache, positions=ints, token_req=ints, req_slot=ints, block_table=ints, page_size=2, hq=1, hkv=1, dim=16)
+    kernels.skinny_gemm(off_by(0, 48, 32), 2, act=off_by(0, 2, 32), epilogue=kernels.EPI_ROPE, rope=rope)
+    assert seen[0][9:11] == (0, 0) and seen[0][28:30] == (0, 0)      # cos, sin; rot_half, interleaved
