@@ -251,18 +251,19 @@ CISR_EXPORT int cisr_moe_rows(const void* h, const void* w_up, const void* w_dow
 
 // ---------------------------------------------------------------- many tokens: rows sorted by expert
 // The (token, chosen expert) pairs of a step are laid out expert by expert, each expert's rows padded to whole tiles of
-// `tile` rows, so that one grouped product serves all experts:
+// `tile` rows (1: not at all, which is what the products by runs take: 16 tokens of eight experts each are 128 rows; padded to 128 they were 8192,
+// 206 MB of scratch at a width of 4096):
 //   row_of[pair]        the row of pair t * top + k in the sorted layout
-//   src_token[row]      the token whose activations row `row` holds, -1 for padding (and for rows beyond the last tile used)
-//   tile_group[i]       the expert of row tile i, -1 for tiles beyond the last one used
-//   tiles[i]            (where asked for; src_token and tile_group may then be absent) (expert, first row, rows, 0): every expert's rows cut into
+//   src_token[row]      (may be absent where tiles is given) the token whose activations row `row` holds, -1 for padding and rows beyond the last
+//   tile_group[i]       (likewise) the expert of row tile i, -1 for tiles beyond the last one used
+//   tiles[i]            (where asked for) (expert, first row, rows, 0): every expert's rows cut into
 //                       equal runs of up to `run` rows, in steps of 16, expert by expert; rows 0 beyond the last one
 // Pairs whose expert has no matrices (chosen >= n_experts: an identity expert) get row_of = -1 and no row.
 // One CTA; shared memory: 4 * n_experts ints.  Which row inside its expert's block a pair gets depends on the order the
 // atomics happen to run in; every row is computed by itself and a token's experts are summed in the router's order, so
 // the result does not.
 // The pairs are read SORT_BATCH per thread at a time, all on their way together: with one at a time the kernel waited for
-// memory once per 1024 pairs, twice over (16,384 pairs: 21 us, then 14; 6.5 without src_token, which only the layout's other readers ask for).
+// memory once per 1024 pairs, twice over (16,384 pairs: 21 us, then 14; 6.5 without src_token, which the products by runs do not ask for).
 constexpr int SORT_THREADS = 1024, SORT_BATCH = 16;
 __global__ void __launch_bounds__(SORT_THREADS)
 moe_sort_kernel(const int* __restrict__ chosen, int n_pairs, int top, int n_experts, int tile, int max_rows,

@@ -1644,7 +1644,7 @@ def moe_grouped_ok(h: torch.Tensor, w_up: torch.Tensor, top: int, gated: bool = 
 
 
 def moe_sorted_rows(tokens: int, top: int, experts: int) -> int:
-    """Rows of the sorted layout: every expert's block padded to whole tiles, in the worst case."""
+    """Rows of the layout in whole tiles: every expert's block padded to MOE_TILE rows, in the worst case."""
     pairs = tokens * top
     return max(MOE_TILE, (pairs + min(pairs, experts) * (MOE_TILE - 1)) // MOE_TILE * MOE_TILE)
 
@@ -1656,23 +1656,25 @@ def moe_tiles(tokens: int, top: int, experts: int) -> int:
 
 def moe_sort(chosen: torch.Tensor, experts: int, row_of: torch.Tensor, src_token: Optional[torch.Tensor], tile_group: Optional[torch.Tensor],
              tiles: Optional[torch.Tensor] = None, rows: Optional[int] = None) -> None:
-    """Lay the (token, chosen expert) pairs out expert by expert, each expert's rows padded to whole tiles of MOE_TILE:
-    row_of[pair] = its row, src_token[row] = the token of that row (-1: padding), tile_group[tile] = its expert (-1: unused).
-    `tiles` int32 [moe_tiles, 4] (src_token and tile_group may then be None, `rows` the layout's rows): (expert, first row, rows, 0) of each run of up to
-    MOE_RUN rows, rows 0 beyond the last."""
+    """Lay the (token, chosen expert) pairs out expert by expert: row_of[pair] = its row.
+    With src_token and tile_group each expert's rows are padded to whole tiles of MOE_TILE: src_token[row] = the token of that row (-1: padding),
+    tile_group[tile] = its expert (-1: unused).  With `tiles` int32 [moe_tiles, 4] alone (src_token and tile_group None, `rows` the layout's rows, at
+    least one per pair) the experts' rows follow one another without padding, and tiles has (expert, first row, rows, 0) of each run of up
+    to MOE_RUN rows, rows 0 beyond the last."""
     _need(chosen, torch.int32, "chosen", 2); _need(row_of, torch.int32, "row_of", 1)
     for name, t in (("src_token", src_token), ("tile_group", tile_group)):
         if t is not None or tiles is None:
             _need(t, torch.int32, name, 1)
     tokens, top = chosen.shape
+    tile = 1 if src_token is None and tile_group is None else MOE_TILE
     rows = src_token.numel() if src_token is not None else rows
-    if (rows is None or row_of.numel() != tokens * top or rows % MOE_TILE or (tile_group is not None and tile_group.numel() != rows // MOE_TILE)):
+    if (rows is None or row_of.numel() != tokens * top or rows % tile or (tile_group is not None and tile_group.numel() != rows // tile)):
         raise KernelError("moe_sort: shapes disagree")
     if tiles is not None:
         _need(tiles, torch.int32, "tiles", 2)
         if tiles.shape[1] != 4:
             raise KernelError("moe_sort: tiles must be [n, 4]")
-    _check(_moe().cisr_moe_sort(_p(chosen), tokens, top, experts, MOE_TILE, rows, _p(row_of), _p(src_token), _p(tile_group), _p(tiles),
+    _check(_moe().cisr_moe_sort(_p(chosen), tokens, top, experts, tile, rows, _p(row_of), _p(src_token), _p(tile_group), _p(tiles),
                                 0 if tiles is None else tiles.shape[0], MOE_RUN, _stream()), "moe_sort")
 
 
@@ -1718,12 +1720,10 @@ def moe_grouped(h: torch.Tensor, w_up: torch.Tensor, w_down: torch.Tensor, chose
     top = chosen.shape[1]
     if w_up.shape[2] != hidden or w_down.shape != (experts, hidden, ff) or out.shape != (tokens, hidden) or weight.shape != chosen.shape:
         raise KernelError("moe_grouped: shapes disagree")
-    rows = moe_sorted_rows(tokens, top, experts)
-    device = h.device
+    rows, device = tokens * top, h.device       # a row per pair: the products take runs that start anywhere
     row_of = torch.empty(tokens * top, dtype=torch.int32, device=device)
     tiles = torch.empty((moe_tiles(tokens, top, experts), 4), dtype=torch.int32, device=device)
     moe_sort(chosen, experts, row_of, None, None, tiles, rows)
-    # a padding row's products are made by no one: the padding is not filled
     sorted_h = moe_scatter(h, row_of, torch.empty((rows, hidden), dtype=torch.bfloat16, device=device))
     act = gemm_tcgen05_experts(sorted_h, w_up, torch.empty((rows, ff), dtype=torch.bfloat16, device=device), tiles, tokens * top, activation, gate_limit)
     sorted_out = gemm_tcgen05_experts(act, w_down, torch.empty((rows, hidden), dtype=torch.float32, device=device), tiles, tokens * top)

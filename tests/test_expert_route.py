@@ -13,3 +13,19 @@ def test_route(experts, top, width, ff, gated, tokens, grouped):
     h, w = torch.empty(tokens, width, dtype=torch.bfloat16, device="meta"), torch.empty(experts, ff * (2 if gated else 1), width, dtype=torch.bfloat16, device="meta")
     assert kernels.moe_grouped_ok(h, w, top, gated=gated) is grouped
     assert not kernels.moe_grouped_ok(h.float(), w.float(), top, gated=gated)
+
+
+@pytest.mark.parametrize("tokens,top,experts,width,ff", [(16, 8, 64, 64, 32), (1, 2, 4, 64, 32), (300, 4, 8, 64, 48)])
+def test_scratch_is_a_row_per_pair(tokens, top, experts, width, ff, monkeypatch):
+    """Padded to whole tiles, 16 tokens of 64 experts held 206 MB for 3 MB of rows at a width of 4096."""
+    from cisr_b200.ops import kernels
+    rows, tiles = [], []
+    monkeypatch.setattr(kernels, "_need", lambda *a, **kw: None)
+    monkeypatch.setattr(kernels, "moe_sort", lambda chosen, experts, row_of, src, group, t, n: (rows.append(n), tiles.append(t)))
+    monkeypatch.setattr(kernels, "moe_scatter", lambda h, row_of, out: rows.append(out.shape[0]) or out)
+    monkeypatch.setattr(kernels, "gemm_tcgen05_experts", lambda a, w, out, *rest: rows.append(out.shape[0]) or out)
+    monkeypatch.setattr(kernels, "moe_combine", lambda rows_out, row_of, weight, out, scale, h: out)
+    t = lambda *s: torch.zeros(*s, dtype=torch.bfloat16)
+    kernels.moe_grouped(t(tokens, width), t(experts, 2 * ff, width), t(experts, width, ff), torch.zeros(tokens, top, dtype=torch.int32),
+                        torch.zeros(tokens, top), torch.zeros(tokens, width), gate_limit=7.0)
+    assert rows == [tokens * top] * 4 and tiles[0].shape == (kernels.moe_tiles(tokens, top, experts), 4)
