@@ -265,6 +265,7 @@ CISR_EXPORT int cisr_moe_rows(const void* h, const void* w_up, const void* w_dow
 // The pairs are read SORT_BATCH per thread at a time, all on their way together: with one at a time the kernel waited for
 // memory once per 1024 pairs, twice over (16,384 pairs: 21 us, then 14; 6.5 without src_token, which the products by runs do not ask for).
 constexpr int SORT_THREADS = 1024, SORT_BATCH = 16;
+constexpr size_t SORT_MAX_SMEM = 192 * 1024;      // 12,288 experts
 __global__ void __launch_bounds__(SORT_THREADS)
 moe_sort_kernel(const int* __restrict__ chosen, int n_pairs, int top, int n_experts, int tile, int max_rows,
                 int* __restrict__ row_of, int* __restrict__ src_token, int* __restrict__ tile_group, int4* __restrict__ tiles, int max_tiles, int run) {
@@ -420,7 +421,15 @@ CISR_EXPORT int cisr_moe_sort(const int* chosen, int tokens, int top, int n_expe
     if (tiles && (run < 16 || run % 16 || max_tiles < pairs / run + in_use || ((uintptr_t)tiles & 15))) return -2;
     if (!tiles && (!src_token || !tile_group)) return -2;
     const size_t smem = (size_t)4 * n_experts * sizeof(int);
-    if (smem > 48 * 1024) return -3;
+    if (smem > SORT_MAX_SMEM) return -3;
+    if (smem > 48 * 1024) {
+        static bool configured = false;
+        if (!configured) {
+            const cudaError_t e = cudaFuncSetAttribute(moe_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SORT_MAX_SMEM);
+            if (e != cudaSuccess) return (int)e;
+            configured = true;
+        }
+    }
     return launch_kernel(moe_sort_kernel, dim3(1), dim3(SORT_THREADS), smem, (cudaStream_t)stream, g_pdl, chosen, tokens * top, top, n_experts, tile,
                          max_rows, row_of, src_token, tile_group, (int4*)tiles, max_tiles, run);
 }

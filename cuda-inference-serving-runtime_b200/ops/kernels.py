@@ -1626,15 +1626,18 @@ MOE_GROUPED_MIN_ROWS = 64        # (token, expert) pairs per expert, on average,
 # token, 32 / 64 / 400 tokens 67 / 127 / 744 and 25 / 25 / 29; 64 experts of 1792 + 4096 x 896, 8 per token, 4 / 16 / 100 tokens 147 / 431 / 2194 and
 # 117 / 227 / 259.
 MOE_GROUPED_MIN_SAVED = 40.0
+MOE_SORT_MAX_EXPERTS = 12288     # four counts per expert in the shared memory of the one CTA that sorts
 
 
-def moe_grouped_ok(h: torch.Tensor, w_up: torch.Tensor, top: int, gated: bool = False) -> bool:
+def moe_grouped_ok(h: torch.Tensor, w_up: torch.Tensor, top: int, gated: bool = False, w_down: Optional[torch.Tensor] = None) -> bool:
     """Whether a step's experts run as tcgen05 products of rows sorted by expert: bfloat16, widths whose rows are 16-byte multiples, and enough
-    (token, expert) pairs."""
+    (token, expert) pairs.  Buffers that do not start on 16 bytes and more experts than the sort counts are `moe_rows`'."""
     experts, ff, hidden = w_up.shape
     if gated:
         ff //= 2
     if h.dtype != torch.bfloat16 or hidden % 8 or ff % 8:
+        return False
+    if (h.data_ptr() | w_up.data_ptr() | (w_down.data_ptr() if w_down is not None else 0)) % 16 or experts > MOE_SORT_MAX_EXPERTS:
         return False
     pairs = h.shape[0] * top
     if pairs >= MOE_GROUPED_MIN_ROWS * experts and h.shape[0] >= TCGEN05_MIN_TOKENS:

@@ -147,7 +147,7 @@ class RoutedExperts(FeedForward):
         out = torch.empty((tokens, self.hidden), dtype=torch.float32, device=h.device)
         if self.shared_size and out_scale is not None:
             raise NotImplementedError("a shared expert under a per-channel output scale is not built")
-        if kernels.moe_grouped_ok(h, self.up, self.top, gated=self.gated):
+        if kernels.moe_grouped_ok(h, self.up, self.top, gated=self.gated, w_down=self.down):
             kernels.moe_grouped(h, self.up, self.down, chosen, weight, out, out_scale, gate_limit=self.limit,
                                 activation=self.activation)                                         # many tokens: sorted by expert, tcgen05
         else:

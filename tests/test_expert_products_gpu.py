@@ -58,3 +58,13 @@ def test_products(counts, n, k, kind):
     rest = torch.ones(a.shape[0], dtype=torch.bool, device="cuda")
     rest[row_of] = False
     assert out[rest].isnan().all()                       # rows outside the runs are not written
+
+
+@pytest.mark.parametrize("experts", [3072, 3073, 4096, 12288])      # counts of up to 48 KB, and beyond
+def test_sort_of_many_experts(experts):
+    from cisr_b200.ops import kernels
+    chosen = torch.randint(0, experts, (500, 3), generator=torch.Generator().manual_seed(experts)).int()
+    row_of, tiles = torch.empty(1500, dtype=torch.int32, device="cuda"), torch.empty(kernels.moe_tiles(500, 3, experts), 4, dtype=torch.int32, device="cuda")
+    kernels.moe_sort(chosen.cuda(), experts, row_of, None, None, tiles, 1500)
+    assert torch.equal(chosen.flatten()[torch.argsort(row_of.cpu())].long(), chosen.flatten().long().sort().values) and row_of.unique().numel() == 1500
+    assert int(tiles[:, 2].sum()) == 1500

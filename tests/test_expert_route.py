@@ -29,3 +29,17 @@ def test_scratch_is_a_row_per_pair(tokens, top, experts, width, ff, monkeypatch)
     kernels.moe_grouped(t(tokens, width), t(experts, 2 * ff, width), t(experts, width, ff), torch.zeros(tokens, top, dtype=torch.int32),
                         torch.zeros(tokens, top), torch.zeros(tokens, width), gate_limit=7.0)
     assert rows == [tokens * top] * 4 and tiles[0].shape == (kernels.moe_tiles(tokens, top, experts), 4)
+
+
+def test_what_the_products_by_expert_do_not_take_stays_with_the_rows():
+    """Buffers that start off a 16-byte boundary, and more experts than the sort has room for, took `moe_rows` before few tokens were sorted."""
+    from cisr_b200.ops import kernels
+    off = lambda *s: torch.zeros(torch.Size(s).numel() + 1, dtype=torch.bfloat16)[1:].view(*s)
+    meta = lambda *s: torch.empty(*s, dtype=torch.bfloat16, device="meta")
+    h, up, down = meta(64, 1024), meta(16, 768, 1024), meta(16, 1024, 384)
+    assert kernels.moe_grouped_ok(h, up, 4, gated=True, w_down=down)
+    assert not kernels.moe_grouped_ok(off(64, 1024), up, 4, gated=True, w_down=down)
+    assert not kernels.moe_grouped_ok(h, off(16, 768, 1024), 4, gated=True, w_down=down)
+    assert not kernels.moe_grouped_ok(h, up, 4, gated=True, w_down=off(16, 1024, 384))
+    most = kernels.MOE_SORT_MAX_EXPERTS
+    assert kernels.moe_grouped_ok(meta(4096, 64), meta(most, 64, 64), 128) and not kernels.moe_grouped_ok(meta(4096, 64), meta(most + 1, 64, 64), 128)
