@@ -442,17 +442,13 @@ int launch(StreamArgs& a, const void* w, cudaStream_t s) {
     }
     CUtensorMap map_w;
     int status = 0;
-        if (EPI == EPI_PLAIN && !a.grouped) {
+    if (EPI == EPI_PLAIN && !a.grouped) {
         status = cached_map(&map_w, w, a.n, a.k, a.block_rows, 64);
     } else {
         // More dimensions than the matrix has: the 64-column groups of K as the last one (`grouped`), and where a block's
-        // rows lie in two places one for the halves (see the producer)
-        static std::unordered_map<MapKey, CUtensorMap, MapKeyHash> maps;
-        const MapKey key{w, a.n, a.k, a.block_rows, EPI + 16 * a.grouped + 64 * a.stage_groups};
-        auto it = maps.find(key);
-        if (it == maps.end()) {
-            if (maps.size() > 4096) maps.clear();
-            CUtensorMap map;
+        // rows lie in two places one for the halves (see the producer).  halves < 0 in the key: such a map, and the head size it is for
+        const MapKey key{w, a.n, a.k, a.block_rows, EPI + 16 * a.grouped + 64 * a.stage_groups, EPI == EPI_ROPE ? -a.dim : -1, 0};
+        status = find_map(&map_w, key, [&](CUtensorMap* map) {
             const cuuint64_t row_bytes = (cuuint64_t)a.k * sizeof(bf16);
             const cuuint32_t half = (cuuint32_t)a.block_rows / 2;
             const cuuint64_t inner = a.grouped ? 64 : (cuuint64_t)a.k, groups = (cuuint64_t)a.k / 64;
@@ -474,10 +470,8 @@ int launch(StreamArgs& a, const void* w, cudaStream_t s) {
                 rank = 4;
             }
             if (a.grouped) { dims[rank] = groups; strides[rank - 1] = 128; box[rank] = (cuuint32_t)a.stage_groups; ++rank; }
-            status = make_map_nd(&map, w, rank, dims, strides, box);
-            if (!status) it = maps.emplace(key, map).first;
-        }
-        if (!status) map_w = it->second;
+            return make_map_nd(map, w, rank, dims, strides, box);
+        });
     }
     if (status) return status;
     const int grid = a.n_blocks < sms ? a.n_blocks : sms;

@@ -123,34 +123,39 @@ int make_map_groups(CUtensorMap* map, const void* base, long long rows, int cols
 }
 
 struct MapKey {
-    const void* base; long long rows; int cols, box_rows, box_cols; long long halves;      // box_cols 128: two groups of 64, rows in `halves` runs
+    const void* base; long long rows; int cols, box_rows, box_cols; long long halves; int box_halves;      // box_cols 128: two groups of 64, rows in `halves` runs
     bool operator==(const MapKey& o) const {
-        return base == o.base && rows == o.rows && cols == o.cols && box_rows == o.box_rows && box_cols == o.box_cols && halves == o.halves;
+        return base == o.base && rows == o.rows && cols == o.cols && box_rows == o.box_rows && box_cols == o.box_cols && halves == o.halves &&
+               box_halves == o.box_halves;
     }
 };
 struct MapKeyHash {
     size_t operator()(const MapKey& k) const {
         return std::hash<const void*>()(k.base) ^ ((size_t)k.rows * 1000003u) ^ ((size_t)k.cols * 7919u) ^
-               ((size_t)k.box_rows << 8) ^ (size_t)k.box_cols ^ ((size_t)k.halves << 20);
+               ((size_t)k.box_rows << 8) ^ (size_t)k.box_cols ^ ((size_t)k.halves << 20) ^ ((size_t)k.box_halves << 40);
     }
 };
 std::unordered_map<MapKey, CUtensorMap, MapKeyHash> g_maps;     // a map describes geometry only, so it stays right while the address does
 size_t g_map_cache_limit = 4096;                                // entries kept before the cache is emptied
 
-// The tensor map for (base, shape, box), encoded once and then found again.  The map is COPIED into the caller's
+// The tensor map of `key`, encoded once (encode(map) returns a status) and then found again.  The map is COPIED into the caller's
 // storage: a launcher asks for several maps in a row, and a later call may empty the cache, so nothing may keep a
 // pointer into it.
-int cached_map(CUtensorMap* out, const void* base, long long rows, int cols, int box_rows, int box_cols = 64, long long halves = 1, int box_halves = 1) {
-    const MapKey key{base, rows, cols, box_rows, box_cols, halves};
+template <typename Encode>
+int find_map(CUtensorMap* out, const MapKey& key, Encode encode) {
     auto it = g_maps.find(key);
     if (it == g_maps.end()) {
         if (g_maps.size() >= g_map_cache_limit) g_maps.clear();
         CUtensorMap map;
-        const int status = box_cols == 128 ? make_map_groups(&map, base, rows, cols, box_rows, halves, box_halves) : make_map(&map, base, rows, cols, box_rows, box_cols);
-        if (status) return status;
+        if (const int status = encode(&map)) return status;
         it = g_maps.emplace(key, map).first;
     }
     *out = it->second;
     return 0;
+}
+int cached_map(CUtensorMap* out, const void* base, long long rows, int cols, int box_rows, int box_cols = 64, long long halves = 1, int box_halves = 1) {
+    return find_map(out, MapKey{base, rows, cols, box_rows, box_cols, halves, box_halves}, [&](CUtensorMap* map) {
+        return box_cols == 128 ? make_map_groups(map, base, rows, cols, box_rows, halves, box_halves) : make_map(map, base, rows, cols, box_rows, box_cols);
+    });
 }
 }  // namespace
