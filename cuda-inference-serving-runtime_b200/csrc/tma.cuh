@@ -10,6 +10,7 @@
 #pragma once
 #include <cuda.h>
 
+#include <mutex>
 #include <unordered_map>
 
 #include "common.cuh"
@@ -137,12 +138,14 @@ struct MapKeyHash {
 };
 std::unordered_map<MapKey, CUtensorMap, MapKeyHash> g_maps;     // a map describes geometry only, so it stays right while the address does
 size_t g_map_cache_limit = 4096;                                // entries kept before the cache is emptied
+std::mutex g_maps_lock;                                         // calls come from several threads at a time
 
 // The tensor map of `key`, encoded once (encode(map) returns a status) and then found again.  The map is COPIED into the caller's
 // storage: a launcher asks for several maps in a row, and a later call may empty the cache, so nothing may keep a
 // pointer into it.
 template <typename Encode>
 int find_map(CUtensorMap* out, const MapKey& key, Encode encode) {
+    const std::lock_guard<std::mutex> locked(g_maps_lock);
     auto it = g_maps.find(key);
     if (it == g_maps.end()) {
         if (g_maps.size() >= g_map_cache_limit) g_maps.clear();

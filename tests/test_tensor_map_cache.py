@@ -8,6 +8,8 @@ from cisr_b200.ops import build
 PROGRAM = r"""
 #include <cstdio>
 #include <cstring>
+#include <thread>
+#include <vector>
 #include "tma.cuh"
 
 // a "map" that holds its arguments: base, rank, the boxes
@@ -25,14 +27,31 @@ int boxes() {
     const int status = cached_map(&one, (void*)4096, 512, 256, 64, 128, 2, 1) | cached_map(&two, (void*)4096, 512, 256, 64, 128, 2, 2);
     return status || word(one, 4) != 1 || word(two, 4) != 2;
 }
-int main() {
+int threads() {
+    g_map_cache_limit = 7;                       // emptied again and again
+    std::vector<std::thread> all;
+    std::vector<int> wrong(8);
+    for (int t = 0; t < 8; ++t)
+        all.emplace_back([&, t] {
+            for (int i = 0; i < 200000; ++i) {
+                const long long rows = 128 * (1 + (i * 7 + t) % 13);
+                CUtensorMap map;
+                if (cached_map(&map, (void*)(4096 * rows), rows, 64, 64) || word(map, 0) != 4096ull * rows || word(map, 9) != (unsigned long long)rows) ++wrong[t];
+            }
+        });
+    for (auto& t : all) t.join();
+    int sum = 0;
+    for (int w : wrong) sum += w;
+    return sum;
+}
+int main(int, char** argv) {
     g_encode = write_down;
-    return (boxes()) != 0;
+    return (argv[1][0] == 'b' ? boxes() : threads()) != 0;
 }
 """
 
 
-@pytest.mark.parametrize("part", ["boxes"])        # boxes of another size are told apart
+@pytest.mark.parametrize("part", ["boxes", "threads"])        # boxes of another size are told apart; threads share the cache
 def test_cache(part, tmp_path):
     (tmp_path / "maps.cu").write_text(PROGRAM)
     made = subprocess.run([build.find_nvcc(), *build.ARCH_FLAGS, "-std=c++17", "--expt-relaxed-constexpr", "-I", str(build.CSRC), "-o", str(tmp_path / "maps"),
