@@ -2103,6 +2103,10 @@ def skinny_mlp(h: torch.Tensor, gate_up: torch.Tensor, down: torch.Tensor, gate:
     if h.data_ptr() % 16:                 # the kernels read rows by 16 bytes
         h = h.clone()
     act, out = h.new_empty((tokens, inter)), h.new_empty((tokens, n), dtype=torch.float32)
+    if _timing["records"] is not None:    # every product between events of its own
+        skinny_gemm(gate_up, tokens, act=h, epilogue=EPI_SWIGLU, out=act, gate=gate, gate_limit=gate_limit)
+        skinny_gemm(down, tokens, act=act, epilogue=EPI_PLAIN, out=out)
+        return out
     gate_act, limit = _gate(gate, gate_limit)
     stream, act_at = _stream(), act.data_ptr()
     try:
