@@ -2318,7 +2318,7 @@ def raise_if_kernel_gave_up() -> None:
 
 
 # ------------------------------------------------------------------ per-launch timing, for measurement only
-_timing = {"records": None}
+_timing = {"records": None, "open": []}
 _timed, _untimed = {}, {}      # the kernel functions bracketed by events, and as they are
 
 
@@ -2326,17 +2326,23 @@ class timed_launches:
     """Inside this context every kernel function of this module is bracketed by two CUDA events on the current stream;
     `records` collects (function name, shape description, begin event, end event).  Used by bench.py for the
     per-kernel figures (launches run one after the other, outside graphs, so these are isolated kernel times); the
-    engine never turns it on.  Read the times with `summary()` after a synchronisation."""
+    engine never turns it on.  A launch belongs to the innermost open context; contexts may end in any order.  The functions are bracketed as they are
+    found in this module: one that a caller has taken from it before is the plain one.  Read the times with `summary()` after a synchronisation."""
 
     def __enter__(self):
         self.records = []
+        _timing["open"].append(self)
         _timing["records"] = self.records
         globals().update(_timed)              # outside the context the functions are the plain ones: a wrapper took 0.5 us of every launch
         return self
 
     def __exit__(self, *exc):
-        globals().update(_untimed)
-        _timing["records"] = None
+        _timing["open"].remove(self)
+        if _timing["open"]:
+            _timing["records"] = _timing["open"][-1].records
+        else:
+            globals().update(_untimed)
+            _timing["records"] = None
         return False
 
     def summary(self) -> dict:

@@ -41,3 +41,19 @@ def test_every_function_that_launches_is_described():
     seen_by_parts = {"skinny_mlp"}                       # as the products it is made of
     not_launches = {"attention_library"}                 # an init call
     assert launches - set(kernels._DESCRIBE) == seen_by_parts | not_launches
+
+
+def test_a_context_inside_another_leaves_the_outer_one_open(stand_ins):
+    x = torch.zeros(4, 8)
+    plain = kernels.scale_
+    with kernels.timed_launches() as outer:
+        kernels.scale_(x, 2.0)
+        with kernels.timed_launches() as inner:
+            kernels.scale_(x, 2.0)
+        kernels.scale_(x, 2.0)
+    assert len(outer.records) == 2 and len(inner.records) == 1 and kernels.scale_ is plain
+    first, second = kernels.timed_launches(), kernels.timed_launches()
+    first.__enter__(), second.__enter__(), first.__exit__()
+    kernels.scale_(x, 2.0)
+    second.__exit__()
+    assert len(second.records) == 1 and not first.records and kernels.scale_ is plain
