@@ -61,13 +61,15 @@ few_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     uint64_t* full = reinterpret_cast<uint64_t*>(ring + STAGES * STAGE);
     uint64_t* empty = full + STAGES;
     uint64_t* acc_full = empty + STAGES;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_full + 1);
+    uint64_t* done = acc_full + 1;                         // giving up: every product issued is done
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const int block = blockIdx.x, share = blockIdx.z, shares = gridDim.z;
     const int kb0 = a.blocks_k * share / shares, blocks = a.blocks_k * (share + 1) / shares - kb0;
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) { mbar_init(full + s, 1); mbar_init(empty + s, 1); }
         mbar_init(acc_full, 1);
+        mbar_init(done, 1);
         mbar_init_fence();
     }
     if (warp == 1) {
@@ -79,7 +81,7 @@ few_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     tcgen05_fence_after();
     const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
     bool ok = true;
-    int issued = 0;                                        // warp 0: blocks of K requested
+    int requested = 0;                                     // warp 0: blocks of K
     pdl_trigger();
 
     const bool whole = EPI == EPI_PLAIN && shares == 1;    // sums that are the results: from tensor memory to the output
@@ -101,7 +103,7 @@ few_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         pdl_wait();
         CISR_TRACE_WAITED();
         for (int kb = 0; kb < early; ++kb) load_a(kb, kb);
-        issued = early;
+        requested = early;
         int s = 0;
         uint32_t turn = 0;
         for (int kb = early; kb < blocks; ++kb) {
@@ -110,7 +112,7 @@ few_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
             mbar_expect_tx_elect(full + s, (uint32_t)STAGE);
             load_w(s, kb);
             load_a(s, kb);
-            ++issued;
+            ++requested;
             if (++s == STAGES) { s = 0; turn ^= 1u; }
         }
     } else if (warp == 1) {
@@ -157,12 +159,13 @@ few_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     __syncwarp();
     tcgen05_fence_before();
     ok = !__syncthreads_or(!ok);
-    if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 32;" ::"r"(tmem) : "memory");
     if (!ok) {
         if (threadIdx.x == 0) atomicExch(error, 4);
-        if (warp == 0)                                     // copies in flight end before the block does
-            for (int j = max(issued - STAGES, 0); j < issued; ++j) mbar_wait(full + j % STAGES, (uint32_t)(j / STAGES & 1));
+        if (warp == 0) wait_for_copies(full, requested, STAGES);
+        if (warp == 1) wait_for_products_elect(done);
+        __syncthreads();
     }
+    if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 32;" ::"r"(tmem) : "memory");
     __syncwarp();
     if (shares > 1) cluster_meet();                        // every share's sums lie in its shared memory
     if (warp >= 2 && ok && !whole) {

@@ -51,11 +51,13 @@ gemm_float_kernel(const float* __restrict__ a, const float* __restrict__ w, floa
     uint64_t* empty = full + 2;                                                // [2]: its products have read them
     uint64_t* acc_full = empty + 2;                                            // [2]: its sums are there
     uint64_t* acc_empty = acc_full + 2;                                        // [2]: and have been added
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+    uint64_t* done = acc_empty + 2;                                            // giving up: every product issued is done
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const int n0 = (int)blockIdx.x * TN, m0 = (int)blockIdx.y * BM, blocks = (k + BK - 1) / BK;
     if (threadIdx.x == 0) {
         for (int b = 0; b < 2; ++b) { mbar_init(full + b, SPLIT_WARPS); mbar_init(empty + b, 1); mbar_init(acc_full + b, 1); mbar_init(acc_empty + b, ADD_WARPS); }
+        mbar_init(done, 1);
         mbar_init_fence();
     }
     if (warp == 0) {
@@ -176,6 +178,10 @@ gemm_float_kernel(const float* __restrict__ a, const float* __restrict__ w, floa
     __syncwarp();
     tcgen05_fence_before();
     const int again = __syncthreads_or(odd);
+    if (__syncthreads_or(!ok)) {
+        if (warp == 0) wait_for_products_elect(done);
+        __syncthreads();
+    }
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(2 * TN) : "memory");
     if (again) plain_tile(a, w, out, m0, n0, TN, m, n, k);
 }

@@ -298,7 +298,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     uint64_t* empty_bar = full_bar + STAGES;
     uint64_t* acc_full = empty_bar + STAGES;       // [2]: the MMAs of a tile are done
     uint64_t* acc_empty = acc_full + 2;            // [2]: the epilogue has read the buffer
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+    uint64_t* done = acc_empty + 2;                // giving up: every product issued is done
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int k_blocks = (k + BK - 1) / BK;
@@ -315,6 +316,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) { mbar_init(full_bar + s, 1); mbar_init(empty_bar + s, 1); }
         for (int b = 0; b < 2; ++b) { mbar_init(acc_full + b, 1); mbar_init(acc_empty + b, 4); }
+        mbar_init(done, 1);
         mbar_init_fence();
     }
     if (warp == 1) {    // one warp allocates two accumulators' columns of tensor memory
@@ -326,6 +328,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     tcgen05_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     bool ok = true;
+    int requested = 0;                             // warp 0: k blocks, over all tiles
     pdl_trigger();      // under programmatic dependent launch the next kernel may begin its own set-up now
 
     if (warp == 0) {
@@ -352,7 +355,6 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             }
             pdl_wait();
             CISR_TRACE_WAITED();
-            int kbg = 0;                                                      // k blocks issued so far, over all tiles
             for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
                 const int m0 = row_tile(tile) * BM, n0 = col_tile(tile) * TILE_N;
                 int w_row = n0;
@@ -361,13 +363,13 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                     if (group < 0) continue;
                     w_row = group * n + n0;
                 }
-                for (int kb = 0; kb < k_blocks; ++kb, ++kbg) {
-                    const int s = kbg % STAGES;
-                    if (kbg < early) {        // this stage's barrier is armed and its weight tile on the way already
+                for (int kb = 0; kb < k_blocks; ++kb, ++requested) {
+                    const int s = requested % STAGES;
+                    if (requested < early) {        // this stage's barrier is armed and its weight tile on the way already
                         tma_load_2d(tiles + s * (S::A_BYTES + S::B_BYTES), &map_a, kb * BK, m0, full_bar + s);
                         continue;
                     }
-                    ok = mbar_wait(empty_bar + s, ((kbg / STAGES) & 1) ^ 1);  // the MMAs that read this stage are done
+                    ok = mbar_wait(empty_bar + s, ((requested / STAGES) & 1) ^ 1);  // the MMAs that read this stage are done
                     if (!ok) break;
                     mbar_expect_tx(full_bar + s, (uint32_t)(S::A_BYTES + S::B_BYTES));
                     tma_load_2d(tiles + s * (S::A_BYTES + S::B_BYTES), &map_a, kb * BK, m0, full_bar + s);
@@ -433,7 +435,11 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     }
     if (!ok && lane == 0) atomicExch(error, 1);
     tcgen05_fence_before();
-    __syncthreads();
+    if (__syncthreads_or(!ok)) {
+        if (threadIdx.x == 0) wait_for_copies(full_bar, requested, STAGES);
+        if (threadIdx.x == 32) wait_for_products(done);
+        __syncthreads();
+    }
     if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(tmem_columns(BN)) : "memory");
 }
 
@@ -478,7 +484,8 @@ gemm_tcgen05_split_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
     uint64_t* empty_bar = full_bar + STAGES;
     uint64_t* acc_full = empty_bar + STAGES;
     uint64_t* inbox_full = acc_full + 1;                                       // the other CTAs' shares have arrived
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(inbox_full + 1);
+    uint64_t* done = inbox_full + 1;                                           // giving up: every product issued is done
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
     constexpr int TILE_N = paired_rows(EPI) ? BN / 2 : BN;
     constexpr int COLUMNS = MT * BN;                                           // of tensor memory: 64 to 512, a power of two
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
@@ -490,6 +497,7 @@ gemm_tcgen05_split_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
         for (int s = 0; s < STAGES; ++s) { mbar_init(full_bar + s, 1); mbar_init(empty_bar + s, 1); }
         mbar_init(acc_full, 1);
         mbar_init(inbox_full, 1);
+        mbar_init(done, 1);
         mbar_init_fence();
     }
     if (warp == 1) {
@@ -501,6 +509,7 @@ gemm_tcgen05_split_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
     tcgen05_fence_after();
     const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
     bool ok = true;
+    int requested = 0;                                                         // warp 0: blocks of K
     pdl_trigger();
 
     if (warp == 0) {
@@ -526,6 +535,7 @@ gemm_tcgen05_split_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
         pdl_wait();
         CISR_TRACE_WAITED();
         for (int kb = 0; kb < early; ++kb) load_a(kb, kb);
+        requested = early;
         RingAt at{0, 1u};                                    // the second turn
         for (int kb = early; kb < k_blocks; ++kb, at.next(STAGES)) {
             ok = __all_sync(0xffffffffu, mbar_wait(empty_bar + at.stage, at.turn ^ 1));
@@ -533,6 +543,7 @@ gemm_tcgen05_split_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
             mbar_expect_tx_elect(full_bar + at.stage, (uint32_t)S::STAGE);
             load_a(at.stage, kb);
             load_b(at.stage, kb);
+            ++requested;
         }
     } else if (warp == 1) {
         constexpr uint32_t idesc = umma_idesc(BN);
@@ -648,7 +659,11 @@ gemm_tcgen05_split_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
     }
     if (!ok && lane == 0) atomicExch(error, 1);
     tcgen05_fence_before();
-    __syncthreads();
+    if (__syncthreads_or(!ok)) {
+        if (warp == 0) wait_for_copies(full_bar, requested, STAGES);
+        if (warp == 1) wait_for_products_elect(done);
+        __syncthreads();
+    }
     if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(COLUMNS) : "memory");
 }
 
@@ -673,6 +688,20 @@ struct PairSmem {
     static constexpr size_t TOTAL = TILES + 1024 /* alignment slack */ + 256 /* barriers */ + 8 * STAGE_BYTES;
 };
 
+// The end of a pair's kernel: neither CTA leaves while the other's products read its tiles or its barriers are told.  Where a wait ran out, the first CTA,
+// on whose barriers the copies of both complete and which issues the products, waits for both before it meets the other.
+__device__ __forceinline__ void meet_pair(bool ok, int rank, int warp, uint64_t* full_bar, int requested, int stages, uint64_t* done, int* error) {
+    if (!ok && (threadIdx.x & 31) == 0) atomicExch(error, 1);
+    __syncwarp();
+    tcgen05_fence_before();
+    if (__syncthreads_or(!ok) && rank == 0) {
+        if (warp == 0) wait_for_copies(full_bar, requested, stages);
+        if (warp == 1) wait_for_products_pair_elect(done);
+        __syncwarp();
+    }
+    cluster_meet();
+}
+
 template <int EPI>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
 gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
@@ -685,7 +714,8 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     uint64_t* empty_bar = full_bar + PAIR_STAGES;
     uint64_t* acc_full = empty_bar + PAIR_STAGES;
     uint64_t* acc_empty = acc_full + 2;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+    uint64_t* done = acc_empty + 2;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
 
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const int rank = (int)blockIdx.x & 1, pair = (int)blockIdx.x >> 1, pairs = (int)gridDim.x >> 1;
@@ -695,6 +725,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     if (threadIdx.x == 0) {
         for (int s = 0; s < PAIR_STAGES; ++s) { mbar_init(full_bar + s, 1); mbar_init(empty_bar + s, 1); }
         for (int b = 0; b < 2; ++b) { mbar_init(acc_full + b, 1); mbar_init(acc_empty + b, 16); }
+        mbar_init(done, 1);
         mbar_init_fence();
     }
     if (warp == 1) {
@@ -706,6 +737,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     tcgen05_fence_after();
     const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
     bool ok = true;
+    int requested = 0;                   // warp 0: blocks of K, over all tiles
     pdl_trigger();
 
     if (warp == 0) {
@@ -740,6 +772,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
                     load_b(at.stage, kb, n0);
                 }
                 load_a(at.stage, kb, m0);
+                ++requested;
             }
         }
     } else if (warp == 1) {
@@ -794,10 +827,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
             if (lane == 0) mbar_arrive_cluster(in_cluster(acc_empty + acc, 0));
         }
     }
-    if (!ok && lane == 0) atomicExch(error, 1);
-    __syncwarp();
-    tcgen05_fence_before();
-    cluster_meet();                      // neither CTA leaves while the other's products read its tiles or its barriers are told
+    meet_pair(ok, rank, warp, full_bar, requested, stages, done, error);
     if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(2 * PAIR_BN) : "memory");
 }
 
@@ -847,7 +877,8 @@ gemm_tcgen05_experts_kernel(const __grid_constant__ ExpertMaps maps, const Epilo
     uint64_t* empty_bar = full_bar + PAIR_STAGES;
     uint64_t* acc_full = empty_bar + PAIR_STAGES;
     uint64_t* acc_empty = acc_full + 2;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+    uint64_t* done = acc_empty + 2;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
 
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const int rank = (int)blockIdx.x & 1, pair = (int)blockIdx.x >> 1, pairs = (int)gridDim.x >> 1;
@@ -858,6 +889,7 @@ gemm_tcgen05_experts_kernel(const __grid_constant__ ExpertMaps maps, const Epilo
     if (threadIdx.x == 0) {
         for (int s = 0; s < PAIR_STAGES; ++s) { mbar_init(full_bar + s, 1); mbar_init(empty_bar + s, 1); }
         for (int b = 0; b < 2; ++b) { mbar_init(acc_full + b, 1); mbar_init(acc_empty + b, 16); }
+        mbar_init(done, 1);
         mbar_init_fence();
     }
     if (warp == 1) {
@@ -869,6 +901,7 @@ gemm_tcgen05_experts_kernel(const __grid_constant__ ExpertMaps maps, const Epilo
     tcgen05_fence_after();
     const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
     bool ok = true;
+    int requested = 0;                   // warp 0: blocks of K, over all tiles
     pdl_trigger();
     pdl_wait();                          // the tiles come from a kernel before
     // item i: the rows of tiles_list[i / tiles_n] with column tile i % tiles_n; every role walks the same items, and asks for the next one's rows early
@@ -903,6 +936,7 @@ gemm_tcgen05_experts_kernel(const __grid_constant__ ExpertMaps maps, const Epilo
                     }
                     tma_load_2d_pair(stage + S::A_BYTES, rows, kb * BK, row0, bar);
                 }
+                ++requested;
             }
         }
     } else if (warp == 1) {
@@ -995,10 +1029,7 @@ gemm_tcgen05_experts_kernel(const __grid_constant__ ExpertMaps maps, const Epilo
             if (lane == 0) mbar_arrive_cluster(in_cluster(acc_empty + acc, 0));
         }
     }
-    if (!ok && lane == 0) atomicExch(error, 1);
-    __syncwarp();
-    tcgen05_fence_before();
-    cluster_meet();
+    meet_pair(ok, rank, warp, full_bar, requested, stages, done, error);
     if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(2 * PAIR_BN) : "memory");
 }
 

@@ -109,6 +109,33 @@ __device__ __forceinline__ void umma_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
+// Giving up.  A kernel whose wait ran out may still have copies on the way into its shared memory and products that read it: before it frees its
+// tensor memory and leaves, the producer waits for the copies of the last blocks it requested, and the warp that issued the products for a barrier
+// (initialised with one arrival, told by nothing else) that they tell.  Both waits are bounded as every other.
+struct BlockAt {                       // where block j of K is in a ring of `stages`: the stage, and the parity of its turn there
+    int stage; uint32_t turn;
+    __host__ __device__ BlockAt(int j, int stages) : stage(j % stages), turn((uint32_t)(j / stages) & 1u) {}
+};
+__host__ __device__ __forceinline__ int first_in_flight(int requested, int stages) { return requested > stages ? requested - stages : 0; }
+__device__ __forceinline__ void wait_for_copies(uint64_t* full, int requested, int stages) {
+    for (int j = first_in_flight(requested, stages); j < requested; ++j) {
+        const BlockAt at(j, stages);
+        mbar_wait(full + at.stage, at.turn);
+    }
+}
+__device__ __forceinline__ void wait_for_products(uint64_t* done) {             // by the lane that issued them
+    umma_commit(done);
+    mbar_wait(done, 0);
+}
+__device__ __forceinline__ void wait_for_products_elect(uint64_t* done) {       // by the warp one lane of which issued them
+    umma_commit_elect(done);
+    mbar_wait(done, 0);
+}
+__device__ __forceinline__ void wait_for_products_pair_elect(uint64_t* done) {  // in the pair's first CTA
+    umma_commit_pair_elect(done);
+    mbar_wait(done, 0);
+}
+
 // 32 consecutive accumulator columns of this thread's lane (its output row)
 __device__ __forceinline__ void tmem_load32(uint32_t taddr, uint32_t (&v)[32]) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 "
