@@ -410,6 +410,7 @@ CISR_EXPORT int cisr_attn_prefill(const void* q, void* out, const void* k_cache,
                                   const float* sink_heads, void* stream) {
     if (n_tiles <= 0) return 0;
     if (hq % hkv || (SOFTCAP ? !(softcap > 0.f) : softcap != 0.f)) return -2;
+    if (((uintptr_t)q | (uintptr_t)k_cache | (uintptr_t)v_cache) & 15) return -2;      // rows are read by 16 bytes
     static bool configured = false;
     if (!configured) {
         cudaError_t e = cudaFuncSetAttribute(attn_prefill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PREFILL_SMEM);
@@ -430,6 +431,7 @@ CISR_EXPORT int cisr_attn_decode(const void* q, void* out, const void* k_cache, 
                                  float sink, const float* sink_heads, void* stream) {
     if (n_dec <= 0) return 0;
     if (hq % hkv || split_size <= 0 || n_splits <= 0 || (SOFTCAP ? !(softcap > 0.f) : softcap != 0.f)) return -2;
+    if (((uintptr_t)q | (uintptr_t)k_cache | (uintptr_t)v_cache) & 15) return -2;      // rows are read by 16 bytes
     const size_t smem = decode_smem_floats(hq / hkv) * sizeof(float);
     if (smem > 220 * 1024) return -3;
     static size_t configured = 48 * 1024;

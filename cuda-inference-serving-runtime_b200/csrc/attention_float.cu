@@ -15,7 +15,7 @@
 // parts) send the CTA through plain_rows, which has float multiply-adds only.
 //
 // Compiled once per HEAD_DIM, a multiple of 16 up to 128; with -DSOFTCAP=1 a score becomes cap tanh(score / cap) before the softmax.  Wider heads,
-// single tokens and buffers that do not start on 16 bytes are attention.cu's, whose formulas these are.
+// and single tokens, are attention.cu's, whose formulas these are.
 #include "split_mma.cuh"
 #include "softcap.cuh"
 

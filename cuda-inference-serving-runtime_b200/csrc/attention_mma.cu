@@ -1021,6 +1021,7 @@ CISR_EXPORT int cisr_attn_prefill(const void* q, void* out, const void* k_cache,
                                   int keep_first, float sink, const float* sink_heads, void* stream) {
     if (n_tiles <= 0) return 0;
     if (hq % hkv || (SOFTCAP ? !(softcap > 0.f) : softcap != 0.f)) return -2;
+    if (((uintptr_t)q | (uintptr_t)k_cache | (uintptr_t)v_cache) & 15 || (uintptr_t)out & 3) return -2;      // rows are read by 16 bytes, written in pairs
     const size_t smem = PREFILL_SMEM + sizeof(int) * ((size_t)table_width + 4);    // a tile's key range spans at most the table
     if (smem > 220 * 1024) return -3;
     static size_t configured = 0;
@@ -1043,6 +1044,7 @@ CISR_EXPORT int cisr_attn_decode(const void* q, void* out, const void* k_cache, 
     // (merge_proj.cu merges them in the prologue of the output projection); `out` is then not written.
     if (n_dec <= 0) return 0;
     if (hq % hkv || split_size <= 0 || n_splits <= 0 || (SOFTCAP ? !(softcap > 0.f) : softcap != 0.f)) return -2;
+    if (((uintptr_t)q | (uintptr_t)k_cache | (uintptr_t)v_cache) & 15) return -2;      // rows are read by 16 bytes
     const size_t smem = DEC_SMEM + sizeof(int) * ((size_t)split_size / page_size + 4);   // + the range's block table entries
     if (smem > 220 * 1024) return -3;
     static size_t configured = 0;
@@ -1099,7 +1101,7 @@ CISR_EXPORT int cisr_attn_decode_tma(const void* q, void* out, const void* k_cac
     if (!merge && g_clusters) return -2;      // the caller's own merge needs every range's partial sum
     if (hq % hkv || n_splits <= 0 || !cisr_attn_decode_tma_ok(page_size, split_size) || (SOFTCAP ? !(softcap > 0.f) : softcap != 0.f)) return -2;
     const long long cache_rows = (long long)n_pages * hkv * page_size;
-    if (cache_rows <= 0 || cache_rows >= (1ll << 31) || (((uintptr_t)k_cache | (uintptr_t)v_cache) & 15)) return -2;
+    if (cache_rows <= 0 || cache_rows >= (1ll << 31) || (((uintptr_t)q | (uintptr_t)k_cache | (uintptr_t)v_cache) & 15)) return -2;
     const int box_rows = page_size < TK ? page_size : TK;
     CUtensorMap map_k, map_v;
     int status = cached_map(&map_k, k_cache, cache_rows, D, box_rows, 64);

@@ -461,8 +461,7 @@ def attn_prefill(q, out, k_cache, v_cache, req_slot, block_table, tile_req, tile
     for name, t in (("req_slot", req_slot), ("block_table", block_table), ("tile_req", tile_req), ("tile_q0", tile_q0), ("q_start", q_start),
                     ("q_len", q_len), ("ctx_len", ctx_len)):
         _need(t, torch.int32, name)
-    if (kind == "auto" and k_cache.dtype == torch.float32 and dim <= FLOAT_PREFILL_MAX_HEAD_DIM
-            and not (q.data_ptr() | k_cache.data_ptr() | v_cache.data_ptr()) % 16):      # that kernel reads rows by 16 bytes
+    if kind == "auto" and k_cache.dtype == torch.float32 and dim <= FLOAT_PREFILL_MAX_HEAD_DIM:
         launch = _attention_float(dim, softcap is not None).cisr_attn_prefill_float
     else:
         launch = attention_library(dim, k_cache.dtype, kind, softcap is not None).cisr_attn_prefill
