@@ -5,8 +5,10 @@
 //     128 or two of 64), or 64 gate rows and the 64 up rows of the same features (SWIGLU)
 //   * warp 0: TMA copies of 128 of K at a time: the block's rows in ONE box of 32 KB and the tokens in one of 4 KB, into a ring of three stages;
 //     the first stages' weights are requested before the wait on the kernel before
-//   * warp 1: tcgen05.mma (M = 128, N = 16); warps 2..5: the sums of a share from tensor memory to shared memory, one barrier.cluster, and each CTA
-//     adds the shares of its part of the rows, in the order of K, and runs the epilogue on them
+//   * warp 1: tcgen05.mma (M = 128, N = 16), the eight products of a block into eight accumulators.  The tensor core cuts a sum instead of
+//     rounding it: with all of K in one accumulator the error against 64 bits was 3.6 to 4.5 times that of stream_gemm.cu's eight slices of K
+//   * warps 2..5: the accumulators, added in float, are a share's sums; they go to shared memory, one barrier.cluster, and each CTA adds the shares of
+//     its part of the rows, in the order of K, and runs the epilogue on them
 // Two CTAs share an SM: one streams while the other starts or ends.
 //
 // What bounds it: the weights at the rate of memory.  The persistent kernel of stream_gemm.cu, whose warps multiply by mma.sync, takes longer with
@@ -23,6 +25,7 @@ namespace {
 typedef __nv_bfloat16 bf16;
 enum : int { EPI_PLAIN = 0, EPI_SWIGLU = 1, EPI_ROPE = 2 };
 constexpr int TN = 16, BK2 = 128, STAGES = 3, THREADS = 192, EPI_THREADS = 128;
+constexpr int SLICES = BK2 / 16, TMEM_COLUMNS = SLICES * TN;      // an accumulator for each sixteen of a block's K
 constexpr size_t A_BYTES = (size_t)BM * BK2 * sizeof(bf16), B_BYTES = (size_t)TN * BK2 * sizeof(bf16), STAGE = A_BYTES + B_BYTES;
 constexpr size_t SMEM = STAGES * STAGE + 1024 /* alignment slack */ + 128 /* barriers */;
 bool g_pdl = false;
@@ -36,13 +39,6 @@ struct FewArgs {
     int n, m, blocks_k, accumulate, gate_act, table_width, page_size, hq, hkv, dim;
 };
 
-__device__ __forceinline__ void tmem_load16(uint32_t taddr, uint32_t (&v)[16]) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-                   "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-                 : "r"(taddr) : "memory");
-    tmem_load_wait();
-}
 __device__ __forceinline__ void cluster_meet() { asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 __device__ __forceinline__ float load_cluster(uint32_t at) {
     float v;
@@ -73,7 +69,7 @@ few_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         mbar_init_fence();
     }
     if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 32;" ::"r"(smem_u32(tmem_slot)) : "memory");
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(TMEM_COLUMNS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     tcgen05_fence_before();
@@ -126,8 +122,9 @@ few_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
             tcgen05_fence_after();
             const uint64_t at = (uint64_t)s * (STAGE >> 4);
 #pragma unroll
-            for (int kk = 0; kk < BK2 / 16; ++kk)
-                umma_bf16_elect(tmem, desc_a + at + kk / 4 * (A_BYTES / 2 >> 4) + 2 * (kk % 4), desc_b + at + kk / 4 * (B_BYTES / 2 >> 4) + 2 * (kk % 4), idesc, (kb | kk) != 0);
+            for (int kk = 0; kk < SLICES; ++kk)
+                umma_bf16_elect(tmem + (uint32_t)(kk * TN), desc_a + at + kk / 4 * (A_BYTES / 2 >> 4) + 2 * (kk % 4), desc_b + at + kk / 4 * (B_BYTES / 2 >> 4) + 2 * (kk % 4),
+                                idesc, kb != 0);
             umma_commit_elect(empty + s);
             if (++s == STAGES) { s = 0; turn ^= 1u; }
         }
@@ -145,14 +142,23 @@ few_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         tcgen05_fence_after();
         const int col = block * BM + quarter * 32 + lane;
         if (ok) {
-            uint32_t v[TN];
-            tmem_load16(tmem + ((uint32_t)(quarter * 32) << 16), v);
+            float v[TN];
+#pragma unroll
+            for (int q = 0; q < SLICES; q += 2) {              // the slices' sums, rounded where they meet
+                uint32_t two[2 * TN];
+                tmem_load32(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(q * TN), two);
+#pragma unroll
+                for (int j = 0; j < TN; ++j) {
+                    const float pair = __uint_as_float(two[j]) + __uint_as_float(two[TN + j]);
+                    v[j] = q ? v[j] + pair : pair;
+                }
+            }
             if (whole) {
 #pragma unroll
-                for (int j = 0; j < TN; ++j) if (j < a.m && col < a.n) put(j, col, __uint_as_float(v[j]));
+                for (int j = 0; j < TN; ++j) if (j < a.m && col < a.n) put(j, col, v[j]);
             } else {
 #pragma unroll
-                for (int j = 0; j < TN; ++j) part[j * BM + quarter * 32 + lane] = __uint_as_float(v[j]);
+                for (int j = 0; j < TN; ++j) part[j * BM + quarter * 32 + lane] = v[j];
             }
         }
     }
@@ -165,7 +171,7 @@ few_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         if (warp == 1) wait_for_products_elect(done);
         __syncthreads();
     }
-    if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 32;" ::"r"(tmem) : "memory");
+    if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLUMNS) : "memory");
     __syncwarp();
     if (shares > 1) cluster_meet();                        // every share's sums lie in its shared memory
     if (warp >= 2 && ok && !whole) {

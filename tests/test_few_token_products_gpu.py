@@ -124,3 +124,20 @@ def test_rule():
     for turn in ((128, 64, True), (128, 32, False), (96, 48, False), (128, 0, False)):
         assert not kernels.few_takes(4, big, turn)
     assert kernels.skinny_ok(16, big) and not kernels.skinny_ok(16, big, (96, 48, False))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,k", [(49152, 576), (8192, 2048), (4096, 4096), (1024, 4160)])
+@pytest.mark.parametrize("tokens", [1, 16])
+def test_sums_are_as_exact_as_the_streaming_kernels(n, k, tokens):
+    """The tensor core cuts what it adds: with K in one accumulator these sums were 3.6 times (K 576) and 4.5 times (K 2048) as far from 64 bits."""
+    g = torch.Generator(device="cuda").manual_seed(k)
+    w = (torch.randn(n, k, generator=g, device="cuda") * k ** -0.5).bfloat16()
+    a = torch.randn(tokens, k, generator=g, device="cuda").bfloat16()
+    want, errors = a.double() @ w.double().T, {}
+    for kind in ("few", "stream"):
+        out = torch.empty(tokens, n, device="cuda")
+        kernels.skinny_gemm(w, tokens, act=a, out=out, kind=kind)
+        errors[kind] = float((out.double() - want).norm() / want.norm())
+    kernels.raise_if_kernel_gave_up()
+    assert errors["few"] <= 1.1 * errors["stream"], errors           # the same number of cuts; a tenth for how they fall
