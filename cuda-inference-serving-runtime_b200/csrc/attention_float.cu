@@ -12,7 +12,8 @@
 // operands in shared memory) 137.
 //
 // Scores or outputs that are not finite (an infinity among the inputs, or a float that rounds to a bfloat16 infinity, has NaN among its
-// parts) send the CTA through plain_rows, which has float multiply-adds only.
+// parts), and outputs other than zero below 2^-64 (values below about 2^-110 run out of exponents for their parts), send the CTA through plain_rows,
+// which has float multiply-adds only.
 //
 // Compiled once per HEAD_DIM, a multiple of 16 up to 128; with -DSOFTCAP=1 a score becomes cap tanh(score / cap) before the softmax.  Wider heads,
 // and single tokens, are attention.cu's, whose formulas these are.
@@ -293,7 +294,12 @@ attn_prefill_split_kernel(const __grid_constant__ SplitAttention a) {
             inv[h] = 1.f / (sk > -INFINITY ? l + expf(sk - m_use) : l);
             if (row0 + 8 * h < r.rows)
 #pragma unroll
-                for (int j = 0; j < D / 8; ++j) odd = fmaf(o[j][2 * h], 0.f, fmaf(o[j][2 * h + 1], 0.f, odd));
+                for (int j = 0; j < D / 8; ++j)
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        const float x = fabsf(o[j][2 * h + e] * inv[h]);
+                        odd = fmaf(o[j][2 * h + e], 0.f, x > 0.f && x < 0x1p-64f ? NAN : odd);
+                    }
         }
     }
     if (__syncthreads_or(odd != 0.f)) {                               // 0 x finite is 0, else NaN, and a NaN stays

@@ -7,8 +7,8 @@
 //   * eight warps add each block's sums to their own in registers, and one of them issues the next block's products before (tcgen05.mma,
 //     kind::f16, a block's 24 into one of two accumulators, the smallest parts first).  The tensor core cuts a sum instead of rounding it, so no sum stays there
 //     for longer than a block: one rounding per 64 terms, and four of the large products between two
-// Sums that are not finite (an infinity, or a float that rounds to a bfloat16 infinity, has NaN among its parts) are made once more by float
-// multiply-adds.
+// Sums that are not finite (an infinity, or a float that rounds to a bfloat16 infinity, has NaN among its parts), and sums other than zero below 2^-64
+// (operands below about 2^-110 run out of exponents for their parts), are made once more by float multiply-adds.
 //
 // What bounds it: shared memory, whose 128 bytes a cycle serve the products (8 KB per 128 x 128 x 16), the parts as they are laid down, and
 // nothing else: 2300 cycles a block, measured 2700 (1.45 us; 64 columns 1.07).  us, cuBLAS and here: 1000 rows of 960 x 576 29 and 15; 512 rows
@@ -29,11 +29,13 @@ struct FloatSmem {
 
 __device__ __forceinline__ void arrive(uint64_t* bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory"); }
 
-// the tile's elements [rows][TN] by float multiply-adds
+// a sum that the parts may not have carried
+__device__ __forceinline__ bool is_odd(float sum) { return !(fabsf(sum) < INFINITY) || (sum != 0.f && fabsf(sum) < 0x1p-64f); }
+// those of the tile's elements [rows][TN] by float multiply-adds
 __device__ __noinline__ void plain_tile(const float* __restrict__ a, const float* __restrict__ w, float* __restrict__ out, int m0, int n0, int tn, int m, int n, int k) {
     for (int e = threadIdx.x; e < BM * tn; e += THREADS) {
         const int row = m0 + e / tn, col = n0 + e % tn;
-        if (row >= m || col >= n) continue;
+        if (row >= m || col >= n || !is_odd(out[(size_t)row * n + col])) continue;
         float sum = 0.f;
         for (int i = 0; i < k; ++i) sum = fmaf(a[(size_t)row * k + i], w[(size_t)col * k + i], sum);
         out[(size_t)row * n + col] = sum;
@@ -116,10 +118,8 @@ gemm_float_kernel(const float* __restrict__ a, const float* __restrict__ w, floa
         }
         const int row = m0 + quarter * 32 + lane, col = n0 + half * COLS;
         if (ok && row < m) {
-            float z = 0.f;                                                     // 0 x finite is 0, else NaN, and a NaN stays
 #pragma unroll
-            for (int j = 0; j < COLS; ++j) z = fmaf(sums[j], 0.f, z);
-            odd = z != 0.f;
+            for (int j = 0; j < COLS; ++j) odd |= is_odd(sums[j]);
             float* dst = out + (size_t)row * n + col;
             const bool runs = (n & 3) == 0 && ((uintptr_t)out & 15) == 0;
 #pragma unroll

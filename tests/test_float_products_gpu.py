@@ -40,6 +40,13 @@ def test_large_and_small_operands():
     assert ((out.double() - want).abs() <= 2.0 ** -20 * size).all()
     a, w = torch.full((3, 64), 3e38, device="cuda"), torch.full((2, 64), 1e-3, device="cuda")
     assert torch.allclose(kernels.gemm_float(a, w, torch.empty(3, 2, device="cuda")), torch.full((3, 2), 64 * 3e35, device="cuda"), rtol=1e-6)
+    for power in (-60, -100, -112, -120):                    # results of about 2^-114 at the least: beside them a term's rounding to a subnormal's last place is 2^-35
+        a, w = operands(130, 70, 192)
+        small, w = a.abs() * 2.0 ** power, w.abs()
+        for left, right in ((small, w), (w, small)):
+            out = kernels.gemm_float(left, right, torch.empty(left.shape[0], right.shape[0], device="cuda"))
+            want = left.double() @ right.double().T
+            assert ((out.double() - want).abs() <= 1e-6 * want).all(), power
 
 
 @pytest.mark.gpu

@@ -81,3 +81,11 @@ def test_values_without_bound():
     bad[71:, :, 3] = True
     assert got[bad].isnan().all()
     near(got[~bad], want[~bad])
+
+
+@pytest.mark.parametrize("power", [-60, -100, -112, -120])
+def test_small_values(power):
+    """Values whose bfloat16 parts run out of exponents."""
+    got, want = attend([(70, 33), (5, 0)], 64, 4, 2, change=lambda q, k, v, table: v.abs_().mul_(2.0 ** power))
+    # as `near`, and the rounding of a probability's product with a value to the last place of a subnormal, 103 keys
+    assert ((got.double() - want).abs() <= 6e-6 * want + 103 * 2.0 ** -149).all()
