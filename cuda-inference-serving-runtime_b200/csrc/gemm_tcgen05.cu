@@ -285,7 +285,7 @@ __device__ __forceinline__ void epilogue_tile(const Epilogue& ep, int bn, Load l
 }
 
 // Persistent: a CTA walks output tiles blockIdx.x, blockIdx.x + gridDim.x, ...; the accumulator is double-buffered in
-// tensor memory, so the MMA thread fills one buffer while the epilogue warps drain the other.
+// tensor memory, so the MMA thread fills one buffer while the epilogue warps drain the other.  For PLAIN and RELU2 epilogues.
 template <int BN, int STAGES, int EPI>
 __global__ void __launch_bounds__(192)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
@@ -304,7 +304,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int k_blocks = (k + BK - 1) / BK;
     const int total_tiles = tiles_m * tiles_n;
-    constexpr int TILE_N = paired_rows(EPI) ? BN / 2 : BN;    // paired: 128 accumulator columns are 64 gate + 64 up features
+    static_assert(EPI == EPI_PLAIN || EPI == EPI_RELU2, "the other epilogues are the split and the pair kernel's");
     // One weight matrix: neighbouring tiles share its rows (and the CTAs running together share few weight tiles and all
     // activations).  Grouped: neighbours share a row tile and its group's weights; in the other order the CTAs running
     // together read every group's activations, more than L2 holds, once per column of tiles (64 experts of 1792 x 4096,
@@ -334,20 +334,14 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     if (warp == 0) {
         if (lane == 0) {
             auto load_b = [&](int s, int kb, int n0) {
-                unsigned char* b_tile = tiles + s * (S::A_BYTES + S::B_BYTES) + S::A_BYTES;
-                if (paired_rows(EPI)) {       // two boxes of BN/2 rows: gate rows n0.., up rows inter + n0..
-                    tma_load_2d(b_tile, &map_w, kb * BK, n0, full_bar + s);
-                    tma_load_2d(b_tile + S::B_BYTES / 2, &map_w, kb * BK, ep.inter + n0, full_bar + s);
-                } else {
-                    tma_load_2d(b_tile, &map_w, kb * BK, n0, full_bar + s);
-                }
+                tma_load_2d(tiles + s * (S::A_BYTES + S::B_BYTES) + S::A_BYTES, &map_w, kb * BK, n0, full_bar + s);
             };
             // The weights do not come from the kernel before this one: the first stages' weight tiles are requested
             // before the wait on that kernel, the activation tiles after it.
             // (a grouped product learns its weight rows from the kernel before: nothing is requested early)
             const int early = ep.tile_group ? 0 : (k_blocks < STAGES ? k_blocks : STAGES);
             if (early && (int)blockIdx.x < total_tiles) {
-                const int n0 = ((int)blockIdx.x / tiles_m) * TILE_N;
+                const int n0 = ((int)blockIdx.x / tiles_m) * BN;
                 for (int kb = 0; kb < early; ++kb) {
                     mbar_expect_tx(full_bar + kb, (uint32_t)(S::A_BYTES + S::B_BYTES));
                     load_b(kb, kb, n0);
@@ -356,7 +350,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             pdl_wait();
             CISR_TRACE_WAITED();
             for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
-                const int m0 = row_tile(tile) * BM, n0 = col_tile(tile) * TILE_N;
+                const int m0 = row_tile(tile) * BM, n0 = col_tile(tile) * BN;
                 int w_row = n0;
                 if (ep.tile_group) {
                     const int group = ep.tile_group[row_tile(tile)];
@@ -408,24 +402,17 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     } else {
         const int quarter = warp & 3;                                          // the 32 lanes this warp may read
         int it = 0;
-        pdl_wait();      // outputs may alias what the kernel before still reads; step metadata is older than that kernel
+        pdl_wait();      // outputs may alias what the kernel before still reads
         for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
             if (grouped && ep.tile_group[row_tile(tile)] < 0) continue;
             const int acc = it & 1;
-            const int m0 = row_tile(tile) * BM, n0 = col_tile(tile) * TILE_N;
+            const int m0 = row_tile(tile) * BM, n0 = col_tile(tile) * BN;
             const int row = m0 + quarter * 32 + lane;
-            // ROPE: where the row's key and value go hangs on four dependent loads of step metadata; they run while
-            // the tile is still being accumulated instead of after it
-            int pos = 0, page = -1;
-            if (EPI == EPI_ROPE && row < m) {
-                pos = ep.positions[row];
-                page = ep.block_table[(size_t)ep.req_slot[ep.token_req[row]] * ep.table_width + pos / ep.page_size];
-            }
             ok = mbar_wait(acc_full + acc, (it >> 1) & 1);
             if (!ok) break;
             tcgen05_fence_after();
             const uint32_t lane_base = tmem_base + (uint32_t)(acc * BN) + ((uint32_t)(quarter * 32) << 16);
-            epilogue_tile<EPI>(ep, BN, [&](int c, uint32_t (&v)[32]) { tmem_load32(lane_base + (uint32_t)c, v); }, 0, epilogue_units<EPI>(BN), row, m, n, n0, pos, page,
+            epilogue_tile<EPI>(ep, BN, [&](int c, uint32_t (&v)[32]) { tmem_load32(lane_base + (uint32_t)c, v); }, 0, epilogue_units<EPI>(BN), row, m, n, n0, 0, -1,
                                         S::PATCHES && EPI == EPI_PLAIN ? tiles + S::TILES + 256 + (warp - 2) * STAGE_BYTES : nullptr);
             tcgen05_fence_before();
             __syncwarp();
@@ -567,6 +554,7 @@ gemm_tcgen05_split_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
     int pos[MT], page[MT];
     if (warp >= 2) {
         pdl_wait();      // outputs may alias what the kernel before still reads; step metadata is older than that kernel
+        // ROPE: where a row's key and value go hangs on four dependent loads of step metadata; they run while the tile is still being accumulated
 #pragma unroll
         for (int t = 0; t < MT; ++t) {
             const int row = m0 + t * BM + quarter * 32 + lane;
@@ -1042,7 +1030,7 @@ int launch(const void* a, const void* w, const Epilogue& ep, int m, int n, int k
     CUtensorMap map_a, map_w;
     int status = cached_map(&map_a, a, m, k, BM);
     if (status) return status;
-    if ((status = cached_map(&map_w, w, (long long)groups * n, k, paired_rows(EPI) ? BN / 2 : BN))) return status;
+    if ((status = cached_map(&map_w, w, (long long)groups * n, k, BN))) return status;
     typedef Smem<BN, STAGES> S;
     static bool configured = false;
     if (!configured) {
