@@ -270,7 +270,6 @@ attn_prefill_split_kernel(const __grid_constant__ SplitAttention a) {
             for (int e = 0; e < 4; ++e) to[32 * (4 + 4 * j + e)] = o[j][e];
     }
     __syncthreads();
-    float inv[2];
     if (!share) {
         const float sk = a.sink_heads ? a.sink_heads[r.head] : a.sink;
 #pragma unroll
@@ -291,15 +290,13 @@ attn_prefill_split_kernel(const __grid_constant__ SplitAttention a) {
                     for (int e = 0; e < 2; ++e) o[j][2 * h + e] = fmaf(in[32 * (4 + 4 * j + 2 * h + e)], w, o[j][2 * h + e]);
             }
             // a sink is one more term of the denominator, exp(sink), with no value (sink -inf: none); one per head where given
-            inv[h] = 1.f / (sk > -INFINITY ? l + expf(sk - m_use) : l);
-            if (row0 + 8 * h < r.rows)
+            const float inv = 1.f / (sk > -INFINITY ? l + expf(sk - m_use) : l);
+            uint32_t most[2] = {};
 #pragma unroll
-                for (int j = 0; j < D / 8; ++j)
+            for (int j = 0; j < D / 8; ++j)
 #pragma unroll
-                    for (int e = 0; e < 2; ++e) {
-                        const float x = fabsf(o[j][2 * h + e] * inv[h]);
-                        odd = fmaf(o[j][2 * h + e], 0.f, x > 0.f && x < 0x1p-64f ? NAN : odd);
-                    }
+                for (int e = 0; e < 2; ++e) most[e] = max(most[e], oddness(o[j][2 * h + e] *= inv));
+            if (row0 + 8 * h < r.rows && max(most[0], most[1]) >= ODD) odd = NAN;
         }
     }
     if (__syncthreads_or(odd != 0.f)) {                               // 0 x finite is 0, else NaN, and a NaN stays
@@ -315,7 +312,7 @@ attn_prefill_split_kernel(const __grid_constant__ SplitAttention a) {
         float* dst = a.out + ((size_t)(r.tok0 + row) * a.hq + r.head) * D + 2 * (lane & 3);
 #pragma unroll
         for (int j = 0; j < D / 8; ++j) {
-            const float x = o[j][2 * h] * inv[h], y = o[j][2 * h + 1] * inv[h];
+            const float x = o[j][2 * h], y = o[j][2 * h + 1];
             if (pairs) *reinterpret_cast<float2*>(dst + 8 * j) = make_float2(x, y);
             else { dst[8 * j] = x; dst[8 * j + 1] = y; }
         }

@@ -29,13 +29,11 @@ struct FloatSmem {
 
 __device__ __forceinline__ void arrive(uint64_t* bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory"); }
 
-// a sum that the parts may not have carried
-__device__ __forceinline__ bool is_odd(float sum) { return !(fabsf(sum) < INFINITY) || (sum != 0.f && fabsf(sum) < 0x1p-64f); }
-// those of the tile's elements [rows][TN] by float multiply-adds
+// the tile's elements [rows][TN] that the parts may not have carried, by float multiply-adds
 __device__ __noinline__ void plain_tile(const float* __restrict__ a, const float* __restrict__ w, float* __restrict__ out, int m0, int n0, int tn, int m, int n, int k) {
     for (int e = threadIdx.x; e < BM * tn; e += THREADS) {
         const int row = m0 + e / tn, col = n0 + e % tn;
-        if (row >= m || col >= n || !is_odd(out[(size_t)row * n + col])) continue;
+        if (row >= m || col >= n || oddness(out[(size_t)row * n + col]) < ODD) continue;
         float sum = 0.f;
         for (int i = 0; i < k; ++i) sum = fmaf(a[(size_t)row * k + i], w[(size_t)col * k + i], sum);
         out[(size_t)row * n + col] = sum;
@@ -118,8 +116,10 @@ gemm_float_kernel(const float* __restrict__ a, const float* __restrict__ w, floa
         }
         const int row = m0 + quarter * 32 + lane, col = n0 + half * COLS;
         if (ok && row < m) {
+            uint32_t most[2] = {};
 #pragma unroll
-            for (int j = 0; j < COLS; ++j) odd |= is_odd(sums[j]);
+            for (int j = 0; j < COLS; ++j) most[j & 1] = max(most[j & 1], oddness(sums[j]));
+            odd = max(most[0], most[1]) >= ODD;
             float* dst = out + (size_t)row * n + col;
             const bool runs = (n & 3) == 0 && ((uintptr_t)out & 15) == 0;
 #pragma unroll

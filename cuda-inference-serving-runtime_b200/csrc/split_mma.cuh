@@ -36,6 +36,13 @@ __device__ __forceinline__ void split_pair(float x, float y, uint32_t (&p)[3]) {
     x -= __uint_as_float(p[1] << 16); y -= __uint_as_float(p[1] & 0xffff0000u);
     p[2] = bf16_pair(x, y);
 }
+// Results that parts may not have carried: those that are not finite, and those other than zero below 2^-64.  Of several, the largest oddness tells whether
+// there is one: from ODD on.
+constexpr uint32_t ODD = 0x7f800000u - 0x1f800000u;
+__device__ __forceinline__ uint32_t oddness(float x) {
+    const uint32_t size = __float_as_uint(x) & 0x7fffffffu;
+    return size ? size - 0x1f800000u : 0u;         // below 2^-64: around to the largest numbers
+}
 // PLAIN: the upper and the lower halves of the floats' bits in the first two parts, zeros in the third
 template <bool PLAIN>
 __device__ __forceinline__ void tile_pair(float x, float y, uint32_t (&p)[3]) {
