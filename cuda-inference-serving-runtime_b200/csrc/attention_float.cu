@@ -291,32 +291,30 @@ attn_prefill_split_kernel(const __grid_constant__ SplitAttention a) {
             }
             // a sink is one more term of the denominator, exp(sink), with no value (sink -inf: none); one per head where given
             const float inv = 1.f / (sk > -INFINITY ? l + expf(sk - m_use) : l);
-            uint32_t most[2] = {};
 #pragma unroll
-            for (int j = 0; j < D / 8; ++j)
-#pragma unroll
-                for (int e = 0; e < 2; ++e) most[e] = max(most[e], oddness(o[j][2 * h + e] *= inv));
-            if (row0 + 8 * h < r.rows && max(most[0], most[1]) >= ODD) odd = NAN;
+            for (int j = 0; j < D / 8; ++j) { o[j][2 * h] *= inv; o[j][2 * h + 1] *= inv; }
         }
     }
-    if (__syncthreads_or(odd != 0.f)) {                               // 0 x finite is 0, else NaN, and a NaN stays
-        plain_rows(a, r);
-        return;
-    }
-    if (share) return;
-    const bool pairs = ((uintptr_t)a.out & 7) == 0;
+    uint32_t most[2] = {};
+    if (!share) {
+        const bool pairs = ((uintptr_t)a.out & 7) == 0;
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        const int row = row0 + 8 * h;
-        if (row >= r.rows) continue;
-        float* dst = a.out + ((size_t)(r.tok0 + row) * a.hq + r.head) * D + 2 * (lane & 3);
+        for (int h = 0; h < 2; ++h) {
+            const int row = row0 + 8 * h;
+            if (row >= r.rows) continue;
+            float* dst = a.out + ((size_t)(r.tok0 + row) * a.hq + r.head) * D + 2 * (lane & 3);
 #pragma unroll
-        for (int j = 0; j < D / 8; ++j) {
-            const float x = o[j][2 * h], y = o[j][2 * h + 1];
-            if (pairs) *reinterpret_cast<float2*>(dst + 8 * j) = make_float2(x, y);
-            else { dst[8 * j] = x; dst[8 * j + 1] = y; }
+            for (int j = 0; j < D / 8; ++j) {
+                const float x = o[j][2 * h], y = o[j][2 * h + 1];
+                most[0] = max(most[0], oddness(x));
+                most[1] = max(most[1], oddness(y));
+                if (pairs) *reinterpret_cast<float2*>(dst + 8 * j) = make_float2(x, y);
+                else { dst[8 * j] = x; dst[8 * j + 1] = y; }
+            }
         }
     }
+    // a score that is not finite (0 x finite is 0, else NaN, and a NaN stays), or such an output or a tiny one: all rows again
+    if (__syncthreads_or(odd != 0.f || max(most[0], most[1]) >= ODD)) plain_rows(a, r);
 }
 }  // namespace
 
