@@ -73,7 +73,7 @@ constexpr int V_STAGES = D == 64 ? 4 : 2;
 constexpr bool OWN_P = D == 64;
 __host__ __device__ constexpr int value_slots(bool shared) { return V_STAGES + (shared && !OWN_P); }
 static_assert(!OWN_P || (K_STAGES % 2 == 0 && value_slots(true) % 2 == 0), "a slot belongs to one stream");
-constexpr size_t SMEM_FIXED = 1024 + 2 * Q_BYTES + (K_STAGES + V_STAGES) * KV_BYTES + 256;
+constexpr size_t SMEM_FIXED = 1024 + 2 * Q_BYTES + (K_STAGES + V_STAGES) * KV_BYTES + 256 + 16;
 constexpr float LOG2E = 1.4426950408889634f;
 constexpr float RESCALE_STEP = 8.f;           // the max may lag by this much (base-2 exponent) before O is rescaled
 constexpr int FIRST_SOFTMAX_WARP = 4;         // warps 0 and 2: key and value producers; warps 1 and 3: the products
@@ -136,6 +136,7 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     static_assert(2 + 2 * (K_STAGES + V_STAGES + 1) + 11 <= 31, "the barriers and the two words behind them fit 256 bytes");
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 31);
     int* abort_flag = reinterpret_cast<int*>(tmem_slot + 1);
+    uint64_t* done = bars + 32;                                 // [2] giving up: the products that warps 1 and 3 issued are done
     float* exchange = reinterpret_cast<float*>(Kring);          // once every product is done: [2][2 streams][128 rows], maxima and sums
 
     pdl_trigger();
@@ -180,6 +181,7 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __g
             mbar_init(p_full + 2 * s, SOFTMAX_THREADS / 64);
             mbar_init(p_full + 2 * s + 1, SOFTMAX_THREADS / 64);
             mbar_init(o_done + s, 1);
+            mbar_init(done + s, 1);
         }
         *abort_flag = 0;
         mbar_init_fence();
@@ -206,6 +208,7 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         gave_up();
         return false;
     };
+    int requested = 0;                                            // producers: tiles
     auto warp_wait = [&](uint64_t* bar, uint32_t parity) { return (bool)__all_sync(0xffffffffu, wait(bar, parity)); };
 
     if (warp == 0 || warp == 2) {
@@ -236,6 +239,7 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                 tma_load_2d(ring + s * KV_BYTES + sub * KV_SUB + i * box_rows * 128, map, sub * 64, row, full + s);
             }
             if (j == 0 && !values && !shared && lane == 0) load_queries(1);
+            requested = j + 1;
         }
         if (values && ok && tile_k0(n_tiles - 1) + BN > k_end) {
             // Value rows beyond the last key were never written, or are left over from another request: they must not
@@ -572,6 +576,16 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     }
     tcgen05_fence_before();
     __syncthreads();
+    if (*(volatile int*)abort_flag) {
+        if (warp == 0) {
+            mbar_wait(q_full, 0);
+            if (!shared && requested) mbar_wait(q_full + 1, 0);
+            wait_for_copies(k_full, requested, K_STAGES);
+        }
+        if (warp == 2) wait_for_copies(v_full, requested, value_slots(shared));
+        if (warp == 1 || (OWN_P && warp == 3)) wait_for_products_elect(done + (warp >> 1));
+        __syncthreads();
+    }
     if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512) : "memory");
 }
 }  // namespace

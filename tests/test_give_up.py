@@ -35,9 +35,9 @@ def test_blocks_in_flight(tmp_path):
 
 
 def test_products_and_copies_are_waited_for_before_tensor_memory_is_freed():
-    """In the text of every matrix product's kernel, between its last role and the instruction that frees its tensor memory."""
+    """In the text of every kernel with products on tcgen05, between its last role and the instruction that frees its tensor memory."""
     kernels = 0
-    for name in ("gemm_tcgen05.cu", "gemm_float.cu", "few_gemm.cu"):
+    for name in ("gemm_tcgen05.cu", "gemm_float.cu", "few_gemm.cu", "attention_tcgen05.cu"):
         text = (build.CSRC / name).read_text()
         shared = "meet_pair(" in text and re.search(r"void meet_pair\(.*?\n}\n", text, re.DOTALL).group(0)
         for part in text.split("__global__")[1:]:
@@ -48,4 +48,4 @@ def test_products_and_copies_are_waited_for_before_tensor_memory_is_freed():
             end = end + shared if "meet_pair(" in end else end
             assert "wait_for_products" in end, (name, part[:120])
             assert "wait_for_copies" in end or "cp.async.bulk" not in part and "tma_load" not in part, (name, part[:120])
-    assert kernels == 6
+    assert kernels == 7
