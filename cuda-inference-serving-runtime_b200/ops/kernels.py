@@ -2188,18 +2188,25 @@ def tcgen05_ok(a: torch.Tensor, w: torch.Tensor, fused: bool = False) -> bool:
             and a.shape[1] % 8 == 0 and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
 
 
-# The gated product replaces two launches as well.  us in a graph, library and activation kernel against fused, 17 / 32 / 64 / 120 tokens: 3072 x 576
-# 4.9 / 4.8 / 5.1 / 5.6 and 4.1 / 3.7 / 3.7 / 3.7; 5120 x 960 7.1 / 7.1 / 7.3 / 8.1 and 6.5 / 6.7 / 6.3 / 5.4; 16384 x 2048 15.0 / 15.2 / 16.7 / 19.2 and
-# 18.7 / 13.3 / 13.4 / 13.8; 28672 x 4096 43.1 / 44.6 / 47.7 / 57.2 and 44.6 / 45.4 / 46.3 / 47.7, and of the largest the library is ahead where the
-# kernel before hides no start: a feed-forward of 4096, 14336 and 40 tokens outside a graph 75 and 83.
-TCGEN05_GATED_MIN_TOKENS, TCGEN05_GATED_SMALL_BYTES, TCGEN05_GATED_LARGE_BYTES = 32, 16 << 20, 80 << 20
+# The gated product replaces two launches as well.  us in a graph, library and activation kernel against fused, 17 / 32 / 64 / 96 / 120 tokens:
+#   3072 x 576       4.9 / 4.8 / 5.1 /   -  / 5.6      4.1 / 3.7 / 3.7 /   -  / 3.7
+#   5120 x 960       7.1 / 7.1 / 7.3 /   -  / 8.1      6.5 / 6.7 / 6.3 /   -  / 5.4
+#   8192 x 1024      7.0 / 7.3 / 8.7 / 9.5 / 9.8       9.4 / 7.8 / 6.2 / 6.2 / 6.3
+#   12288 x 1536    11.3 / 11.6 / 12.6 / 13.6 / 13.7  13.9 / 12.6 / 9.8 / 10.1 / 10.3
+#   16384 x 2048    15.1 / 15.5 / 17.1 / 19.1 / 19.5  18.3 / 13.5 / 13.6 / 13.6 / 13.8
+#   20480 x 2560    21.7 / 22.7 / 24.8 / 29.2 / 30.3  36.4 / 25.4 / 25.8 / 26.1 / 26.3
+#   24576 x 3072    30.0 / 31.3 / 34.6 / 37.2 / 37.5  39.1 / 32.2 / 32.9 / 33.5 / 33.9
+#   28672 x 4096    43.4 / 44.7 / 48.6 / 56.2 / 58.0  47.0 / 47.8 / 48.9 / 49.6 / 50.3
+# From 16 MB of weights on fewer than 128 KB of activations are read slowly (a tensor map whose boxes lie mostly outside it); from there the fused one
+# is ahead below 80 MB.  The largest matrices keep the library to 127 tokens, as before: fused is behind to some 64 tokens and ahead from 96.
+TCGEN05_GATED_SMALL_BYTES, TCGEN05_GATED_LARGE_BYTES, TCGEN05_GATED_MIN_ACTIVATION_BYTES = 16 << 20, 80 << 20, 128 << 10
 
 
 def tcgen05_gated_ok(a: torch.Tensor, w: torch.Tensor) -> bool:
     """Whether the gated product of `a` with the stacked `w` is better one launch of the tcgen05 kernel."""
     size = w.numel() * 2
-    least = 0 if size < TCGEN05_GATED_SMALL_BYTES else TCGEN05_GATED_MIN_TOKENS if size < TCGEN05_GATED_LARGE_BYTES else TCGEN05_MIN_TOKENS
-    return tcgen05_ok(a, w, fused=True) and a.shape[0] >= min(TCGEN05_MIN_TOKENS, least)
+    return tcgen05_ok(a, w, fused=True) and (a.shape[0] >= TCGEN05_MIN_TOKENS or size < TCGEN05_GATED_SMALL_BYTES
+                                             or (size < TCGEN05_GATED_LARGE_BYTES and a.numel() * 2 >= TCGEN05_GATED_MIN_ACTIVATION_BYTES))
 
 
 def gemm_tcgen05(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, accumulate: bool = False, out_mult: float = 1.0) -> torch.Tensor:

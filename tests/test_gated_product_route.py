@@ -12,6 +12,8 @@ def test_rule():
     assert not ok(16, 3072, 576) and ok(17, 3072, 576) and ok(127, 3072, 576)
     assert not ok(31, 16384, 2048) and ok(32, 16384, 2048)
     assert not ok(127, 28672, 4096) and ok(128, 28672, 4096)
+    # 16 MB of weights and more: fewer than 128 KB of activations are the library's, which is ahead there by up to 1 us
+    assert not ok(63, 8192, 1024) and ok(64, 8192, 1024) and not ok(42, 12288, 1536) and ok(43, 12288, 1536)
     assert not ok(64, 3072, 576, torch.float32) and not ok(64, 3072, 572)
 
 
