@@ -2380,7 +2380,7 @@ _DESCRIBE = {
     "latent_values": lambda mixed, v_up, *a, **kw: (int(mixed.shape[0]), int(v_up.shape[0]), int(v_up.shape[1]), int(v_up.shape[2])),
     "moe_select": lambda logits, *a, **kw: (int(logits.shape[0]), int(logits.shape[1])),
     "moe_rows": lambda h, w_up, w_down, chosen, *a, **kw: (int(h.shape[0]), int(w_up.shape[0]), int(w_up.shape[1]), int(w_up.shape[2]), int(chosen.shape[1])),
-    "moe_sort": lambda chosen, experts, *a: (int(chosen.shape[0]), int(chosen.shape[1]), int(experts)),
+    "moe_sort": lambda chosen, experts, *a, **kw: (int(chosen.shape[0]), int(chosen.shape[1]), int(experts)),
     "moe_scatter": lambda h, row_of, sorted_h: (int(row_of.numel()), int(sorted_h.shape[1])),
     "moe_combine": lambda sorted_out, row_of, weight, out, out_scale=None, h=None: (int(out.shape[0]), int(weight.shape[1]), int(out.shape[1])),
     "gemm_tcgen05_grouped": lambda a, w, out, tile_group, rows_in_use=None, activation="relu_squared":

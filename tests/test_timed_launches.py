@@ -1,4 +1,5 @@
 """What the event brackets around launches see (no GPU needed: events and libraries are stand-ins)."""
+import inspect
 import re
 
 import pytest
@@ -57,3 +58,10 @@ def test_a_context_inside_another_leaves_the_outer_one_open(stand_ins):
     kernels.scale_(x, 2.0)
     second.__exit__()
     assert len(second.records) == 1 and not first.records and kernels.scale_ is plain
+
+
+def test_a_description_takes_every_call_that_its_function_takes():
+    for name, describe in kernels._DESCRIBE.items():
+        parameters = inspect.signature(kernels._untimed[name]).parameters.values()
+        given = [object() for p in parameters if p.kind == p.POSITIONAL_OR_KEYWORD and p.default is p.empty]
+        inspect.signature(describe).bind(*given, **{p.name: p.default for p in parameters if p.kind == p.KEYWORD_ONLY or p.default is not p.empty})
