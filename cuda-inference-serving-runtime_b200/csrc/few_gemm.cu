@@ -6,7 +6,8 @@
 //   * warp 0: TMA copies of 128 of K at a time: the block's rows in ONE box of 32 KB and the tokens in one of 4 KB, into a ring of three stages;
 //     the first stages' weights are requested before the wait on the kernel before
 //   * warp 1: tcgen05.mma (M = 128, N = 16), the eight products of a block into eight accumulators.  The tensor core cuts a sum instead of
-//     rounding it: with all of K in one accumulator the error against 64 bits was 3.6 to 4.5 times that of stream_gemm.cu's eight slices of K
+//     rounding it: with all of K in one accumulator the error against 64 bits was 3.6 to 4.5 times that of stream_gemm.cu's eight slices of K (49152 x
+//     576 5.2e-7, there 1.5e-7, so 0.9e-7; 16 tokens 13.5 us with one, 13.8 with eight)
 //   * warps 2..5: the accumulators, added in float, are a share's sums; they go to shared memory, one barrier.cluster, and each CTA adds the shares of
 //     its part of the rows, in the order of K, and runs the epilogue on them
 // Two CTAs share an SM: one streams while the other starts or ends.

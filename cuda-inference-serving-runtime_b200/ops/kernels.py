@@ -1617,7 +1617,7 @@ def moe_rows(h: torch.Tensor, w_up: torch.Tensor, w_down: torch.Tensor, chosen: 
 
 
 EXPERT_ACTIVATIONS = {"relu_squared": 0, "gelu": 1}      # ungated expert activations as the kernels number them
-MOE_TILE = 128                   # rows per tile of the grouped product: each expert's rows are padded to whole tiles
+MOE_TILE = 128                   # rows per tile of the grouped product, whose groups are padded to whole tiles
 MOE_RUN = 256                    # most rows of a run of one expert's rows that the tensor-core products take as one tile
 MOE_GROUPED_MIN_ROWS = 64        # (token, expert) pairs per expert, on average, from which sorting and the products by expert pay for any width
 # Below that: `moe_rows` brings an expert's matrices once per pair (8 TB/s: mostly from L2), the products by expert once per expert in use (5 TB/s); they
